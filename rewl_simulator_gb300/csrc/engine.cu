@@ -350,6 +350,9 @@ __device__ __forceinline__ int chunk_dm(unsigned acc, unsigned plus, int j)
     return -2 * ((int)__popc(acc & plus & le) - (int)__popc(acc & ~plus & le));
 }
 
+struct SweepParams;
+using SweepKernel = void (*)(const SweepParams);
+
 struct SweepParams {
     DevPtrs P;
     const int32_t* slots;    // walkers of this launch
@@ -357,6 +360,8 @@ struct SweepParams {
     int nsweeps;
     int smem_per_warp;       // bytes
     int nbcap;               // table capacity per warp (Ising, shared memory)
+    int counts;              // bin-tracking kernel: visit counts beside g in shared memory
+    int moments;             // bin-tracking kernel with observables: moment sums in shared memory
 };
 
 // Per-warp staging of one chunk for the lane-0 resolver: energy change without /
@@ -622,46 +627,40 @@ __global__ void __launch_bounds__(256) k_sweep_ising(const SweepParams p)
 
 // ---------------------------------------------------------------------------
 // Bin-tracking Ising sweeps (used when every energy change is a whole number of
-// bins: 4|J| divisible by the bin width, as for J = 1 and width 4).  The chain
-// then carries only the bin index b and the logDoS value g[b].
+// bins: 4|J| divisible by the bin width, as for J = 1 and width 4).
 //
-// G walkers share a warp (P = 32/G lanes each).  For each chunk the walker's
-// lanes first form, per site: the integer acceptance threshold, the packed bin
-// changes (without / with the left neighbour flipped, wrap term for x = L-1)
-// and the spin.
+// The chain of accept decisions of one walker is serial, but a few decisions
+// ahead there are few outcomes: G walkers share a warp, P = 32 / G lanes each,
+// and a walker's lanes are the nodes of the binary tree of its next D = log2(P)
+// decisions (lane 1 the first decision, lanes 2k and 2k + 1 the decision after
+// lane k's rejection / acceptance; lane 0 idles).  A block of D sites is then:
+//   * every node forms its own position relative to the block's start (the sum
+//     of the bin changes its ancestors accepted), its proposal, and how often
+//     the path to it visits either bin within the block -- all independent of
+//     where the block starts, so this is done while the block before it is
+//     being decided;
+//   * once the start is known, every node loads g at its two bins (two shared
+//     loads for D decisions instead of D dependent ones), decides, and one vote
+//     hands all decisions to all lanes;
+//   * a node is on the path if its ancestors decided its way (one masked
+//     compare); the D nodes on the path commit g + visits x ln f, in order of
+//     their sites, and the last of them publishes the new position.
+// Energy changes are multiples of 4|J|: with a = the number of neighbours that
+// agree, a flip moves the walker by (a - 2) x q bins (q = 4 J / width), and a
+// left neighbour flipped just before changes a by one.  Positions inside a block
+// are sums of at most five such steps and live in the four bytes of a register:
+// a byte-wise prefix sum is one multiplication by 0x01010101.
+//
+// The lattice is one bit per spin (1: spin -1), a row being nch chunks of at most
+// 32 sites, one word each; chunks are cut into blocks of D sites (the last one
+// shorter).  The agreement counts of a chunk come from its words by bit-sliced
+// addition and are handed to the nodes through shared memory (`slots`).
+//
+// The table carries kGuard sentinel bins on each side holding INT64_MAX: a
+// proposal outside the window fails the compare by itself, and nodes below an
+// out-of-window proposal (never on the path) still read inside the table.
 // ---------------------------------------------------------------------------
-struct __align__(16) SiteRec {
-    long long T;    // accept iff d < T
-    int pk;         // bytes: bin change, same with left neighbour flipped, wrap term
-    int s;          // spin
-};
-
-
-// The accept chain, all lanes of a walker in lockstep, with the table reads one
-// site ahead.  While site j is being decided, the two bins site j+1 may propose
-// (one if site j is rejected, one if it is accepted -- which moves the walker
-// and flips the left neighbour of site j+1) are already being loaded, so the
-// load latency overlaps the decision.  Per site the dependent work is then:
-// one 64-bit compare of g(proposal) against g(current) + threshold, a select of
-// the taken branch and one add.
-//
-// A prefetched load follows the commit store of the site before it, so it is
-// stale only when it reads the bin the next commit writes, i.e. exactly when
-// its proposal keeps the bin (offset change 0); the value is then the one just
-// committed.
-//
-// The table carries kGuard sentinel bins on each side holding INT64_MAX, so a
-// proposal outside the window fails the compare by itself whatever g holds (no
-// range checks): the current bin never leaves the window, and prefetches issued
-// from an out-of-window proposal stay inside the table.  Bin
-// positions are byte offsets into the table.
-//
-// The chain runs without a break from chunk to chunk: the first offsets of the
-// next chunk are formed from the lattice before the current chunk's flips, then
-// corrected for the neighbours the current chunk flips as soon as those are
-// decided, and handed to all lanes by shuffle; thresholds come from one Philox
-// block per four sites, 4C sites at a time, one batch ahead.
-constexpr int kGuard = 8;
+constexpr int kGuard = 20;                                // 2 x 5 decisions x |q| <= 2 bins
 constexpr long long kGuardValue = 0x7FFFFFFFFFFFFFFFLL;   // never below g + threshold
 
 __device__ __forceinline__ long long lds64(const char* base, int off)
@@ -670,21 +669,69 @@ __device__ __forceinline__ long long lds64(const char* base, int off)
 }
 __device__ __forceinline__ void sts64(char* base, int off, long long v) { *reinterpret_cast<long long*>(base + off) = v; }
 
+// acc + n f for an int64 f = f_hi 2^32 + f_lo (f_lo signed): two multiply-adds
+__device__ __forceinline__ long long mad_units(long long acc, int n, int f_lo, int f_hi)
+{
+    long long r;
+    asm("{\n\t.reg .b32 lo, hi;\n\tmad.wide.s32 %0, %1, %2, %4;\n\tmov.b64 {lo, hi}, %0;\n\tmad.lo.s32 hi, %1, %3, hi;\n\t"
+        "mov.b64 %0, {lo, hi};\n\t}"
+        : "=&l"(r) : "r"(n), "r"(f_lo), "r"(f_hi), "l"(acc));
+    return r;
+}
+
+// adds 1 to the 32-bit word at shared address `addr`
+__device__ __forceinline__ void red_shared_inc(unsigned addr)
+{
+    asm volatile("red.shared.add.u32 [%0], 1;" :: "r"(addr) : "memory");
+}
+
+// chunk layout of a row of L sites: `n` words, the first `rem` of `base` + 1 sites, the others of `base`
+struct RowChunks {
+    int n, base, rem;
+    __host__ __device__ explicit RowChunks(int L) : n((L + 31) / 32), base(L / n), rem(L % n) {}
+    __host__ __device__ int len(int c) const { return base + (c < rem ? 1 : 0); }
+    __host__ __device__ int start(int c) const { return c * base + (c < rem ? c : rem); }
+    __host__ __device__ int of(int x) const { return x < rem * (base + 1) ? x / (base + 1) : rem + (x - rem * (base + 1)) / base; }
+};
+
+template <int G>
+struct BinsTree {
+    static constexpr int kLanes = 32 / G;
+    static constexpr int kDepth = G == 1 ? 5 : G == 2 ? 4 : 3;
+    static constexpr int kBlocks = (32 + kDepth - 1) / kDepth;      // blocks of the longest chunk
+    static constexpr int kSlot = kDepth == 5 ? 16 : 8;              // bytes per block: agreement counts, then left terms
+    static constexpr int kRing = G == 4 ? 128 : 256;                // thresholds kept per walker
+    static_assert(kLanes == 1 << kDepth, "one lane per node");
+};
+
+constexpr int kObsWords = 8;      // Ising moments as integers: |M|, M^2 and M^4 in halves of 28 bits, 64 bits each
+
+// 64-bit sum in two shared words, lo then hi
+__device__ __forceinline__ void add_carry(unsigned* s, unsigned x)
+{
+    const unsigned old = atomicAdd(s, x);
+    if (old + x < old) atomicAdd(s + 1, 1u);
+}
+
+// shared memory of one walker: table with guards, lattice words, thresholds, two chunks' slots;
+// with observables the bins of a chunk's steps and (acc) the
+// moments' integer sums, with correlators row and column sums and counts
+template <int G>
+__host__ __device__ inline int bins_smem(int nbcap, int L, bool obs, bool corr, bool cnt, bool acc)
+{
+    const RowChunks rc(L);
+    return (nbcap + 2 * kGuard) * (cnt ? 16 : 8) + ((rc.n * L * 4 + 15) & ~15) + BinsTree<G>::kRing * 8 +
+           2 * BinsTree<G>::kBlocks * BinsTree<G>::kSlot + 16 + (obs ? 32 * 4 : 0) + (corr ? 8 * L + 4 * nbcap : 0) + (acc ? 4 * kObsWords * nbcap : 0);
+}
+
 // The sweeps of one warp's G walkers (launch position warp_index; its shared memory starts at
 // warp_base, one region of p.smem_per_warp bytes per walker).
-template <int G, int C, bool OBS, bool LEAN>
+template <int G, bool OBS, bool CNT>
 __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int warp_index, unsigned char* warp_base)
 {
-    constexpr int P = 32 / G;
-    constexpr int SPL = (C + P - 1) / P;          // sites per lane in a chunk
-    constexpr int BPL = (C + P - 1) / P;          // Philox blocks per lane in a batch of 4C sites
-    constexpr int kAhead = 4;                     // per-site inputs are read this many sites early
-    // LEAN: each step reads g at the next proposal after its own write (no candidate prefetch,
-    // no staleness select): five fewer ALU instructions per step and a dependent shared-memory
-    // load on the chain, which pays where enough warps share an SM to hide it
-    constexpr bool kLean = LEAN;
-    static_assert(!LEAN || G > 1, "the lean chain is for warps of several walkers");
-    static_assert(C % 4 == 0 && C >= 4 && C <= 32 && P >= 4, "chunk");
+    using T = BinsTree<G>;
+    constexpr int RS = CNT ? 16 : 8, RW = RS / 8;            // table record: g, with CNT followed by the launch's visits
+    constexpr int P = T::kLanes, D = T::kDepth, SPL = 32 / P, RING = T::kRing;
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31;
     const int grp = lane / P, q = lane - grp * P, gbase = grp * P;
@@ -697,44 +744,77 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
     const int w = P_.slot_win[s];
     const WinDev W = P_.win[w];
     const int L = I.L, N = I.N, nb = W.nb;
+    const RowChunks rc(L);
     unsigned char* base = warp_base + (size_t)grp * p.smem_per_warp;
-    const int gs_bytes = ((p.nbcap + 2 * kGuard) * 8 + 15) & ~15;
-    long long* gs = reinterpret_cast<long long*>(base) + kGuard;     // gs[-kGuard .. nb+kGuard)
-    int8_t* lat = reinterpret_cast<int8_t*>(base + gs_bytes);
-    long long* Tb = reinterpret_cast<long long*>(base + gs_bytes + ((N + 15) & ~15));   // 2 x 4C thresholds
-    int2* Db = reinterpret_cast<int2*>(Tb + 8 * C);                                   // 2 x C offset pairs
-    int* seqb = reinterpret_cast<int*>(Db + 2 * C);                                   // C bins (observables)
-    int* rsum = seqb + C;                                                             // correlators: row sums,
-    int* csum = rsum + L;                                                             // column sums,
-    int* bcnt = csum + L;                                                             // bin counts mod 1000
+    long long* gs = reinterpret_cast<long long*>(base) + RW * kGuard;            // records -kGuard .. nb+kGuard-1
+    uint32_t* lat = reinterpret_cast<uint32_t*>(base + (p.nbcap + 2 * kGuard) * RS);   // [L][rc.n] words
+    long long* Tb = reinterpret_cast<long long*>(reinterpret_cast<unsigned char*>(lat) + ((rc.n * L * 4 + 15) & ~15));
+    unsigned char* slots = reinterpret_cast<unsigned char*>(Tb + RING);          // 2 chunks of T::kBlocks slots
+    int* seqb = reinterpret_cast<int*>(slots + 2 * T::kBlocks * T::kSlot) + 4;   // a chunk's bins (observables)
+    int* rsum = seqb + (OBS ? 32 : 0);                                           // correlators: row sums,
+    int* csum = rsum + L;                                                        // column sums,
+    int* bcnt = csum + L;                                                        // bin counts mod 1000
+    const bool corr = OBS && P_.corr, moments = OBS && p.moments;
+    unsigned* mom = reinterpret_cast<unsigned*>(corr ? bcnt + p.nbcap : rsum);   // moment sums (observables)
     // table positions are byte offsets from the start of shared memory, so that the
     // accesses need no address arithmetic
     char* const sm = reinterpret_cast<char*>(smem);
     const int gsoff = (int)(reinterpret_cast<char*>(gs) - sm);
+    const unsigned smbase = (unsigned)__cvta_generic_to_shared(sm);
+    const int sink = (int)(reinterpret_cast<char*>(seqb - 4) - sm);
 
     const int cfg = P_.slot_cfg[s];
     int8_t* gl = P_.spins + P_.cfg_off[cfg];
     long long* gg = reinterpret_cast<long long*>(P_.g + P_.slot_tab[s]);
-    for (int i = q; i < N; i += P) lat[i] = gl[i];
-    for (int k = q; k < nb; k += P) gs[k] = gg[k];
-    for (int k = q; k < kGuard; k += P) { gs[-1 - k] = kGuardValue; gs[nb + k] = kGuardValue; }
+    for (int k = q - kGuard; k < nb + kGuard; k += P) {
+        gs[RW * k] = k >= 0 && k < nb ? gg[k] : kGuardValue;
+        if (CNT) gs[RW * k + 1] = 0;
+    }
+    // every slot starts as "no change" (count 2, left term 1), so that a short block's missing
+    // sites keep positions inside the table; bytes past a slot's D sites stay zero
+    for (int k = q; k < 2 * T::kBlocks * T::kSlot; k += P) {
+        const int half = k % T::kSlot / (T::kSlot / 2), j = k % (T::kSlot / 2);
+        slots[k] = j < D ? (unsigned char)(half ? 1 : 2) : (unsigned char)0;
+    }
+    int minus = 0;                                             // spins -1 seen by this walker (all its lanes agree)
+    for (int c = 0, i = 0; c < rc.n * L; ++c) {
+        const int len = rc.len(c % rc.n);
+        uint32_t bits = 0;
+#pragma unroll
+        for (int k = 0; k < SPL; ++k) {
+            const int jj = q + k * P;
+            const unsigned bal = __ballot_sync(kFull, jj < len && gl[i + jj] < 0);
+            bits |= (P == 32 ? bal : ((bal >> gbase) & (0xFFFFFFFFu >> (32 - P)))) << (k * P % 32);
+        }
+        if (q == 0) lat[c] = bits;
+        minus += __popc(bits);
+        i += len;
+    }
     __syncwarp();
-    const bool corr = OBS && P_.corr;
+    auto spin = [&](int i) {
+        const int y = i / L, x = i - y * L, c = rc.of(x);
+        return (lat[y * rc.n + c] >> (x - rc.start(c))) & 1u ? -1 : 1;
+    };
+    const double invN = 1.0 / (double)N;
+    double* ob = OBS ? P_.obs + (size_t)P_.slot_tab[s] * P_.obs_stride : nullptr;
+    if (moments)
+        for (int k = q; k < nb * kObsWords; k += P) mom[k] = 0;
     if (corr) {
-        plane_sums(rsum, csum, L, q, [&](int i) { return (int)lat[i]; }, P);
+        plane_sums(rsum, csum, L, q, spin, P);
         const uint64_t* gv0 = P_.visits + P_.slot_tab[s];
         for (int k = q; k < nb; k += P) bcnt[k] = (int)(gv0[k] % kCountsPerTransform);
         __syncwarp();
     }
 
-    const int J = (int)I.J_u;
-    const int sh = I.bin_shift;                        // energy change -> bin change (x8: byte offset)
+    const int sh = I.bin_shift;
+    const int q8 = (int)((4 * I.J_u) >> sh) * RS;              // table bytes per agreeing neighbour
     const int Ewlo = (int)W.elo_u;
     const long long lnf = P_.win_lnf[w];
+    const int lnf_lo = (int)(uint32_t)lnf;                     // ln f = lnf_hi 2^32 + lnf_lo, lnf_lo signed
+    const int lnf_hi = (int)((lnf - (long long)lnf_lo) >> 32);
     const uint64_t sweeps0 = P_.slot_sweeps[s];
     const uint32_t uid = (uint32_t)(s - I.first_slot);
     const uint32_t k0 = (uint32_t)I.seed ^ uid, k1 = (uint32_t)(I.seed >> 32);
-    const bool wraps = C == L;                         // a row is one chunk: its last site sees the row start
 
     const int E0 = (int)P_.cfg_E[cfg];
     const int b0 = (E0 - Ewlo) >> sh;
@@ -743,336 +823,429 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
         if (lane == 0) atomicOr(&P_.counters[0], ERR_BOUNDS);
         return;
     }
-    int M = P_.cfg_M[3 * cfg];
+    int M = N - 2 * minus;
 
-    // thresholds (+ ln f) of the 4C sites from attempt A0 on into Tb[buf]
-    auto draw = [&](uint64_t A0, int buf) {
-        longlong2* dst = reinterpret_cast<longlong2*>(Tb + buf * 4 * C);
-#pragma unroll
-        for (int k = 0; k < BPL; ++k) {
-            const int bi = q + k * P;
-            if (bi < C) {
-                const uint64_t a = A0 + (uint64_t)(4 * bi);
-                const Philox4 r = philox4x32_10(Philox4{(uint32_t)(a >> 2), (uint32_t)(a >> 34), kStreamWL, 0u}, k0, k1);
-                longlong2 t01, t23;
-                t01.x = accept_threshold(neglog_u32(r.x)) + lnf;
-                t01.y = accept_threshold(neglog_u32(r.y)) + lnf;
-                t23.x = accept_threshold(neglog_u32(r.z)) + lnf;
-                t23.y = accept_threshold(neglog_u32(r.w)) + lnf;
-                dst[2 * bi] = t01;
-                dst[2 * bi + 1] = t23;
-            }
-        }
-    };
-
-    // Inputs of a chunk formed from the lattice as it stands, before the flips of the
-    // chunk processed meanwhile (which starts at site c0prev, or -1): per site the
-    // spin, the energy change without / with the previous site of the sequence
-    // flipped, and for the neighbours lying in the chunk at c0prev (other than the
-    // previous site) their bit there and the correction 4 J s s_nbr if it flips.
-    int ns[SPL], nd0[SPL], nd1[SPL], nbit[SPL][2], ncoef[SPL][2], nwrap = 0;
-    auto prepare = [&](int y, int x0, int c0prev) {
-        const int row = y * L;
-        const int up = (y == 0 ? L - 1 : y - 1) * L, down = (y == L - 1 ? 0 : y + 1) * L;
-        nwrap = 0;
-#pragma unroll
-        for (int k = 0; k < SPL; ++k) {
-            const int jj = q + k * P;
-            ns[k] = 0; nd0[k] = 0; nd1[k] = 0;
-            nbit[k][0] = nbit[k][1] = -1; ncoef[k][0] = ncoef[k][1] = 0;
-            if (jj < C) {
-                const int x = x0 + jj;
-                const int xl = x == 0 ? L - 1 : x - 1, xr = x == L - 1 ? 0 : x + 1;
-                const int si = lat[row + x];
-                const int su = lat[up + x], sl = lat[row + xl], sr = lat[row + xr];
-                const int d0 = 2 * J * si * (su + sl + sr + lat[down + x]);
-                ns[k] = si;
-                nd0[k] = d0;
-                nd1[k] = x > 0 ? d0 - 4 * J * si * sl : d0;        // x > 0: the left site comes just before
-                if (jj == C - 1 && wraps) nwrap = -4 * J * si * sr;
-                const int ou = up + x - c0prev, orr = row + xr - c0prev;
-                if (c0prev >= 0 && (unsigned)ou < (unsigned)C) { nbit[k][0] = ou; ncoef[k][0] = 4 * J * si * su; }
-                if (c0prev >= 0 && xr == 0 && (unsigned)orr < (unsigned)C) { nbit[k][1] = orr; ncoef[k][1] = 4 * J * si * sr; }
-            }
-        }
-    };
-    // offsets of prepared site slot k once the bits of `acc` it depends on are known
-    auto finish = [&](int k, unsigned acc) {
-        int corr = 0;
-#pragma unroll
-        for (int n = 0; n < 2; ++n)
-            if (nbit[k][n] >= 0 && ((acc >> nbit[k][n]) & 1u)) corr += ncoef[k][n];
-        return make_int2(((nd0[k] - corr) >> sh) * 8, ((nd1[k] - corr) >> sh) * 8);
-    };
-
-    // ---- chunk 0 ----
-    int cs[SPL];                                        // spins of the current chunk
-    int2 E_[4];                                         // offsets of the first 4 sites of the chunk
-    long long T_[4];                                    // thresholds of the first 4 sites of the chunk
-    int cwrap;
-    draw(sweeps0 * (uint64_t)N, 0);
-    prepare(0, 0, -1);
+    // this lane's node: level (decisions before it), the ancestors' decisions that lead to it
+    const int lvl = q == 0 ? 0 : 31 - __clz(q);
+    const int lvla = q == 0 ? 32 : lvl;                        // the idle lane is beyond every block
+    unsigned want = 0, anc = 0;                                // ancestors' vote bits: needed value, mask
+    unsigned mA = 0, mB = 0, K = 0, L80 = 0;                   // byte masks of accepted / twice accepted steps, biases
+    bool first = false, last = false;                          // first decision accepted; the one before this node's
     {
+        int bias = 0;
+        bool prev = false;
+        for (int i = 0; i < lvl; ++i) {
+            const int node = q >> (lvl - i);
+            const bool a = (q >> (lvl - 1 - i)) & 1;
+            anc |= 1u << node;
+            if (a) want |= 1u << node;
+            if (a) { mA |= 0xFFu << (8 * i); bias += 2; }
+            if (a && prev) { mB |= 0xFFu << (8 * i); bias += 1; }
+            K |= (unsigned)(16 - bias) << (8 * i);
+            L80 |= 0x80u << (8 * i);
+            if (i == 0) first = a;
+            prev = a;
+        }
+        last = prev;
+        if (q == 0) { anc = 1u; want = 1u; }                   // its vote is always 0: never on the path
+    }
+    const unsigned selC = lvl == 0 ? 0x5554u : 0x5550u | (unsigned)(lvl - 1);
+    const unsigned selE = 0x7770u | (unsigned)lvl, selX = last ? 0x7770u | (unsigned)lvl : 0x7777u;
+    const int pbias = 2 + (last ? 1 : 0);
+    const unsigned KP = 0u - (unsigned)pbias * 0x01010101u;
+    const int kC = -16 * q8, kP = -(16 + pbias) * q8;
+    const int shiftC = first ? -1 : 0, shiftP = (first || lvl == 0) ? -1 : 0;    // left neighbour of the block's first site
+    const bool leaf = lvl == D - 1 && q != 0;
+    // what a leaf publishes with its position: the decisions of its path in bits 20.. (its own: bit 20 + D - 1)
+    int pathc = 0;
+    for (int i = 0; i < lvl; ++i)
+        if ((q >> (lvl - 1 - i)) & 1) pathc |= 1 << (20 + i);
+
+    // thresholds of P Philox blocks (four attempts each) from block `blk` on into the ring
+    auto draw = [&](uint64_t blk) {
+        const uint64_t a = blk + (uint64_t)q;
+        const Philox4 r = philox4x32_10(Philox4{(uint32_t)a, (uint32_t)(a >> 32), kStreamWL, 0u}, k0, k1);
+        longlong2* dst = reinterpret_cast<longlong2*>(Tb + (((uint32_t)a * 4u) & (RING - 1)));
+        longlong2 t01, t23;
+        t01.x = word_threshold(r.x);
+        t01.y = word_threshold(r.y);
+        t23.x = word_threshold(r.z);
+        t23.y = word_threshold(r.w);
+        dst[0] = t01;
+        dst[1] = t23;
+    };
+
+    // Agreement counts and left terms of the chunk (y, c), into slots `buf`.  The words are read as
+    // they stand, before the flips of the chunk being processed (word index cprev) except for its
+    // decisions `acc` known by now -- the left neighbour of the chunk's first site excepted, whose
+    // flip the nodes add themselves.
+    constexpr int kBuf = T::kBlocks * T::kSlot;
+    int myslot[SPL];
+#pragma unroll
+    for (int k = 0; k < SPL; ++k) {
+        const int jj = q + k * P;
+        myslot[k] = (jj / D) * T::kSlot + jj % D;
+    }
+    struct Planes {
+        unsigned sw, su, al, t1, c1;                           // the chunk's word; up disagreements; partial sums
+    };
+    auto write_slots = [&](const Planes& f, unsigned up_flips, int c, int len, int from, int buf) {
+        const unsigned au = ~(f.su ^ up_flips);
+        const unsigned t0 = au ^ f.al, c0 = au & f.al;
+        const unsigned a0 = t0 ^ f.t1, a1 = c0 ^ f.c1 ^ (t0 & f.t1), a2 = c0 & f.c1;
+        unsigned char* dst = slots + buf * kBuf;
 #pragma unroll
         for (int k = 0; k < SPL; ++k) {
             const int jj = q + k * P;
-            cs[k] = ns[k];
-            if (jj < C) Db[jj] = finish(k, 0u);
+            const unsigned e = ((a0 >> jj) & 1u) + 2u * ((a1 >> jj) & 1u) + 4u * ((a2 >> jj) & 1u);
+            const unsigned x = jj == 0 && c == 0 ? 1u : 2u - 2u * ((f.al >> jj) & 1u);
+            if (jj < len && jj >= from) {
+                dst[myslot[k]] = (unsigned char)e;
+                dst[myslot[k] + T::kSlot / 2] = (unsigned char)x;
+            }
         }
-        cwrap = __shfl_sync(kFull, (nwrap >> sh) * 8, gbase + (C - 1) % P);
-    }
-    __syncwarp();
+    };
+    auto publish = [&](int y, int c, int buf, int cprev, unsigned acc) {
+        const int up = y == 0 ? L - 1 : y - 1, dn = y == L - 1 ? 0 : y + 1;
+        const int cl = c == 0 ? rc.n - 1 : c - 1, cr = c == rc.n - 1 ? 0 : c + 1;
+        const int len = rc.len(c), row = y * rc.n;
+        const unsigned sw = lat[row + c], uw = lat[up * rc.n + c], dw = lat[dn * rc.n + c], lw = lat[row + cl];
+        const unsigned rw = lat[row + cr] ^ (row + cr == cprev ? acc : 0u);
+        const unsigned lb = (sw << 1) | ((lw >> (rc.len(cl) - 1)) & 1u);
+        const unsigned rb = (sw >> 1) | ((rw & 1u) << (len - 1));
+        const unsigned ar = ~(sw ^ rb), ad = ~(sw ^ dw);
+        Planes f;
+        f.sw = sw;
+        f.su = sw ^ uw;
+        f.al = ~(sw ^ lb);
+        f.t1 = ar ^ ad;
+        f.c1 = ar & ad;
+        write_slots(f, up * rc.n + c == cprev ? acc : 0u, c, len, 0, buf);
+        return f;
+    };
+
+    // A node's part of a block that does not depend on where the block starts: the slots and the
+    // threshold it reads, then its positions, then the visits of its path to either bin.
+    struct Slot {
+        unsigned e0, e1, x0, x1;
+        long long t;
+    };
+    struct Node {
+        int rC, rP, nC, nP, x0;
+        long long t;
+    };
+    auto fetch = [&](const unsigned char* slot, uint32_t attempt) {
+        Slot f;
+        if (D == 5) {
+            const uint4 v = *reinterpret_cast<const uint4*>(slot);
+            f.e0 = v.x; f.e1 = v.y; f.x0 = v.z; f.x1 = v.w;
+        } else {
+            const uint2 v = *reinterpret_cast<const uint2*>(slot);
+            f.e0 = v.x; f.e1 = 0u; f.x0 = v.y; f.x1 = 0u;
+        }
+        f.t = Tb[(attempt + (uint32_t)lvl) & (RING - 1)];
+        return f;
+    };
+    auto node = [&](const Slot& f) {
+        const unsigned S = ((f.e0 & mA) + (f.x0 & mB)) * 0x01010101u + K;        // positions after each step, + 16
+        const unsigned cb = __byte_perm(S, 0x10u, selC);
+        const unsigned pb = cb + __byte_perm(f.e0, f.e1, selE) + __byte_perm(f.x0, f.x1, selX);
+        Node n;
+        n.rC = (int)cb * q8 + kC;
+        n.rP = (int)pb * q8 + kP;
+        n.x0 = ((int)(f.x0 & 0xFFu) - 1) * q8;
+        n.nC = __popc(~((S ^ (cb * 0x01010101u)) + 0x7F7F7F7Fu) & L80);          // steps of the path that ended here
+        n.nP = __popc(~((S ^ (pb * 0x01010101u + KP)) + 0x7F7F7F7Fu) & L80);
+        n.t = f.t;
+        return n;
+    };
+
+    // what the last block left: the position (byte offset, bits 0-19), its decisions (from bit 20 on),
+    // and in the sign whether its last site flipped
+    unsigned state = (unsigned)(gsoff + b0 * RS);
+    unsigned acc = 0;                                          // the current chunk's decisions so far
+    // one block of nlev sites (at the chunk's site j0): its nodes `n`; the next block's slots are
+    // read (ahead()) between the loads and the decision, its node work is done behind the vote
+    auto block = [&](const Node n, const int nlev, int j0, auto ahead) {
+        const int root = (int)(state & 0xFFFFFu);
+        const int shift = ((int)state >> 31) & n.x0;
+        const int aC = root + n.rC + (shift & shiftC), aP = root + n.rP + (shift & shiftP);
+        long long gC, gP;
+        int dn = n.nC - n.nP;
+        if (CNT) {
+            const longlong2 c = *reinterpret_cast<const longlong2*>(sm + aC), d = *reinterpret_cast<const longlong2*>(sm + aP);
+            gC = c.x; gP = d.x;
+            dn += (int)c.y - (int)d.y;
+        } else {
+            gC = lds64(sm, aC);
+            gP = lds64(sm, aP);
+        }
+        const Slot f = ahead();
+        const bool live = lvla < nlev;
+        const bool a = gP < mad_units(gC + n.t, dn, lnf_lo, lnf_hi) && live;
+        const unsigned B = __ballot_sync(kFull, a) >> gbase;
+        const bool on = ((B ^ want) & anc) == 0;
+        const unsigned vC = (unsigned)(aC + pathc), vP = (unsigned)(aP + pathc) + (0x80000000u | 1u << (20 + D - 1));
+        unsigned v = a ? vP : vC;
+        const int fin = a ? aP : aC;
+        if (G <= 2) {
+            v = on && leaf ? v : 0u;
+            if (G == 1) v = __reduce_max_sync(kFull, v);
+            else {
+                const unsigned v0 = __reduce_max_sync(kFull, grp == 0 ? v : 0u), v1 = __reduce_max_sync(kFull, grp == 0 ? 0u : v);
+                v = grp == 0 ? v0 : v1;
+            }
+        } else {
+            const unsigned O = __ballot_sync(kFull, on && leaf) & ((0xFFFFFFFFu >> (32 - P)) << gbase);
+            v = __shfl_sync(kFull, v, 31 - __clz(O));
+        }
+        if (OBS && on && live) seqb[j0 + lvl] = fin;
+        if (CNT) {
+            // lanes off the path count in a word nobody reads (a predicated reduction costs a branch)
+            red_shared_inc(smbase + (unsigned)(on && live ? fin + 8 : sink));
+        } else {
+            const int vis = (a ? n.nP : n.nC) + 1;
+            const long long gn = mad_units(a ? gP : gC, vis, lnf_lo, lnf_hi);
+            const int sl = on && live ? lvl : -1;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { E_[i] = Db[i]; T_[i] = Tb[i]; }
+            for (int i = 0; i < D; ++i) {
+                if (sl == i) sts64(sm, fin, gn);
+                __syncwarp();                                  // a later visit's value replaces an earlier one's
+            }
+        }
+        const Node next = node(f);
+        __syncwarp();
+        const unsigned path = (v >> 20) & ((1u << D) - 1u);
+        acc |= path << j0;
+        state = nlev == D ? v : (v & 0x7FFFFFFFu) | (path << (32 - nlev) & 0x80000000u);
+        return next;
+    };
 
-    int bc = gsoff + b0 * 8;                            // shared offset of the current bin
-    long long gcv = gs[b0];                             // g at the current bin
-    int bp = bc + E_[0].x;                              // site 0: proposal (left neighbour unprocessed)
-    long long LD = lds64(sm, bp);                       // g at the proposed bin
-    int q0 = bc + E_[1].x, q1 = bp + E_[1].y;           // site 1 if site 0 is rejected / accepted
-    long long l0 = 0, l1 = 0;
-    if (!kLean) { l0 = lds64(sm, q0); l1 = lds64(sm, q1); }
-    long long gcT = gcv - lnf + T_[0];                  // g at the current bin + threshold
-
-    const int nch = N / C;
-    const int total = p.nsweeps * nch;
-    int y = 0, x0 = 0;                                  // position of the current chunk
-    for (int t = 0; t < total; ++t) {
-        const int tn = t + 1;                           // the next chunk (wraps into the next sweep)
-        int yn = y, xn = x0 + C;
-        if (xn == L) { xn = 0; yn = y + 1 == L ? 0 : y + 1; }
-        const int c0 = y * L + x0;
-        const long long* Tc = Tb + ((t >> 2) & 1) * 4 * C + (t & 3) * C;
-        const long long* Tn = Tb + ((tn >> 2) & 1) * 4 * C + (tn & 3) * C;
-        const int2* Dc = Db + (t & 1) * C;
-        int2* Dn = Db + (tn & 1) * C;
-        if ((tn & 3) == 0 && tn < total) {
-            // the next chunk opens a batch: draw it now (its buffer is not in use)
-            const int swn = tn / nch;
-            draw((sweeps0 + (uint64_t)swn) * (uint64_t)N + (uint64_t)((tn - swn * nch) * C), (tn >> 2) & 1);
+    const uint64_t A0 = sweeps0 * (uint64_t)N;                 // first attempt
+    uint64_t drawn = A0 >> 2;                                  // first Philox block not drawn
+    int ready = -(int)(A0 & 3);                                // thresholds in the ring from the current chunk on
+    for (; ready < 64; ready += 4 * P, drawn += P) draw(drawn);
+    Planes next_planes = publish(0, 0, 0, -1, 0u);
+    unsigned up_flips = 0;                                     // the flips of the chunk above (whole-row chunks)
+    __syncwarp();
+    const bool wraps = rc.n == 1;                              // a row is one chunk: its last site sees its first
+    int y = 0, ci = 0, buf = 0;
+    uint32_t at = (uint32_t)A0;                                // the current chunk's first attempt (ring index)
+    uint64_t left = (uint64_t)p.nsweeps * (uint64_t)N;
+    // the change of a whole-row chunk's last count when the row's first site has flipped
+    auto wrap_term = [&](int yy) {
+        const unsigned sw = lat[yy * rc.n];
+        return (((sw >> (L - 1)) ^ sw) & 1u) ? 1 : -1;         // first and last disagree: a flip makes them agree
+    };
+    const int blocks_min = (rc.base + D - 1) / D;
+    // rows of one block: the last site's wrap term depends on the block's own first decision
+    auto node_row = [&](const unsigned char* slot, uint32_t attempt, int len, int yy) {
+        unsigned w0 = 0, w1 = 0;
+        if (first) (len < 5 ? w0 : w1) = (unsigned)wrap_term(yy) << (len < 5 ? 8 * (len - 1) : 0);
+        Slot f = fetch(slot, attempt);
+        f.e0 += w0;
+        f.e1 += w1;
+        return node(f);
+    };
+    Node n = blocks_min == 1 ? node_row(slots, at, L, 0) : node(fetch(slots, at));
+    while (left > 0) {
+        const int len = rc.len(ci), nblk = (len + D - 1) / D;
+        const int cw = y * rc.n + ci;
+        int yn = y, cn = ci + 1;
+        if (cn == rc.n) { cn = 0; yn = y + 1 == L ? 0 : y + 1; }
+        if (ready < 64) {
+            draw(drawn);
+            drawn += P;
+            ready += 4 * P;
             __syncwarp();
         }
-        prepare(yn, xn, c0);
-        long long Tnext0 = Tn[0];
-
-        long long Tr[C + 1];
-        int2 Er[C];
-        Tr[0] = T_[0];
-#pragma unroll
-        for (int i = 1; i < 4; ++i) Tr[i] = T_[i];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) Er[i] = E_[i];
-        unsigned acc = 0;
-#pragma unroll
-        for (int j = 0; j < C; ++j) {
-            if ((j & 1) == 0 && j + kAhead + 2 <= C) {
-                const int jn = j + kAhead;
-                const longlong2 tv = reinterpret_cast<const longlong2*>(Tc)[jn >> 1];
-                Tr[jn] = tv.x; Tr[jn + 1] = tv.y;
-                const int4 d = reinterpret_cast<const int4*>(Dc)[jn >> 1];
-                Er[jn] = make_int2(d.x, d.y); Er[jn + 1] = make_int2(d.z, d.w);
-            }
-            if (j == C - 1) Tr[C] = Tnext0;
-            const bool a = LD < gcT;
-            const long long sel = a ? LD : gcv;
-            const long long gnew = sel + lnf;
-            const int bnew = a ? bp : bc;
-            sts64(sm, bnew, gnew);
-            if (OBS) seqb[j] = bnew;
-            if (a) acc |= 1u << j;
-            if (j == 1 || j == 3) {
-                // next chunk's sites j-1, j: the neighbours they have in this chunk are decided
-#pragma unroll
-                for (int i = j - 1; i <= j; ++i) {
-                    const int2 v = finish(i / P, acc);
-                    E_[i] = make_int2(__shfl_sync(kFull, v.x, gbase + i % P), __shfl_sync(kFull, v.y, gbase + i % P));
+        acc = 0;
+        const unsigned char* cur = slots + buf * kBuf;
+        const unsigned char* nxt = slots + (buf ^ 1) * kBuf;
+        const Planes planes = next_planes;
+        const unsigned old = planes.sw;
+        auto none = [&] { return Slot{}; };
+        // the change of the last site's count where the row's first site has flipped (its right neighbour)
+        auto wrap_byte = [&] {
+            const unsigned t = ((old >> (len - 1)) ^ old) & 1u ? 1u : 0xFFFFFFFFu;
+            return wraps && (acc & 1u) ? t << (8 * (((len - 1) % D) & 3)) : 0u;
+        };
+        const bool fifth = D == 5 && (len - 1) % D == 4;
+        if (blocks_min >= 3) {
+            // three blocks or more: every block's node work runs while the block before it decides.
+            // The next chunk's slots are published during the last block but one; where the chunk
+            // above it is this one, the counts of its last two blocks are written again during its
+            // first block, with this chunk's last decisions.
+            uint32_t k = at + D;
+            const unsigned char* slot = cur + T::kSlot;
+            const int late = (nblk - 2) * D;
+            n = block(n, D, 0, [&] {
+                if (nblk == 3) {
+                    if (wraps) write_slots(planes, up_flips, ci, len, late, buf);
+                    __syncwarp();
+                    return fetch(slot, k);
                 }
-            }
-            gcT = sel + Tr[j + 1];                     // gnew + threshold of site j+1
-            bp = a ? q1 : q0;
-            if (kLean) {
-                LD = lds64(sm, bp);                    // read after this step's write: current
-            } else {
-                const long long lt = a ? l1 : l0;
-                LD = bp == bnew ? gnew : lt;           // the prefetch read the bin just committed
-            }
-            const int2 ev = (j + 2 < C) ? Er[j + 2] : E_[j + 2 - C];
-            int e0 = ev.x, e1 = ev.y;
-            if (j + 2 == C - 1) {                      // a row's last site sees the row start
-                const int wv = (wraps && (acc & 1u)) ? cwrap : 0;
-                e0 += wv; e1 += wv;
-            }
-            q0 = bnew + e0;
-            q1 = bp + e1;
-            if (!kLean) {
-                l0 = lds64(sm, q0);
-                l1 = lds64(sm, q1);
-            }
-            bc = bnew;
-            gcv = gnew;
+                const Slot m = fetch(slot, k);
+                if (wraps) write_slots(planes, up_flips, ci, len, late, buf);
+                return m;
+            });
+            k += D;
+            slot += T::kSlot;
+            int j0 = D;
+#pragma unroll 2
+            for (; j0 < late; j0 += D, k += D, slot += T::kSlot)
+                n = block(n, D, j0, [&] { return fetch(slot, k); });
+            n = block(n, D, j0, [&] {
+                const unsigned wr = wrap_byte();
+                Slot m = fetch(slot, k);
+                m.e0 += fifth ? 0u : wr;
+                m.e1 += fifth ? wr : 0u;
+                next_planes = publish(yn, cn, buf ^ 1, cw, acc);
+                return m;
+            });
+            j0 += D;
+            n = block(n, len - j0, j0, [&] { return fetch(nxt, at + (uint32_t)len); });
+        } else if (nblk == 2) {
+            n = block(n, D, 0, none);
+            const unsigned wr = wrap_byte();
+            Slot f = fetch(cur + T::kSlot, at + D);
+            f.e0 += fifth ? 0u : wr;
+            f.e1 += fifth ? wr : 0u;
+            n = node(f);
+            publish(yn, cn, buf ^ 1, cw, acc);
+            __syncwarp();
+            n = block(n, len - D, D, [&] { return fetch(nxt, at + (uint32_t)len); });
+        } else {
+            n = block(n, len, 0, none);
         }
-        // apply the chunk's flips and the magnetisation change
-        {
-            unsigned plus = 0;
+        // the chunk's flips
+        if (q == 0) lat[cw] = old ^ acc;
+        __syncwarp();
+        up_flips = acc;
+        if (blocks_min < 3) {
+            // short rows: the next row's counts with all of this one's decisions
+            next_planes = publish(yn, cn, buf ^ 1, -1, 0u);
+            __syncwarp();
+            if (nblk == 1) n = node_row(nxt, at + (uint32_t)len, L, yn);
+        }
+        if (OBS) {
+            // the chunk's moments and correlators, one step per lane
+            const unsigned plus = ~old & (0xFFFFFFFFu >> (32 - len));
+            const int x0 = rc.start(ci);
 #pragma unroll
-            for (int k = 0; k < SPL; ++k) {
-                const int jj = q + k * P;
-                const unsigned bal = __ballot_sync(kFull, jj < C && cs[k] > 0);
-                const unsigned mine = P == 32 ? bal : ((bal >> gbase) & ((1u << P) - 1u));
-                plus |= (k * P < 32) ? (mine << (k * P)) : 0u;
-                if (jj < C && ((acc >> jj) & 1u)) lat[c0 + jj] = (int8_t)(-cs[k]);
-            }
-            const unsigned full = C == 32 ? 0xFFFFFFFFu : ((1u << C) - 1u);
-            if (OBS) __syncwarp();
-            if (OBS && valid) {
-                double* ob = P_.obs + (size_t)P_.slot_tab[s] * P_.obs_stride;
-#pragma unroll
-                for (int k = 0; k < SPL; ++k) {
-                    const int jj = q + k * P;
-                    if (jj < C)
-                    {
-                        const int32_t Mv[1] = {M + chunk_dm(acc, plus, jj)};
-                        Ising2dModel::add_observables(ob + (size_t)((seqb[jj] - gsoff) >> 3) * P_.obs_stride, Mv,
-                                                      1.0 / (double)N, P_.corr);
+            for (int i = 0; i < SPL; ++i) {
+                const int jj = q + i * P;
+                const bool mine = valid && jj < len;
+                const int off = mine ? seqb[jj] : -1 - lane;
+                const int b = mine ? (off - gsoff) / RS : 0;
+                if (mine) {
+                    const int32_t Mv[1] = {M + chunk_dm(acc, plus, jj)};
+                    if (moments) {
+                        const unsigned m = (unsigned)abs(Mv[0]), m2 = m * m;
+                        const unsigned long long m4 = (unsigned long long)m2 * m2;
+                        unsigned* t = mom + kObsWords * b;
+                        add_carry(t, m);
+                        add_carry(t + 2, m2);
+                        add_carry(t + 4, (unsigned)(m4 & 0xFFFFFFFu));
+                        add_carry(t + 6, (unsigned)(m4 >> 28));
+                    } else {
+                        Ising2dModel::add_observables(ob + (size_t)b * P_.obs_stride, Mv, invN, P_.corr);
                     }
                 }
-            }
-            if (corr) {
-                // G(q_min) at the steps whose bin count before the visit is a multiple of 1000:
-                // bcnt holds every bin's count before this chunk (mod 1000), to which the chunk's
-                // earlier visits to the bin are added.  The chunk's bins are read once into
-                // registers (broadcast loads) and compared there.  The lattice already holds the
-                // chunk's flips: an accepted site's value before the chunk is minus its value now.
-                int first[SPL], total[SPL];
-#pragma unroll
-                for (int k = 0; k < SPL; ++k) { first[k] = 0; total[k] = 0; }
-                if (valid) {
-                    int sq[C];
-#pragma unroll
-                    for (int j2 = 0; j2 < C; j2 += 4) {
-                        const int4 v = reinterpret_cast<const int4*>(seqb)[j2 >> 2];
-                        sq[j2] = v.x; sq[j2 + 1] = v.y; sq[j2 + 2] = v.z; sq[j2 + 3] = v.w;
-                    }
-                    const double invN = 1.0 / (double)N;
-                    double* ob = P_.obs + (size_t)P_.slot_tab[s] * P_.obs_stride;
-#pragma unroll
-                    for (int k = 0; k < SPL; ++k) {
-                        const int jj = q + k * P;
-                        if (jj >= C) continue;
-                        const int off = seqb[jj], b = (off - gsoff) >> 3;
-                        int earlier = 0, all = 0;
-#pragma unroll
-                        for (int j2 = 0; j2 < C; ++j2) {
-                            const int eq = sq[j2] == off ? 1 : 0;
-                            earlier += j2 < jj ? eq : 0;
-                            all += eq;
-                        }
-                        first[k] = earlier == 0;
-                        total[k] = all;
-                        if ((bcnt[b] + earlier) % (int)kCountsPerTransform == 0) {
+                if (corr) {
+                    // G(q_min) at the steps whose bin count before the visit is a multiple of 1000: the
+                    // count before this strip of steps plus the strip's earlier visits to the bin
+                    const unsigned same = __match_any_sync(kFull, off), earlier = same & ((1u << lane) - 1u);
+                    if (mine) {
+                        const int seen = bcnt[b] + __popc(earlier);
+                        if (seen == 0 || seen == (int)kCountsPerTransform) {
                             const double Gq = plane_corr(rsum, csum, P_.qtab + I.qtab_off, L, y, chunk_dm(acc, plus, jj), x0,
-                                                         jj, acc, [&](int kk) { return -(int)lat[c0 + kk]; });
+                                                         jj, acc, [&](int kk) { return (old >> kk) & 1u ? -1 : 1; });
                             atomicAdd(ob + (size_t)b * P_.obs_stride + 3, invN * invN * Gq);
                         }
                     }
+                    __syncwarp();
+                    if (mine && earlier == 0) {
+                        const int n2 = bcnt[b] + __popc(same);
+                        bcnt[b] = n2 >= (int)kCountsPerTransform ? n2 - (int)kCountsPerTransform : n2;
+                    }
+                    __syncwarp();
                 }
-                __syncwarp();
-                // the chunk's flips into the row and column sums, its visits into the counts (by
-                // the first step at each bin)
-#pragma unroll
-                for (int k = 0; k < SPL; ++k) {
-                    const int jj = q + k * P;
-                    if (valid && jj < C && ((acc >> jj) & 1u)) csum[x0 + jj] += 2 * (int)lat[c0 + jj];
-                    if (valid && jj < C && first[k]) bcnt[(seqb[jj] - gsoff) >> 3] += total[k];
-                }
-                if (valid && q == 0) rsum[y] += -2 * ((int)__popc(acc & plus) - (int)__popc(acc & ~plus & full));
-                __syncwarp();
             }
-            M += -2 * ((int)__popc(acc & plus) - (int)__popc(acc & ~plus & full));
-        }
-        // publish the next chunk: spins, offsets, wrap term, first thresholds
+            if (corr) {
+                // the chunk's flips into the row and column sums
 #pragma unroll
-        for (int k = 0; k < SPL; ++k) {
-            const int jj = q + k * P;
-            cs[k] = ns[k];
-            if (jj < C) Dn[jj] = finish(k, acc);
+                for (int i = 0; i < SPL; ++i) {
+                    const int jj = q + i * P;
+                    if (valid && jj < len && ((acc >> jj) & 1u)) csum[x0 + jj] -= 2 * ((old >> jj) & 1u ? -1 : 1);
+                }
+                if (valid && q == 0) rsum[y] += chunk_dm(acc, plus, 31);
+            }
+            M += chunk_dm(acc, plus, 31);
+            __syncwarp();
         }
-        cwrap = __shfl_sync(kFull, (nwrap >> sh) * 8, gbase + (C - 1) % P);
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) T_[i] = Tn[i];
-        y = yn; x0 = xn;
+        left -= (uint64_t)len;
+        at += (uint32_t)len;
+        ready -= len;
+        y = yn; ci = cn; buf ^= 1;
     }
     __syncwarp();
+    int down = 0;                                              // spins -1 at the end
+    for (int c = 0, i = 0; c < rc.n * L; ++c) {
+        const int len = rc.len(c % rc.n);
+        const unsigned bits = lat[c];
+        down += __popc(bits);
+        if (valid)
+            for (int jj = q; jj < len; jj += P) gl[i + jj] = (bits >> jj) & 1u ? -1 : 1;
+        i += len;
+    }
     if (valid) {
-        for (int i = q; i < N; i += P) gl[i] = lat[i];
         uint32_t* gH = P_.H + P_.slot_tab[s];
         uint64_t* gv = P_.visits + P_.slot_tab[s];
         for (int k = q; k < nb; k += P) {
-            const long long gnew = gs[k];
-            const long long dv = (gnew - gg[k]) / lnf;
+            const long long dv = CNT ? gs[RW * k + 1] : (gs[k] - gg[k]) / lnf;
+            const long long gnew = CNT ? gs[RW * k] + dv * lnf : gs[k];
             const int e = commit_visits(gH, gv, k, dv, gnew);
             if (e) atomicOr(&P_.counters[0], e);
             gg[k] = gnew;
         }
+        if (moments) {
+            // m = |M| / N: the launch's sums are whole numbers until here
+            const double in2 = invN * invN;
+            for (int k = q; k < nb; k += P) {
+                const unsigned* t = mom + kObsWords * k;
+                auto sum = [&](int j) { return (double)(((unsigned long long)t[j + 1] << 32) | t[j]); };
+                double* o = ob + (size_t)k * P_.obs_stride;
+                if ((t[0] | t[1]) == 0) continue;
+                o[0] += invN * sum(0);
+                o[1] += in2 * sum(2);
+                o[2] += in2 * in2 * (268435456.0 * sum(6) + sum(4));
+            }
+        }
         if (q == 0) {
-            if ((unsigned)(bc - gsoff) >= (unsigned)(nb * 8)) atomicOr(&P_.counters[0], ERR_BOUNDS);
-            P_.cfg_E[cfg] = (long long)Ewlo + ((long long)((bc - gsoff) >> 3) << sh);
-            P_.cfg_M[3 * cfg] = M;
+            const int root = (int)(state & 0xFFFFFu);
+            if ((unsigned)(root - gsoff) >= (unsigned)(nb * RS)) atomicOr(&P_.counters[0], ERR_BOUNDS);
+            P_.cfg_E[cfg] = (long long)Ewlo + ((long long)((root - gsoff) / RS) << sh);
+            P_.cfg_M[3 * cfg] = N - 2 * down;
             P_.slot_sweeps[s] = sweeps0 + (uint64_t)p.nsweeps;
         }
     }
 }
 
-template <int G, int C, bool OBS, bool LEAN>
+template <int G, bool OBS, bool CNT>
 __global__ void __launch_bounds__(128, 1) k_sweep_ising_bins(const SweepParams p)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int wib = threadIdx.x >> 5;
-    sweep_bins_warp<G, C, OBS, LEAN>(p, blockIdx.x * (blockDim.x >> 5) + wib, smem + (size_t)wib * G * p.smem_per_warp);
+    sweep_bins_warp<G, OBS, CNT>(p, blockIdx.x * (blockDim.x >> 5) + wib, smem + (size_t)wib * G * p.smem_per_warp);
 }
 
-template <int G, bool OBS, bool LEAN>
-void launch_bins_t(int C, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const SweepParams& sp)
+SweepKernel bins_kernel(int G, bool obs, bool cnt)
 {
-    switch (C) {
-    case 32: k_sweep_ising_bins<G, 32, OBS, LEAN><<<grid, block, smem, st>>>(sp); break;
-    case 24: k_sweep_ising_bins<G, 24, OBS, LEAN><<<grid, block, smem, st>>>(sp); break;
-    case 16: k_sweep_ising_bins<G, 16, OBS, LEAN><<<grid, block, smem, st>>>(sp); break;
-    case 8: k_sweep_ising_bins<G, 8, OBS, LEAN><<<grid, block, smem, st>>>(sp); break;
-    default: k_sweep_ising_bins<G, 4, OBS, LEAN><<<grid, block, smem, st>>>(sp); break;
-    }
-}
-
-// lean: the chain without the candidate prefetch (several walkers per warp, enough warps per SM
-// to hide the shared-memory latency it exposes; observables off)
-template <int G>
-void launch_bins(int C, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const SweepParams& sp, bool lean)
-{
-    if (sp.P.obs) launch_bins_t<G, true, false>(C, grid, block, smem, st, sp);
-    else if (G > 1 && lean) launch_bins_t<G, false, (G > 1)>(C, grid, block, smem, st, sp);
-    else launch_bins_t<G, false, false>(C, grid, block, smem, st, sp);
-}
-
-template <int G, bool OBS, bool LEAN>
-cudaError_t allow_bins_smem_t()
-{
-    cudaError_t e = cudaSuccess;
-    e = e != cudaSuccess ? e : cudaFuncSetAttribute(k_sweep_ising_bins<G, 32, OBS, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    e = e != cudaSuccess ? e : cudaFuncSetAttribute(k_sweep_ising_bins<G, 24, OBS, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    e = e != cudaSuccess ? e : cudaFuncSetAttribute(k_sweep_ising_bins<G, 16, OBS, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    e = e != cudaSuccess ? e : cudaFuncSetAttribute(k_sweep_ising_bins<G, 8, OBS, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    e = e != cudaSuccess ? e : cudaFuncSetAttribute(k_sweep_ising_bins<G, 4, OBS, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
-    return e;
-}
-
-template <int G>
-cudaError_t allow_bins_smem()
-{
-    cudaError_t e = allow_bins_smem_t<G, false, false>();
-    e = e != cudaSuccess ? e : allow_bins_smem_t<G, true, false>();
-    if (G > 1) e = e != cudaSuccess ? e : allow_bins_smem_t<G, false, (G > 1)>();
-    return e;
+    if (!cnt) return obs ? k_sweep_ising_bins<1, true, false> : k_sweep_ising_bins<1, false, false>;
+    if (G == 1) return obs ? k_sweep_ising_bins<1, true, true> : k_sweep_ising_bins<1, false, true>;
+    if (G == 2) return obs ? k_sweep_ising_bins<2, true, true> : k_sweep_ising_bins<2, false, true>;
+    return obs ? k_sweep_ising_bins<4, true, true> : k_sweep_ising_bins<4, false, true>;
 }
 
 // Ashkin-Teller: sweep = sigma pass then tau pass (wang_landau.hpp:109-119); the
@@ -1393,14 +1566,13 @@ __global__ void __launch_bounds__(256, 2) k_sweep_tables(const SweepParams p)
 // fused kernel's registers are those of its dispatch loop plus the largest callee.
 // --------------------------------------------------------------------------
 enum FusedKind : int {
-    kFusedBins32 = 0, kFusedBins24 = 1, kFusedBins16 = 2, kFusedBins8 = 3, kFusedBins4 = 4,
-    kFusedTablesIsing = 5, kFusedTablesAT = 6
+    kFusedBins = 0, kFusedTablesIsing = 1, kFusedTablesAT = 2
 };
 constexpr int kMaxFusedGroups = 16;
 
 struct FusedGroup {
     const int32_t* slots;
-    int nslots, smem_per_warp, nbcap, kind, first_task, pad;
+    int nslots, smem_per_warp, nbcap, kind, first_task, counts, moments;
 };
 
 struct FusedParams {
@@ -1410,10 +1582,11 @@ struct FusedParams {
     FusedGroup g[kMaxFusedGroups];
 };
 
-template <int C, bool OBS>
+template <bool OBS>
 __device__ __noinline__ void fused_bins(const SweepParams& p, int unit, unsigned char* base)
 {
-    sweep_bins_warp<1, C, OBS, false>(p, unit, base);
+    if (p.counts) sweep_bins_warp<1, OBS, true>(p, unit, base);
+    else sweep_bins_warp<1, OBS, false>(p, unit, base);
 }
 
 template <class Model, bool OBS>
@@ -1438,14 +1611,10 @@ __global__ void __launch_bounds__(128) k_sweep_fused(const FusedParams fp)
         const FusedGroup& G = fp.g[gi];
         SweepParams sp;
         sp.P = fp.P; sp.slots = G.slots; sp.nslots = G.nslots; sp.nsweeps = fp.nsweeps;
-        sp.smem_per_warp = G.smem_per_warp; sp.nbcap = G.nbcap;
+        sp.smem_per_warp = G.smem_per_warp; sp.nbcap = G.nbcap; sp.counts = G.counts; sp.moments = G.moments;
         const int unit = t - G.first_task;
         switch (G.kind) {
-        case kFusedBins32: fused_bins<32, OBS>(sp, unit, base); break;
-        case kFusedBins24: fused_bins<24, OBS>(sp, unit, base); break;
-        case kFusedBins16: fused_bins<16, OBS>(sp, unit, base); break;
-        case kFusedBins8: fused_bins<8, OBS>(sp, unit, base); break;
-        case kFusedBins4: fused_bins<4, OBS>(sp, unit, base); break;
+        case kFusedBins: fused_bins<OBS>(sp, unit, base); break;
         case kFusedTablesIsing: fused_tables<Ising2dModel, OBS>(sp, unit, base); break;
         default: fused_tables<AshkinTeller2dModel, OBS>(sp, unit, base); break;
         }
@@ -1766,15 +1935,14 @@ struct Launch {
     int smem_per_warp = 0;  // per walker for the bin-tracking kernel, per warp otherwise
     int nbcap = 0;
     int wpb = 1;            // warps per block
-    int bins = 0;           // Ising bin-tracking kernel with `walkers_per_warp` walkers per warp and chunk `chunk`
+    int bins = 0;           // Ising bin-tracking kernel with `walkers_per_warp` walkers per warp
     int walkers_per_warp = 1;
-    int chunk = 32;
+    int counts = 0;         // bin-tracking kernel: visit counts beside g in shared memory (16 bytes per bin)
+    int moments = 0;        // bin-tracking kernel with observables: moment sums in shared memory
     int tables = 0;         // the global-table kernel (k_sweep_tables)
     int carveout = -1;      // global-table kernel: shared-memory carveout (percent) that leaves the rest to L1
     DBuf<int32_t> d_slots;
 };
-
-using SweepKernel = void (*)(const SweepParams);
 
 template <class Model>
 SweepKernel table_kernel_t(bool replay, bool obs)
@@ -1831,7 +1999,6 @@ struct rewl_engine {
     int64_t kernel_launches = 0;        // sweep-kernel launches since the last timing read
     int64_t launches_total = 0;         // every engine kernel since creation
     int sweep_variant = 3;              // REWL_SWEEP_VARIANT: 3 all-lane Ising resolver (default), 2 lane-0, 4 global tables
-    int bins_lean = -1;                 // REWL_BINS_LEAN: 1 / 0 forces the lean bin-tracking chain on / off (-1: by occupancy)
 
     DBuf<InstDev> d_inst;
     DBuf<WinDev> d_win;
@@ -2189,22 +2356,22 @@ int upload_all(rewl_engine* e)
 
 bool bins_eligible(const InstDev& I, const rewl_batch_desc& D, int max_window_bins)
 {
-    if (I.model != REWL_MODEL_ISING2D || D.rng_mode != REWL_RNG_PHILOX) return false;
+    if (I.model != REWL_MODEL_ISING2D || D.rng_mode != REWL_RNG_PHILOX || I.L < 3) return false;
     // the window table, with its guard bins, and the lattice live in shared memory (with the
     // correlators also the bin counts and the row and column sums)
-    const size_t need = (size_t)(max_window_bins + 2 + 2 * kGuard) * 8 + I.N + 4096 +
-                        (D.observables == 2 ? (size_t)4 * (max_window_bins + 2) + 8 * I.L : 0);
+    const size_t need = (size_t)bins_smem<1>((max_window_bins + 3) & ~1, I.L, D.observables != 0, D.observables == 2, false, false) + 256;
     if (need > 200 * 1024) return false;
-    const int C = I.chunk;
-    if (!(C == 32 || C == 24 || C == 16 || C == 8 || C == 4)) return false;
     const long long step = 4 * std::llabs(I.J_u);            // every energy change is a multiple of 4|J|
     if (step % (1LL << I.bin_shift) != 0) return false;
-    // the thresholds are drawn four sites per Philox block, 4C sites at a time
-    if (I.N % (4 * C) != 0) return false;
-    // a proposal lands at most 8|J| / width bins away, and a prefetch issued from an
-    // out-of-window proposal twice that: the guard bins cover both
+    // a proposal lands at most 2 x 4|J| / width bins away; the guard bins cover five of them
     const long long maxbins = (8 * std::llabs(I.J_u)) >> I.bin_shift;
-    if (2 * maxbins > kGuard) return false;
+    if (5 * maxbins > kGuard) return false;
+    // energies are -2 N J plus multiples of 4|J|: the bins' lower edges have to be energies
+    if (((-2 * (long long)I.N * I.J_u - I.eglo_u) & ((1LL << I.bin_shift) - 1)) != 0) {
+        // lattices cut into whole chunks of 4, 8, 16, 24 or 32 sites report this as an energy off its bin
+        const int C = I.chunk;
+        return (C == 32 || C == 24 || C == 16 || C == 8 || C == 4) && I.N % (4 * C) == 0;
+    }
     return true;
 }
 
@@ -2267,10 +2434,9 @@ int plan_fused(rewl_engine* e, int nsm)
     for (size_t k = 0; k < order.size(); ++k) {
         const Launch& l = e->launches[order[k].second];
         FusedGroup& G = F.g[k];
-        G.slots = l.d_slots.p; G.nslots = (int)l.slots.size(); G.smem_per_warp = l.smem_per_warp; G.nbcap = l.nbcap;
+        G.slots = l.d_slots.p; G.nslots = (int)l.slots.size(); G.smem_per_warp = l.smem_per_warp; G.nbcap = l.nbcap; G.counts = l.counts; G.moments = l.moments;
         if (l.bins)
-            G.kind = l.chunk == 32 ? kFusedBins32 : l.chunk == 24 ? kFusedBins24 : l.chunk == 16 ? kFusedBins16
-                   : l.chunk == 8 ? kFusedBins8 : kFusedBins4;
+            G.kind = kFusedBins;
         else if (l.tables)
             G.kind = l.model == REWL_MODEL_ISING2D ? kFusedTablesIsing : kFusedTablesAT;
         else
@@ -2306,7 +2472,7 @@ int plan_launches(rewl_engine* e)
     const int nsm = sm_count(e);
     // group walkers by (model, bin-tracking kernel, chunk, sites) so each launch has one
     // kernel shape and the walkers sharing a warp run the same number of chunks
-    struct Key { int model, bins, chunk, sites; };
+    struct Key { int model, bins, sites; };
     std::vector<Key> keys;
     std::vector<Launch> plans;
     for (int s = 0; s < e->nslots; ++s) {
@@ -2314,16 +2480,15 @@ int plan_launches(rewl_engine* e)
         int max_nb = 0;
         for (const auto& wd : H.wins) max_nb = std::max(max_nb, wd.nb);
         const int bins = bins_eligible(H.dev, e->desc, max_nb) && getenv("REWL_SWEEP_VARIANT") == nullptr ? 1 : 0;
-        Key k{H.d.model, bins, bins ? H.dev.chunk : 0, bins ? H.dev.N : 0};
+        Key k{H.d.model, bins, bins ? H.dev.N : 0};
         size_t idx = 0;
         for (; idx < keys.size(); ++idx)
-            if (keys[idx].model == k.model && keys[idx].bins == k.bins && keys[idx].chunk == k.chunk &&
-                keys[idx].sites == k.sites)
+            if (keys[idx].model == k.model && keys[idx].bins == k.bins && keys[idx].sites == k.sites)
                 break;
         if (idx == keys.size()) {
             keys.push_back(k);
             Launch l;
-            l.model = k.model; l.bins = k.bins; l.chunk = k.chunk ? k.chunk : 32;
+            l.model = k.model; l.bins = k.bins;
             plans.push_back(std::move(l));
         }
         plans[idx].slots.push_back(s);
@@ -2346,12 +2511,20 @@ int plan_launches(rewl_engine* e)
                 // 3072); four only for still larger batches
                 G = n <= 4 * nsm ? 1 : (n <= 32 * nsm ? 2 : 4);
             }
-            l.walkers_per_warp = G;
             l.nbcap = (maxnb + 1) & ~1;
-            int raw = (((l.nbcap + 2 * kGuard) * 8 + 15) & ~15) + ((maxN + 15) & ~15) + 8 * l.chunk * 8 + 2 * l.chunk * 8 + l.chunk * 4
-                      + (corr ? 8 * maxL + 4 * l.nbcap : 0);
-            l.smem_per_warp = ((raw + 127) & ~127) + 16;           // per walker; +16 skews the walkers' banks
-            if ((size_t)l.smem_per_warp * G > 220 * 1024) return fail(REWL_EINVAL, "a walker needs %d bytes of shared memory", l.smem_per_warp);
+            const bool obs = e->desc.observables != 0;
+            // per walker, the largest of the shapes the autotuner may pick; +16 skews the walkers' banks
+            auto raw = [&](bool cnt, bool acc) {
+                return std::max({bins_smem<1>(l.nbcap, maxL, obs, corr, cnt, acc), bins_smem<2>(l.nbcap, maxL, obs, corr, cnt, acc),
+                                 bins_smem<4>(l.nbcap, maxL, obs, corr, cnt, acc)});
+            };
+            if ((size_t)raw(false, false) * G > 220 * 1024)
+                return fail(REWL_EINVAL, "a walker needs %d bytes of shared memory", raw(false, false));
+            l.counts = raw(true, false) + 144 <= 200 * 1024 / G;
+            if (!l.counts) G = 1;                                  // g alone: one walker per warp only
+            l.moments = obs && raw(l.counts, true) + 144 <= 200 * 1024 / G;
+            l.walkers_per_warp = G;
+            l.smem_per_warp = ((raw(l.counts, l.moments) + 127) & ~127) + 16;
             int wpb = e->desc.warps_per_block;
             if (wpb == 0) {
                 const int warps = (n + G - 1) / G;
@@ -2400,9 +2573,9 @@ int plan_launches(rewl_engine* e)
         if (l.tables && !e->gsnap.p && e->table_total > 0)
             if (int rc = e->gsnap.alloc(e->table_total)) return rc;
     }
-    CUDA_TRY(allow_bins_smem<1>());
-    CUDA_TRY(allow_bins_smem<2>());
-    CUDA_TRY(allow_bins_smem<4>());
+    for (int G : {1, 2, 4})
+        for (int o = 0; o < 4; ++o)
+            CUDA_TRY(cudaFuncSetAttribute(bins_kernel(G, o & 1, o & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     if (e->desc.persistent) return plan_fused(e, nsm);
     if (e->launches.size() > 1) {
         CUDA_TRY(cudaEventCreateWithFlags(&e->fork_ev, cudaEventDisableTiming));
@@ -2457,19 +2630,13 @@ int launch_group(rewl_engine* e, Launch& l, cudaStream_t stream, int nsweeps, co
     const bool replay = e->desc.rng_mode == REWL_RNG_REPLAY;
     SweepParams sp;
     sp.P = P; sp.slots = l.d_slots.p; sp.nslots = (int)l.slots.size(); sp.nsweeps = nsweeps;
-    sp.smem_per_warp = l.smem_per_warp; sp.nbcap = l.nbcap;
+    sp.smem_per_warp = l.smem_per_warp; sp.nbcap = l.nbcap; sp.counts = l.counts; sp.moments = l.moments;
     if (l.bins) {
         const int G = l.walkers_per_warp;
         const int warps = (sp.nslots + G - 1) / G;
         const int blocks = (warps + l.wpb - 1) / l.wpb;
         const size_t smem = (size_t)l.wpb * G * l.smem_per_warp;
-        // the lean chain from 5 warps per SM on (measured at L = 64, two walkers per warp: 2048
-        // walkers 3.78e10 against 3.55e10 flips/s, 3072 4.62e10 against 3.78e10; 1024 walkers,
-        // 3.4 warps per SM, 2.15e10 against 2.43e10)
-        const bool lean = e->bins_lean < 0 ? warps >= 5 * sm_count(e) : e->bins_lean == 1;
-        if (G == 1) launch_bins<1>(l.chunk, blocks, 32 * l.wpb, smem, stream, sp, false);
-        else if (G == 2) launch_bins<2>(l.chunk, blocks, 32 * l.wpb, smem, stream, sp, lean);
-        else launch_bins<4>(l.chunk, blocks, 32 * l.wpb, smem, stream, sp, lean);
+        bins_kernel(G, P.obs != nullptr, l.counts)<<<blocks, 32 * l.wpb, smem, stream>>>(sp);
     } else {
         const int blocks = (sp.nslots + l.wpb - 1) / l.wpb;
         const size_t smem = (size_t)l.wpb * l.smem_per_warp;
@@ -2502,7 +2669,8 @@ cudaError_t record_timing(rewl_engine* e)
 int max_launch_sweeps(const rewl_engine* e)
 {
     const int64_t visits = kLaunchGrowth / std::max<int64_t>(1, e->lnf_bound_u) - 1;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(1 << 20, visits / std::max<int64_t>(1, e->ndof_max)));
+    // the bin-tracking kernel counts a launch's visits in 31 bits
+    return (int)std::max<int64_t>(1, std::min<int64_t>(1 << 20, std::min<int64_t>(visits, INT32_MAX) / std::max<int64_t>(1, e->ndof_max)));
 }
 
 // Raise the ln f bound (rewl_set_lnf, rewl_restore); a captured check interval split its sweeps
@@ -2726,9 +2894,6 @@ int rewl_create(const rewl_batch_desc* desc, rewl_engine** out)
         const int k = std::atoi(v);
         e->sweep_variant = (k == 2 || k == 4) ? k : 3;
     }
-    // REWL_BINS_LEAN: 1 / 0 forces the lean chain of the bin-tracking kernel on / off for warps
-    // of several walkers (tests; by default it is taken from 5 warps per SM on)
-    if (const char* v = std::getenv("REWL_BINS_LEAN")) e->bins_lean = std::atoi(v) == 1 ? 1 : 0;
     int rc = build_host(e);               // descriptor validation and layout: host only
     if (rc) { delete e; return rc; }
     int ndev = 0;
@@ -3665,7 +3830,7 @@ int rewl_autotune(rewl_engine* e, int32_t sweeps)
         // the bin-tracking kernel takes at most 4 warps per block (its launch bounds); 4 walkers
         // per warp is left to the planner's rule for very large batches
         for (int G : {1, 2}) {
-            if ((!l.bins && G > 1) || (l.bins && G > (int)l.slots.size())) continue;
+            if ((!l.counts && G > 1) || (l.bins && G > (int)l.slots.size())) continue;
             if (e->desc.walkers_per_warp && l.bins && G != e->desc.walkers_per_warp) continue;
             for (int W : {1, 2, 4, 8}) {
                 if (l.bins && W > 4) continue;
