@@ -45,6 +45,7 @@
 #include <random>
 #include <sstream>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/rewl.h"
@@ -362,6 +363,8 @@ struct SweepParams {
     int nbcap;               // table capacity per warp (Ising, shared memory)
     int counts;              // bin-tracking kernel: visit counts beside g in shared memory
     int moments;             // bin-tracking kernel with observables: moment sums in shared memory
+    int cache;               // global-table kernel: bins of each walker's table in shared memory
+    int replay;              // global-table kernel, serial chain: recorded uniforms
 };
 
 // Per-warp staging of one chunk for the lane-0 resolver: energy change without /
@@ -1248,23 +1251,20 @@ SweepKernel bins_kernel(int G, bool obs, bool cnt)
     return obs ? k_sweep_ising_bins<4, true, true> : k_sweep_ising_bins<4, false, true>;
 }
 
-// Ashkin-Teller: sweep = sigma pass then tau pass (wang_landau.hpp:109-119); the
-// flavour toggles after each pass.  A window holds tens of thousands of bins, so
-// its logDoS stays in global memory: each step reads g at the proposal and writes
-// g at the current bin, nothing else.  The counts and visits of the launch are
-// derived at its end from the change of g against a copy taken at its start
-// (every visit adds the same ln f), and the chain loads both possible proposals
-// of the next step one step ahead, so a load's latency overlaps a decision.
-// bins either side of the walker's bin prefetched into L1 per chunk (measured on the Ashkin-Teller
-// benchmark: 256 / 384 / 512 / 768 / 1024 bins 43.5 / 43.3 / 43.4 / 43.9 / 44.1 ms per launch)
-constexpr int kTableReach = 512;
+// Ashkin-Teller: sweep = sigma pass then tau pass (wang_landau.hpp:109-119); the flavour toggles
+// after each pass.  A window holds tens of thousands of bins, so its logDoS stays in global memory;
+// the part around the walker is held in shared memory (TableCache below).
+constexpr int kMinCache = 2048;
 
 struct TableStage {
-    longlong2 du[32];        // per site: {proposal, proposal after its left neighbour flipped in this chunk}
-    long long T[32];         // acceptance thresholds of the chunk's sites
+    longlong2 du[32 + 8];    // per site: {proposal, proposal after its left neighbour flipped in this chunk}
+    long long T[2][32 + 8];  // acceptance thresholds of two chunks' sites (the last block of a chunk reads past its sites)
     long long wcu;           // row-wrap correction of the last site when the chunk is a whole row
     int seq[32];             // bin after each step (observables)
+    unsigned sink;           // counts the lanes off the path, read by nobody
+    unsigned pad[3];
 };
+static_assert(sizeof(TableStage) % 16 == 0, "what follows is 16-byte aligned");
 
 // Chain state of one Ashkin-Teller walker (lane 0).  The energy is carried as its
 // position v = (E - E_lo) * bin_mul - gblo << bin_shift, in units of the bin
@@ -1273,34 +1273,31 @@ struct TableStage {
 struct TableChain {
     long long v, vn, gc, draws;
     long long G0, G1;        // logDoS loaded for step j's proposal if step j-1 was rejected / accepted
-    long long T;             // step j's threshold
     longlong2 q;             // step j+1's proposals
     int b, bn, err;
     bool inr, ap;            // step j's proposal in the window; step j-1 accepted
     unsigned acc;
 };
 
-// One step j of the chunk, software-pipelined two deep.  On entry (vn, bn, inr) is
-// step j's proposal, and its logDoS is G1 or G0 (as step j-1 was accepted or not),
-// loaded during step j-1.  With PREFETCH the two proposals of step j+1 (step j
-// rejected: from v; accepted: from vn) are loaded first, before step j waits on
-// its own loads, so two steps' loads are in flight at once.  A value loaded before
-// step j-1's write to bin b is stale exactly when the proposal is b: gc replaces
-// it.  LOADQ: step j+2 exists and its proposals are read from shared memory now.
-// WRAPFIX: step j+1 is the last site of a whole-row chunk, whose right neighbour
-// is the row's first site, flipped in this chunk iff bit 0 of acc.
-template <bool REPLAY, bool OBS, bool PREFETCH, bool LOADQ, bool WRAPFIX>
-__device__ __forceinline__ void table_step(TableChain& c, const int j, TableStage* st, long long* gg, const int nb,
-                                        const int sh, const long long lnf, const DevPtrs& P,
+// One step j of a chunk decided serially by lane 0, software-pipelined two deep: replayed runs,
+// whose recorded uniforms are consumed on demand, and windows whose bins the tree below cannot hold
+// in a register's high word.  On entry (vn, bn, inr) is step j's proposal, and its logDoS is G1 or G0
+// (as step j-1 was accepted or not), loaded during step j-1.  With PREFETCH the two proposals of step
+// j+1 (step j rejected: from v; accepted: from vn) are loaded first.  A value loaded before step j-1's
+// write to bin b is stale exactly when the proposal is b: gc replaces it.  LOADQ: step j+2 exists and
+// its proposals are read from shared memory now.  WRAPFIX: step j+1 is the last site of a whole-row
+// chunk, whose right neighbour is the row's first site, flipped in this chunk iff bit 0 of acc.
+template <bool OBS, bool PREFETCH, bool LOADQ, bool WRAPFIX>
+__device__ __forceinline__ void serial_step(TableChain& c, const int j, TableStage* st, long long* gg, const int nb,
+                                        const int sh, const long long lnf, const DevPtrs& P, const bool replay,
                                         const long long thr_off, const long long thr_n)
 {
-    long long t0 = 0, t1 = 0, G0 = 0, G1 = 0, Tn = 0;
+    long long t0 = 0, t1 = 0, G0 = 0, G1 = 0;
     longlong2 qn = make_longlong2(0, 0);
     int b0 = 0, b1 = 0;
     bool i0 = false, i1 = false;
     if (LOADQ) qn = st->du[j + 2];
     if (PREFETCH) {
-        if (!REPLAY) Tn = st->T[j + 1];
         t0 = c.v + c.q.x;
         t1 = c.vn + c.q.y;
         if (WRAPFIX) {
@@ -1318,8 +1315,8 @@ __device__ __forceinline__ void table_step(TableChain& c, const int j, TableStag
     const long long gn = c.bn == c.b ? c.gc : (c.ap ? c.G1 : c.G0);
     const long long d = gn - c.gc;
     bool a;
-    if (!REPLAY) {
-        a = c.inr && (d < c.T);
+    if (!replay) {
+        a = c.inr && d < st->T[0][j];
     } else if (c.inr && d > 0) {
         if (c.draws >= thr_n) { c.err = ERR_REPLAY_EXHAUSTED; a = false; }
         else { a = d < P.thr[thr_off + c.draws]; ++c.draws; }
@@ -1335,17 +1332,126 @@ __device__ __forceinline__ void table_step(TableChain& c, const int j, TableStag
         c.bn = a ? b1 : b0;
         c.inr = a ? i1 : i0;
         c.G0 = G0; c.G1 = G1; c.ap = a;
-        c.T = Tn;
         c.q = qn;
     }
 }
+
+// The same chunk decided five sites at a time on the binary tree of outcomes, as the bin-tracking
+// kernel does it (above), one walker per warp: lane q >= 1 is the node at level log2(q), lane 0 stands
+// for the walker's present bin.  Positions are bin numerators shifted so that the bin is the high word
+// of a 64-bit integer; the path's bins come from the ancestor lanes by shuffle.
+struct TableTree {
+    static constexpr int D = 5;
+    int lvl, lvla;                         // level, level for the length check
+    unsigned want, anc, path;              // ancestors' votes: needed value, mask; the decisions that lead here
+    int up[D - 1];                         // the ancestor at each level (beyond the node's own: itself)
+    int dwell[D];                          // steps of the way here that end at the block's first bin, and at the
+                                           // proposal accepted at each level
+    bool first, last, leaf;                // first decision on the way here; the one before this node
+    __device__ explicit TableTree(int q)
+    {
+        lvl = q == 0 ? 0 : 31 - __clz(q);
+        lvla = q == 0 ? 32 : lvl;
+        want = anc = path = 0;
+#pragma unroll
+        for (int i = 0; i < D - 1; ++i) {
+            const bool above = i < lvl, a = above && ((q >> (lvl - 1 - i)) & 1);
+            up[i] = above ? q >> (lvl - i) : q;
+            if (above) anc |= 1u << up[i];
+            if (a) { want |= 1u << up[i]; path |= 1u << i; }
+        }
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            bool here = k == 0;            // k: the first bin, then the proposals of levels 0 ..
+            dwell[k] = 0;
+#pragma unroll
+            for (int i = 0; i < D - 1; ++i) {
+                if (accepts(i)) here = k == i + 1;
+                dwell[k] += here && i < lvl ? 1 : 0;
+            }
+        }
+        first = accepts(0);
+        last = lvl > 0 && accepts(lvl - 1);
+        if (q == 0) { anc = 1u; want = 1u; }                   // its vote is always 0: never on the path
+        leaf = lvl == D - 1;
+        // lane constants: kept in registers, not worked out again in every block
+        keep(want); keep(anc); keep(path); keep(lvl); keep(lvla);
+#pragma unroll
+        for (int i = 0; i < D - 1; ++i) keep(up[i]);
+#pragma unroll
+        for (int k = 0; k < D; ++k) keep(dwell[k]);
+    }
+    template <class T>
+    __device__ static void keep(T& x) { asm volatile("" : "+r"(x)); }
+    __device__ bool accepts(int i) const { return (path >> i) & 1u; }
+};
+
+// The part of a walker's table around its present bin, in shared memory: bins [lo, lo + size) at slot
+// bin mod size, g when the bin came in and the visits since (g now = g + visits x ln f).  A bin's
+// visits are booked (g, per-stage count, cumulative visits) when it leaves; bins outside are always
+// up to date in global memory.
+struct TableCache {
+    long long* g;
+    unsigned* n;
+    int size, lo, nb;                      // size: a power of two
+    long long* gg;
+    uint32_t* gH;
+    uint64_t* gv;
+    long long lnf;
+    int err;
+    __device__ __forceinline__ bool holds(int b) const { return (unsigned)(b - lo) < (unsigned)size; }
+    // the window's bins up to `margin` from b are all cached
+    __device__ __forceinline__ bool within(int b, int margin) const
+    {
+        return (lo == 0 || b - margin >= lo) && (lo + size >= nb || b + margin < lo + size);
+    }
+    __device__ void fill(int first, int last, int lane)
+    {
+        for (int b = first + lane; b < last; b += 32) {
+            const int k = b & (size - 1);
+            g[k] = b < nb ? gg[b] : 0;
+            n[k] = 0;
+        }
+    }
+    __device__ void book(int first, int last, int lane)
+    {
+        for (int b = first + lane; b < last; b += 32) {
+            const int k = b & (size - 1);
+            const unsigned v = n[k];
+            if (v == 0) continue;
+            const long long gnew = g[k] + (long long)v * lnf;
+            gg[b] = gnew;
+            err |= commit_visits(gH, gv, b, v, gnew);
+        }
+    }
+    // around bin b (all lanes)
+    __device__ void centre(int b, int lane)
+    {
+        const int to = max(0, min(b - size / 2, nb - size));
+        if (to == lo) return;
+        __syncwarp();
+        const int out0 = to > lo ? lo : max(to + size, lo), out1 = to > lo ? min(to, lo + size) : lo + size;
+        const int in0 = to > lo ? max(lo + size, to) : to, in1 = to > lo ? to + size : min(lo, to + size);
+        book(out0, out1, lane);
+        lo = to;
+        __syncwarp();
+        fill(in0, in1, lane);
+        __syncwarp();
+    }
+};
 
 // Sweeps of any model type of models.cuh with the window tables in global memory (the
 // Ashkin-Teller instances, whose windows hold tens of thousands of bins, and Ising windows too
 // large for shared memory).  One warp per walker; the planes sweep in turn (sigma then tau for
 // Ashkin-Teller, wang_landau.hpp:109-119), the flipped plane toggling after each pass.
 // The sweeps of one walker (launch position li; the warp's shared memory starts at warp_base).
-template <class Model, bool REPLAY, bool OBS>
+//
+// Bound: the latency of one block of five decisions (about 640 cycles at one warp per scheduler:
+// shared loads and shuffles of the bins, 64-bit positions, vote and reductions), once per five flips;
+// with many walkers per SM the 46 instructions per flip, and the cached bins that fit.  Ashkin-Teller
+// L = 32, bins of 0.05, 8 windows x 4 walkers: 32 walkers 178 -> 157 cycles per flip, 512 walkers 381
+// -> 195, 2048 walkers 772 -> 517 (from one dependent global load and store per flip).
+template <class Model, bool TREE, bool OBS>
 __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const int li, unsigned char* warp_base)
 {
     constexpr int NP = Model::kPlanes, NM = Model::kMags, NC = Model::kCorrPlanes;
@@ -1356,8 +1462,12 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
     const InstDev I = P.inst[P.slot_inst[s]];
     const int w = P.slot_win[s];
     const WinDev W = P.win[w];
-    const int L = I.L, N = I.N, C = I.chunk, nb = W.nb;
-    unsigned char* base = warp_base;
+    const int L = I.L, N = I.N, nb = W.nb;
+    const RowChunks rc(L);
+    // from the start of shared memory, so that the accesses below are shared-memory accesses
+    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned char* base = smem + (int)(warp_base - smem);
+    const bool replay = !TREE && p.replay;
     TableStage* st = reinterpret_cast<TableStage*>(base);
     int8_t* sp = reinterpret_cast<int8_t*>(st + 1);       // NP planes of N spins
     const int64_t* hf = I.field_off >= 0 ? P.fields + I.field_off : nullptr;
@@ -1366,11 +1476,22 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
     int8_t* gl = P.spins + P.cfg_off[cfg];
     for (int i = lane; i < NP * N; i += 32) sp[i] = gl[i];
     long long* gg = reinterpret_cast<long long*>(P.g + P.slot_tab[s]);
-    long long* g0 = reinterpret_cast<long long*>(P.gsnap + P.slot_tab[s]);
-    for (int k = lane; k < nb; k += 32) g0[k] = gg[k];
+    // the serial chain works on the table in global memory and derives the visits from a copy of it
+    long long* g0 = !TREE ? reinterpret_cast<long long*>(P.gsnap + P.slot_tab[s]) : nullptr;
+    if (!TREE)
+        for (int k = lane; k < nb; k += 32) g0[k] = gg[k];
     __syncwarp();
     // correlators: row sums rs[p] and column sums cs[p] of every correlator plane
     int* sums = reinterpret_cast<int*>(sp + ((NP * N + 15) & ~15));
+    TableCache tab;
+    tab.size = p.cache;
+    tab.g = reinterpret_cast<long long*>(reinterpret_cast<unsigned char*>(sums) + (P.corr ? (8 * NP * L + 15) & ~15 : 0));
+    tab.n = reinterpret_cast<unsigned*>(tab.g + tab.size);
+    tab.nb = nb;
+    tab.gg = gg;
+    tab.gH = P.H + P.slot_tab[s];
+    tab.gv = P.visits + P.slot_tab[s];
+    tab.err = 0;
     const bool corr = OBS && P.corr;
     const double invN = 1.0 / (double)N;
     if (corr) {
@@ -1380,7 +1501,6 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
         __syncwarp();
     }
 
-    const Couplings cpl{I.J_u, I.K_u};
     const long long lnf = P.win_lnf[w];
     const uint64_t sweeps0 = P.slot_sweeps[s];
     const uint32_t uid = (uint32_t)(s - I.first_slot);
@@ -1388,112 +1508,241 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
     const long long eglo = I.eglo_u, mul = I.bin_mul;
     const int sh = I.bin_shift;
     const long long vlo = (long long)W.gblo << sh;     // window start in bin-numerator units
-    const bool wraps = C == L;
+    // couplings and fields in position units: the tree's positions have the bin in their high word
+    const int up = TREE ? 32 - sh : 0;
+    const Couplings cpl{(I.J_u * mul) << up, (I.K_u * mul) << up};
+    auto field = [&](int i) { return hf ? ((long long)hf[i] * mul) << up : 0ll; };
+    const bool wraps = rc.n == 1;                      // a row is one chunk: its last site sees its first
     int flavour = NP == 1 ? 0 : P.slot_flavour[s];
 
-    TableChain c{};
-    int32_t M[3] = {0, 0, 0};                          // lane 0: the magnetisations
+    TableChain c{};                                    // serial chain, lane 0
+    int32_t M[3] = {0, 0, 0};                          // the magnetisations
     long long thr_off = 0, thr_n = 0;
-    int err = 0;
-    if (lane == 0) {
-        const long long E = P.cfg_E[cfg];
-        for (int m = 0; m < NM; ++m) M[m] = P.cfg_M[3 * cfg + m];
-        c.v = (E - eglo) * mul - vlo;
-        const long long gb = c.v >> sh;
-        if (gb < 0 || gb >= nb) err = ERR_BOUNDS;
-        c.b = (int)(err ? 0 : gb);
-        c.gc = gg[c.b];
-        if (REPLAY) { c.draws = P.slot_draws[s]; thr_off = P.slot_thr_off[s]; thr_n = P.slot_thr_n[s]; }
-    }
-    err = __shfl_sync(kFull, err, 0);
-    if (err) {
-        if (lane == 0) atomicOr(&P.counters[0], err);
+    long long vr = ((long long)P.cfg_E[cfg] - eglo) * mul - vlo;       // the walker's position
+    for (int m = 0; m < NM; ++m) M[m] = P.cfg_M[3 * cfg + m];
+    if ((vr >> sh) < 0 || (vr >> sh) >= nb) {
+        if (lane == 0) atomicOr(&P.counters[0], ERR_BOUNDS);
         return;
     }
+    if (!TREE && lane == 0) {
+        c.v = vr;
+        c.b = (int)(vr >> sh);
+        c.gc = gg[c.b];
+        if (replay) { c.draws = P.slot_draws[s]; thr_off = P.slot_thr_off[s]; thr_n = P.slot_thr_n[s]; }
+    }
+    vr <<= up;
+    if (TREE) {
+        tab.lnf = lnf;
+        tab.lo = max(0, min((int)(vr >> 32) - tab.size / 2, nb - tab.size));
+        tab.fill(tab.lo, tab.lo + tab.size, lane);
+    }
+    const unsigned sink = (unsigned)__cvta_generic_to_shared(&st->sink);
+    const TableTree tree(lane);
+    constexpr int D = TableTree::D;
+    const int lnf_lo = (int)(uint32_t)lnf, lnf_hi = (int)((lnf - (long long)(int)(uint32_t)lnf) >> 32);
+    const uint64_t attempts0 = sweeps0 * (uint64_t)NP * (uint64_t)N;   // the launch's first attempt
+    uint64_t attempt = attempts0;                      // of the current chunk
+    int tbuf = 0;
+    long long hnext = TREE ? field(min(lane, N - 1)) : 0;      // field of the chunk's site
+    auto draw = [&](uint64_t from, int len, int buf) { // thresholds of the len attempts from `from` on
+        if (lane < len) st->T[buf][lane] = word_threshold(philox_word(seed, uid, from + (uint64_t)lane, kStreamWL));
+    };
+    if (TREE) draw(attempt, rc.len(0), 0);
+
+    struct Node { long long rC, rP, x0, T; };          // position and proposal relative to the block's start
+    auto node = [&](int j0) {
+        const char* d = reinterpret_cast<const char*>(st->du + j0);
+        auto at = [&](int i, bool left) { return *reinterpret_cast<const long long*>(d + 16 * i + (left ? 8 : 0)); };
+        Node n;
+        n.x0 = at(0, true) - at(0, false);
+        n.rC = tree.accepts(0) ? at(0, false) : 0;
+#pragma unroll
+        for (int i = 1; i < D - 1; ++i) {
+            const long long v = at(i, tree.accepts(i - 1));
+            n.rC += tree.accepts(i) ? v : 0;
+        }
+        const long long v = at(tree.lvl, tree.last);
+        n.rP = n.rC + (lane == 0 ? 0 : v);
+        n.T = st->T[tbuf][j0 + tree.lvl];
+        return n;
+    };
 
     for (int sw = 0; sw < p.nsweeps; ++sw) {
         for (int pass = 0; pass < NP; ++pass) {
             const int plane = NP == 1 ? 0 : flavour;
             int8_t* A = sp + plane * N;
             const int8_t* B = NP == 1 ? A : sp + (plane ^ 1) * N;
-            const uint64_t A0 = ((sweeps0 + (uint64_t)sw) * (uint64_t)NP + (uint64_t)pass) * (uint64_t)N;
-            for (int c0 = 0; c0 < N; c0 += C) {
-                {
-                    // bring the lines of g within kTableReach bins of the walker's bin into L1
-                    // (the chunk's proposals mostly fall there), one line per lane per 512 bins
-                    const int bcur = __shfl_sync(kFull, c.b, 0);
-                    for (int k = lane * 16 - kTableReach; k <= kTableReach; k += 32 * 16) {
-                        const int bb = bcur + k;
-                        if ((unsigned)bb < (unsigned)nb) asm volatile("prefetch.global.L1 [%0];" ::"l"(gg + bb));
-                    }
+            for (int ch = 0, cc = 0, y = 0, c0 = 0, C = rc.len(0); ch < L * rc.n; ++ch) {
+                const int x0 = c0 - y * L;
+                if (TREE) {
+                    const int b = (int)(vr >> 32);
+                    if (!tab.within(b, tab.size / 8)) tab.centre(b, lane);
                 }
-                int ai = 0, sg[NM];
+                int ai = 0, sg[NM], far = 0;
                 for (int m = 0; m < NM; ++m) sg[m] = 0;
+                const long long h = hnext;             // (read while the chunk before it was decided)
                 if (lane < C) {
-                    const int i = c0 + lane;
+                    const int i = c0 + lane, x = x0 + lane;
+                    const Neighbours nbr{y == 0 ? i + (L - 1) * L : i - L, x == 0 ? i + L - 1 : i - 1,
+                                         x == L - 1 ? i - (L - 1) : i + 1, y == L - 1 ? i - (L - 1) * L : i + L};
                     ai = A[i];
                     Model::flip_signs(ai, B[i], plane, sg);
-                    const long long d0 = Model::delta_energy(A, B, i, L, cpl, hf ? hf[i] : 0);
-                    const long long d1 = lane > 0 ? Model::left_flipped(A, B, i, L, cpl, d0) : d0;
-                    st->du[lane] = make_longlong2(d0 * mul, d1 * mul);
-                    if (wraps && lane == C - 1) st->wcu = Model::right_flipped(A, B, i, L, cpl) * mul;
-                    if (!REPLAY) {
-                        const uint32_t word = philox_word(seed, uid, A0 + (uint64_t)i, kStreamWL);
-                        st->T[lane] = accept_threshold(neglog_u32(word));
-                    }
+                    const long long d0 = Model::delta_at(A, B, i, nbr, cpl, TREE ? h : field(i));
+                    const long long d1 = lane > 0 ? d0 + Model::flipped_at(A, B, i, nbr.left, cpl) : d0;
+                    const longlong2 d = make_longlong2(d0, d1);
+                    st->du[lane] = d;
+                    if (TREE) far = max(abs((int)(d.x >> 32)), abs((int)(d.y >> 32))) + 1;
+                    if (wraps && lane == C - 1) st->wcu = Model::flipped_at(A, B, i, nbr.right, cpl);
+                    if (!TREE && !replay) st->T[0][lane] = word_threshold(philox_word(seed, uid, attempt + (uint64_t)lane, kStreamWL));
                 }
+                // bins a block's nodes can lie away from its start: five steps (and a row's wrap term, part of
+                // an energy change as large)
+                const int reach = TREE ? (D + 1) * (int)__reduce_max_sync(kFull, (unsigned)far) : 0;
                 __syncwarp();
-                if (lane == 0) {
-                    c.acc = 0;
-                    c.vn = c.v + st->du[0].x;
-                    c.bn = (int)(c.vn >> sh);
-                    c.inr = (unsigned)c.bn < (unsigned)nb;
-                    c.G0 = c.G1 = gg[min((unsigned)c.bn, (unsigned)(nb - 1))];
-                    c.ap = false;
-                    if (!REPLAY) c.T = st->T[0];
-                    if (C == 1) {
-                        table_step<REPLAY, OBS, false, false, false>(c, 0, st, gg, nb, sh, lnf, P, thr_off, thr_n);
-                    } else {
-                        c.q = st->du[1];
-#pragma unroll 4
-                        for (int j = 0; j < C - 2; ++j)
-                            table_step<REPLAY, OBS, true, true, false>(c, j, st, gg, nb, sh, lnf, P, thr_off, thr_n);
-                        if (wraps) table_step<REPLAY, OBS, true, false, true>(c, C - 2, st, gg, nb, sh, lnf, P, thr_off, thr_n);
-                        else table_step<REPLAY, OBS, true, false, false>(c, C - 2, st, gg, nb, sh, lnf, P, thr_off, thr_n);
-                        table_step<REPLAY, OBS, false, false, false>(c, C - 1, st, gg, nb, sh, lnf, P, thr_off, thr_n);
+                // the next chunk: position, first site, length
+                int cn = cc + 1, yn = y;
+                if (cn == rc.n) { cn = 0; ++yn; }
+                const int Cn = rc.len(cn);
+                unsigned acc = 0;
+                if (!TREE) {
+                    if (lane == 0) {
+                        c.acc = 0;
+                        c.vn = c.v + st->du[0].x;
+                        c.bn = (int)(c.vn >> sh);
+                        c.inr = (unsigned)c.bn < (unsigned)nb;
+                        c.G0 = c.G1 = gg[min((unsigned)c.bn, (unsigned)(nb - 1))];
+                        c.ap = false;
+                        if (C == 1) {
+                            serial_step<OBS, false, false, false>(c, 0, st, gg, nb, sh, lnf, P, replay, thr_off, thr_n);
+                        } else {
+                            c.q = st->du[1];
+                            for (int j = 0; j < C - 2; ++j)
+                                serial_step<OBS, true, true, false>(c, j, st, gg, nb, sh, lnf, P, replay, thr_off, thr_n);
+                            if (wraps) serial_step<OBS, true, false, true>(c, C - 2, st, gg, nb, sh, lnf, P, replay, thr_off, thr_n);
+                            else serial_step<OBS, true, false, false>(c, C - 2, st, gg, nb, sh, lnf, P, replay, thr_off, thr_n);
+                            serial_step<OBS, false, false, false>(c, C - 1, st, gg, nb, sh, lnf, P, replay, thr_off, thr_n);
+                        }
                     }
+                    acc = __shfl_sync(kFull, c.acc, 0);
+                } else {
+                    int flipped = 0;                   // the block's left neighbour flipped just before it
+                    // one block of nlev sites from the chunk's site j0, `ahead` the work that does not wait for
+                    // it.  NEAR: every bin its lanes can name is cached.
+                    auto block = [&](auto near, const Node& n, int nlev, int j0, long long wC, long long wP, auto ahead) {
+                        constexpr bool NEAR = decltype(near)::value;
+                        const long long sC = flipped && tree.first ? n.x0 : 0;
+                        const long long sP = flipped && (tree.first || lane == 1) ? n.x0 : 0;
+                        const long long vC = vr + (n.rC + sC + wC), vP = vr + (n.rP + sP + wP);
+                        const int bP = (int)(vP >> 32), bC = (int)(vC >> 32);
+                        const int kP = bP & (tab.size - 1), kC = bC & (tab.size - 1);
+                        long long gP = tab.g[kP], gC = tab.g[kC];
+                        int cP = (int)tab.n[kP], cC = (int)tab.n[kC];
+                        // (a node below an out-of-window proposal is never on the path: what it reads does not matter)
+                        const bool inr = (unsigned)bP < (unsigned)nb;
+                        if (!NEAR) {
+                            if (inr && !tab.holds(bP)) { gP = gg[bP]; cP = 0; }
+                            if ((unsigned)bC < (unsigned)nb && !tab.holds(bC)) { gC = gg[bC]; cC = 0; }
+                        }
+                        // visits to this node's two bins on the way here: its path stays `dwell` steps at the
+                        // block's first bin and at every accepted proposal
+                        const int b0 = (int)(vr >> 32);
+                        int nC = b0 == bC ? tree.dwell[0] : 0, nP = b0 == bP ? tree.dwell[0] : 0;
+#pragma unroll
+                        for (int i = 0; i < D - 1; ++i) {
+                            const int b = __shfl_sync(kFull, bP, tree.up[i]);
+                            nC += b == bC ? tree.dwell[i + 1] : 0;
+                            nP += b == bP ? tree.dwell[i + 1] : 0;
+                        }
+                        const bool live = tree.lvla < nlev;
+                        const long long bound = mad_units(gC + n.T, (cC + nC) - (cP + nP), lnf_lo, lnf_hi);
+                        const bool a = (gP < bound) & live & inr;
+                        const unsigned vote = __ballot_sync(kFull, a);
+                        const bool on = ((vote ^ tree.want) & tree.anc) == 0;
+                        const long long v = a ? vP : vC;
+                        const bool mine = on && live, end = on && tree.leaf;
+                        const int bin = a ? bP : bC;
+                        // the last node of the path has the walker's position and the block's decisions
+                        const unsigned lo = __reduce_max_sync(kFull, end ? (unsigned)(unsigned long long)v : 0u);
+                        const unsigned hi = __reduce_max_sync(kFull, end ? (unsigned)bin : 0u);
+                        const unsigned path = __reduce_max_sync(kFull, end ? tree.path | (a ? 1u << (D - 1) : 0u) : 0u);
+                        if (OBS && mine) st->seq[j0 + tree.lvl] = bin;
+                        if (!NEAR && __any_sync(kFull, mine && !tab.holds(bin))) {
+                            // a step outside the cached bins: booked at once, in order
+                            const int sl = mine ? tree.lvl : -1;
+                            for (int i = 0; i < D; ++i) {
+                                if (sl == i) {
+                                    if (tab.holds(bin)) tab.n[bin & (tab.size - 1)] += 1u;
+                                    else {
+                                        const long long gnew = gg[bin] + lnf;
+                                        gg[bin] = gnew;
+                                        tab.err |= commit_visits(tab.gH, tab.gv, bin, 1, gnew);
+                                    }
+                                }
+                                __syncwarp();
+                            }
+                        } else {
+                            red_shared_inc(mine ? (unsigned)__cvta_generic_to_shared(tab.n + (bin & (tab.size - 1))) : sink);
+                        }
+                        ahead();
+                        __syncwarp();
+                        vr = (long long)(((unsigned long long)hi << 32) | lo);
+                        acc |= path << j0;
+                        flipped = (int)(path >> (nlev - 1)) & 1;
+                    };
+                    auto decide = [&](const Node& n, int nlev, int j0, long long wC, long long wP, auto ahead) {
+                        if (tab.within((int)(vr >> 32), reach)) block(std::true_type{}, n, nlev, j0, wC, wP, ahead);
+                        else block(std::false_type{}, n, nlev, j0, wC, wP, ahead);
+                    };
+                    Node n = node(0);
+                    int j0 = 0;
+                    for (; j0 + D < C; j0 += D) {
+                        Node next;
+                        decide(n, D, j0, 0, 0, [&] { next = node(j0 + D); });
+                        n = next;
+                    }
+                    // the chunk's last block; where the chunk is a row, its last site sees the first one's flip
+                    long long wC = 0, wP = 0;
+                    if (wraps) {
+                        const int li = C - 1 - j0;
+                        const long long t = (j0 > 0 ? (acc & 1u) != 0 : tree.first) ? st->wcu : 0;
+                        if (tree.lvla == li) wP = t;           // (not the idle lane)
+                        else if (tree.accepts(li)) wC = wP = t;
+                    }
+                    decide(n, C - j0, j0, wC, wP, [&] {
+                        draw(attempt + (uint64_t)C, Cn, tbuf ^ 1);
+                        hnext = field(min((ch + 1 == L * rc.n ? 0 : c0 + C) + lane, N - 1));
+                    });
                 }
-                const unsigned acc = __shfl_sync(kFull, c.acc, 0);
                 // per magnetisation: the steps whose accepted flip lowers it (its term was +1)
                 // and raises it; the change after step j is -2 (lowered - raised) up to j
                 unsigned plus[NM], minus[NM];
-                for (int m = 0; m < NM; ++m) {
-                    plus[m] = __ballot_sync(kFull, lane < C && sg[m] > 0);
-                    minus[m] = __ballot_sync(kFull, lane < C && sg[m] < 0);
-                }
+                if (OBS)
+                    for (int m = 0; m < NM; ++m) {
+                        plus[m] = __ballot_sync(kFull, lane < C && sg[m] > 0);
+                        minus[m] = __ballot_sync(kFull, lane < C && sg[m] < 0);
+                    }
                 auto dm = [&](int m, int j) {
                     const unsigned le = j >= 31 ? 0xFFFFFFFFu : ((2u << j) - 1u);
                     return -2 * ((int)__popc(acc & plus[m] & le) - (int)__popc(acc & minus[m] & le));
                 };
                 if (OBS) {
-                    int32_t M0[3] = {0, 0, 0};
-                    for (int m = 0; m < NM; ++m) M0[m] = __shfl_sync(kFull, M[m], 0);
                     __syncwarp();
                     if (lane < C) {
                         int32_t Mv[3] = {0, 0, 0};
-                        for (int m = 0; m < NM; ++m) Mv[m] = M0[m] + dm(m, lane);
+                        for (int m = 0; m < NM; ++m) Mv[m] = M[m] + dm(m, lane);
                         Model::add_observables(P.obs + (size_t)(P.slot_tab[s] + st->seq[lane]) * P.obs_stride, Mv, invN,
                                                P.corr);
                     }
                     if (corr) {
-                        const int y = c0 / L, x0 = c0 - y * L, row = y * L;
+                        const int row = y * L;
                         const int bin = lane < C ? st->seq[lane] : -1 - lane;
                         const unsigned grp = __match_any_sync(kFull, bin);
                         if (lane < C) {
-                            // the bin's count before step `lane`: its visits at the launch's start
-                            // plus the change of g over ln f, less the chunk's visits from this step on
-                            const unsigned long long after =
-                                P.visits[P.slot_tab[s] + bin] + (unsigned long long)((gg[bin] - g0[bin]) / lnf);
+                            // the bin's count before step `lane`: its visits booked so far and those not
+                            // booked yet, less the chunk's visits from this step on
+                            const unsigned long long after = P.visits[P.slot_tab[s] + bin] +
+                                (!TREE ? (unsigned long long)((gg[bin] - g0[bin]) / lnf)
+                                        : tab.holds(bin) ? (unsigned long long)tab.n[bin & (tab.size - 1)] : 0ull);
                             const unsigned long long seen = after - (unsigned long long)__popc(grp >> lane);
                             if (seen % kCountsPerTransform == 0) {
                                 const double* q = P.qtab + I.qtab_off;
@@ -1518,42 +1767,54 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
                     }
                 }
                 if (lane < C && ((acc >> lane) & 1u)) A[c0 + lane] = (int8_t)(-ai);
-                if (lane == 0)
+                if (OBS)
                     for (int m = 0; m < NM; ++m) M[m] += dm(m, 31);
                 __syncwarp();
+                attempt += (uint64_t)C;
+                tbuf ^= 1;
+                c0 += C;
+                cc = cn; y = yn; C = Cn;
             }
             if (NP == 2) flavour ^= 1;
         }
     }
     for (int i = lane; i < NP * N; i += 32) gl[i] = sp[i];
-    // counts and visits from the logDoS change (lane 0's stores to g are ordered
-    // before the other lanes' loads by the barrier)
-    __syncwarp();
-    uint32_t* gH = P.H + P.slot_tab[s];
-    uint64_t* gv = P.visits + P.slot_tab[s];
-    for (int k = lane; k < nb; k += 32) {
-        const long long gnew = gg[k], dg = gnew - g0[k];
-        if (dg != 0) {
-            const int e = commit_visits(gH, gv, k, dg / lnf, gnew);
-            if (e) atomicOr(&P.counters[0], e);
-        }
+    int sum[NM];
+    for (int m = 0; m < NM; ++m) sum[m] = 0;
+    for (int i = lane; i < N; i += 32) {
+        int t[NM];
+        Model::mag_terms(sp, N, i, t);
+        for (int m = 0; m < NM; ++m) sum[m] += t[m];
     }
+    for (int m = 0; m < NM; ++m) M[m] = __reduce_add_sync(kFull, sum[m]);
+    __syncwarp();
+    if (!TREE) {
+        for (int k = lane; k < nb; k += 32) {
+            const long long gnew = gg[k], dg = gnew - g0[k];
+            if (dg != 0) tab.err |= commit_visits(tab.gH, tab.gv, k, dg / lnf, gnew);
+        }
+    } else {
+        tab.book(tab.lo, min(tab.lo + tab.size, nb), lane);
+    }
+    if (tab.err) atomicOr(&P.counters[0], tab.err);
     if (lane == 0) {
-        P.cfg_E[cfg] = eglo + (c.v + vlo) / mul;
+        if (!TREE) vr = c.v;
+        vr >>= up;
+        P.cfg_E[cfg] = eglo + (vr + vlo) / mul;
         for (int m = 0; m < NM; ++m) P.cfg_M[3 * cfg + m] = M[m];
         P.slot_sweeps[s] = sweeps0 + (uint64_t)p.nsweeps;
         if (NP == 2) P.slot_flavour[s] = flavour;
-        if (REPLAY) P.slot_draws[s] = c.draws;
+        if (replay) P.slot_draws[s] = c.draws;
         if (c.err) atomicOr(&P.counters[0], c.err);
     }
 }
 
-template <class Model, bool REPLAY, bool OBS>
+template <class Model, bool TREE, bool OBS>
 __global__ void __launch_bounds__(256, 2) k_sweep_tables(const SweepParams p)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int wib = threadIdx.x >> 5;
-    sweep_tables_warp<Model, REPLAY, OBS>(p, blockIdx.x * (blockDim.x >> 5) + wib, smem + (size_t)wib * p.smem_per_warp);
+    sweep_tables_warp<Model, TREE, OBS>(p, blockIdx.x * (blockDim.x >> 5) + wib, smem + (size_t)wib * p.smem_per_warp);
 }
 
 // --------------------------------------------------------------------------
@@ -1572,7 +1833,7 @@ constexpr int kMaxFusedGroups = 16;
 
 struct FusedGroup {
     const int32_t* slots;
-    int nslots, smem_per_warp, nbcap, kind, first_task, counts, moments;
+    int nslots, smem_per_warp, nbcap, kind, first_task, counts, moments, cache;
 };
 
 struct FusedParams {
@@ -1592,7 +1853,8 @@ __device__ __noinline__ void fused_bins(const SweepParams& p, int unit, unsigned
 template <class Model, bool OBS>
 __device__ __noinline__ void fused_tables(const SweepParams& p, int unit, unsigned char* base)
 {
-    sweep_tables_warp<Model, false, OBS>(p, unit, base);
+    if (p.cache) sweep_tables_warp<Model, true, OBS>(p, unit, base);
+    else sweep_tables_warp<Model, false, OBS>(p, unit, base);
 }
 
 template <bool OBS>
@@ -1611,7 +1873,7 @@ __global__ void __launch_bounds__(128) k_sweep_fused(const FusedParams fp)
         const FusedGroup& G = fp.g[gi];
         SweepParams sp;
         sp.P = fp.P; sp.slots = G.slots; sp.nslots = G.nslots; sp.nsweeps = fp.nsweeps;
-        sp.smem_per_warp = G.smem_per_warp; sp.nbcap = G.nbcap; sp.counts = G.counts; sp.moments = G.moments;
+        sp.smem_per_warp = G.smem_per_warp; sp.nbcap = G.nbcap; sp.counts = G.counts; sp.moments = G.moments; sp.cache = G.cache; sp.replay = 0;
         const int unit = t - G.first_task;
         switch (G.kind) {
         case kFusedBins: fused_bins<OBS>(sp, unit, base); break;
@@ -1939,22 +2201,24 @@ struct Launch {
     int walkers_per_warp = 1;
     int counts = 0;         // bin-tracking kernel: visit counts beside g in shared memory (16 bytes per bin)
     int moments = 0;        // bin-tracking kernel with observables: moment sums in shared memory
+    int tree = 0;           // the global-table kernel may decide on the tree of outcomes
     int tables = 0;         // the global-table kernel (k_sweep_tables)
+    int cache = 0;          // its bins of each walker's table in shared memory (a power of two); 0: the serial chain
     int carveout = -1;      // global-table kernel: shared-memory carveout (percent) that leaves the rest to L1
     DBuf<int32_t> d_slots;
 };
 
 template <class Model>
-SweepKernel table_kernel_t(bool replay, bool obs)
+SweepKernel table_kernel_t(bool tree, bool obs)
 {
-    if (replay) return obs ? k_sweep_tables<Model, true, true> : k_sweep_tables<Model, true, false>;
+    if (tree) return obs ? k_sweep_tables<Model, true, true> : k_sweep_tables<Model, true, false>;
     return obs ? k_sweep_tables<Model, false, true> : k_sweep_tables<Model, false, false>;
 }
 
-SweepKernel table_kernel(int model, bool replay, bool obs)
+SweepKernel table_kernel(int model, bool tree, bool obs)
 {
-    return model == REWL_MODEL_ISING2D ? table_kernel_t<Ising2dModel>(replay, obs)
-                                       : table_kernel_t<AshkinTeller2dModel>(replay, obs);
+    return model == REWL_MODEL_ISING2D ? table_kernel_t<Ising2dModel>(tree, obs)
+                                       : table_kernel_t<AshkinTeller2dModel>(tree, obs);
 }
 
 } // namespace
@@ -2335,7 +2599,6 @@ int upload_all(rewl_engine* e)
     }
     bool any_at = false;
     for (const auto& hi : e->inst) any_at = any_at || hi.d.model == REWL_MODEL_ASHKIN_TELLER2D;
-    if (any_at && tab && (rc = e->gsnap.alloc(tab))) return rc;
     if (D.observables && tab) {
         e->obs_stride = any_at ? (D.observables == 2 ? 16 : 12) : (D.observables == 2 ? 4 : 3);
         if ((rc = e->obs.alloc((size_t)tab * e->obs_stride))) return rc;
@@ -2375,6 +2638,17 @@ bool bins_eligible(const InstDev& I, const rewl_batch_desc& D, int max_window_bi
     return true;
 }
 
+// The global-table kernel's tree keeps the bin in the high word of a position and adds up to six
+// energy changes: bins of at most 2^32 numerator units, and no single flip across 2^26 bins.
+int tree_eligible(const HostInst& H, const rewl_batch_desc& D)
+{
+    if (D.rng_mode != REWL_RNG_PHILOX || H.dev.bin_shift > 32) return 0;
+    double h = 0;
+    for (double f : H.fields) h = std::max(h, std::fabs(f));
+    const double move = 2.0 * (4.0 * std::fabs((double)H.dev.J_u) + 4.0 * std::fabs((double)H.dev.K_u) + std::ldexp(h, H.dev.escale));
+    return move * (double)H.dev.bin_mul < std::ldexp(1.0, 26 + H.dev.bin_shift) ? 1 : 0;
+}
+
 // Streaming multiprocessors of the engine's device (152 on a GB300).
 int sm_count(const rewl_engine* e)
 {
@@ -2383,14 +2657,15 @@ int sm_count(const rewl_engine* e)
     return n;
 }
 
-// The logDoS tables of the Ashkin-Teller kernel live in global memory and are read through L1,
-// so its shared-memory carveout is the smallest that still holds the blocks resident on an SM
-// (the CUDA runtime's default split leaves L1 far less).
+// The serial chain reads the tables in global memory through L1, so its shared-memory carveout is
+// the smallest that still holds the blocks resident on an SM (the CUDA runtime's default split leaves
+// L1 far less); the tree keeps the walkers' surroundings in shared memory and takes all of it (with a
+// carveout just large enough, 512 walkers at L = 24 ran in two waves: 388 against 205 cycles per flip).
 int at_carveout(rewl_engine* e, Launch& l)
 {
     if (!l.tables) return REWL_OK;
     const int nsm = sm_count(e);
-    const SweepKernel fn = table_kernel(l.model, e->desc.rng_mode == REWL_RNG_REPLAY, e->desc.observables != 0);
+    const SweepKernel fn = table_kernel(l.model, l.cache > 0, e->desc.observables != 0);
     const int threads = 32 * l.wpb;
     const size_t smem = (size_t)l.wpb * l.smem_per_warp;
     int occ = 0;
@@ -2400,7 +2675,7 @@ int at_carveout(rewl_engine* e, Launch& l)
     int smem_sm = 0;
     CUDA_TRY(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, e->desc.device));
     const size_t need = (size_t)per_sm * (smem + 1024);
-    l.carveout = (int)std::min<size_t>(100, (need * 100 + smem_sm - 1) / (size_t)smem_sm);
+    l.carveout = l.cache ? 100 : (int)std::min<size_t>(100, (need * 100 + smem_sm - 1) / (size_t)smem_sm);
     return REWL_OK;
 }
 
@@ -2434,7 +2709,7 @@ int plan_fused(rewl_engine* e, int nsm)
     for (size_t k = 0; k < order.size(); ++k) {
         const Launch& l = e->launches[order[k].second];
         FusedGroup& G = F.g[k];
-        G.slots = l.d_slots.p; G.nslots = (int)l.slots.size(); G.smem_per_warp = l.smem_per_warp; G.nbcap = l.nbcap; G.counts = l.counts; G.moments = l.moments;
+        G.slots = l.d_slots.p; G.nslots = (int)l.slots.size(); G.smem_per_warp = l.smem_per_warp; G.nbcap = l.nbcap; G.counts = l.counts; G.moments = l.moments; G.cache = l.cache;
         if (l.bins)
             G.kind = kFusedBins;
         else if (l.tables)
@@ -2472,7 +2747,7 @@ int plan_launches(rewl_engine* e)
     const int nsm = sm_count(e);
     // group walkers by (model, bin-tracking kernel, chunk, sites) so each launch has one
     // kernel shape and the walkers sharing a warp run the same number of chunks
-    struct Key { int model, bins, sites; };
+    struct Key { int model, bins, sites, tree; };
     std::vector<Key> keys;
     std::vector<Launch> plans;
     for (int s = 0; s < e->nslots; ++s) {
@@ -2480,15 +2755,16 @@ int plan_launches(rewl_engine* e)
         int max_nb = 0;
         for (const auto& wd : H.wins) max_nb = std::max(max_nb, wd.nb);
         const int bins = bins_eligible(H.dev, e->desc, max_nb) && getenv("REWL_SWEEP_VARIANT") == nullptr ? 1 : 0;
-        Key k{H.d.model, bins, bins ? H.dev.N : 0};
+        Key k{H.d.model, bins, bins ? H.dev.N : 0, tree_eligible(H, e->desc)};
         size_t idx = 0;
         for (; idx < keys.size(); ++idx)
-            if (keys[idx].model == k.model && keys[idx].bins == k.bins && keys[idx].sites == k.sites)
+            if (keys[idx].model == k.model && keys[idx].bins == k.bins && keys[idx].sites == k.sites &&
+                keys[idx].tree == k.tree)
                 break;
         if (idx == keys.size()) {
             keys.push_back(k);
             Launch l;
-            l.model = k.model; l.bins = k.bins;
+            l.model = k.model; l.bins = k.bins; l.tree = k.tree;
             plans.push_back(std::move(l));
         }
         plans[idx].slots.push_back(s);
@@ -2545,13 +2821,23 @@ int plan_launches(rewl_engine* e)
             } else {
                 const int planes = l.model == REWL_MODEL_ISING2D ? 1 : 2;
                 l.nbcap = 0;
-                l.smem_per_warp = (int)(sizeof(TableStage) + ((planes * maxN + 15) & ~15) + (corr ? 8 * planes * maxL : 0));
+                const int fixed = (int)(sizeof(TableStage) + ((planes * maxN + 15) & ~15) + (corr ? (8 * planes * maxL + 15) & ~15 : 0));
+                // as much of every walker's table as the walkers sharing an SM leave room for, but no less than
+                // 2048 bins (the rest of the walkers then wait for a second wave): Ashkin-Teller L = 32 at bins
+                // of 0.05, 2048 walkers, 512 / 1024 / 2048 / 4096 bins 5.5 / 5.8 / 7.6 / 5.6e9 flips/s; 512
+                // walkers, 1024 / 2048 / 4096 / 8192 bins 3.0 / 4.1 / 5.1 / 3.1e9
+                const int per_sm = e->desc.persistent ? 8 : std::max(1, std::min(32, (e->nslots + nsm - 1) / nsm));
+                l.cache = l.tree ? 256 : 0;
+                while (l.cache && l.cache < maxnb && fixed + 24 * l.cache <= 200 * 1024 &&
+                       (l.cache < kMinCache || fixed + 24 * l.cache + 1040 <= 225 * 1024 / per_sm))
+                    l.cache *= 2;
+                l.smem_per_warp = fixed + 12 * l.cache;
             }
         }
         if (!l.bins) {
             l.smem_per_warp = (l.smem_per_warp + 15) & ~15;
             int wpb = e->desc.warps_per_block;
-            if (wpb == 0) wpb = n <= nsm * 2 ? 1 : n <= nsm * 8 ? 2 : 4;
+            if (wpb == 0) wpb = l.tables || n <= nsm * 2 ? 1 : n <= nsm * 8 ? 2 : 4;
             while (wpb > 1 && (size_t)wpb * l.smem_per_warp > 200 * 1024) wpb >>= 1;
             if ((size_t)l.smem_per_warp > 220 * 1024) return fail(REWL_EINVAL, "a walker needs %d bytes of shared memory (limit 220 KiB)", l.smem_per_warp);
             l.wpb = wpb;
@@ -2569,8 +2855,8 @@ int plan_launches(rewl_engine* e)
                 CUDA_TRY(cudaFuncSetAttribute(table_kernel(m, r, o), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     for (auto& l : e->launches) {
         if (int rc = at_carveout(e, l)) return rc;
-        // the global-table kernel copies each walker's logDoS at the start of a launch
-        if (l.tables && !e->gsnap.p && e->table_total > 0)
+        // the serial chain copies each walker's logDoS at the start of a launch
+        if (l.tables && !l.cache && !e->gsnap.p && e->table_total > 0)
             if (int rc = e->gsnap.alloc(e->table_total)) return rc;
     }
     for (int G : {1, 2, 4})
@@ -2587,6 +2873,27 @@ int plan_launches(rewl_engine* e)
             CUDA_TRY(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
             e->join_ev.push_back(ev);
         }
+    }
+    return REWL_OK;
+}
+
+// New fields whose energy changes the tree of the global-table kernel cannot hold: the instance's
+// launch group goes over to the serial chain.
+int leave_tree(rewl_engine* e, int ii)
+{
+    if (tree_eligible(e->inst[ii], e->desc)) return REWL_OK;
+    for (auto& l : e->launches) {
+        if (!l.cache) continue;
+        bool here = false;
+        for (int s : l.slots) here = here || e->h_slot_inst[s] == ii;
+        if (!here) continue;
+        if (!e->gsnap.p)
+            if (int rc = e->gsnap.alloc(e->table_total)) return rc;
+        l.cache = 0;
+        for (int g = 0; g < e->fused_p.ngroups; ++g)
+            if (e->fused_p.g[g].slots == l.d_slots.p) e->fused_p.g[g].cache = 0;
+        if (int rc = at_carveout(e, l)) return rc;
+        e->drop_graph();
     }
     return REWL_OK;
 }
@@ -2630,7 +2937,7 @@ int launch_group(rewl_engine* e, Launch& l, cudaStream_t stream, int nsweeps, co
     const bool replay = e->desc.rng_mode == REWL_RNG_REPLAY;
     SweepParams sp;
     sp.P = P; sp.slots = l.d_slots.p; sp.nslots = (int)l.slots.size(); sp.nsweeps = nsweeps;
-    sp.smem_per_warp = l.smem_per_warp; sp.nbcap = l.nbcap; sp.counts = l.counts; sp.moments = l.moments;
+    sp.smem_per_warp = l.smem_per_warp; sp.nbcap = l.nbcap; sp.counts = l.counts; sp.moments = l.moments; sp.cache = l.cache; sp.replay = replay;
     if (l.bins) {
         const int G = l.walkers_per_warp;
         const int warps = (sp.nslots + G - 1) / G;
@@ -2641,7 +2948,7 @@ int launch_group(rewl_engine* e, Launch& l, cudaStream_t stream, int nsweeps, co
         const int blocks = (sp.nslots + l.wpb - 1) / l.wpb;
         const size_t smem = (size_t)l.wpb * l.smem_per_warp;
         if (l.tables) {
-            const SweepKernel fn = table_kernel(l.model, replay, e->desc.observables != 0);
+            const SweepKernel fn = table_kernel(l.model, l.cache > 0, e->desc.observables != 0);
             if (l.carveout >= 0) CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, l.carveout));
             fn<<<blocks, 32 * l.wpb, smem, stream>>>(sp);
         } else {
@@ -3034,6 +3341,7 @@ int rewl_import_disorder(rewl_engine* e, int32_t ii, const double* fields)
         q[i] = (int64_t)v; H.fields[i] = std::ldexp(v, -20);
     }
     cudaSetDevice(e->desc.device);
+    if (int rc = leave_tree(e, ii)) return rc;
     CUDA_TRY(cudaMemcpyAsync(e->fields.p + H.dev.field_off, q.data(), q.size() * 8, cudaMemcpyHostToDevice, e->stream));
     const int n = H.dev.nwin * H.dev.R;
     std::vector<int32_t> cfgs(n), insts(n, ii);

@@ -4,9 +4,10 @@
 // model type provides, for a configuration held as int8 +-1 planes (Ising: one
 // plane; Ashkin-Teller: sigma then tau) on the L x L periodic square lattice with
 // site = y L + x:
-//   delta_energy      energy change of flipping plane a's spin at a site (b the other plane)
-//   left_flipped      the same after the site's left neighbour in plane a has flipped
-//   right_flipped     the correction for a right neighbour in plane a that has flipped
+//   delta_at          energy change of flipping plane a's spin at a site (b the other plane), given its
+//                     neighbours; delta_energy works them out
+//   flipped_at        the change of that where the neighbour j in plane a has flipped (left_flipped,
+//                     right_flipped: the same for a site's left and right neighbour)
 //   recalculate       energy and magnetisations from scratch
 //   flip              apply a flip and update the magnetisations
 //   add_observables   the per-bin moments of update_observables for the current magnetisations
@@ -15,6 +16,7 @@
 //   flip_signs        for each magnetisation, the sign of the site's term before a flip of
 //                     plane a (the flip changes it by -2 sign; 0: unchanged)
 //   corr_site         a site's value in each correlator plane
+//   mag_terms         a site's term in each magnetisation
 //   add_transforms    the G(q_min) of each correlator plane into the observable columns
 // kPlanes spin planes, kMags magnetisations, kCorrPlanes correlator planes, corr_mag[p]
 // the magnetisation whose terms are correlator plane p's values.
@@ -30,6 +32,12 @@ __host__ __device__ inline int nb_up(int i, int L) { int x = i % L, y = i / L; r
 __host__ __device__ inline int nb_left(int i, int L) { int x = i % L, y = i / L; return y * L + (x == 0 ? L - 1 : x - 1); }
 __host__ __device__ inline int nb_right(int i, int L) { int x = i % L, y = i / L; return y * L + (x == L - 1 ? 0 : x + 1); }
 __host__ __device__ inline int nb_down(int i, int L) { int x = i % L, y = i / L; return (y == L - 1 ? 0 : y + 1) * L + x; }
+
+// a site's neighbours (site indices)
+struct Neighbours {
+    int up, left, right, down;
+};
+__host__ __device__ inline Neighbours neighbours(int i, int L) { return {nb_up(i, L), nb_left(i, L), nb_right(i, L), nb_down(i, L)}; }
 
 struct Couplings {
     int64_t J, K;            // nearest-neighbour and four-spin couplings in energy units
@@ -67,20 +75,29 @@ struct Ising2dModel {
 
     __host__ __device__ static void flip_signs(int a, int, int, int* sg) { sg[0] = a; }
     __host__ __device__ static int corr_site(const int8_t* sp, int, int i, int) { return sp[i]; }
+    __host__ __device__ static void mag_terms(const int8_t* sp, int, int i, int* t) { t[0] = sp[i]; }
     __device__ static void add_transforms(double* o, const double* G, double in2) { atomicAdd(o + 3, in2 * G[0]); }
 
-    __host__ __device__ static int64_t delta_energy(const int8_t* a, const int8_t*, int i, int L, Couplings c, int64_t)
+    __host__ __device__ static int64_t delta_at(const int8_t* a, const int8_t*, int i, Neighbours n, Couplings c, int64_t)
     {
-        const int sum = a[nb_up(i, L)] + a[nb_left(i, L)] + a[nb_right(i, L)] + a[nb_down(i, L)];
+        const int sum = a[n.up] + a[n.left] + a[n.right] + a[n.down];
         return 2 * (int64_t)a[i] * c.J * sum;
     }
-    __host__ __device__ static int64_t left_flipped(const int8_t* a, const int8_t*, int i, int L, Couplings c, int64_t d0)
+    __host__ __device__ static int64_t flipped_at(const int8_t* a, const int8_t*, int i, int j, Couplings c)
     {
-        return d0 - 4 * (int64_t)a[i] * a[nb_left(i, L)] * c.J;
+        return -4 * (int64_t)a[i] * a[j] * c.J;
     }
-    __host__ __device__ static int64_t right_flipped(const int8_t* a, const int8_t*, int i, int L, Couplings c)
+    __host__ __device__ static int64_t delta_energy(const int8_t* a, const int8_t* b, int i, int L, Couplings c, int64_t h)
     {
-        return -4 * (int64_t)a[i] * a[nb_right(i, L)] * c.J;
+        return delta_at(a, b, i, neighbours(i, L), c, h);
+    }
+    __host__ __device__ static int64_t left_flipped(const int8_t* a, const int8_t* b, int i, int L, Couplings c, int64_t d0)
+    {
+        return d0 + flipped_at(a, b, i, nb_left(i, L), c);
+    }
+    __host__ __device__ static int64_t right_flipped(const int8_t* a, const int8_t* b, int i, int L, Couplings c)
+    {
+        return flipped_at(a, b, i, nb_right(i, L), c);
     }
     // E recomputed as sum_i -1/2 s_i J sum_nb s_nb (ising2d_hamiltonian.hpp:191-210)
     __host__ __device__ static void recalculate(const int8_t* sp, int L, Couplings c, const int64_t*, int64_t& E, int32_t* M)
@@ -138,6 +155,12 @@ struct AshkinTeller2dModel {
     {
         return p == 0 ? sp[i] : sp[i] * sp[N + i];
     }
+    __host__ __device__ static void mag_terms(const int8_t* sp, int N, int i, int* t)
+    {
+        t[0] = sp[i];
+        t[1] = sp[N + i];
+        t[2] = sp[i] * sp[N + i];
+    }
     // the tau correlator is computed from sigma, as the reference does (ashkin_teller2d_hamiltonian.hpp:
     // 298-299); phi's is the sum of the two
     __device__ static void add_transforms(double* o, const double* G, double in2)
@@ -146,22 +169,20 @@ struct AshkinTeller2dModel {
         atomicAdd(o + 3, gs); atomicAdd(o + 7, gs); atomicAdd(o + 11, gs + gs); atomicAdd(o + 15, gb);
     }
 
-    __host__ __device__ static int64_t delta_energy(const int8_t* a, const int8_t* b, int i, int L, Couplings c, int64_t h)
+    __host__ __device__ static int64_t delta_at(const int8_t* a, const int8_t* b, int i, Neighbours n, Couplings c, int64_t h)
     {
-        const int u = nb_up(i, L), l = nb_left(i, L), r = nb_right(i, L), d = nb_down(i, L);
+        const int u = n.up, l = n.left, r = n.right, d = n.down;
         const int sa = a[u] + a[l] + a[r] + a[d];
         const int sab = a[u] * b[u] + a[l] * b[l] + a[r] * b[r] + a[d] * b[d];
         return 2 * (int64_t)a[i] * (h * b[i] + c.J * sa + c.K * (int64_t)b[i] * sab);
     }
-    __host__ __device__ static int64_t left_flipped(const int8_t* a, const int8_t* b, int i, int L, Couplings c, int64_t d0)
+    __host__ __device__ static int64_t flipped_at(const int8_t* a, const int8_t* b, int i, int j, Couplings c)
     {
-        const int l = nb_left(i, L);
-        return d0 - 4 * (int64_t)a[i] * a[l] * (c.J + c.K * (int64_t)b[i] * b[l]);
+        return -4 * (int64_t)a[i] * a[j] * (c.J + c.K * (int64_t)b[i] * b[j]);
     }
-    __host__ __device__ static int64_t right_flipped(const int8_t* a, const int8_t* b, int i, int L, Couplings c)
+    __host__ __device__ static int64_t delta_energy(const int8_t* a, const int8_t* b, int i, int L, Couplings c, int64_t h)
     {
-        const int r = nb_right(i, L);
-        return -4 * (int64_t)a[i] * a[r] * (c.J + c.K * (int64_t)b[i] * b[r]);
+        return delta_at(a, b, i, neighbours(i, L), c, h);
     }
     __host__ __device__ static void recalculate(const int8_t* sp, int L, Couplings c, const int64_t* h, int64_t& E, int32_t* M)
     {

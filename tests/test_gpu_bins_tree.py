@@ -66,3 +66,70 @@ OBS = [
 @pytest.mark.parametrize("case", OBS, ids=[c[0] for c in OBS])
 def test_observables_match_the_oracle(engine_lib, oracle_lib, case):
     _run_observables_case(engine_lib, oracle_lib, case)
+
+
+AT = [
+    # L, K, sigma_h, bin width, windows, replicas, sweeps per exchange / check, observables
+    (2, 0.5, 0.5, 0.05, 1, 2, 50, 100, 0), (3, 0.25, 0.3, 0.05, 2, 2, 40, 80, 0), (9, 0.75, 0.0, 0.25, 2, 2, 10, 20, 0),
+    (10, 0.5, 0.5, 0.05, 3, 2, 10, 20, 2), (11, 0.5, 0.5, 1.0, 2, 2, 10, 20, 1), (17, 0.25, 0.3, 0.05, 4, 2, 4, 8, 0),
+    (33, 0.5, 0.5, 0.05, 4, 2, 2, 4, 0), (37, 0.5, 0.5, 0.05, 3, 1, 2, 4, 1), (20, 0.5, 3.0, 0.0625, 2, 2, 4, 8, 0),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", AT, ids=lambda c: f"L{c[0]}_bw{c[3]:g}_obs{c[8]}")
+def test_ashkin_teller_tree_matches_the_oracle(engine_lib, oracle_lib, case):
+    """Whole-row and cut rows, one block and several, windows smaller and larger than the bins held
+    in shared memory, strong fields (energy changes far beyond them)."""
+    L, K, sig, bw, nwin, R, se, sc, obs = case
+    _run_observables_case(engine_lib, oracle_lib, ("", 1, L, -5.0 * L * L, 0.0, bw, nwin, R, se, sc, 300 + L, 2, 0, sig, 1, obs)) \
+        if obs else _at_case(engine_lib, oracle_lib, case)
+
+
+def _at_case(rg, po, case):
+    L, K, sig, bw, nwin, R, se, sc, _ = case
+    h = np.round(np.random.default_rng(L).normal(0, sig, L * L) * 2**20) / 2**20 if sig else None
+    eng, orc = _pair(rg, po, 1, L, -np.ceil(2 * (2 + K)) * L * L, 0.0, bw, nwin, R, se, sc, 300 + L, K=K, fields=h, mask=1)
+    try:
+        for k in range(2):
+            eng.run_cycles(1)
+            orc.cycle()
+            _compare(eng, orc, f"cycle {k}")
+    finally:
+        eng.close()
+        orc.close()
+
+
+@pytest.mark.gpu
+def test_fields_beyond_the_tree_run_the_serial_chain(engine_lib, oracle_lib):
+    """One site's field carries an energy change across more than 2^26 bins: the launch group decides
+    serially, and so it does when such fields are imported later."""
+    rg, po = engine_lib, oracle_lib
+    h = np.zeros(36)
+    h[7] = 4.0e6
+    big = dict(K=0.5, fields=h, mask=1)
+    eng, orc = _pair(rg, po, 1, 6, -180.0 - 4.0e6, -4.0e6, 0.05, 2, 2, 10, 20, 61, **big)
+    try:
+        eng.run_cycles(1)
+        orc.cycle()
+        _compare(eng, orc, "created")
+    finally:
+        eng.close()
+        orc.close()
+    ins = rg.Instance(model=rg.MODEL_ASHKIN_TELLER2D, L=6, K=0.5, fields=np.zeros(36), energy_min=-180.0, energy_max=0.0,
+                      bin_width=0.05, num_windows=2, replicas_per_window=2, seed=61)
+    with rg.Engine(rg.Batch(instances=[ins], sweeps_per_exchange=10, sweeps_per_check=20, mask_mode=rg.MASK_VISITED)) as a, \
+            rg.Engine(rg.Batch(instances=[ins], sweeps_per_exchange=10, sweeps_per_check=20, mask_mode=rg.MASK_VISITED)) as b:
+        a.run_cycles(1)
+        b.run_cycles(1)
+        a.import_disorder(0, np.zeros(36))          # the same fields: still the tree
+        h[7] = 4.0e6
+        b.import_disorder(0, h)                     # serial from here on ...
+        b.import_disorder(0, np.zeros(36))          # ... with the same energies as before
+        for k in range(2):
+            a.run_cycles(1)
+            b.run_cycles(1)
+        for s in range(4):
+            x, y = a.export_walker(s), b.export_walker(s)
+            for key in x:
+                np.testing.assert_array_equal(x[key], y[key], err_msg=f"walker {s} {key}")
