@@ -46,6 +46,8 @@ constexpr int kExpTable = 1 << kExpBits;
 struct ThermoArgs {
     const double *E, *lng;             // nb levels
     const float2* x32;                 // {-E, ln g} in single precision
+    const long long *Ei, *gi;          // E 2^se and ln g / ln 2 2^sg as integers (62 bits)
+    int se, sg;
     const double* obs;                 // K columns of nb values
     int nb, K, counts_col, nT, trapezoid;
     double N, Tmin, dT, counts_mean;
@@ -60,45 +62,65 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
-// exp(d) for -700 <= d <= 700 by table look-up (P. T. P. Tang, "Table-driven implementation of the
-// exponential function in IEEE floating-point arithmetic", ACM TOMS 15, 1989): d = (2048 k + j) ln 2 /
-// 2048 + r, exp(d) = 2^k 2^(j/2048) (1 + r + r^2/2 + r^3/6), |r| <= 1.7e-4 (the next term is 3.5e-17).
-// Eight FP64 instructions.
-__device__ __forceinline__ double exp_table(double d, const double* tab)
+// 2^(i / 2048) in units of 2^-63, from 2^(1/2), 2^(1/4), ... 2^(1/2048)
+__device__ unsigned long long pow2_fraction(int i)
 {
-    constexpr double kMagic = 6755399441055744.0;                      // 1.5 x 2^52: adding it rounds to an integer
-    constexpr double kStep = 0.69314718055994530942 / kExpTable;
-    constexpr double kHi = 0x1.62e42fefp-12;                           // ln 2 / 2048 to 33 bits: d - n kHi is exact
-    constexpr double kLo = 0x1.473de6af278edp-45;                      // the rest of it
-    const double y = fma(d, 1.0 / kStep, kMagic);
-    const int n = __double2loint(y);
-    const double nd = y - kMagic;
-    const double r = fma(-nd, kLo, fma(-nd, kHi, d));
-    const double p = fma(r * r, fma(r, 1.0 / 6.0, 0.5), r);
-    const double t = tab[n & (kExpTable - 1)];
-    const double scaled = __hiloint2double(__double2hiint(t) + ((n >> kExpBits) << 20), __double2loint(t));
-    return fma(scaled, p, scaled);
+    constexpr unsigned long long kRoot[kExpBits] = {
+        0xb504f333f9de6484ull, 0x9837f0518db8a96full, 0x8b95c1e3ea8bd6e7ull, 0x85aac367cc487b15ull, 0x82cd8698ac2ba1d7ull,
+        0x8164d1f3bc030773ull, 0x80b1ed4fd999ab6cull, 0x8058d7d2d5e5f6b1ull, 0x802c6436d0e04f51ull, 0x8016302f17467628ull,
+        0x800b179c82028fd1ull};
+    unsigned long long v = 1ull << 63;
+#pragma unroll
+    for (int k = 0; k < kExpBits; ++k)
+        if ((i >> (kExpBits - 1 - k)) & 1) {
+            const unsigned long long hi = __umul64hi(v, kRoot[k]), lo = v * kRoot[k];
+            v = (hi << 1) + (lo >> 63) + ((lo >> 62) & 1ull);
+        }
+    return v;
 }
 
-// One warp per temperature.  Bound: the FP64 pipe (two lanes per clock and SM), so what the sums do
-// not need stays off it:
+// 2^(d 2^-F) as a double, for -1020 <= d 2^-F < 1000, in integer arithmetic: the fraction is split into
+// a table index j and a rest g < 2^-11 (P. T. P. Tang, "Table-driven implementation of the exponential
+// function in IEEE floating-point arithmetic", ACM TOMS 15, 1989), 2^g = 1 + t + t^2/2 + t^3/6 + t^4/24 with
+// t = g ln 2 in units of 2^-75 (the next term is below 2^-64), and the product is rounded to 53 bits once.
+__device__ __forceinline__ double pow2_fixed(long long d, int F, const unsigned long long* tab)
+{
+    const int k = (int)(d >> F);
+    const unsigned long long fr = (unsigned long long)d << (64 - F);
+    const unsigned long long t = __umul64hi(fr << kExpBits, 0xb17217f7d1cf79acull);      // 2^-75
+    const unsigned th = (unsigned)(t >> 32);                                             // 2^-43
+    const unsigned long long t2 = __umul64hi(t, t);                                      // 2^-86
+    const unsigned t2h = (unsigned)(t2 >> 32);                                           // 2^-54
+    const unsigned t3 = __umulhi(__umulhi(t2h, th), 0x2AAAAAABu);                        // t^3 / 6, 2^-65
+    const unsigned t4 = __umulhi(__umulhi(t2h, t2h), 0x0AAAAAABu);                       // t^4 / 24, 2^-76
+    const unsigned long long p = t + (t2 >> 12) + ((unsigned long long)t3 << 10) + (t4 >> 1);
+    const unsigned long long m = tab[(int)(fr >> (64 - kExpBits))];
+    const unsigned long long w = m + (__umul64hi(m, p) >> 11);                           // [1, 2) in 2^-63
+    return __longlong_as_double(((long long)(k + 1022) << 52) + (long long)((w >> 11) + ((w >> 10) & 1ull)));
+}
+
+// One warp per temperature.  Bound: the FP64 pipe -- an FP64 warp instruction occupies it for 32
+// cycles of the SM, as long as some sixty integer ones -- so what the sums do not need stays off it:
 //   * a level whose weight is zero in FP64 (more than 746 below the maximum) is found in single
 //     precision, with its rounding error bounded and added to the margin, and skipped: half of the
 //     levels of an L = 64 spectrum over the default ladder;
-//   * E / T is the quotient by the reciprocal with one residual correction (Markstein, 1990) instead of a
-//     division, x is formed once, exp is by table (above), E^2 comes from memory.
-// 21 FP64 instructions per weighted level with four observables, where division twice and exp took
-// about 50 for every level: 4,095 levels x 50,000 temperatures x 5 columns 23.4 -> 7.9 ms (with the copies; the FP64 pipe
-// at 86 %).
-// STAGED: levels in shared memory.
-template <bool STAGED>
+//   * the exponents of the others, relative to the largest, are differences of 62-bit integers, and
+//     their exponentials are formed by integer arithmetic to the last bit of a double (above).
+// What is left is one addition and three products for the sums and one per observable: 4,095 levels x
+// 50,000 temperatures x 5 columns 23.4 -> 2.9 ms (with the copies) from two divisions and a library
+// exponential for every level; the same sums with a table exponential in FP64 took 7.9 ms.
+// Where the integers could be coarser than FP64 -- energies whose largest values dwarf those that
+// count -- a temperature takes the FP64 form of the same sums.
+// STAGED: levels in shared memory.  KO: room for observable columns.
+template <bool STAGED, int KO>
 __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
 {
     extern __shared__ __align__(16) double sm[];
-    double* tab = sm;
+    unsigned long long* tab = reinterpret_cast<unsigned long long*>(sm);
     double *sE = sm + kExpTable, *sG = sE + a.nb, *sE2 = sG + a.nb;
     float2* sX = reinterpret_cast<float2*>(sE2 + a.nb);
-    for (int j = threadIdx.x; j < kExpTable; j += blockDim.x) tab[j] = exp2((double)j / kExpTable);
+    long long *sEi = reinterpret_cast<long long*>(sX + a.nb), *sgi = sEi + a.nb;
+    for (int j = threadIdx.x; j < kExpTable; j += blockDim.x) tab[j] = pow2_fraction(j);
     if (STAGED)
         for (int b = threadIdx.x; b < a.nb; b += blockDim.x) {
             const double e = a.E[b];
@@ -106,19 +128,21 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
             sE2[b] = e * e;
             sG[b] = a.lng[b];
             sX[b] = a.x32[b];
+            sEi[b] = a.Ei[b];
+            sgi[b] = a.gi[b];
         }
     __syncthreads();
     const double* E = STAGED ? sE : a.E;
     const double* G = STAGED ? sG : a.lng;
     const float2* X = STAGED ? sX : a.x32;
+    const long long* Ei = STAGED ? sEi : a.Ei;
+    const long long* gi = STAGED ? sgi : a.gi;
+    constexpr double kLog2e = 0x1.71547652b82fep+0, kLog2eLo = 0x1.777d0ffda0d24p-56;
     const int lane = threadIdx.x & 31, nb = a.nb;
     for (int t = blockIdx.x * kWarps + (threadIdx.x >> 5); t < a.nT; t += gridDim.x * kWarps) {
         const double T = __dadd_rn(a.Tmin, __dmul_rn(a.dT, (double)t));    // rounded as the reference's Tmin + dT * i
         const double rT = 1.0 / T;
-        auto exponent = [&](int b) {
-            const double e = E[b], q0 = e * rT;
-            return G[b] - fma(fma(-q0, T, e), rT, q0);
-        };
+        auto exponent = [&](int b) { return G[b] - E[b] / T; };
         // the largest exponent, to the single-precision error `err` of every x32 (three times what its
         // roundings add up to): the exponent of the level found is the reference point, which need not be
         // the largest one to the last bit
@@ -127,22 +151,44 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
         const bool filter = a.e_max >= 0.f && err < 50.f;
         double m;
         float floor32 = -INFINITY;
+        int F = 0, top = 0;
+        long long c = 0;
         if (filter) {
             float best = -INFINITY;
-            int at = 0;
             for (int b = lane; b < nb; b += 32) {
                 const float2 v = X[b];
                 const float x = fmaf(v.x, r32, v.y);
-                if (x > best) { best = x; at = b; }
+                if (x > best) { best = x; top = b; }
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 const float x = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-                const int i = __shfl_xor_sync(0xFFFFFFFFu, at, o);
-                if (x > best || (x == best && i < at)) { best = x; at = i; }
+                const int i = __shfl_xor_sync(0xFFFFFFFFu, top, o);
+                if (x > best || (x == best && i < top)) { best = x; top = i; }
             }
-            m = exponent(at);
+            m = exponent(top);
             floor32 = best - 746.f - 2.f * err;
+            // fixed point for the levels that count: their energies lie within `span` of the reference's
+            float span = 0.f;
+            const float2 ref = X[top];
+            for (int b = lane; b < nb; b += 32) {
+                const float2 v = X[b];
+                if (!(fmaf(v.x, r32, v.y) < floor32)) span = fmaxf(span, fabsf(v.x - ref.x));
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) span = fmaxf(span, __shfl_xor_sync(0xFFFFFFFFu, span, o));
+            span = 1.0001f * span + 2e-7f * a.e_max;
+            const double ch = kLog2e * rT, cl = fma(kLog2e, rT, -ch) + (kLog2e * (fma(-rT, T, 1.0) * rT) + kLog2eLo * rT);
+            const float bits = 1.45f * (2.f * span * r32 + 750.f + 2.f * err);     // bound of every exponent difference
+            F = min(min(60 - ilogbf(bits), a.se - 3 - ilogb(ch)), min(a.sg, 52));
+            // the roundings of the integers against those of x = ln g - E / T and of a weight in FP64
+            const double coarse = ldexp(ch, -a.se) + ldexp(1.0, -a.sg) + ldexp(1.0, -F);
+            if (F >= 24 && coarse <= 0x1p-53 * (1.0 + (fabs(E[top]) * rT + fabs(m)))) {
+                const int up = F + 64 - a.se;
+                c = __double2ll_rn(ldexp(ch, up)) + __double2ll_rn(ldexp(cl, up));
+            } else {
+                F = 0;
+            }
         } else {
             m = -INFINITY;
             for (int b = lane; b < nb; b += 32) m = fmax(m, exponent(b));
@@ -150,9 +196,10 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
             for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
         }
 
-        double z = 0.0, u = 0.0, u2 = 0.0, s = 0.0, o[kMaxObs];
+        double z = 0.0, u = 0.0, u2 = 0.0, s = 0.0, o[KO + 1];
 #pragma unroll
-        for (int k = 0; k < kMaxObs; ++k) o[k] = 0.0;
+        for (int k = 0; k < KO; ++k) o[k] = 0.0;
+        const long long etop = Ei[top], gtop = gi[top];
         for (int b0 = 0; b0 < nb; b0 += 32) {
             const int b = b0 + lane;
             bool counts = b < nb;
@@ -162,15 +209,21 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
             }
             if (!__any_sync(0xFFFFFFFFu, counts)) continue;
             if (counts) {
-                const double e = E[b], d = exponent(b) - m;
-                double w = d > -700.0 ? exp_table(d, tab) : exp(d);
+                double w;
+                if (F) {
+                    const long long d = ((gi[b] - gtop) >> (a.sg - F)) - __mul64hi(Ei[b] - etop, c);
+                    w = (d >> F) >= -1020 ? pow2_fixed(d, F, tab) : 0.0;
+                } else {
+                    w = exp(exponent(b) - m);
+                }
                 if (a.trapezoid && (b == 0 || b == nb - 1)) w *= 0.5;
+                const double e = E[b];
                 z += w;
                 u = fma(e, w, u);
                 u2 = fma(STAGED ? sE2[b] : e * e, w, u2);
                 s = fma(G[b], w, s);
 #pragma unroll
-                for (int k = 0; k < kMaxObs; ++k)
+                for (int k = 0; k < KO; ++k)
                     if (k < a.K && k != a.counts_col) o[k] = fma(a.obs[(size_t)k * nb + b], w, o[k]);
             }
         }
@@ -180,7 +233,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
         s = warp_sum(s);
         double* row = a.out + (size_t)t * (5 + a.K);
 #pragma unroll
-        for (int k = 0; k < kMaxObs; ++k)
+        for (int k = 0; k < KO; ++k)
             if (k < a.K) {
                 if (k == a.counts_col) o[k] = a.counts_mean;
                 else o[k] = warp_sum(o[k]) / z;
@@ -216,8 +269,8 @@ int rewl_thermodynamics(const double* E, const double* lng, const double* obs, i
     if (cudaSetDevice(device) != cudaSuccess) return tfail(REWL_EDEVICE, "cannot use device %d", device);
     const size_t nrow = 5 + (size_t)num_obs, nb = (size_t)nbins;
     // one buffer on the host and one on the device: E, ln g, observables by column, {-E, ln g} in
-    // single precision; then (device) temperatures and rows
-    const size_t in = nb * (3 + num_obs), all = in + (size_t)num_T * (1 + nrow);
+    // single precision, E and ln g / ln 2 as integers; then (device) temperatures and rows
+    const size_t in = nb * (5 + num_obs), all = in + (size_t)num_T * (1 + nrow);
     std::vector<double> h(in);
     std::copy(E, E + nb, h.begin());
     std::copy(lng, lng + nb, h.begin() + nb);
@@ -231,7 +284,20 @@ int rewl_thermodynamics(const double* E, const double* lng, const double* obs, i
         if (counts_col >= 0) counts += obs[b * num_obs + counts_col];
         x32[b] = make_float2((float)-E[b], (float)lng[b]);
     }
+    // the integers: 2^62 above the largest energy, 2^60 above the largest ln g / ln 2 (formed to 106 bits)
+    int xe = 0, xg = 0;
+    std::frexp(e_max, &xe);
+    std::frexp(g_max * 1.45, &xg);
+    const int se = std::min(std::max(62 - xe, -900), 900), sg = std::min(std::max(60 - xg, -900), 900);
+    long long* ints = reinterpret_cast<long long*>(h.data() + nb * (3 + num_obs));
+    constexpr double kLog2e = 0x1.71547652b82fep+0, kLog2eLo = 0x1.777d0ffda0d24p-56;
+    for (size_t b = 0; b < nb; ++b) {
+        const double g = lng[b] * kLog2e, rest = std::fma(lng[b], kLog2e, -g) + lng[b] * kLog2eLo;
+        ints[b] = std::llrint(std::ldexp(E[b], se));
+        ints[nb + b] = std::llrint(std::ldexp(g, sg)) + std::llrint(std::ldexp(rest, sg));
+    }
     ThermoArgs a{};
+    a.se = se; a.sg = sg;
     a.nb = nbins; a.K = num_obs; a.counts_col = counts_col; a.nT = num_T; a.trapezoid = trapezoid ? 1 : 0;
     a.N = system_size; a.Tmin = Tmin; a.dT = (Tmax - Tmin) / (double)num_T; a.counts_mean = counts / (double)nbins;
     // single precision locates the levels that count while it can hold them
@@ -246,18 +312,20 @@ int rewl_thermodynamics(const double* E, const double* lng, const double* obs, i
     if (e == cudaSuccess) {
         a.E = d; a.lng = d + nb; a.obs = d + 2 * nb;
         a.x32 = reinterpret_cast<const float2*>(d + nb * (2 + num_obs));
+        a.Ei = reinterpret_cast<const long long*>(d + nb * (3 + num_obs)); a.gi = a.Ei + nb;
         a.temps = d + in; a.out = a.temps + num_T;
         int nsm = 0;
         if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || nsm < 1) nsm = 152;
-        const size_t table = kExpTable * sizeof(double), staged = table + nb * 32;
-        const bool fits = staged <= 200 * 1024;        // levels up to 5,900 in shared memory
-        const void* fn = fits ? reinterpret_cast<const void*>(k_thermo<true>) : reinterpret_cast<const void*>(k_thermo<false>);
-        const size_t smem = fits ? staged : table;
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        const size_t table = kExpTable * sizeof(double), staged = table + nb * 48;
+        const bool fits = staged <= 220 * 1024;        // levels up to 4,352 in shared memory
+        using Kernel = void (*)(const ThermoArgs);
+        const Kernel kernels[2][3] = {{k_thermo<false, 0>, k_thermo<false, 6>, k_thermo<false, kMaxObs>},
+                                      {k_thermo<true, 0>, k_thermo<true, 6>, k_thermo<true, kMaxObs>}};
+        const Kernel fn = kernels[fits ? 1 : 0][num_obs == 0 ? 0 : num_obs <= 6 ? 1 : 2];
+        e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
         if (e == cudaSuccess) {
             const int grid = std::min((num_T + kWarps - 1) / kWarps, nsm);
-            if (fits) k_thermo<true><<<grid, 32 * kWarps, smem, st>>>(a);
-            else k_thermo<false><<<grid, 32 * kWarps, smem, st>>>(a);
+            fn<<<grid, 32 * kWarps, fits ? staged : table, st>>>(a);
             e = cudaGetLastError();
         }
     }

@@ -9,9 +9,9 @@ CASES = [
     # levels, N, energy scale, Tmin, Tmax, temperatures, columns, counts column, trapezoid
     (2, 4, 8.0, 0.5, 5.0, 7, 0, -1, True), (31, 16, 32.0, 0.1, 10.0, 33, 3, 2, False),
     (33, 16, 32.0, 0.01, 50.01, 200, 1, -1, True), (1000, 1024, 2048.0, 0.01, 50.01, 1000, 17, 16, True),
-    (5888, 4096, 8192.0, 0.05, 20.0, 300, 4, 3, True), (5913, 4096, 8192.0, 0.05, 20.0, 300, 4, 3, False),
+    (4352, 4096, 8192.0, 0.05, 20.0, 300, 4, 3, True), (4353, 4096, 8192.0, 0.05, 20.0, 300, 4, 3, False),
     (20001, 4096, 8192.0, 0.5, 50.0, 100, 5, 4, True), (500, 256, 1e9, 0.01, 1.0, 50, 2, 1, True),
-    (500, 256, 1e20, 1e17, 1e19, 50, 2, -1, True),
+    (500, 256, 1e20, 1e17, 1e19, 50, 2, -1, True), (300, 1, 1e-9, 0.01, 1.0, 20, 1, -1, False),
 ]
 
 
@@ -48,3 +48,19 @@ def test_ladder(engine_lib, case):
         for k in range(K):
             ref = obs[:, k].mean() if k == counts else p @ obs[:, k]
             assert abs(out[i, 5 + k] - ref) <= rel * ref
+
+
+@pytest.mark.gpu
+def test_ground_state_at_zero_energy(engine_lib):
+    """Energies from 0 to 10^9 at temperatures of order 1: the integers that span them are coarser than
+    FP64 near the ground state, and the ladder keeps FP64's precision there."""
+    from rewl_simulator_gb300.thermo import thermodynamics
+    nb = 700
+    E = np.concatenate([[0.0, 0.3, 0.7, 1.1, 1.9, 2.3], np.geomspace(3.0, 1e9, nb - 6)])
+    lng = np.log1p(E)
+    T, out = thermodynamics(E, lng, 16, Tmin=0.1, Tmax=4.1, num_T=40, trapezoid=False)
+    for i, t in enumerate(T):
+        x = lng - E / t
+        w = np.exp(x - x.max())
+        U = (w * E).sum() / w.sum() / 16
+        assert abs(out[i, 1] - U) <= 4e-15 * U + 1e-300
