@@ -326,7 +326,7 @@ int rewl_mlp_launches(const rewl_mlp* mlp, int64_t* count);
 /* Allocation-free prediction (no counterpart in the reference).  Same result as
  * rewl_mlp_predict, but X (n x in_dim floats) and y (n floats) are DEVICE
  * pointers and the work is enqueued on `stream` (a cudaStream_t; NULL = legacy
- * default stream) without waiting for it.  Activations live in a static 9.5 MiB
+ * default stream) without waiting for it.  Activations live in a static 5.5 MiB
  * device array that every GPU loading this library holds until exit, so no call
  * allocates device memory.  It is for callers that cannot call cudaMalloc: a host
  * program whose own allocator already holds the device's memory, a loop at its
