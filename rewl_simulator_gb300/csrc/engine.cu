@@ -173,6 +173,7 @@ struct DevPtrs {
     int obs_stride;          // 3 (Ising) or 12 (a batch with Ashkin-Teller instances); 4 or 16 with correlators
     int corr;                // observables carry the G(q_min) correlators
     const double* qtab;      // per instance: cos(q_min x) then sin(q_min x), x < L
+    const int2* qfix;        // the same in units of 2^-30 (x) and 2^-60 (y)
 };
 
 // --------------------------------------------------------------------------
@@ -330,6 +331,53 @@ __device__ double plane_corr(const int* rs, const int* cs, const double* q, int 
         iy += (double)cl * sn;
     }
     return 0.5 * ((rx * rx + ix * ix) + (ry * ry + iy * iy));
+}
+
+// The same by P lanes together, for the step that all of them name: lane l takes the quantity
+// l % (4 NC) -- of its plane l / 4 % NC: the cosine and sine sums over rows, then over columns --
+// and of its terms every P / (4 NC)-th.  rs, cs, flips (accepted flips of the chunk that change
+// the lane's plane, up to the step), up (the steps whose term was +1 before) are the lane's
+// plane's; the plane's four lanes return 2 G.  The sums are whole numbers (sums times table
+// entries of 60 binary places), so a term costs two integer multiplications instead of five FP64
+// instructions at 32 cycles of an SM each, and the only rounding is of the table and of the
+// final squares.
+template <int P, int NC>
+__device__ double plane_power(const int* rs, const int* cs, const int2* q, int L, int y, int x0, unsigned flips,
+                              unsigned up, int lane)
+{
+    constexpr int NQ = 4 * NC;
+    const bool col = (lane & 2) != 0;
+    const int* v = col ? cs : rs;
+    if (lane & 1) q += L;
+    const int dr = -2 * ((int)__popc(flips & up) - (int)__popc(flips & ~up));
+    long long hi = 0, lo = 0;                              // below 2^14 sites x 2^30
+#pragma unroll 4
+    for (int t = lane / NQ; t < L; t += P / NQ) {
+        const int2 c = q[t];
+        const int k = t - x0;
+        const bool in = (unsigned)k < 32u && ((flips >> k) & 1u) != 0;
+        int r = v[t];
+        if (col) r -= !in ? 0 : (up >> k) & 1u ? 2 : -2;
+        else r += t == y ? dr : 0;
+        hi += (long long)r * c.x;
+        lo += (long long)r * c.y;
+    }
+#pragma unroll
+    for (int m = NQ; m < P; m *= 2) {
+        hi += __shfl_xor_sync(kFull, hi, m);
+        lo += __shfl_xor_sync(kFull, lo, m);
+    }
+    const double x = fma(whole_double(hi), 1.0 / 1073741824.0, whole_double(lo) * (1.0 / 1152921504606846976.0));
+    double g = x * x;
+    g += __shfl_xor_sync(kFull, g, 1);
+    g += __shfl_xor_sync(kFull, g, 2);
+    return g;
+}
+
+__device__ __forceinline__ int mod_transform(unsigned long long x)     // x % kCountsPerTransform
+{
+    static_assert(kCountsPerTransform == 1000, "2^32 = 296 modulo 1000");
+    return (int)(((unsigned)(x >> 32) % 1000u * 296u + (unsigned)x % 1000u) % 1000u);
 }
 
 // Row and column sums of a plane (value(i) for site i) into rs, cs, by `stride` lanes.
@@ -682,10 +730,14 @@ __device__ __forceinline__ long long mad_units(long long acc, int n, int f_lo, i
     return r;
 }
 
-// adds 1 to the 32-bit word at shared address `addr`
+// adds 1 (v) to the 32-bit word at shared address `addr`
 __device__ __forceinline__ void red_shared_inc(unsigned addr)
 {
     asm volatile("red.shared.add.u32 [%0], 1;" :: "r"(addr) : "memory");
+}
+__device__ __forceinline__ void red_shared_add(unsigned addr, int v)
+{
+    asm volatile("red.shared.add.s32 [%0], %1;" :: "r"(addr), "r"(v) : "memory");
 }
 
 // chunk layout of a row of L sites: `n` words, the first `rem` of `base` + 1 sites, the others of `base`
@@ -707,14 +759,16 @@ struct BinsTree {
     static_assert(kLanes == 1 << kDepth, "one lane per node");
 };
 
-constexpr int kObsWords = 8;      // Ising moments as integers: |M|, M^2 and M^4 in halves of 28 bits, 64 bits each
-
-// 64-bit sum in two shared words, lo then hi
-__device__ __forceinline__ void add_carry(unsigned* s, unsigned x)
-{
-    const unsigned old = atomicAdd(s, x);
-    if (old + x < old) atomicAdd(s + 1, 1u);
-}
+// Ising moments of a bin as whole numbers, in words that reductions add to without looking: |M|,
+// M^2 in two parts, M^4 in four, `bits` binary digits each (the last ones what is left).  `visits`
+// visits cannot overflow a word; after as many the words are added to the observable sums in
+// global memory and start at zero again.
+constexpr int kObsWords = 7;
+struct MomentParts {
+    int bits;
+    unsigned visits;
+    __host__ __device__ explicit MomentParts(int N) : bits(N <= 8192 ? 18 : 16), visits(1u << (32 - bits)) {}
+};
 
 // shared memory of one walker: table with guards, lattice words, thresholds, two chunks' slots;
 // with observables the bins of a chunk's steps and (acc) the
@@ -756,7 +810,7 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
     int* seqb = reinterpret_cast<int*>(slots + 2 * T::kBlocks * T::kSlot) + 4;   // a chunk's bins (observables)
     int* rsum = seqb + (OBS ? 32 : 0);                                           // correlators: row sums,
     int* csum = rsum + L;                                                        // column sums,
-    int* bcnt = csum + L;                                                        // bin counts mod 1000
+    int* bcnt = csum + L;                                                        // visits before a bin's next transform
     const bool corr = OBS && P_.corr, moments = OBS && p.moments;
     unsigned* mom = reinterpret_cast<unsigned*>(corr ? bcnt + p.nbcap : rsum);   // moment sums (observables)
     // table positions are byte offsets from the start of shared memory, so that the
@@ -800,12 +854,37 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
     };
     const double invN = 1.0 / (double)N;
     double* ob = OBS ? P_.obs + (size_t)P_.slot_tab[s] * P_.obs_stride : nullptr;
+    const MomentParts parts(N);
+    unsigned booked = 0;                                       // visits in the moments' words
+    const int reach2 = (int)(((unsigned long long)N * N) >> parts.bits) != 0 ? 2 : 1;      // parts of M^2, M^4
+    int reach4 = 1;
+    for (unsigned long long x = (unsigned long long)N * N * N * N; (x >>= parts.bits) != 0;) ++reach4;
     if (moments)
         for (int k = q; k < nb * kObsWords; k += P) mom[k] = 0;
+    // the words into the sums of m = |M| / N
+    auto book_moments = [&] {
+        const double in2 = invN * invN, unit = (double)(1u << parts.bits);
+        __syncwarp();
+        if (valid)
+            for (int k = q; k < nb; k += P) {
+                unsigned* t = mom + kObsWords * k;
+                double* o = ob + (size_t)k * P_.obs_stride;
+                if ((t[0] | t[1] | t[2]) != 0) {               // (M = 0 adds nothing)
+                    o[0] += invN * (double)t[0];
+                    o[1] += in2 * (unit * (double)t[2] + (double)t[1]);
+                    o[2] += in2 * in2 * (((unit * (double)t[6] + (double)t[5]) * unit + (double)t[4]) * unit + (double)t[3]);
+                    for (int j = 0; j < kObsWords; ++j) t[j] = 0;
+                }
+            }
+        __syncwarp();
+    };
     if (corr) {
         plane_sums(rsum, csum, L, q, spin, P);
         const uint64_t* gv0 = P_.visits + P_.slot_tab[s];
-        for (int k = q; k < nb; k += P) bcnt[k] = (int)(gv0[k] % kCountsPerTransform);
+        for (int k = q; k < nb; k += P) {
+            const int r = mod_transform(gv0[k]);
+            bcnt[k] = r == 0 ? 0 : (int)kCountsPerTransform - r;
+        }
         __syncwarp();
     }
 
@@ -1132,46 +1211,62 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
             if (nblk == 1) n = node_row(nxt, at + (uint32_t)len, L, yn);
         }
         if (OBS) {
-            // the chunk's moments and correlators, one step per lane
+            // the chunk's moments and correlators, one step per lane, by reductions that return nothing and
+            // with no look at the chunk's own repeats of a bin unless a transform may be due (16 steps
+            // of L = 16: 1370 -> 650 cycles beside the 1500 of their decisions)
             const unsigned plus = ~old & (0xFFFFFFFFu >> (32 - len));
             const int x0 = rc.start(ci);
+            if (moments && (booked += (unsigned)len) > parts.visits) {
+                book_moments();
+                booked = (unsigned)len;
+            }
 #pragma unroll
             for (int i = 0; i < SPL; ++i) {
                 const int jj = q + i * P;
                 const bool mine = valid && jj < len;
                 const int off = mine ? seqb[jj] : -1 - lane;
                 const int b = mine ? (off - gsoff) / RS : 0;
-                if (mine) {
-                    const int32_t Mv[1] = {M + chunk_dm(acc, plus, jj)};
-                    if (moments) {
-                        const unsigned m = (unsigned)abs(Mv[0]), m2 = m * m;
-                        const unsigned long long m4 = (unsigned long long)m2 * m2;
-                        unsigned* t = mom + kObsWords * b;
-                        add_carry(t, m);
-                        add_carry(t + 2, m2);
-                        add_carry(t + 4, (unsigned)(m4 & 0xFFFFFFFu));
-                        add_carry(t + 6, (unsigned)(m4 >> 28));
-                    } else {
-                        Ising2dModel::add_observables(ob + (size_t)b * P_.obs_stride, Mv, invN, P_.corr);
-                    }
+                const int Mj = M + chunk_dm(acc, plus, jj);
+                // visits of the bin before its next transform (correlators), ahead of the chunk
+                const int before = corr && mine ? bcnt[b] : 32;
+                if (moments) {
+                    const unsigned m = (unsigned)abs(Mj), m2 = m * m, low = (1u << parts.bits) - 1u;
+                    const unsigned long long m4 = (unsigned long long)m2 * m2;
+                    const unsigned t = mine ? (unsigned)__cvta_generic_to_shared(mom + kObsWords * b) : 0u;
+                    auto add = [&](int k, unsigned v) { red_shared_add(mine ? t + 4 * k : smbase + (unsigned)sink, (int)v); };
+                    add(0, m);
+                    add(1, m2 & low);
+                    if (reach2 > 1) add(2, m2 >> parts.bits);
+                    add(3, (unsigned)m4 & low);
+                    if (reach4 > 1) add(4, (unsigned)(m4 >> parts.bits) & low);
+                    if (reach4 > 2) add(5, (unsigned)(m4 >> (2 * parts.bits)) & low);
+                    if (reach4 > 3) add(6, (unsigned)(m4 >> (3 * parts.bits)));
+                } else if (mine) {
+                    const int32_t Mv[1] = {Mj};
+                    Ising2dModel::add_observables(ob + (size_t)b * P_.obs_stride, Mv, invN, P_.corr);
                 }
                 if (corr) {
-                    // G(q_min) at the steps whose bin count before the visit is a multiple of 1000: the
-                    // count before this strip of steps plus the strip's earlier visits to the bin
-                    const unsigned same = __match_any_sync(kFull, off), earlier = same & ((1u << lane) - 1u);
-                    if (mine) {
-                        const int seen = bcnt[b] + __popc(earlier);
-                        if (seen == 0 || seen == (int)kCountsPerTransform) {
-                            const double Gq = plane_corr(rsum, csum, P_.qtab + I.qtab_off, L, y, chunk_dm(acc, plus, jj), x0,
-                                                         jj, acc, [&](int kk) { return (old >> kk) & 1u ? -1 : 1; });
-                            atomicAdd(ob + (size_t)b * P_.obs_stride + 3, invN * invN * Gq);
+                    // G(q_min) at the steps whose bin count before the visit is a multiple of 1000
+                    bool due = false;
+                    if (__any_sync(kFull, before < len)) {
+                        const unsigned same = __match_any_sync(kFull, off), earlier = same & ((1u << lane) - 1u);
+                        due = mine && before == __popc(earlier);
+                        bool todo = due;
+                        for (unsigned all; (all = __ballot_sync(kFull, todo)) != 0;) {
+                            // one step of each walker of the warp
+                            const unsigned own = (all >> gbase) & (0xFFFFFFFFu >> (32 - P));
+                            const int e = own ? __ffs((int)own) - 1 : 0, je = e + i * P;
+                            const unsigned le = je >= 31 ? 0xFFFFFFFFu : ((2u << je) - 1u);
+                            const double Gq = plane_power<P, 1>(rsum, csum, P_.qfix + I.qtab_off, L, y, x0, acc & le, plus, q);
+                            if (own != 0 && q == e) {
+                                red_global_add(ob + (size_t)b * P_.obs_stride + 3, 0.5 * invN * invN * Gq);
+                                todo = false;
+                            }
                         }
                     }
-                    __syncwarp();
-                    if (mine && earlier == 0) {
-                        const int n2 = bcnt[b] + __popc(same);
-                        bcnt[b] = n2 >= (int)kCountsPerTransform ? n2 - (int)kCountsPerTransform : n2;
-                    }
+                    __syncwarp();                              // every lane has read its bin's count
+                    red_shared_add(mine ? (unsigned)__cvta_generic_to_shared(bcnt + b) : smbase + (unsigned)sink,
+                                   due ? (int)kCountsPerTransform - 1 : -1);
                     __syncwarp();
                 }
             }
@@ -1180,9 +1275,12 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
 #pragma unroll
                 for (int i = 0; i < SPL; ++i) {
                     const int jj = q + i * P;
-                    if (valid && jj < len && ((acc >> jj) & 1u)) csum[x0 + jj] -= 2 * ((old >> jj) & 1u ? -1 : 1);
+                    const bool flipped = valid && jj < len && ((acc >> jj) & 1u);
+                    red_shared_add(flipped ? (unsigned)__cvta_generic_to_shared(csum + x0 + jj) : smbase + (unsigned)sink,
+                                   (old >> jj) & 1u ? 2 : -2);
                 }
-                if (valid && q == 0) rsum[y] += chunk_dm(acc, plus, 31);
+                const int dr = chunk_dm(acc, plus, 31);
+                if (valid && q == 0) red_shared_add((unsigned)__cvta_generic_to_shared(rsum + y), dr);
             }
             M += chunk_dm(acc, plus, 31);
             __syncwarp();
@@ -1212,19 +1310,7 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
             if (e) atomicOr(&P_.counters[0], e);
             gg[k] = gnew;
         }
-        if (moments) {
-            // m = |M| / N: the launch's sums are whole numbers until here
-            const double in2 = invN * invN;
-            for (int k = q; k < nb; k += P) {
-                const unsigned* t = mom + kObsWords * k;
-                auto sum = [&](int j) { return (double)(((unsigned long long)t[j + 1] << 32) | t[j]); };
-                double* o = ob + (size_t)k * P_.obs_stride;
-                if ((t[0] | t[1]) == 0) continue;
-                o[0] += invN * sum(0);
-                o[1] += in2 * sum(2);
-                o[2] += in2 * in2 * (268435456.0 * sum(6) + sum(4));
-            }
-        }
+        if (moments) book_moments();
         if (q == 0) {
             const int root = (int)(state & 0xFFFFFu);
             if ((unsigned)(root - gsoff) >= (unsigned)(nb * RS)) atomicOr(&P_.counters[0], ERR_BOUNDS);
@@ -1494,6 +1580,7 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
     tab.err = 0;
     const bool corr = OBS && P.corr;
     const double invN = 1.0 / (double)N;
+    double* const ob = OBS ? P.obs + (size_t)P.slot_tab[s] * P.obs_stride : nullptr;
     if (corr) {
         for (int cp = 0; cp < NC; ++cp)
             plane_sums(sums + 2 * L * cp, sums + 2 * L * cp + L, L, lane,
@@ -1713,62 +1800,80 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
                         hnext = field(min((ch + 1 == L * rc.n ? 0 : c0 + C) + lane, N - 1));
                     });
                 }
-                // per magnetisation: the steps whose accepted flip lowers it (its term was +1)
-                // and raises it; the change after step j is -2 (lowered - raised) up to j
-                unsigned plus[NM], minus[NM];
+                // per magnetisation that the plane's flips change: the steps whose accepted flip lowers it
+                // (its term was +1; the others raise it); the change after step j is -2 (lowered - raised)
+                // up to j
+                unsigned plus[NM] = {};
+                int total[NM] = {};                    // by the whole chunk
+                auto changes = [&](int m) { return m == NM - 1 || m == plane; };
+                auto dm = [&](int m, int j) {
+                    const unsigned le = acc & (0xFFFFFFFFu >> (31 - j));
+                    return changes(m) ? 2 * (int)__popc(le) - 4 * (int)__popc(le & plus[m]) : 0;
+                };
                 if (OBS)
                     for (int m = 0; m < NM; ++m) {
                         plus[m] = __ballot_sync(kFull, lane < C && sg[m] > 0);
-                        minus[m] = __ballot_sync(kFull, lane < C && sg[m] < 0);
+                        total[m] = dm(m, 31);
                     }
-                auto dm = [&](int m, int j) {
-                    const unsigned le = j >= 31 ? 0xFFFFFFFFu : ((2u << j) - 1u);
-                    return -2 * ((int)__popc(acc & plus[m] & le) - (int)__popc(acc & minus[m] & le));
-                };
                 if (OBS) {
                     __syncwarp();
-                    if (lane < C) {
+                    const int bin = lane < C ? st->seq[lane] : -1 - lane;
+                    // correlators: the bin's visits booked so far and those not booked yet (this chunk's
+                    // are among them), read ahead of the moments
+                    unsigned long long after = 1;
+                    if (corr && lane < C)
+                        after = tab.gv[bin] +
+                                (!TREE ? (unsigned long long)((gg[bin] - g0[bin]) / lnf)
+                                       : tab.holds(bin) ? (unsigned long long)tab.n[bin & (tab.size - 1)] : 0ull);
+                    // Moments: short chunks leave lanes for two groups of them at once.  Moments and
+                    // correlators are FP64's latency: 12 steps of L = 12, 4300 -> 2200 cycles beside the 3400
+                    // of their decisions, with a transform in one chunk of six (1100 cycles; a lane alone 2500).
+                    const int per = Model::kGroups > 1 && C <= 16 ? 16 : 32;
+                    const int step = lane & (per - 1);
+                    if (step < C) {
                         int32_t Mv[3] = {0, 0, 0};
-                        for (int m = 0; m < NM; ++m) Mv[m] = M[m] + dm(m, lane);
-                        Model::add_observables(P.obs + (size_t)(P.slot_tab[s] + st->seq[lane]) * P.obs_stride, Mv, invN,
-                                               P.corr);
+                        for (int m = 0; m < NM; ++m) Mv[m] = M[m] + dm(m, step);
+                        double* o = ob + (size_t)((unsigned)st->seq[step] * (unsigned)P.obs_stride);
+                        for (int g = lane / per; g < Model::kGroups; g += 32 / per)
+                            Model::add_group(o, g, Mv, invN, invN * invN, P.corr);
                     }
                     if (corr) {
-                        const int row = y * L;
-                        const int bin = lane < C ? st->seq[lane] : -1 - lane;
-                        const unsigned grp = __match_any_sync(kFull, bin);
-                        if (lane < C) {
-                            // the bin's count before step `lane`: its visits booked so far and those not
-                            // booked yet, less the chunk's visits from this step on
-                            const unsigned long long after = P.visits[P.slot_tab[s] + bin] +
-                                (!TREE ? (unsigned long long)((gg[bin] - g0[bin]) / lnf)
-                                        : tab.holds(bin) ? (unsigned long long)tab.n[bin & (tab.size - 1)] : 0ull);
-                            const unsigned long long seen = after - (unsigned long long)__popc(grp >> lane);
-                            if (seen % kCountsPerTransform == 0) {
-                                const double* q = P.qtab + I.qtab_off;
+                        // steps whose bin count before the visit is a multiple of 1000: the count after
+                        // the chunk less the chunk's visits from the step on
+                        const int last = mod_transform(after - 1);
+                        if (__any_sync(kFull, lane < C && last < C)) {
+                            const unsigned grp = __match_any_sync(kFull, bin);
+                            unsigned todo = __ballot_sync(kFull, lane < C && last == __popc(grp >> lane) - 1);
+                            const int cp = lane / 4 % NC, m = Model::corr_mag(cp);
+                            unsigned up = 0;
+                            for (int k = 0; k < NM; ++k)
+                                if (k == m) up = plus[k];
+                            for (; todo != 0; todo &= todo - 1) {
+                                const int j = __ffs((int)todo) - 1;
+                                // a correlator plane changes where its magnetisation's terms do
+                                const unsigned flips = changes(m) ? acc & (0xFFFFFFFFu >> (31 - j)) : 0u;
+                                const double g = plane_power<32, NC>(sums + 2 * L * cp, sums + 2 * L * cp + L,
+                                                                     P.qfix + I.qtab_off, L, y, x0, flips, up, lane);
                                 double G[NC];
-                                for (int cp = 0; cp < NC; ++cp) {
-                                    const int m = Model::corr_mag(cp);
-                                    // a correlator plane changes where its magnetisation's terms do
-                                    G[cp] = plane_corr(sums + 2 * L * cp, sums + 2 * L * cp + L, q, L, y, dm(m, lane), x0, lane,
-                                                       acc & (plus[m] | minus[m]),
-                                                       [&](int k) { return Model::corr_site(sp, N, row + x0 + k, cp); });
-                                }
-                                Model::add_transforms(P.obs + (size_t)(P.slot_tab[s] + bin) * P.obs_stride, G, invN * invN);
+                                for (int k = 0; k < NC; ++k) G[k] = __shfl_sync(kFull, g, 4 * k);
+                                if (lane == j)
+                                    Model::add_transforms(ob + (size_t)bin * P.obs_stride, G, 0.5 * invN * invN);
                             }
                         }
                         __syncwarp();
                         // the chunk's flips into the sums
                         for (int cp = 0; cp < NC; ++cp) {
                             const int m = Model::corr_mag(cp);
-                            if (lane < C && ((acc >> lane) & 1u)) sums[2 * L * cp + L + x0 + lane] -= 2 * sg[m];
-                            if (lane == 0) sums[2 * L * cp + y] += dm(m, 31);
+                            if (!changes(m)) continue;
+                            if (lane < C && ((acc >> lane) & 1u))
+                                red_shared_add((unsigned)__cvta_generic_to_shared(sums + 2 * L * cp + L + x0 + lane), -2 * sg[m]);
+                            if (lane == 0) red_shared_add((unsigned)__cvta_generic_to_shared(sums + 2 * L * cp + y), total[m]);
                         }
                     }
                 }
                 if (lane < C && ((acc >> lane) & 1u)) A[c0 + lane] = (int8_t)(-ai);
                 if (OBS)
-                    for (int m = 0; m < NM; ++m) M[m] += dm(m, 31);
+                    for (int m = 0; m < NM; ++m) M[m] += total[m];
                 __syncwarp();
                 attempt += (uint64_t)C;
                 tbuf ^= 1;
@@ -2278,6 +2383,7 @@ struct rewl_engine {
     DBuf<double> obs;           // per-bin observable sums (observables on)
     DBuf<int64_t> gsnap;        // Ashkin-Teller engines: logDoS copy taken by each sweep launch
     DBuf<double> qtab;          // correlator kernels (observables == 2)
+    DBuf<int2> qfix;
     DBuf<unsigned long long> xround;   // exchange round and the exchange kernel's done-block count
     std::vector<cudaStream_t> gstreams; // one per launch group when there are several (they run concurrently)
     cudaEvent_t fork_ev = nullptr;
@@ -2287,6 +2393,7 @@ struct rewl_engine {
     std::vector<int64_t> h_fields;
     std::vector<uint8_t> h_mask;
     std::vector<double> h_qtab;
+    std::vector<int2> h_qfix;
 
     DevPtrs ptrs() const
     {
@@ -2301,7 +2408,7 @@ struct rewl_engine {
         P.win_sweepctr = win_sweepctr.p; P.pairs = nullptr; P.counters = counters.p; P.stats = stats.p;
         P.xround = xround.p;
         P.obs = obs.p; P.obs_stride = obs_stride;
-        P.corr = desc.observables == 2 ? 1 : 0; P.qtab = qtab.p;
+        P.corr = desc.observables == 2 ? 1 : 0; P.qtab = qtab.p; P.qfix = qfix.p;
         return P;
     }
 
@@ -2318,7 +2425,7 @@ struct rewl_engine {
         d_inst.free_(); d_win.free_();
         slot_inst.free_(); slot_win.free_(); slot_cfg.free_(); slot_nb.free_(); slot_flavour.free_();
         pairs[0].free_(); pairs[1].free_();
-        obs.free_(); gsnap.free_(); qtab.free_(); xround.free_(); fused_counter.free_();
+        obs.free_(); gsnap.free_(); qtab.free_(); qfix.free_(); xround.free_(); fused_counter.free_();
         for (cudaStream_t st : gstreams) cudaStreamDestroy(st);
         gstreams.clear();
         for (cudaEvent_t ev : join_ev) cudaEventDestroy(ev);
@@ -2555,6 +2662,10 @@ int build_host(rewl_engine* e)
             for (int lw = dir; lw + 1 < D.instances[ii].num_windows; lw += 2) { e->pairs_dir[dir].push_back(ii); e->pairs_dir[dir].push_back(lw); }
     }
     e->h_fields = std::move(h_fields);
+    for (const double c : h_qtab) {
+        const double units = std::ldexp(c, 30), whole = std::nearbyint(units);
+        e->h_qfix.push_back(make_int2((int)whole, (int)std::nearbyint(std::ldexp(units - whole, 30))));
+    }
     e->h_qtab = std::move(h_qtab);
     e->h_mask = std::move(h_mask);
     return REWL_OK;
@@ -2573,7 +2684,7 @@ int upload_all(rewl_engine* e)
         (rc = upload(e->slot_inst, e->h_slot_inst, s)) || (rc = upload(e->slot_win, e->h_slot_win, s)) ||
         (rc = upload(e->slot_nb, e->h_slot_nb, s)) || (rc = upload(e->slot_tab, e->h_slot_tab, s)) ||
         (rc = upload(e->cfg_off, e->h_cfg_off, s)) || (rc = upload(e->fields, e->h_fields, s)) ||
-        (rc = upload(e->qtab, e->h_qtab, s)) ||
+        (rc = upload(e->qtab, e->h_qtab, s)) || (rc = upload(e->qfix, e->h_qfix, s)) ||
         (rc = upload(e->mask, e->h_mask, s)) || (rc = upload(e->pairs[0], e->pairs_dir[0], s)) ||
         (rc = upload(e->pairs[1], e->pairs_dir[1], s)))
         return rc;

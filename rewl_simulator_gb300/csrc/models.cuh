@@ -39,6 +39,37 @@ struct Neighbours {
 };
 __host__ __device__ inline Neighbours neighbours(int i, int L) { return {nb_up(i, L), nb_left(i, L), nb_right(i, L), nb_down(i, L)}; }
 
+// adds v to *p in global memory (atomicAdd on a pointer whose address space the compiler does not know
+// asks for it at every use, and takes a compare-and-swap loop for shared memory along)
+__device__ __forceinline__ void red_global_add(double* p, double v)
+{
+    asm volatile("red.global.add.f64 [%0], %1;" :: "l"(__cvta_generic_to_global(p)), "d"(v) : "memory");
+}
+
+// Conversions to FP64 without the conversion instructions (95 cycles each, and FP64's pipe): a
+// whole number |v| < 2^51 as the low bits of 1.5 x 2^52 + v, less 1.5 x 2^52; a positive normal float by its
+// exponent and fraction fields (zero stays zero).
+__device__ __forceinline__ double whole_double(long long v)
+{
+    return __longlong_as_double(0x4338000000000000ll + v) - 6755399441055744.0;
+}
+__device__ __forceinline__ double float_double(float f)
+{
+    const unsigned u = __float_as_uint(f);
+    return __hiloint2double(u == 0 ? 0 : (int)((u >> 3) + (896u << 20)), (int)(u << 29));
+}
+
+// Square root of a whole number below 2^31 to FP64's last place: Newton's iteration on x^2 = k with the residual
+// in one fused operation, twice, from the single-precision root (22 -> 43 -> more than 53 places)
+__device__ inline double whole_root(unsigned k)
+{
+    const float y = k == 0 ? 0.f : rsqrtf((float)k);
+    const double kd = whole_double(k), half = float_double(0.5f * y);
+    double x = float_double((float)k * y);
+    x = fma(fma(-x, x, kd), half, x);
+    return fma(fma(-x, x, kd), half, x);
+}
+
 struct Couplings {
     int64_t J, K;            // nearest-neighbour and four-spin couplings in energy units
 };
@@ -69,6 +100,7 @@ __device__ inline double full_corr(const int8_t* a, const int8_t* b, const doubl
 struct Ising2dModel {
     static constexpr int kPlanes = 1;
     static constexpr int kMoments = 3;
+    static constexpr int kGroups = 1;
     static constexpr int kMags = 1;
     static constexpr int kCorrPlanes = 1;
     __host__ __device__ static constexpr int corr_mag(int) { return 0; }
@@ -76,7 +108,7 @@ struct Ising2dModel {
     __host__ __device__ static void flip_signs(int a, int, int, int* sg) { sg[0] = a; }
     __host__ __device__ static int corr_site(const int8_t* sp, int, int i, int) { return sp[i]; }
     __host__ __device__ static void mag_terms(const int8_t* sp, int, int i, int* t) { t[0] = sp[i]; }
-    __device__ static void add_transforms(double* o, const double* G, double in2) { atomicAdd(o + 3, in2 * G[0]); }
+    __device__ static void add_transforms(double* o, const double* G, double in2) { red_global_add(o + 3, in2 * G[0]); }
 
     __host__ __device__ static int64_t delta_at(const int8_t* a, const int8_t*, int i, Neighbours n, Couplings c, int64_t)
     {
@@ -122,14 +154,22 @@ struct Ising2dModel {
     __device__ static void add_observables(double* o, const int32_t* M, double invN, int)
     {
         const double m = invN * fabs((double)M[0]);
-        atomicAdd(o, m);
-        atomicAdd(o + 1, m * m);
-        atomicAdd(o + 2, m * m * m * m);
+        red_global_add(o, m);
+        red_global_add(o + 1, m * m);
+        red_global_add(o + 2, m * m * m * m);
+    }
+    // the same from whole numbers, one group of moments (kGroups) at a time
+    __device__ static void add_group(double* o, int, const int32_t* M, double invN, double, int)
+    {
+        const double m = invN * (double)(unsigned)abs(M[0]), m2 = m * m;
+        red_global_add(o, m);
+        red_global_add(o + 1, m2);
+        red_global_add(o + 2, m2 * m2);
     }
     // CORRELATION_LENGTHS (ising2d_hamiltonian.hpp:246-252): G after the three moments
     __device__ static void add_correlators(double* o, const int8_t* sp, int, int L, const double* q, double in2)
     {
-        atomicAdd(o + 3, in2 * full_corr(sp, nullptr, q, L));
+        red_global_add(o + 3, in2 * full_corr(sp, nullptr, q, L));
     }
 };
 
@@ -140,6 +180,7 @@ struct Ising2dModel {
 struct AshkinTeller2dModel {
     static constexpr int kPlanes = 2;
     static constexpr int kMoments = 12;
+    static constexpr int kGroups = 2;
     static constexpr int kMags = 3;          // sigma, tau, Baxter
     static constexpr int kCorrPlanes = 2;    // sigma, sigma * tau
     __host__ __device__ static constexpr int corr_mag(int p) { return p == 0 ? 0 : 2; }
@@ -166,7 +207,7 @@ struct AshkinTeller2dModel {
     __device__ static void add_transforms(double* o, const double* G, double in2)
     {
         const double gs = in2 * G[0], gb = in2 * G[1];
-        atomicAdd(o + 3, gs); atomicAdd(o + 7, gs); atomicAdd(o + 11, gs + gs); atomicAdd(o + 15, gb);
+        red_global_add(o + 3, gs); red_global_add(o + 7, gs); red_global_add(o + 11, gs + gs); red_global_add(o + 15, gb);
     }
 
     __host__ __device__ static int64_t delta_at(const int8_t* a, const int8_t* b, int i, Neighbours n, Couplings c, int64_t h)
@@ -219,13 +260,29 @@ struct AshkinTeller2dModel {
         const double a = invN * fabs((double)M[0]), t = invN * fabs((double)M[1]), b = invN * fabs((double)M[2]);
         const double p2 = a * a + t * t;
         const int g = corr ? 1 : 0;
-        atomicAdd(o + 0, a); atomicAdd(o + 1, a * a); atomicAdd(o + 2, a * a * a * a);
+        red_global_add(o + 0, a); red_global_add(o + 1, a * a); red_global_add(o + 2, a * a * a * a);
         o += g;
-        atomicAdd(o + 3, t); atomicAdd(o + 4, t * t); atomicAdd(o + 5, t * t * t * t);
+        red_global_add(o + 3, t); red_global_add(o + 4, t * t); red_global_add(o + 5, t * t * t * t);
         o += g;
-        atomicAdd(o + 6, sqrt(p2)); atomicAdd(o + 7, p2); atomicAdd(o + 8, p2 * p2);
+        red_global_add(o + 6, sqrt(p2)); red_global_add(o + 7, p2); red_global_add(o + 8, p2 * p2);
         o += g;
-        atomicAdd(o + 9, b); atomicAdd(o + 10, b * b); atomicAdd(o + 11, b * b * b * b);
+        red_global_add(o + 9, b); red_global_add(o + 10, b * b); red_global_add(o + 11, b * b * b * b);
+    }
+    // The same from whole numbers, in two groups: sigma and tau, Baxter and phi.  FP64 bounds it (an
+    // instruction takes 32 cycles of an SM, its result 65), and CUDA's sqrt most of all (670 cycles):
+    // twelve instructions a group, the root included, which leave room for one another.
+    // Magnetisations are at most 128 x 128.
+    __device__ static void add_group(double* o, int group, const int32_t* M, double invN, double in2, int corr)
+    {
+        const int c = 3 + (corr ? 1 : 0);
+        const unsigned m = (unsigned)abs(group == 0 ? M[0] : M[2]);
+        const unsigned k = (unsigned)(M[1] * M[1]) + (group == 0 ? 0u : (unsigned)(M[0] * M[0]));
+        // (m is exact in single precision)
+        const double a = invN * float_double((float)m), b = invN * whole_root(k), a2 = a * a, b2 = in2 * whole_double(k);
+        double* const oa = o + (group == 0 ? 0 : 3 * c);
+        double* const ob = o + (group == 0 ? c : 2 * c);
+        red_global_add(oa, a); red_global_add(oa + 1, a2); red_global_add(oa + 2, a2 * a2);
+        red_global_add(ob, b); red_global_add(ob + 1, b2); red_global_add(ob + 2, b2 * b2);
     }
     // CORRELATION_LENGTHS (ashkin_teller2d_hamiltonian.hpp:295-315): the tau correlator is
     // computed from sigma as in the reference (:298-299); phi's is the sum of the two
@@ -233,6 +290,6 @@ struct AshkinTeller2dModel {
     {
         const double gs = in2 * full_corr(sp, nullptr, q, L);
         const double gb = in2 * full_corr(sp, sp + N, q, L);
-        atomicAdd(o + 3, gs); atomicAdd(o + 7, gs); atomicAdd(o + 11, gs + gs); atomicAdd(o + 15, gb);
+        red_global_add(o + 3, gs); red_global_add(o + 7, gs); red_global_add(o + 11, gs + gs); red_global_add(o + 15, gb);
     }
 };
