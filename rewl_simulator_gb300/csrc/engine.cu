@@ -41,6 +41,7 @@
 #include <fstream>
 #include <iomanip>
 #include <limits>
+#include <mutex>
 #include <new>
 #include <random>
 #include <sstream>
@@ -2252,6 +2253,74 @@ __global__ void __launch_bounds__(256) k_flat(const FlatParams fp)
     }
 }
 
+// What the host reads after a check interval, in one go.
+struct Report {
+    unsigned long long stats[2];   // exchanges attempted, accepted
+    int32_t counters[2];           // error word, flat events of the last check
+    int32_t windows_done;
+};
+
+// (one block) into host memory
+__global__ void k_report(DevPtrs P, int nwin, Report* out)
+{
+    __shared__ int done;
+    if (threadIdx.x == 0) done = 0;
+    __syncthreads();
+    int n = 0;
+    for (int w = threadIdx.x; w < nwin; w += blockDim.x) n += P.win_done[w];
+    if (n) atomicAdd(&done, n);
+    __syncthreads();
+    if (threadIdx.x == 0) *out = Report{{P.stats[0], P.stats[1]}, {P.counters[0], P.counters[1]}, done};
+}
+
+// Observable columns of a model, before the count column: Ising |m|, m^2, m^4 (+ G(q_min));
+// Ashkin-Teller 12 moments (+ a G(q_min) after each group of three).
+__host__ __device__ inline int obs_columns(int model, bool corr) { return model == REWL_MODEL_ISING2D ? (corr ? 4 : 3) : (corr ? 16 : 12); }
+__host__ __device__ inline bool is_corr_column(int model, bool corr, int k) { return corr && (model == REWL_MODEL_ISING2D ? k == 3 : (k & 3) == 3); }
+
+// Rows b0 .. b0 + rows - 1 of [nb][K + 1]: K averages and the update count, from the sums of slots
+// first .. first + count - 1, into host memory (a thread per entry).  Moments: sum over the slots /
+// total count (the count-weighted mean of the replicas' running means).  G(q_min): each slot's sum
+// over its transforms, ceil(count / 1000) of them, weighted by the slot's count in the same way.
+__global__ void k_export_observables(DevPtrs P, int model, int first, int count, int b0, int rows, double* out)
+{
+    const int K = obs_columns(model, P.corr != 0);
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)rows * (K + 1)) return;
+    const int b = b0 + (int)(i / (K + 1)), k = (int)(i % (K + 1));
+    const bool transform = is_corr_column(model, P.corr != 0, k);
+    double sum = 0.0;
+    unsigned long long cnt = 0;
+    for (int s = first; s < first + count; ++s) {
+        const int64_t o = P.slot_tab[s] + b;
+        const unsigned long long v = P.visits[o];
+        cnt += v;
+        if (k == K || (transform && !v)) continue;
+        const double x = P.obs[(size_t)o * P.obs_stride + k];
+        if (!transform) { sum = __dadd_rn(sum, x); continue; }
+        const double mean = x / (double)((v + kCountsPerTransform - 1) / kCountsPerTransform);
+        sum = __dadd_rn(sum, count == 1 ? mean : __dmul_rn((double)v, mean));
+    }
+    out[i] = k == K ? (double)cnt : !cnt ? 0.0 : (count == 1 && transform) ? sum : sum / (double)cnt;
+}
+
+// A window's logDoS, the replicas weighted by their visits, into host memory.
+__global__ void k_export_logdos(DevPtrs P, int first, int count, int b0, int rows, double* out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= rows) return;
+    const int b = b0 + i;
+    double total = 0.0, acc = 0.0;
+    for (int s = first; s < first + count; ++s) total = __dadd_rn(total, (double)P.visits[P.slot_tab[s] + b]);
+    if (total == 0.0 || count == 1) acc = (double)P.g[P.slot_tab[first] + b] / kLogdosScale;
+    else
+        for (int s = first; s < first + count; ++s) {
+            const int64_t o = P.slot_tab[s] + b;
+            acc = __dadd_rn(acc, __dmul_rn((double)P.visits[o] / total, (double)P.g[o] / kLogdosScale));
+        }
+    out[i] = acc;
+}
+
 __global__ void k_reset_window(DevPtrs P, int w, int reduce)
 {
     const WinDev W = P.win[w];
@@ -2420,8 +2489,16 @@ struct rewl_engine {
         g_events.clear();
     }
 
+    // pinned host memory that kernels write results to: a Report, then rows of an export
+    static constexpr size_t kReportBytes = 256, kExportBytes = 4u << 20;
+    char* pinned = nullptr;
+    size_t export_doubles = 0;
+    std::mutex export_mu;
+
     void release()
     {
+        if (pinned) cudaFreeHost(pinned);
+        pinned = nullptr;
         d_inst.free_(); d_win.free_();
         slot_inst.free_(); slot_win.free_(); slot_cfg.free_(); slot_nb.free_(); slot_flavour.free_();
         pairs[0].free_(); pairs[1].free_();
@@ -3009,19 +3086,68 @@ int leave_tree(rewl_engine* e, int ii)
     return REWL_OK;
 }
 
-int check_device_error(rewl_engine* e)
+int device_error(int word)
 {
-    int32_t h[4];
-    CUDA_TRY(cudaMemcpyAsync(h, e->counters.p, sizeof h, cudaMemcpyDeviceToHost, e->stream));
-    CUDA_TRY(cudaStreamSynchronize(e->stream));
-    if (h[0] & ERR_BOUNDS) return fail(REWL_EBOUNDS, "a walker's energy left its window (device error word %d)", h[0]);
-    if (h[0] & ERR_ADJUST) return fail(REWL_EINVAL, "a walker could not reach its window");
-    if (h[0] & ERR_REPLAY_EXHAUSTED) return fail(REWL_EINVAL, "replay uniform stream exhausted");
-    if (h[0] & ERR_RANGE)
+    if (word & ERR_BOUNDS) return fail(REWL_EBOUNDS, "a walker's energy left its window (device error word %d)", word);
+    if (word & ERR_ADJUST) return fail(REWL_EINVAL, "a walker could not reach its window");
+    if (word & ERR_REPLAY_EXHAUSTED) return fail(REWL_EINVAL, "replay uniform stream exhausted");
+    if (word & ERR_RANGE)
         return fail(REWL_ESTATE, "a window's logDoS passed 2^62 units (6.7e7 nats) without a flat event: "
                                  "a replica is trapped away from part of its window");
-    if (h[0] & ERR_COUNT)
+    if (word & ERR_COUNT)
         return fail(REWL_ESTATE, "a per-stage histogram count passed 2^32 - 1 without a flat event");
+    return REWL_OK;
+}
+
+// Waits for the stream and reads the device's counters.  One kernel that writes to pinned memory and
+// one wait; a copy to pageable memory is a wait of its own (a check interval ended with eight of them
+// and four waits: L = 8, 3 windows x 2 walkers, 2 x 20 sweeps, 285 -> 214 us an interval).
+int read_report(rewl_engine* e, Report* r)
+{
+    std::lock_guard<std::mutex> lock(e->export_mu);
+    k_report<<<1, 128, 0, e->stream>>>(e->ptrs(), e->nwin_total, reinterpret_cast<Report*>(e->pinned));
+    CUDA_TRY(cudaGetLastError());
+    CUDA_TRY(cudaStreamSynchronize(e->stream));
+    std::memcpy(r, e->pinned, sizeof *r);
+    return REWL_OK;
+}
+
+int check_device_error(rewl_engine* e)
+{
+    Report r;
+    if (int rc = read_report(e, &r)) return rc;
+    return device_error(r.counters[0]);
+}
+
+int alloc_pinned(rewl_engine* e)
+{
+    size_t most = 1;
+    for (int s = 0; s < e->nslots; ++s) {
+        const int width = e->desc.observables ? obs_columns(e->inst[e->h_slot_inst[s]].d.model, e->desc.observables == 2) + 1 : 1;
+        most = std::max(most, (size_t)e->h_slot_nb[s] * width);
+    }
+    e->export_doubles = std::max<size_t>(64, std::min(most, rewl_engine::kExportBytes / 8));
+    if (cudaHostAlloc(reinterpret_cast<void**>(&e->pinned), rewl_engine::kReportBytes + e->export_doubles * 8, cudaHostAllocDefault) != cudaSuccess) {
+        e->pinned = nullptr;
+        return fail(REWL_ENOMEM, "pinned host memory for exports");
+    }
+    return REWL_OK;
+}
+
+// [nb][width] doubles from a kernel that launch(first row, rows, destination) starts, through pinned memory
+template <class F>
+int export_rows(rewl_engine* e, int nb, int width, double* out, F launch)
+{
+    std::lock_guard<std::mutex> lock(e->export_mu);
+    double* staged = reinterpret_cast<double*>(e->pinned + rewl_engine::kReportBytes);
+    const int most = (int)(e->export_doubles / (size_t)width);
+    for (int b0 = 0; b0 < nb; b0 += most) {
+        const int rows = std::min(most, nb - b0);
+        launch(b0, rows, staged);
+        CUDA_TRY(cudaGetLastError());
+        CUDA_TRY(cudaStreamSynchronize(e->stream));
+        std::memcpy(out + (size_t)b0 * width, staged, (size_t)rows * width * 8);
+    }
     return REWL_OK;
 }
 
@@ -3321,6 +3447,7 @@ int rewl_create(const rewl_batch_desc* desc, rewl_engine** out)
         delete e; return fail(REWL_EDEVICE, "cannot open device %d", desc->device);
     }
     rc = upload_all(e);
+    if (!rc) rc = alloc_pinned(e);
     if (!rc) rc = plan_launches(e);
     if (!rc) {
         k_init<<<(e->nslots + 63) / 64, 64, 0, e->stream>>>(e->ptrs(), e->nslots, 0);
@@ -3563,15 +3690,35 @@ int rewl_exchange(rewl_engine* e)
 
 namespace {
 // After k_flat: the number of windows that went flat, and the device error word.
-int finish_check(rewl_engine* e, int32_t* num_flat)
+int finish_check(rewl_engine* e, Report* r)
 {
-    int32_t h[2];
-    CUDA_TRY(cudaMemcpyAsync(h, e->counters.p, sizeof h, cudaMemcpyDeviceToHost, e->stream));
-    CUDA_TRY(cudaStreamSynchronize(e->stream));
-    e->flat_events += h[1];
+    if (int rc = read_report(e, r)) return rc;
+    e->flat_events += r->counters[1];
     e->cycles++;
-    if (num_flat) *num_flat = h[1];
-    return check_device_error(e);
+    return device_error(r->counters[0]);
+}
+
+void fill_status(const rewl_engine* e, const Report& r, rewl_status* st)
+{
+    std::memset(st, 0, sizeof *st);
+    st->sweeps = e->sweeps_total;
+    st->cycles = e->cycles;
+    st->flat_events = e->flat_events;
+    st->windows_total = e->nwin_total;
+    st->windows_done = r.windows_done;
+    st->all_done = st->windows_done == st->windows_total;
+    st->exchanges_attempted = (int64_t)r.stats[0];
+    st->exchanges_accepted = (int64_t)r.stats[1];
+    st->attempted_flips = e->flips_total;
+    st->device_error = r.counters[0];
+    st->kernel_launches = e->launches_total;
+}
+
+int check_flat(rewl_engine* e, Report* r)
+{
+    CUDA_TRY(cudaMemsetAsync(e->counters.p + 1, 0, 4, e->stream));
+    if (int rc = launch_flat(e)) return rc;
+    return finish_check(e, r);
 }
 
 // Capture one check interval (rounds x (sweeps + exchange), then the flatness step) as a CUDA
@@ -3613,7 +3760,7 @@ int capture_cycle(rewl_engine* e)
 }
 
 // One check interval by replaying the captured graph.
-int replay_cycle(rewl_engine* e, int32_t* num_flat)
+int replay_cycle(rewl_engine* e, Report* r)
 {
     if (!e->cycle_exec)
         if (int rc = capture_cycle(e)) return rc;
@@ -3622,7 +3769,7 @@ int replay_cycle(rewl_engine* e, int32_t* num_flat)
     e->launches_total += e->g_launches; e->kernel_launches += e->g_kernel_launches;
     e->exch_round += (uint64_t)e->g_rounds;
     e->direction ^= (int)(e->g_rounds & 1);
-    int rc = finish_check(e, num_flat);     // synchronises the stream
+    int rc = finish_check(e, r);            // synchronises the stream
     for (size_t k = 0; k + 1 < e->g_events.size(); k += 2) {
         float t = 0;                        // timing only: a failed read leaves it out
         if (cudaEventElapsedTime(&t, e->g_events[k], e->g_events[k + 1]) == cudaSuccess) e->graph_sweep_ms += t;
@@ -3636,10 +3783,10 @@ int rewl_check_flat(rewl_engine* e, int32_t* num_flat)
 {
     if (!e) return fail(REWL_EINVAL, "null engine");
     cudaSetDevice(e->desc.device);
-    CUDA_TRY(cudaMemsetAsync(e->counters.p + 1, 0, 4, e->stream));
-    int rc = launch_flat(e);
-    if (rc) return rc;
-    return finish_check(e, num_flat);
+    Report r{};
+    const int rc = check_flat(e, &r);
+    if (num_flat) *num_flat = r.counters[1];
+    return rc;
 }
 
 int rewl_reset_histograms(rewl_engine* e, int32_t ii, int32_t w, int32_t reduce)
@@ -3657,25 +3804,9 @@ int rewl_get_status(rewl_engine* e, rewl_status* st)
 {
     if (!e || !st) return fail(REWL_EINVAL, "null argument");
     cudaSetDevice(e->desc.device);
-    std::vector<int32_t> done(e->nwin_total);
-    unsigned long long stats[2];
-    int32_t counters[4];
-    CUDA_TRY(cudaMemcpyAsync(done.data(), e->win_done.p, done.size() * 4, cudaMemcpyDeviceToHost, e->stream));
-    CUDA_TRY(cudaMemcpyAsync(stats, e->stats.p, sizeof stats, cudaMemcpyDeviceToHost, e->stream));
-    CUDA_TRY(cudaMemcpyAsync(counters, e->counters.p, sizeof counters, cudaMemcpyDeviceToHost, e->stream));
-    CUDA_TRY(cudaStreamSynchronize(e->stream));
-    std::memset(st, 0, sizeof *st);
-    st->sweeps = e->sweeps_total;
-    st->cycles = e->cycles;
-    st->flat_events = e->flat_events;
-    st->windows_total = e->nwin_total;
-    for (int d : done) st->windows_done += d;
-    st->all_done = st->windows_done == st->windows_total;
-    st->exchanges_attempted = (int64_t)stats[0];
-    st->exchanges_accepted = (int64_t)stats[1];
-    st->attempted_flips = e->flips_total;
-    st->device_error = counters[0];
-    st->kernel_launches = e->launches_total;
+    Report r;
+    if (int rc = read_report(e, &r)) return rc;
+    fill_status(e, r, st);
     return REWL_OK;
 }
 
@@ -3688,21 +3819,21 @@ int rewl_run_cycles(rewl_engine* e, int64_t ncycles, int64_t timeout_ms, rewl_st
     int rc = REWL_OK;
     if (e->desc.autotune && !e->tuned && (rc = rewl_autotune(e, 0))) return rc;
     for (int64_t c = 0; c < ncycles; ++c) {
-        int32_t nflat = 0;
+        Report report;
         // a whole check interval replays as one graph unless sweeps were run by hand since the
         // last check (the captured flatness step assumes exactly one interval of sweeps)
         const bool graph = e->desc.graphs && e->desc.rng_mode != REWL_RNG_REPLAY && e->sweeps_since_check == 0;
         if (graph) {
-            if ((rc = replay_cycle(e, &nflat))) return rc;
+            if ((rc = replay_cycle(e, &report))) return rc;
         } else {
             for (int r = 0; r < rounds; ++r) {
                 if ((rc = launch_sweeps(e, se))) return rc;
                 if ((rc = launch_exchange(e))) return rc;
             }
-            if ((rc = rewl_check_flat(e, &nflat))) return rc;
+            if ((rc = check_flat(e, &report))) return rc;
         }
         rewl_status s;
-        if ((rc = rewl_get_status(e, &s))) return rc;
+        fill_status(e, report, &s);
         if (st) *st = s;
         if (s.all_done) break;
         if (timeout_ms > 0) {
@@ -3710,55 +3841,21 @@ int rewl_run_cycles(rewl_engine* e, int64_t ncycles, int64_t timeout_ms, rewl_st
             if (ms > timeout_ms) return fail(REWL_ETIMEDOUT, "run_cycles deadline of %lld ms passed", (long long)timeout_ms);
         }
     }
-    if (st) return rewl_get_status(e, st);
+    if (st && ncycles == 0) return rewl_get_status(e, st);
     return REWL_OK;
 }
 
 namespace {
-// Observable columns of a model, before the count column: Ising |m|, m^2, m^4 (+ G(q_min));
-// Ashkin-Teller 12 moments (+ a G(q_min) after each group of three).
-int obs_columns(int model, bool corr) { return model == REWL_MODEL_ISING2D ? (corr ? 4 : 3) : (corr ? 16 : 12); }
-bool is_corr_column(int model, bool corr, int k) { return corr && (model == REWL_MODEL_ISING2D ? k == 3 : (k & 3) == 3); }
-
-// [nb][K + 1] rows of K averages and the update count, from the sums of the given slots.
-// Moments: sum over the slots / total count (the count-weighted mean of the replicas' running
-// means).  G(q_min): each slot's sum over its transforms, ceil(count / 1000) of them, weighted
-// by the slot's count in the same way.
-int export_obs(rewl_engine* e, int ii, const std::vector<int>& slots, double* out)
+// Observables of slots first .. first + count - 1 (k_export_observables): the sums stay on the device, only
+// the averages cross (L = 12, K + 1 = 17 columns of 8228 bins, 4 replicas: 4.3 MB and four waits, 660 us;
+// 1.1 MB and one, 146 us).
+int export_obs(rewl_engine* e, int ii, int first, int count, double* out)
 {
     if (!e->obs.p) return fail(REWL_ESTATE, "the engine was created without observables (rewl_batch_desc.observables)");
-    const int model = e->inst[ii].d.model;
-    const bool corr = e->desc.observables == 2;
-    const int K = obs_columns(model, corr);
-    const int nb = e->h_slot_nb[slots[0]];
-    const bool single = slots.size() == 1;
-    std::vector<double> sum((size_t)nb * K, 0.0), part((size_t)nb * e->obs_stride);
-    std::vector<uint64_t> cnt(nb, 0), v(nb);
-    for (int s : slots) {
-        const int64_t off = e->h_slot_tab[s];
-        CUDA_TRY(cudaMemcpyAsync(part.data(), e->obs.p + (size_t)off * e->obs_stride, part.size() * 8,
-                                 cudaMemcpyDeviceToHost, e->stream));
-        CUDA_TRY(cudaMemcpyAsync(v.data(), e->visits.p + off, nb * 8, cudaMemcpyDeviceToHost, e->stream));
-        CUDA_TRY(cudaStreamSynchronize(e->stream));
-        for (int b = 0; b < nb; ++b) {
-            for (int k = 0; k < K; ++k) {
-                const double x = part[(size_t)b * e->obs_stride + k];
-                if (!is_corr_column(model, corr, k)) { sum[(size_t)b * K + k] += x; continue; }
-                if (!v[b]) continue;
-                const double mean = x / (double)((v[b] + kCountsPerTransform - 1) / kCountsPerTransform);
-                sum[(size_t)b * K + k] += single ? mean : (double)v[b] * mean;
-            }
-            cnt[b] += v[b];
-        }
-    }
-    for (int b = 0; b < nb; ++b) {
-        for (int k = 0; k < K; ++k) {
-            const double x = sum[(size_t)b * K + k];
-            out[(size_t)b * (K + 1) + k] = !cnt[b] ? 0.0 : (single && is_corr_column(model, corr, k)) ? x : x / (double)cnt[b];
-        }
-        out[(size_t)b * (K + 1) + K] = (double)cnt[b];
-    }
-    return REWL_OK;
+    const int model = e->inst[ii].d.model, width = obs_columns(model, e->desc.observables == 2) + 1;
+    return export_rows(e, e->h_slot_nb[first], width, out, [&](int b0, int rows, double* to) {
+        k_export_observables<<<(unsigned)(((long long)rows * width + 127) / 128), 128, 0, e->stream>>>(e->ptrs(), model, first, count, b0, rows, to);
+    });
 }
 } // namespace
 
@@ -3766,7 +3863,7 @@ int rewl_export_observables(rewl_engine* e, int32_t w, double* out)
 {
     if (!valid_walker(e, w) || !out) return fail(REWL_EINVAL, "walker %d out of range or null output", w);
     cudaSetDevice(e->desc.device);
-    return export_obs(e, e->h_slot_inst[w], {w}, out);
+    return export_obs(e, e->h_slot_inst[w], w, 1, out);
 }
 
 int rewl_export_window_observables(rewl_engine* e, int32_t ii, int32_t w, double* out)
@@ -3774,9 +3871,7 @@ int rewl_export_window_observables(rewl_engine* e, int32_t ii, int32_t w, double
     if (window_index(e, ii, w) < 0 || !out) return fail(REWL_EINVAL, "bad window or null output");
     cudaSetDevice(e->desc.device);
     const InstDev& I = e->inst[ii].dev;
-    std::vector<int> slots;
-    for (int r = 0; r < I.R; ++r) slots.push_back(I.first_slot + w * I.R + r);
-    return export_obs(e, ii, slots, out);
+    return export_obs(e, ii, I.first_slot + w * I.R, I.R, out);
 }
 
 int rewl_export_walker(rewl_engine* e, int32_t w, int8_t* dofs, double* state, uint64_t* counts, double* logdos, uint64_t* visits)
@@ -3816,24 +3911,9 @@ int rewl_export_window_logdos(rewl_engine* e, int32_t ii, int32_t w, double* out
     if (wi < 0 || !out) return fail(REWL_EINVAL, "bad window or null output");
     cudaSetDevice(e->desc.device);
     const InstDev& I = e->inst[ii].dev;
-    const int nb = e->h_wins[wi].nb, R = I.R;
-    std::vector<int64_t> g((size_t)R * nb);
-    std::vector<uint64_t> v((size_t)R * nb);
-    for (int r = 0; r < R; ++r) {
-        const int s = I.first_slot + w * R + r;
-        CUDA_TRY(cudaMemcpyAsync(g.data() + (size_t)r * nb, e->g.p + e->h_slot_tab[s], nb * 8, cudaMemcpyDeviceToHost, e->stream));
-        CUDA_TRY(cudaMemcpyAsync(v.data() + (size_t)r * nb, e->visits.p + e->h_slot_tab[s], nb * 8, cudaMemcpyDeviceToHost, e->stream));
-    }
-    CUDA_TRY(cudaStreamSynchronize(e->stream));
-    for (int b = 0; b < nb; ++b) {
-        double tot = 0;
-        for (int r = 0; r < R; ++r) tot += (double)v[(size_t)r * nb + b];
-        double acc = 0;
-        if (tot == 0 || R == 1) acc = (double)g[b] / kLogdosScale;
-        else for (int r = 0; r < R; ++r) acc = acc + ((double)v[(size_t)r * nb + b] / tot) * ((double)g[(size_t)r * nb + b] / kLogdosScale);
-        out[b] = acc;
-    }
-    return REWL_OK;
+    return export_rows(e, e->h_wins[wi].nb, 1, out, [&](int b0, int rows, double* to) {
+        k_export_logdos<<<(rows + 127) / 128, 128, 0, e->stream>>>(e->ptrs(), I.first_slot + w * I.R, I.R, b0, rows, to);
+    });
 }
 
 int rewl_export_window_mask(rewl_engine* e, int32_t ii, int32_t w, uint8_t* out)
