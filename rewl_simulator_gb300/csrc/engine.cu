@@ -34,6 +34,7 @@
 #include <cmath>
 #include <cfloat>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
@@ -107,15 +108,20 @@ __device__ __forceinline__ bool engine_failed_warp(const int32_t* counters)
 // A launch's derived visits to bin k (its logDoS change over ln f) into the per-stage count
 // (uint32, the reference keeps uint64: a count that would pass 2^32 - 1 saturates and is
 // reported) and the cumulative visits; also checks the new logDoS against the range limit.
-__device__ __forceinline__ int commit_visits(uint32_t* gH, uint64_t* gv, int k, long long dv, long long gnew)
+__device__ __forceinline__ int commit_visits(uint32_t* gH, uint64_t* gv, int k, uint32_t h, uint64_t v, long long dv,
+                                             long long gnew)           // (h, v: what gH[k], gv[k] hold)
 {
     int err = 0;
-    const unsigned long long h = (unsigned long long)gH[k] + (unsigned long long)dv;
-    if (h > 0xFFFFFFFFull) { err |= ERR_COUNT; gH[k] = 0xFFFFFFFFu; }
-    else gH[k] = (uint32_t)h;
-    gv[k] += (uint64_t)dv;
+    const unsigned long long sum = (unsigned long long)h + (unsigned long long)dv;
+    if (sum > 0xFFFFFFFFull) err |= ERR_COUNT;
+    gH[k] = sum > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)sum;
+    gv[k] = v + (uint64_t)dv;
     if (gnew >= kLogdosLimit) err |= ERR_RANGE;
     return err;
+}
+__device__ __forceinline__ int commit_visits(uint32_t* gH, uint64_t* gv, int k, long long dv, long long gnew)
+{
+    return commit_visits(gH, gv, k, gH[k], gv[k], dv, gnew);
 }
 
 struct InstDev {
@@ -1343,15 +1349,19 @@ SweepKernel bins_kernel(int G, bool obs, bool cnt)
 // the part around the walker is held in shared memory (TableCache below).
 constexpr int kMinCache = 2048;
 
+// a Philox block gives four attempts' words, so that a warp draws 128 thresholds at a time (32 at a
+// time, one word a lane, was 700 cycles a chunk)
+constexpr int kTableRing = 256;
 struct TableStage {
-    longlong2 du[32 + 8];    // per site: {proposal, proposal after its left neighbour flipped in this chunk}
-    long long T[2][32 + 8];  // acceptance thresholds of two chunks' sites (the last block of a chunk reads past its sites)
+    longlong2 du[32 + 8];    // per site: {proposal, proposal after its left neighbour flipped in this chunk};
+                             // tree: 32-bit, {proposal, change of it when the left neighbour flips}
+    long long T[kTableRing]; // acceptance thresholds, by attempt modulo kTableRing (serial chain: the chunk's)
     long long wcu;           // row-wrap correction of the last site when the chunk is a whole row
     int seq[32];             // bin after each step (observables)
     unsigned sink;           // counts the lanes off the path, read by nobody
     unsigned pad[3];
 };
-static_assert(sizeof(TableStage) % 16 == 0, "what follows is 16-byte aligned");
+static_assert(offsetof(TableStage, T) % 16 == 0 && sizeof(TableStage) % 16 == 0, "what follows is 16-byte aligned");
 
 // Chain state of one Ashkin-Teller walker (lane 0).  The energy is carried as its
 // position v = (E - E_lo) * bin_mul - gblo << bin_shift, in units of the bin
@@ -1403,7 +1413,7 @@ __device__ __forceinline__ void serial_step(TableChain& c, const int j, TableSta
     const long long d = gn - c.gc;
     bool a;
     if (!replay) {
-        a = c.inr && d < st->T[0][j];
+        a = c.inr && d < st->T[j];
     } else if (c.inr && d > 0) {
         if (c.draws >= thr_n) { c.err = ERR_REPLAY_EXHAUSTED; a = false; }
         else { a = d < P.thr[thr_off + c.draws]; ++c.draws; }
@@ -1425,13 +1435,18 @@ __device__ __forceinline__ void serial_step(TableChain& c, const int j, TableSta
 
 // The same chunk decided five sites at a time on the binary tree of outcomes, as the bin-tracking
 // kernel does it (above), one walker per warp: lane q >= 1 is the node at level log2(q), lane 0 stands
-// for the walker's present bin.  Positions are bin numerators shifted so that the bin is the high word
-// of a 64-bit integer; the path's bins come from the ancestor lanes by shuffle.
+// for the walker's present bin.  Positions are 32-bit bin numerators relative to the bin the block
+// starts in, without the trailing binary zeros that all energy changes share (the bin multiplier's);
+// a node's is a sum of its path's changes, each times a lane constant 0 or 1 (integer multiply-adds,
+// which leave the ALU to the rest).  The path's bins come from the ancestor lanes by shuffle.
 struct TableTree {
     static constexpr int D = 5;
     int lvl, lvla;                         // level, level for the length check
     unsigned want, anc, path;              // ancestors' votes: needed value, mask; the decisions that lead here
     int up[D - 1];                         // the ancestor at each level (beyond the node's own: itself)
+    int took[D - 1], both[D - 1];          // 0/1: the decision at a level was to flip; so was the one before it
+    int own, ownx;                         // 0/1: there is a proposal (not in lane 0); its left neighbour flipped
+    int firstP;                            // 0/1: the proposal sees the flip of the block's left neighbour
     int dwell[D];                          // steps of the way here that end at the block's first bin, and at the
                                            // proposal accepted at each level
     bool first, last, leaf;                // first decision on the way here; the one before this node
@@ -1461,6 +1476,17 @@ struct TableTree {
         last = lvl > 0 && accepts(lvl - 1);
         if (q == 0) { anc = 1u; want = 1u; }                   // its vote is always 0: never on the path
         leaf = lvl == D - 1;
+#pragma unroll
+        for (int i = 0; i < D - 1; ++i) {
+            took[i] = accepts(i) ? 1 : 0;
+            both[i] = i > 0 && accepts(i) && accepts(i - 1) ? 1 : 0;
+            keep(took[i]);
+            keep(both[i]);
+        }
+        own = q == 0 ? 0 : 1;
+        ownx = own && last ? 1 : 0;
+        firstP = first || q == 1 ? 1 : 0;
+        keep(own); keep(ownx); keep(firstP);
         // lane constants: kept in registers, not worked out again in every block
         keep(want); keep(anc); keep(path); keep(lvl); keep(lvla);
 #pragma unroll
@@ -1492,23 +1518,50 @@ struct TableCache {
     {
         return (lo == 0 || b - margin >= lo) && (lo + size >= nb || b + margin < lo + size);
     }
+    // (kBatch bins of a lane at a time, their loads before their stores: a walker at high energies recentres
+    // once per 1700 flips: 51,000 cycles with one bin's loads and stores after another's, 15,000 so)
+    static constexpr int kBatch = 4;
     __device__ void fill(int first, int last, int lane)
     {
-        for (int b = first + lane; b < last; b += 32) {
-            const int k = b & (size - 1);
-            g[k] = b < nb ? gg[b] : 0;
-            n[k] = 0;
+        for (int b = first + lane; b < last; b += 32 * kBatch) {
+            long long x[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int k = b + 32 * i;
+                x[i] = k < min(last, nb) ? gg[k] : 0;
+            }
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int k = b + 32 * i;
+                if (k < last) {
+                    g[k & (size - 1)] = x[i];
+                    n[k & (size - 1)] = 0;
+                }
+            }
         }
     }
     __device__ void book(int first, int last, int lane)
     {
-        for (int b = first + lane; b < last; b += 32) {
-            const int k = b & (size - 1);
-            const unsigned v = n[k];
-            if (v == 0) continue;
-            const long long gnew = g[k] + (long long)v * lnf;
-            gg[b] = gnew;
-            err |= commit_visits(gH, gv, b, v, gnew);
+        for (int b = first + lane; b < last; b += 32 * kBatch) {
+            unsigned v[kBatch];
+            uint32_t h[kBatch];
+            uint64_t c[kBatch];
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int k = b + 32 * i;
+                v[i] = k < last ? n[k & (size - 1)] : 0u;
+                h[i] = v[i] ? gH[k] : 0u;
+                c[i] = v[i] ? gv[k] : 0u;
+            }
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int k = b + 32 * i;
+                if (v[i]) {
+                    const long long gnew = g[k & (size - 1)] + (long long)v[i] * lnf;
+                    gg[k] = gnew;
+                    err |= commit_visits(gH, gv, k, h[i], c[i], v[i], gnew);
+                }
+            }
         }
     }
     // around bin b (all lanes)
@@ -1533,11 +1586,12 @@ struct TableCache {
 // Ashkin-Teller, wang_landau.hpp:109-119), the flipped plane toggling after each pass.
 // The sweeps of one walker (launch position li; the warp's shared memory starts at warp_base).
 //
-// Bound: the latency of one block of five decisions (about 640 cycles at one warp per scheduler:
-// shared loads and shuffles of the bins, 64-bit positions, vote and reductions), once per five flips;
-// with many walkers per SM the 46 instructions per flip, and the cached bins that fit.  Ashkin-Teller
-// L = 32, bins of 0.05, 8 windows x 4 walkers: 32 walkers 178 -> 157 cycles per flip, 512 walkers 381
-// -> 195, 2048 walkers 772 -> 517 (from one dependent global load and store per flip).
+// Bound: the latency of one block of five decisions (about 400 cycles at one warp per scheduler:
+// shared loads and shuffles of the bins, vote and reductions, half of it instruction issue), once per five
+// flips, and about 900 cycles a chunk of energy changes, thresholds and loop; with many walkers per SM the
+// instructions and the cached bins that fit.  Ashkin-Teller L = 32, bins of 0.05, 8 windows x 4 walkers,
+// cycles per flip: 32 walkers 178 as a chain of dependent global loads and stores, 157 as a tree of 64-bit
+// positions with 32 thresholds a draw, 116 now; 512 walkers 381, 195, 138; 2048 walkers 772, 517, 381.
 template <class Model, bool TREE, bool OBS>
 __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const int li, unsigned char* warp_base)
 {
@@ -1596,10 +1650,15 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
     const long long eglo = I.eglo_u, mul = I.bin_mul;
     const int sh = I.bin_shift;
     const long long vlo = (long long)W.gblo << sh;     // window start in bin-numerator units
-    // couplings and fields in position units: the tree's positions have the bin in their high word
-    const int up = TREE ? 32 - sh : 0;
-    const Couplings cpl{(I.J_u * mul) << up, (I.K_u * mul) << up};
-    auto field = [&](int i) { return hf ? ((long long)hf[i] * mul) << up : 0ll; };
+    // couplings and fields in position units, for the tree without their common trailing zeros
+    using Pos = std::conditional_t<TREE, int, long long>;
+    // (the multiplier's, and one more: a flip changes the energy by an even number)
+    const int zm = TREE ? min(__ffsll(mul) - 1, sh) : 0, even = TREE && zm < sh ? 1 : 0;
+    const int zeros = zm + even, shz = sh - zeros;
+    const long long mulz = mul >> zm;
+    const CouplingsOf<Pos> cpl{(Pos)(I.J_u * mulz), (Pos)(I.K_u * mulz)};
+    auto field = [&](int i) { return hf ? (Pos)(hf[i] * mulz) : Pos(0); };
+    int2* const dx = reinterpret_cast<int2*>(st->du);
     const bool wraps = rc.n == 1;                      // a row is one chunk: its last site sees its first
     int flavour = NP == 1 ? 0 : P.slot_flavour[s];
 
@@ -1618,10 +1677,12 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
         c.gc = gg[c.b];
         if (replay) { c.draws = P.slot_draws[s]; thr_off = P.slot_thr_off[s]; thr_n = P.slot_thr_n[s]; }
     }
-    vr <<= up;
+    // the tree's position: bin, numerator within it in units of 2^zeros, and what is below them for good
+    int b0 = (int)(vr >> sh), fr = (int)((vr >> zeros) & ((1ll << shz) - 1));
+    const long long below = vr & ((1ll << zeros) - 1);
     if (TREE) {
         tab.lnf = lnf;
-        tab.lo = max(0, min((int)(vr >> 32) - tab.size / 2, nb - tab.size));
+        tab.lo = max(0, min(b0 - tab.size / 2, nb - tab.size));
         tab.fill(tab.lo, tab.lo + tab.size, lane);
     }
     const unsigned sink = (unsigned)__cvta_generic_to_shared(&st->sink);
@@ -1630,28 +1691,36 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
     const int lnf_lo = (int)(uint32_t)lnf, lnf_hi = (int)((lnf - (long long)(int)(uint32_t)lnf) >> 32);
     const uint64_t attempts0 = sweeps0 * (uint64_t)NP * (uint64_t)N;   // the launch's first attempt
     uint64_t attempt = attempts0;                      // of the current chunk
-    int tbuf = 0;
-    long long hnext = TREE ? field(min(lane, N - 1)) : 0;      // field of the chunk's site
-    auto draw = [&](uint64_t from, int len, int buf) { // thresholds of the len attempts from `from` on
-        if (lane < len) st->T[buf][lane] = word_threshold(philox_word(seed, uid, from + (uint64_t)lane, kStreamWL));
+    Pos hnext = TREE ? field(min(lane, N - 1)) : Pos(0);      // field of the chunk's site
+    uint64_t drawn = attempts0 >> 2;                   // next Philox block
+    int ready = -(int)(attempts0 & 3);                 // thresholds in the ring from the current chunk on
+    auto draw = [&] {
+        const uint64_t blk = drawn + (uint64_t)lane;
+        const Philox4 r = philox4x32_10(Philox4{(uint32_t)blk, (uint32_t)(blk >> 32), kStreamWL, 0u}, (uint32_t)seed ^ uid,
+                                        (uint32_t)(seed >> 32));
+        longlong2* t = reinterpret_cast<longlong2*>(st->T + (((uint32_t)blk * 4u) & (kTableRing - 1)));
+        t[0] = make_longlong2(word_threshold(r.x), word_threshold(r.y));
+        t[1] = make_longlong2(word_threshold(r.z), word_threshold(r.w));
+        drawn += 32;
+        ready += 128;
     };
-    if (TREE) draw(attempt, rc.len(0), 0);
+    if (TREE) draw();
 
-    struct Node { long long rC, rP, x0, T; };          // position and proposal relative to the block's start
+    struct Node { int rC, rP, x0; long long T; };      // position and proposal relative to the block's start
     auto node = [&](int j0) {
-        const char* d = reinterpret_cast<const char*>(st->du + j0);
-        auto at = [&](int i, bool left) { return *reinterpret_cast<const long long*>(d + 16 * i + (left ? 8 : 0)); };
+        const int2* d = dx + j0;
         Node n;
-        n.x0 = at(0, true) - at(0, false);
-        n.rC = tree.accepts(0) ? at(0, false) : 0;
+        const int2 d0 = d[0];
+        n.x0 = d0.y;
+        n.rC = tree.took[0] * d0.x;
 #pragma unroll
         for (int i = 1; i < D - 1; ++i) {
-            const long long v = at(i, tree.accepts(i - 1));
-            n.rC += tree.accepts(i) ? v : 0;
+            const int2 v = d[i];
+            n.rC += tree.took[i] * v.x + tree.both[i] * v.y;
         }
-        const long long v = at(tree.lvl, tree.last);
-        n.rP = n.rC + (lane == 0 ? 0 : v);
-        n.T = st->T[tbuf][j0 + tree.lvl];
+        const int2 v = d[tree.lvl];
+        n.rP = n.rC + tree.own * v.x + tree.ownx * v.y;
+        n.T = st->T[((uint32_t)attempt + (uint32_t)(j0 + tree.lvl)) & (kTableRing - 1)];
         return n;
     };
 
@@ -1662,26 +1731,27 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
             const int8_t* B = NP == 1 ? A : sp + (plane ^ 1) * N;
             for (int ch = 0, cc = 0, y = 0, c0 = 0, C = rc.len(0); ch < L * rc.n; ++ch) {
                 const int x0 = c0 - y * L;
-                if (TREE) {
-                    const int b = (int)(vr >> 32);
-                    if (!tab.within(b, tab.size / 8)) tab.centre(b, lane);
-                }
+                if (TREE && !tab.within(b0, tab.size / 8)) tab.centre(b0, lane);
                 int ai = 0, sg[NM], far = 0;
                 for (int m = 0; m < NM; ++m) sg[m] = 0;
-                const long long h = hnext;             // (read while the chunk before it was decided)
+                const Pos h = hnext;                   // (read while the chunk before it was decided)
                 if (lane < C) {
                     const int i = c0 + lane, x = x0 + lane;
                     const Neighbours nbr{y == 0 ? i + (L - 1) * L : i - L, x == 0 ? i + L - 1 : i - 1,
                                          x == L - 1 ? i - (L - 1) : i + 1, y == L - 1 ? i - (L - 1) * L : i + L};
                     ai = A[i];
                     Model::flip_signs(ai, B[i], plane, sg);
-                    const long long d0 = Model::delta_at(A, B, i, nbr, cpl, TREE ? h : field(i));
-                    const long long d1 = lane > 0 ? d0 + Model::flipped_at(A, B, i, nbr.left, cpl) : d0;
-                    const longlong2 d = make_longlong2(d0, d1);
-                    st->du[lane] = d;
-                    if (TREE) far = max(abs((int)(d.x >> 32)), abs((int)(d.y >> 32))) + 1;
-                    if (wraps && lane == C - 1) st->wcu = Model::flipped_at(A, B, i, nbr.right, cpl);
-                    if (!TREE && !replay) st->T[0][lane] = word_threshold(philox_word(seed, uid, attempt + (uint64_t)lane, kStreamWL));
+                    const Pos d0 = Model::delta_at(A, B, i, nbr, cpl, TREE ? h : field(i));
+                    const Pos dl = lane > 0 ? Model::flipped_at(A, B, i, nbr.left, cpl) : Pos(0);
+                    if constexpr (TREE) {
+                        const int2 d = make_int2(d0 >> even, dl >> even);
+                        dx[lane] = d;
+                        far = (max(abs(d.x), abs(d.x + d.y)) >> shz) + 1;
+                    } else {
+                        st->du[lane] = make_longlong2(d0, d0 + dl);
+                    }
+                    if (wraps && lane == C - 1) st->wcu = Model::flipped_at(A, B, i, nbr.right, cpl) >> even;
+                    if (!TREE && !replay) st->T[lane] = word_threshold(philox_word(seed, uid, attempt + (uint64_t)lane, kStreamWL));
                 }
                 // bins a block's nodes can lie away from its start: five steps (and a row's wrap term, part of
                 // an energy change as large)
@@ -1713,15 +1783,20 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
                     }
                     acc = __shfl_sync(kFull, c.acc, 0);
                 } else {
-                    int flipped = 0;                   // the block's left neighbour flipped just before it
+                    // first bins from which a block stays among the cached ones (none: a span of 0 far away)
+                    int near0 = tab.lo == 0 ? 0 : tab.lo + reach;
+                    const int near1 = tab.lo + tab.size >= nb ? nb - 1 : tab.lo + tab.size - 1 - reach;
+                    const unsigned nears = near1 >= near0 ? (unsigned)(near1 - near0) : 0u;
+                    if (near1 < near0) near0 = nb;
+                    int flipped = 0;                   // all ones: the block's left neighbour flipped just before it
                     // one block of nlev sites from the chunk's site j0, `ahead` the work that does not wait for
                     // it.  NEAR: every bin its lanes can name is cached.
-                    auto block = [&](auto near, const Node& n, int nlev, int j0, long long wC, long long wP, auto ahead) {
+                    auto block = [&](auto near, const Node& n, int nlev, int j0, int wC, int wP, auto ahead) {
                         constexpr bool NEAR = decltype(near)::value;
-                        const long long sC = flipped && tree.first ? n.x0 : 0;
-                        const long long sP = flipped && (tree.first || lane == 1) ? n.x0 : 0;
-                        const long long vC = vr + (n.rC + sC + wC), vP = vr + (n.rP + sP + wP);
-                        const int bP = (int)(vP >> 32), bC = (int)(vC >> 32);
+                        const int x0 = flipped & n.x0;
+                        const int vC = tree.took[0] * x0 + (fr + n.rC + wC), vP = tree.firstP * x0 + (fr + n.rP + wP);
+                        const int oC = vC >> shz, oP = vP >> shz;          // bins from the block's first one
+                        const int bC = b0 + oC, bP = b0 + oP;
                         const int kP = bP & (tab.size - 1), kC = bC & (tab.size - 1);
                         long long gP = tab.g[kP], gC = tab.g[kC];
                         int cP = (int)tab.n[kP], cC = (int)tab.n[kC];
@@ -1733,25 +1808,23 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
                         }
                         // visits to this node's two bins on the way here: its path stays `dwell` steps at the
                         // block's first bin and at every accepted proposal
-                        const int b0 = (int)(vr >> 32);
-                        int nC = b0 == bC ? tree.dwell[0] : 0, nP = b0 == bP ? tree.dwell[0] : 0;
+                        int nC = oC == 0 ? tree.dwell[0] : 0, nP = oP == 0 ? tree.dwell[0] : 0;
 #pragma unroll
                         for (int i = 0; i < D - 1; ++i) {
-                            const int b = __shfl_sync(kFull, bP, tree.up[i]);
-                            nC += b == bC ? tree.dwell[i + 1] : 0;
-                            nP += b == bP ? tree.dwell[i + 1] : 0;
+                            const int o = __shfl_sync(kFull, oP, tree.up[i]);
+                            nC += o == oC ? tree.dwell[i + 1] : 0;
+                            nP += o == oP ? tree.dwell[i + 1] : 0;
                         }
                         const bool live = tree.lvla < nlev;
                         const long long bound = mad_units(gC + n.T, (cC + nC) - (cP + nP), lnf_lo, lnf_hi);
                         const bool a = (gP < bound) & live & inr;
                         const unsigned vote = __ballot_sync(kFull, a);
                         const bool on = ((vote ^ tree.want) & tree.anc) == 0;
-                        const long long v = a ? vP : vC;
+                        const unsigned v = (unsigned)(a ? vP : vC) ^ 0x80000000u;      // (in order as unsigned)
                         const bool mine = on && live, end = on && tree.leaf;
                         const int bin = a ? bP : bC;
                         // the last node of the path has the walker's position and the block's decisions
-                        const unsigned lo = __reduce_max_sync(kFull, end ? (unsigned)(unsigned long long)v : 0u);
-                        const unsigned hi = __reduce_max_sync(kFull, end ? (unsigned)bin : 0u);
+                        const int to = (int)(__reduce_max_sync(kFull, end ? v : 0u) ^ 0x80000000u);
                         const unsigned path = __reduce_max_sync(kFull, end ? tree.path | (a ? 1u << (D - 1) : 0u) : 0u);
                         if (OBS && mine) st->seq[j0 + tree.lvl] = bin;
                         if (!NEAR && __any_sync(kFull, mine && !tab.holds(bin))) {
@@ -1773,12 +1846,13 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
                         }
                         ahead();
                         __syncwarp();
-                        vr = (long long)(((unsigned long long)hi << 32) | lo);
+                        b0 += to >> shz;
+                        fr = to & ((1 << shz) - 1);
                         acc |= path << j0;
-                        flipped = (int)(path >> (nlev - 1)) & 1;
+                        flipped = -((int)(path >> (nlev - 1)) & 1);
                     };
-                    auto decide = [&](const Node& n, int nlev, int j0, long long wC, long long wP, auto ahead) {
-                        if (tab.within((int)(vr >> 32), reach)) block(std::true_type{}, n, nlev, j0, wC, wP, ahead);
+                    auto decide = [&](const Node& n, int nlev, int j0, int wC, int wP, auto ahead) {
+                        if ((unsigned)(b0 - near0) <= nears) block(std::true_type{}, n, nlev, j0, wC, wP, ahead);
                         else block(std::false_type{}, n, nlev, j0, wC, wP, ahead);
                     };
                     Node n = node(0);
@@ -1789,15 +1863,16 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
                         n = next;
                     }
                     // the chunk's last block; where the chunk is a row, its last site sees the first one's flip
-                    long long wC = 0, wP = 0;
+                    int wC = 0, wP = 0;
                     if (wraps) {
                         const int li = C - 1 - j0;
-                        const long long t = (j0 > 0 ? (acc & 1u) != 0 : tree.first) ? st->wcu : 0;
+                        const int t = (j0 > 0 ? (acc & 1u) != 0 : tree.first) ? (int)st->wcu : 0;
                         if (tree.lvla == li) wP = t;           // (not the idle lane)
                         else if (tree.accepts(li)) wC = wP = t;
                     }
                     decide(n, C - j0, j0, wC, wP, [&] {
-                        draw(attempt + (uint64_t)C, Cn, tbuf ^ 1);
+                        if (ready < C + Cn) draw();
+                        ready -= C;
                         hnext = field(min((ch + 1 == L * rc.n ? 0 : c0 + C) + lane, N - 1));
                     });
                 }
@@ -1877,7 +1952,6 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
                     for (int m = 0; m < NM; ++m) M[m] += total[m];
                 __syncwarp();
                 attempt += (uint64_t)C;
-                tbuf ^= 1;
                 c0 += C;
                 cc = cn; y = yn; C = Cn;
             }
@@ -1904,8 +1978,7 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
     }
     if (tab.err) atomicOr(&P.counters[0], tab.err);
     if (lane == 0) {
-        if (!TREE) vr = c.v;
-        vr >>= up;
+        vr = TREE ? ((long long)b0 << sh) + ((long long)fr << zeros) + below : c.v;
         P.cfg_E[cfg] = eglo + (vr + vlo) / mul;
         for (int m = 0; m < NM; ++m) P.cfg_M[3 * cfg + m] = M[m];
         P.slot_sweeps[s] = sweeps0 + (uint64_t)p.nsweeps;
@@ -2826,15 +2899,20 @@ bool bins_eligible(const InstDev& I, const rewl_batch_desc& D, int max_window_bi
     return true;
 }
 
-// The global-table kernel's tree keeps the bin in the high word of a position and adds up to six
-// energy changes: bins of at most 2^32 numerator units, and no single flip across 2^26 bins.
+// The global-table kernel's tree adds up to five energy changes to a position within a bin in 32 bits,
+// in numerator units without the zeros that all changes end in (three changes more leave room for the
+// terms on the way): bins of 0.05 take single flips of up to 100 energy units, bins of 1 of up to 500.
+// Beyond that, the serial chain.
 int tree_eligible(const HostInst& H, const rewl_batch_desc& D)
 {
-    if (D.rng_mode != REWL_RNG_PHILOX || H.dev.bin_shift > 32) return 0;
+    if (D.rng_mode != REWL_RNG_PHILOX) return 0;
+    int zeros = 0;
+    while (zeros < H.dev.bin_shift && (H.dev.bin_mul >> zeros & 1) == 0) ++zeros;
     double h = 0;
     for (double f : H.fields) h = std::max(h, std::fabs(f));
     const double move = 2.0 * (4.0 * std::fabs((double)H.dev.J_u) + 4.0 * std::fabs((double)H.dev.K_u) + std::ldexp(h, H.dev.escale));
-    return move * (double)H.dev.bin_mul < std::ldexp(1.0, 26 + H.dev.bin_shift) ? 1 : 0;
+    const int even = zeros < H.dev.bin_shift ? 1 : 0;
+    return 8.0 * std::ldexp(move, -even) * (double)(H.dev.bin_mul >> zeros) + std::ldexp(1.0, H.dev.bin_shift - zeros - even) < 2147483648.0 ? 1 : 0;
 }
 
 // Streaming multiprocessors of the engine's device (152 on a GB300).

@@ -70,9 +70,13 @@ __device__ inline double whole_root(unsigned k)
     return fma(fma(-x, x, kd), half, x);
 }
 
-struct Couplings {
-    int64_t J, K;            // nearest-neighbour and four-spin couplings in energy units
+// nearest-neighbour and four-spin couplings in energy units (T: 64 bits, or 32 where the caller knows
+// that four times their sum fits)
+template <class T>
+struct CouplingsOf {
+    T J, K;
 };
+using Couplings = CouplingsOf<int64_t>;
 
 // Fourier_Correlator::compute_correlator (src/Hamiltonians/Correlations/fourier_correlator.hpp:
 // 65-118) of plane a, or of the product plane a * b, in the reference's order (one thread):
@@ -110,14 +114,16 @@ struct Ising2dModel {
     __host__ __device__ static void mag_terms(const int8_t* sp, int, int i, int* t) { t[0] = sp[i]; }
     __device__ static void add_transforms(double* o, const double* G, double in2) { red_global_add(o + 3, in2 * G[0]); }
 
-    __host__ __device__ static int64_t delta_at(const int8_t* a, const int8_t*, int i, Neighbours n, Couplings c, int64_t)
+    template <class T>
+    __host__ __device__ static T delta_at(const int8_t* a, const int8_t*, int i, Neighbours n, CouplingsOf<T> c, T)
     {
         const int sum = a[n.up] + a[n.left] + a[n.right] + a[n.down];
-        return 2 * (int64_t)a[i] * c.J * sum;
+        return 2 * (T)a[i] * c.J * sum;
     }
-    __host__ __device__ static int64_t flipped_at(const int8_t* a, const int8_t*, int i, int j, Couplings c)
+    template <class T>
+    __host__ __device__ static T flipped_at(const int8_t* a, const int8_t*, int i, int j, CouplingsOf<T> c)
     {
-        return -4 * (int64_t)a[i] * a[j] * c.J;
+        return -4 * (T)a[i] * a[j] * c.J;
     }
     __host__ __device__ static int64_t delta_energy(const int8_t* a, const int8_t* b, int i, int L, Couplings c, int64_t h)
     {
@@ -210,16 +216,18 @@ struct AshkinTeller2dModel {
         red_global_add(o + 3, gs); red_global_add(o + 7, gs); red_global_add(o + 11, gs + gs); red_global_add(o + 15, gb);
     }
 
-    __host__ __device__ static int64_t delta_at(const int8_t* a, const int8_t* b, int i, Neighbours n, Couplings c, int64_t h)
+    template <class T>
+    __host__ __device__ static T delta_at(const int8_t* a, const int8_t* b, int i, Neighbours n, CouplingsOf<T> c, T h)
     {
         const int u = n.up, l = n.left, r = n.right, d = n.down;
         const int sa = a[u] + a[l] + a[r] + a[d];
         const int sab = a[u] * b[u] + a[l] * b[l] + a[r] * b[r] + a[d] * b[d];
-        return 2 * (int64_t)a[i] * (h * b[i] + c.J * sa + c.K * (int64_t)b[i] * sab);
+        return 2 * (T)a[i] * (h * b[i] + c.J * sa + c.K * (T)b[i] * sab);
     }
-    __host__ __device__ static int64_t flipped_at(const int8_t* a, const int8_t* b, int i, int j, Couplings c)
+    template <class T>
+    __host__ __device__ static T flipped_at(const int8_t* a, const int8_t* b, int i, int j, CouplingsOf<T> c)
     {
-        return -4 * (int64_t)a[i] * a[j] * (c.J + c.K * (int64_t)b[i] * b[j]);
+        return -4 * (T)a[i] * a[j] * (c.J + c.K * (T)b[i] * b[j]);
     }
     __host__ __device__ static int64_t delta_energy(const int8_t* a, const int8_t* b, int i, int L, Couplings c, int64_t h)
     {
