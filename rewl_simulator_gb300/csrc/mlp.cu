@@ -90,6 +90,28 @@ __device__ __forceinline__ float dgelu_f(float dy, float z)
     return __bfloat162float(__float2bfloat16_rn(dy)) * (cdf + z * pdf);
 }
 
+// Kernels of a chain are launched with programmatic dependence (launch_next): the next one's blocks
+// may start, and set themselves up, while this one's finish.  It waits for all of its predecessor's
+// results -- and so, the predecessor having waited likewise, for everything before -- before its first
+// access to global memory.  A GEMM lets the next one start once its own results are on their way: a
+// training step of 4096 rows, hidden 256 x 4, takes 103 us so, 106 without that, 111 where the next may
+// start before the epilogue, 131 from the start (blocks that wait take the side streams' room), and 113
+// with no programmatic dependence at all.
+__device__ __forceinline__ void step_ready() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void step_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... Params, class... Args>
+cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, int block, size_t smem, cudaStream_t st, Args... args)
+{
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 __device__ __forceinline__ void ldsm_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* p)
 {
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
@@ -339,6 +361,7 @@ __global__ void __launch_bounds__(tc::THREADS) k_gemm_tc(const GemmArgs g, const
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tslot;
+    step_wait();                                         // the operands, and what the outputs replace
 
     constexpr int S = tc::STAGES;
     constexpr uint32_t kId = tc::idesc(A_KM, !B_NK);
@@ -449,6 +472,7 @@ __global__ void __launch_bounds__(tc::THREADS) k_gemm_tc(const GemmArgs g, const
             }
         }
     }
+    step_ready();
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     if (warp == 0) {
@@ -502,7 +526,7 @@ bool use_tcgen05()
 }
 
 template <bool A_KM, bool B_NK, int EPI>
-cudaError_t launch_gemm(cudaStream_t st, const GemmArgs& g, int splits)
+cudaError_t launch_gemm(cudaStream_t st, const GemmArgs& g, int splits, bool next)
 {
     if (use_tcgen05()) {
         static_assert(tc::BN == kBN, "tile widths agree");
@@ -512,7 +536,9 @@ cudaError_t launch_gemm(cudaStream_t st, const GemmArgs& g, int splits)
         const bool ok = (A_KM ? encode_operand(&ma, g.A, g.M, g.K, g.lda, tc::BK) : encode_operand(&ma, g.A, g.K, g.M, g.lda, tc::BM)) &&
                         (B_NK ? encode_operand(&mb, g.B, g.K, g.N, g.ldb, tc::BN) : encode_operand(&mb, g.B, g.N, g.K, g.ldb, tc::BK));
         if (!ok) return cudaErrorInvalidValue;
-        k_gemm_tc<A_KM, B_NK, EPI><<<dim3(g.N / tc::BN, (g.M + tc::BM - 1) / tc::BM, splits), tc::THREADS, tc::SMEM_BYTES, st>>>(g, ma, mb);
+        const dim3 grid(g.N / tc::BN, (g.M + tc::BM - 1) / tc::BM, splits);
+        if (next) return launch_next(k_gemm_tc<A_KM, B_NK, EPI>, grid, tc::THREADS, tc::SMEM_BYTES, st, g, ma, mb);
+        k_gemm_tc<A_KM, B_NK, EPI><<<grid, tc::THREADS, tc::SMEM_BYTES, st>>>(g, ma, mb);
     } else {
         k_gemm<A_KM, B_NK, EPI><<<dim3(g.N / kBN, g.M / kBM, splits), 128, 0, st>>>(g);
     }
@@ -552,14 +578,29 @@ int take_tc_error()
 constexpr int kColChunk = 256;                                 // rows per column-sum partial
 
 // column sums over chunks of kColChunk rows: part[chunk][n] = sum_{b in chunk} G[b][n]
+// (B a multiple of kColBatch, N even; two columns a thread).  The rows are added in order, but kColBatch of them are on their way
+// at a time: bound by that latency, a step of 4096 rows
+// took 125 us with a row at a time (its bias gradients longer than the chain beside them), 113 so.
+constexpr int kColBatch = 32;                                  // divides kBM, and with it every batch
+static_assert(kBM % kColBatch == 0 && kColChunk % kColBatch == 0, "whole batches of rows");
 __global__ void k_colsum(const bf16* G, int B, int N, float* part)
 {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b0 = blockIdx.y * kColChunk;
+    const int n = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
+    const int b0 = blockIdx.y * kColChunk, b1 = min(b0 + kColChunk, B);
     if (n >= N) return;
-    float s = 0.f;
-    for (int b = b0; b < b0 + kColChunk && b < B; ++b) s += __bfloat162float(G[(size_t)b * N + n]);
-    part[(size_t)blockIdx.y * N + n] = s;
+    float s0 = 0.f, s1 = 0.f;
+    for (int b = b0; b < b1; b += kColBatch) {
+        __nv_bfloat162 x[kColBatch];
+#pragma unroll
+        for (int i = 0; i < kColBatch; ++i)
+            x[i] = *reinterpret_cast<const __nv_bfloat162*>(G + (size_t)(b + i) * N + n);
+#pragma unroll
+        for (int i = 0; i < kColBatch; ++i) {
+            s0 += __low2float(x[i]);
+            s1 += __high2float(x[i]);
+        }
+    }
+    *reinterpret_cast<float2*>(part + (size_t)blockIdx.y * N + n) = make_float2(s0, s1);
 }
 
 // dst[i] = sum_p parts[p * stride + i], p in order: gradients are reproducible run to run
@@ -582,14 +623,20 @@ int weight_splits(int B)
 }
 
 // loss gradient of the mean squared error mean((out[:,0] - y)^2); each row's share of the loss
-// goes to rows[b] (summed in a fixed order by k_loss_sum)
+// goes to rows[b] (summed in a fixed order by k_loss_sum).  Eight threads a row, 16 bytes each.
+constexpr int kRowThreads = kOut / 8;
 __global__ void k_loss_grad(const float* out, const float* y, int B, bf16* dOut, float* rows)
 {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    step_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, b = i / kRowThreads, c = i % kRowThreads;
     if (b >= B) return;
-    const float e = out[(size_t)b * kOut] - y[b];
-    for (int c = 0; c < kOut; ++c) dOut[(size_t)b * kOut + c] = __float2bfloat16_rn(c == 0 ? 2.0f * e / (float)B : 0.f);
-    rows[b] = e * e / (float)B;
+    uint4 v = make_uint4(0, 0, 0, 0);                          // the padding's gradients
+    if (c == 0) {
+        const float e = out[(size_t)b * kOut] - y[b];
+        v.x = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(2.0f * e / (float)B));
+        rows[b] = e * e / (float)B;
+    }
+    *reinterpret_cast<uint4*>(dOut + (size_t)b * kOut + 8 * c) = v;
 }
 
 // loss = sum of rows[0..B): one block of 256 threads, strided partial sums, then a fixed tree
@@ -613,17 +660,26 @@ __global__ void __launch_bounds__(256) k_loss_sum(const float* rows, int B, floa
 struct TrainCursor {
     unsigned long long step;
     int k;
-    int pad;
+    unsigned done;                 // k_adam's blocks that are through with this step
 };
 
 // Adam with the bias corrections of the cursor's step (c1 = 1 - b1^t, c2 = 1 - b2^t, computed on
 // the host for every step of the call, two floats per step).
 __global__ void k_adam(float* p, float* m, float* v, const float* grad, const float* mask, bf16* pb, size_t n,
-                       float lr, float b1, float b2, float eps, const float* ctab, const TrainCursor* cur)
+                       float lr, float b1, float b2, float eps, const float* ctab, TrainCursor* cur, const float* loss,
+                       float* losses)
 {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
     const int k = cur->k;
+    // the end of a training step, by the last block to have read the cursor: keep its loss, advance
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&cur->done, 1u) == gridDim.x - 1) {
+        losses[k] = *loss;
+        cur->step += 1;
+        cur->k = k + 1;
+        cur->done = 0;
+    }
+    if (i >= n) return;
     const float c1 = ctab[2 * k], c2 = ctab[2 * k + 1];
     const float gi = grad[i] * mask[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -638,22 +694,15 @@ __global__ void k_adam(float* p, float* m, float* v, const float* grad, const fl
 __global__ void k_gather(const bf16* X, const float* y, int n, bf16* Xb, float* yb, int B, uint64_t seed,
                          const TrainCursor* cur)
 {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    static_assert(kIn / 8 == kRowThreads, "16 bytes a thread");
+    step_wait();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, b = t / kRowThreads, c = 8 * (t % kRowThreads);
     if (b >= B) return;
     const uint64_t step = cur->step;
     const uint32_t w = rewl::philox_word(seed, 0x4D4C5000u, step * (uint64_t)B + (uint64_t)b, 0x4D4C5001u);
     const int i = (int)rewl::mulhi32(w, (uint32_t)n);
-    for (int c = 0; c < kIn; c += 8)
-        *reinterpret_cast<uint4*>(Xb + (size_t)b * kIn + c) = *reinterpret_cast<const uint4*>(X + (size_t)i * kIn + c);
-    yb[b] = y[i];
-}
-
-// End of a training step: keep its loss, advance the cursor.
-__global__ void k_train_advance(TrainCursor* cur, const float* loss, float* losses)
-{
-    losses[cur->k] = *loss;
-    cur->step += 1;
-    cur->k += 1;
+    *reinterpret_cast<uint4*>(Xb + (size_t)b * kIn + c) = *reinterpret_cast<const uint4*>(X + (size_t)i * kIn + c);
+    if (c == 0) yb[b] = y[i];
 }
 
 template <typename T>
@@ -794,7 +843,7 @@ int gemm(rewl_mlp* m, cudaStream_t st, const bf16* A, const bf16* B, int M, int 
     if (M % kBM || N % kBN || K % (kBK * splits)) return mfail(REWL_EINVAL, "gemm shape %d x %d x %d (split %d)", M, N, K, splits);
     GemmArgs g{A, B, M, N, K, lda, ldb, K / splits, Cf, Cb, ldc, bias, Z};
     m->launches++;
-    MCUDA((launch_gemm<A_KM, B_NK, EPI>(st, g, splits)));
+    MCUDA((launch_gemm<A_KM, B_NK, EPI>(st, g, splits, st == m->stream)));
     return REWL_OK;
 }
 
@@ -838,7 +887,7 @@ int bias_grad(rewl_mlp* m, cudaStream_t st, int l, const bf16* G, int B)
 {
     const int N = m->dout[l], chunks = (int)bias_chunks(B);
     float* part = m->Bpart.p;
-    k_colsum<<<dim3((N + 127) / 128, chunks), 128, 0, st>>>(G, B, N, part);
+    k_colsum<<<dim3((N + 63) / 64, chunks), 32, 0, st>>>(G, B, N, part);
     k_sum_parts<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(part, chunks, (size_t)N, (size_t)N, m->Gr.p + m->boff[l]);
     m->launches += 2;
     MCUDA(cudaGetLastError());
@@ -846,16 +895,16 @@ int bias_grad(rewl_mlp* m, cudaStream_t st, int l, const bf16* G, int B)
 }
 
 // backward of the mean squared error on m->yb; every gradient entry is written once into Gr
-// (zeroed here, so that padding entries stay zero).  The layer gradients are a chain of L products
+// (the gaps between its blocks are zero from the start).  The layer gradients are a chain of L products
 // on the network's stream; a layer's weight and bias gradients need only its own link of it and
 // run on the side streams, which the chain waits for at its end.  A launch fills the GPU for a few
 // microseconds at most, so a step is bound by the number of launches that wait on one another:
-// 4096 rows, hidden 256 x 4: 30 launches in a row, 217 us a step; 14 in a row, 136 us.
+// 4096 rows, hidden 256 x 4: 30 launches in a row, 217 us a step; 14 in a row, 125 us; the chain with
+// programmatic dependence and shorter side work 103 us.
 int backward(rewl_mlp* m, int B)
 {
     const int L = m->layers;
-    MCUDA(cudaMemsetAsync(m->Gr.p, 0, m->nparams * sizeof(float), m->stream));
-    k_loss_grad<<<(B + 127) / 128, 128, 0, m->stream>>>(m->out.p, m->yb.p, B, m->dOut.p, m->lossrow.p);
+    MCUDA(launch_next(k_loss_grad, dim3((B * kRowThreads + 127) / 128), 128, 0, m->stream, m->out.p, m->yb.p, B, m->dOut.p, m->lossrow.p));
     m->launches++;
     // gradients of layer l from A (its outputs' gradient), once event `ev` says that A is there
     auto side_work = [&](int l, const bf16* A, cudaEvent_t ev) -> int {
@@ -906,6 +955,7 @@ __global__ void k_stage(const float* X, int n, int in_dim, int rows, bf16* H0)
 // the first column of the padded outputs; NaN while a GEMM's bounded wait has run out
 __global__ void k_take(const float* out, int n, float* y)
 {
+    step_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool timed_out = *reinterpret_cast<const volatile int*>(&g_tc_error) != 0;
     if (i < n) y[i] = timed_out ? __int_as_float(0x7FC00000) : out[(size_t)i * kOut];
@@ -913,7 +963,8 @@ __global__ void k_take(const float* out, int n, float* y)
 
 // the caller's n rows as they are to the device, and from there into rows x kIn bf16: the copy is
 // of in_dim floats a row, not of a row padded on the host (predicting 7900 rows, 7 features:
-// 224 us with padding on the host and all kOut columns back, 117 us with k_stage and k_take)
+// 224 us with padding on the host and all kOut columns back, 117 us with k_stage and k_take, 94 with
+// programmatic dependence and the status in k_take)
 int upload_features(rewl_mlp* m, const float* X, int n, int in_dim, int rows, bf16* dst)
 {
     const size_t need = (size_t)n * in_dim;
@@ -1050,12 +1101,11 @@ int rewl_mlp_predict(rewl_mlp* m, const float* X, int32_t n, int32_t in_dim, flo
     if ((rc = upload_features(m, X, n, in_dim, Bp, m->H[0].p)) || (rc = forward(m, Bp, false))) return rc;
     // the last hidden layer's buffer is read by now: the first column goes there, n floats to the host
     float* first = reinterpret_cast<float*>(m->H[m->layers].p);
-    k_take<<<(unsigned)((n + 255) / 256), 256, 0, m->stream>>>(m->out.p, n, first);
-    MCUDA(cudaGetLastError());
+    MCUDA(launch_next(k_take, dim3((n + 255) / 256), 256, 0, m->stream, m->out.p, n, first));
     m->launches++;
     MCUDA(cudaMemcpyAsync(y, first, (size_t)n * 4, cudaMemcpyDeviceToHost, m->stream));
     MCUDA(cudaStreamSynchronize(m->stream));
-    return take_tc_error();
+    return y[0] == y[0] ? REWL_OK : take_tc_error();       // (NaN everywhere while the flag stands)
 }
 
 // One forward + backward on the given rows (no update); gradients readable with
@@ -1114,7 +1164,7 @@ int rewl_mlp_train(rewl_mlp* m, int32_t steps, int32_t batch, float lr, float* l
         ct[2 * s] = 1.f - std::pow(b1, t);
         ct[2 * s + 1] = 1.f - std::pow(b2, t);
     }
-    const TrainCursor c0{(unsigned long long)m->step, 0, 0};
+    const TrainCursor c0{(unsigned long long)m->step, 0, 0u};
     MCUDA(cudaMemcpyAsync(m->ctab.p, ct.data(), ct.size() * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     MCUDA(cudaMemcpyAsync(m->cursor.p, &c0, sizeof c0, cudaMemcpyHostToDevice, m->stream));
     MCUDA(cudaStreamSynchronize(m->stream));       // the host copies above leave scope
@@ -1123,16 +1173,15 @@ int rewl_mlp_train(rewl_mlp* m, int32_t steps, int32_t batch, float lr, float* l
     // a CUDA graph and replayed `steps` times (about 30 launches a step, launch-bound otherwise)
     const int64_t l0 = m->launches;
     auto enqueue_step = [&]() -> int {
-        k_gather<<<(batch + 127) / 128, 128, 0, m->stream>>>(m->Xall.p, m->yall.p, m->nall, m->H[0].p, m->yb.p, batch,
+        k_gather<<<(batch * kRowThreads + 127) / 128, 128, 0, m->stream>>>(m->Xall.p, m->yall.p, m->nall, m->H[0].p, m->yb.p, batch,
                                                              m->seed, m->cursor.p);
         m->launches++;
         int r;
         if ((r = forward(m, batch, true)) || (r = backward(m, batch))) return r;
         k_adam<<<(unsigned)((m->nparams + 255) / 256), 256, 0, m->stream>>>(m->P.p, m->Mm.p, m->Vm.p, m->Gr.p, m->Mask.p,
                                                                             m->Pb.p, m->nparams, lr, b1, b2, eps,
-                                                                            m->ctab.p, m->cursor.p);
-        k_train_advance<<<1, 1, 0, m->stream>>>(m->cursor.p, m->loss.p, m->lossv.p);
-        m->launches += 2;
+                                                                            m->ctab.p, m->cursor.p, m->loss.p, m->lossv.p);
+        m->launches++;
         MCUDA(cudaGetLastError());
         return REWL_OK;
     };
@@ -1235,7 +1284,7 @@ cudaError_t noalloc_layer(cudaStream_t st, const bf16* A, const bf16* W, int M, 
                           const float* bias)
 {
     const GemmArgs g{A, W, M, N, K, K, K, K, Cf, Cb, N, bias, nullptr};
-    return launch_gemm<false, true, EPI>(st, g, 1);
+    return launch_gemm<false, true, EPI>(st, g, 1, false);         // (the caller's stream, perhaps under capture)
 }
 
 int predict_noalloc_on_device(rewl_mlp* m, const float* X, int32_t n, int32_t in_dim, float* y, void* stream);
