@@ -737,10 +737,19 @@ __device__ __forceinline__ long long mad_units(long long acc, int n, int f_lo, i
     return r;
 }
 
-// adds 1 (v) to the 32-bit word at shared address `addr`
+// a b + c on the multiply-add pipe, whatever a and b are: the integer ALU is the busier one
+__device__ __forceinline__ unsigned mad32(unsigned a, unsigned b, unsigned c)
+{
+    unsigned r;
+    asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+
+// adds 1 (v) to the 32-bit word at shared address `addr` (+ OFFSET)
+template <int OFFSET = 0>
 __device__ __forceinline__ void red_shared_inc(unsigned addr)
 {
-    asm volatile("red.shared.add.u32 [%0], 1;" :: "r"(addr) : "memory");
+    asm volatile("red.shared.add.u32 [%0 + %1], 1;" :: "r"(addr), "n"(OFFSET) : "memory");
 }
 __device__ __forceinline__ void red_shared_add(unsigned addr, int v)
 {
@@ -949,6 +958,16 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
     int pathc = 0;
     for (int i = 0; i < lvl; ++i)
         if ((q >> (lvl - 1 - i)) & 1) pathc |= 1 << (20 + i);
+    const unsigned pathP = (unsigned)pathc + (0x80000000u | 1u << (20 + D - 1));
+    // Sums on the multiply-add pipe and fewer of them where one walker has the warp: its instructions
+    // wait for the integer ALU (L = 64, 55.1 -> 54.0 cycles per flip).  Several walkers' warps take turns
+    // and do better with the plain sums (125.5 against 128.1), as do observables (117.0, 117.6).
+    constexpr bool kMad = G == 1 && !OBS;
+    unsigned one = 1;                                          // (not to be folded)
+    if (kMad) asm volatile("" : "+r"(one));
+    auto mad = [&](unsigned a, unsigned b, unsigned c) { return kMad ? mad32(a, b, c) : a * b + c; };
+    auto sum = [&](unsigned a, unsigned b) { return kMad ? mad32(a, one, b) : a + b; };
+    const unsigned tboff = (unsigned)(reinterpret_cast<char*>(Tb) - sm);
 
     // thresholds of P Philox blocks (four attempts each) from block `blk` on into the ring
     auto draw = [&](uint64_t blk) {
@@ -1032,19 +1051,21 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
             const uint2 v = *reinterpret_cast<const uint2*>(slot);
             f.e0 = v.x; f.e1 = 0u; f.x0 = v.y; f.x1 = 0u;
         }
-        f.t = Tb[(attempt + (uint32_t)lvl) & (RING - 1)];
+        if (kMad) f.t = lds64(sm, (int)sum(mad(attempt, 8u, (unsigned)(8 * lvl)) & (8 * RING - 1), tboff));
+        else f.t = Tb[(attempt + (uint32_t)lvl) & (RING - 1)];
         return f;
     };
     auto node = [&](const Slot& f) {
-        const unsigned S = ((f.e0 & mA) + (f.x0 & mB)) * 0x01010101u + K;        // positions after each step, + 16
+        const unsigned S = kMad ? mad32(f.e0 & mA, 0x01010101u, mad32(f.x0 & mB, 0x01010101u, K))   // positions after each step, + 16
+                                : ((f.e0 & mA) + (f.x0 & mB)) * 0x01010101u + K;
         const unsigned cb = __byte_perm(S, 0x10u, selC);
         const unsigned pb = cb + __byte_perm(f.e0, f.e1, selE) + __byte_perm(f.x0, f.x1, selX);
         Node n;
         n.rC = (int)cb * q8 + kC;
         n.rP = (int)pb * q8 + kP;
         n.x0 = ((int)(f.x0 & 0xFFu) - 1) * q8;
-        n.nC = __popc(~((S ^ (cb * 0x01010101u)) + 0x7F7F7F7Fu) & L80);          // steps of the path that ended here
-        n.nP = __popc(~((S ^ (pb * 0x01010101u + KP)) + 0x7F7F7F7Fu) & L80);
+        n.nC = __popc(~sum(S ^ (cb * 0x01010101u), 0x7F7F7F7Fu) & L80);         // steps of the path that ended here
+        n.nP = __popc(~sum(S ^ (pb * 0x01010101u + KP), 0x7F7F7F7Fu) & L80);
         n.t = f.t;
         return n;
     };
@@ -1074,9 +1095,10 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
         const bool a = gP < mad_units(gC + n.t, dn, lnf_lo, lnf_hi) && live;
         const unsigned B = __ballot_sync(kFull, a) >> gbase;
         const bool on = ((B ^ want) & anc) == 0;
-        const unsigned vC = (unsigned)(aC + pathc), vP = (unsigned)(aP + pathc) + (0x80000000u | 1u << (20 + D - 1));
-        unsigned v = a ? vP : vC;
         const int fin = a ? aP : aC;
+        constexpr unsigned kFlip = 0x80000000u | 1u << (20 + D - 1);       // the node's own decision
+        unsigned v = kMad ? (unsigned)fin + (a ? pathP : (unsigned)pathc)
+                          : a ? (unsigned)(aP + pathc) + kFlip : (unsigned)(aC + pathc);
         if (G <= 2) {
             v = on && leaf ? v : 0u;
             if (G == 1) v = __reduce_max_sync(kFull, v);
@@ -1091,7 +1113,8 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
         if (OBS && on && live) seqb[j0 + lvl] = fin;
         if (CNT) {
             // lanes off the path count in a word nobody reads (a predicated reduction costs a branch)
-            red_shared_inc(smbase + (unsigned)(on && live ? fin + 8 : sink));
+            if (kMad) red_shared_inc<8>(smbase + (unsigned)(on && live ? fin : sink - 8));
+            else red_shared_inc(smbase + (unsigned)(on && live ? fin + 8 : sink));
         } else {
             const int vis = (a ? n.nP : n.nC) + 1;
             const long long gn = mad_units(a ? gP : gC, vis, lnf_lo, lnf_hi);
