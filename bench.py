@@ -56,10 +56,11 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 METRIC = "time to ln g within 1e-2 of exact, MLP warm-start vs plain WL, 1 GB300; flips/s"
-# Cycles per attempted flip of one walker's accept chain at the speed of light of the
-# bin-tracking kernel's design, from probe kernels on a GB300: a dependent shared-memory load
-# (29 cycles) plus a 64-bit compare and select (11 cycles).
-CHAIN_FLOOR_CYCLES = 40.0
+# Cycles per attempted flip of one walker at the speed of light of the sweep kernels' design, a
+# block of five decisions at a time, from probe kernels on a GB300: a dependent shared-memory load
+# of 16 bytes (33 cycles), a vote (12), a maximum over the warp (26) and fifteen dependent integer
+# instructions (4.5 each).
+CHAIN_FLOOR_CYCLES = 28.0
 
 
 def _ising_workload(name, L, nwin, R, se, sc, lnf_final, one_over_t, init_mode, profile):
@@ -905,12 +906,12 @@ def run_gpu(args):
     roofline = {"bound": WORKLOAD["bound"], "kernel": WORKLOAD["kernel"], "avg_launch_ms": avg_launch_ms,
                 "flips_per_launch": flips_per_launch, "launch_shapes": shapes}
     if WORKLOAD["model"] != "mixed":
-        # the serial accept chain of one walker: cycles per attempted flip against the design's floor
+        # one walker's blocks of decisions: cycles per attempted flip against the design's floor
         walker_flips = WORKLOAD["sweeps_per_exchange"] * ndof(WORKLOAD)
         cycles = avg_launch_ms * 1e-3 * sm_mhz * 1e6 / walker_flips
-        kind = "chain floor: dependent shared load (29) + 64-bit compare/select (11), measured on a GB300"
+        kind = "block floor: shared load (33) + vote (12) + warp maximum (26) + 15 dependent integer instructions (68) per five flips, measured on a GB300"
         if WORKLOAD["model"] != "ising2d":
-            kind += "; this kernel's dependent loads come from L1/L2 (tables of tens of thousands of bins)"
+            kind += "; this kernel holds only the bins around each walker in shared memory (tables of tens of thousands of bins)"
         roofline.update({"unit": "cycles/flip", "achieved": cycles, "peak": CHAIN_FLOOR_CYCLES,
                          "frac": CHAIN_FLOOR_CYCLES / cycles, "walkers_per_warp": int(shapes[0][2]) if shapes else 1,
                          "peak_kind": kind,

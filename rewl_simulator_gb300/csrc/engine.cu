@@ -16,14 +16,20 @@
 // Kernels
 //   k_init          one thread per walker: initial spins from Philox, then the
 //                   deterministic walk into the window (rewl_walker.hpp:79-115)
+//   k_sweep_ising_bins  one, two or four walkers per warp; lattice, window table and
+//                   thresholds in shared memory; several sites decided at a time on
+//                   a binary tree of outcomes (the default Ising kernel)
 //   k_sweep_ising   one warp per walker; lattice, g and H staged in shared
 //                   memory; lanes precompute a row-aligned chunk of <= 32 sites
 //                   (energy change with and without the left neighbour flipped,
 //                   integer acceptance threshold), lane 0 resolves the serial
-//                   Wang-Landau chain in integer arithmetic only
-//   k_sweep_tables  the same for any model type of models.cuh with the tables in
-//                   global memory (Ashkin-Teller: one plane per pass; Ising windows
-//                   too large for shared memory)
+//                   Wang-Landau chain in integer arithmetic only (replay, bin
+//                   widths that do not divide 4J)
+//   k_sweep_tables  any model type of models.cuh with the tables in global memory
+//                   (Ashkin-Teller: one plane per pass; Ising windows too large for
+//                   shared memory): the tree, with the bins around the walker in
+//                   shared memory, or the serial chain
+//   k_export_*, k_report  results and counters into pinned host memory
 //   k_exchange      one thread per window pair (rewl_simulation.hpp:228-346)
 //   k_flat          one block per window: flatness vote, FP64 count-weighted
 //                   averaging, histogram reset, REDUCE_LOGDOS, ln f schedule
@@ -797,6 +803,13 @@ __host__ __device__ inline int bins_smem(int nbcap, int L, bool obs, bool corr, 
            2 * BinsTree<G>::kBlocks * BinsTree<G>::kSlot + 16 + (obs ? 32 * 4 : 0) + (corr ? 8 * L + 4 * nbcap : 0) + (acc ? 4 * kObsWords * nbcap : 0);
 }
 
+// Bound: a warp alone on its scheduler by the latency of a block (about 265 cycles per five decisions:
+// shared loads, vote, warp maximum and the integer instructions between them; 23 instructions per
+// flip), several by instruction issue (16 per flip with two walkers each, the ALU 77 % busy on the
+// busiest scheduler).  Measured against one decision after another: L = 64, 512 walkers 70 -> 58
+// cycles per flip, 3072 walkers 4.62 -> 4.70e10 flips/s; L = 20, 32 walkers, whose rows had no chunk of
+// eight, 376 -> 71.
+//
 // The sweeps of one warp's G walkers (launch position warp_index; its shared memory starts at
 // warp_base, one region of p.smem_per_warp bytes per walker).
 template <int G, bool OBS, bool CNT>
@@ -960,8 +973,8 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
         if ((q >> (lvl - 1 - i)) & 1) pathc |= 1 << (20 + i);
     const unsigned pathP = (unsigned)pathc + (0x80000000u | 1u << (20 + D - 1));
     // Sums on the multiply-add pipe and fewer of them where one walker has the warp: its instructions
-    // wait for the integer ALU (L = 64, 55.1 -> 54.0 cycles per flip).  Several walkers' warps take turns
-    // and do better with the plain sums (125.5 against 128.1), as do observables (117.0, 117.6).
+    // wait for the integer ALU (L = 64, 59.4 -> 58.1 cycles per flip).  Several walkers' warps take turns
+    // and do better with the plain sums (135 against 138), as do observables (126.1, 126.8).
     constexpr bool kMad = G == 1 && !OBS;
     unsigned one = 1;                                          // (not to be folded)
     if (kMad) asm volatile("" : "+r"(one));
@@ -1613,8 +1626,10 @@ struct TableCache {
 // shared loads and shuffles of the bins, vote and reductions, half of it instruction issue), once per five
 // flips, and about 900 cycles a chunk of energy changes, thresholds and loop; with many walkers per SM the
 // instructions and the cached bins that fit.  Ashkin-Teller L = 32, bins of 0.05, 8 windows x 4 walkers,
-// cycles per flip: 32 walkers 178 as a chain of dependent global loads and stores, 157 as a tree of 64-bit
-// positions with 32 thresholds a draw, 116 now; 512 walkers 381, 195, 138; 2048 walkers 772, 517, 381.
+// cycles per flip from flat tables: 32 walkers 192 as a chain of dependent global loads and stores, 169 as a
+// tree of 64-bit positions with 32 thresholds a draw, 122 now; 512 walkers 411, 210, 149; 2048 walkers 832,
+// 557, 411 (with the tables of a longer run 432, the chain 439: two waves of seven warps per SM, each with
+// its cached bins).
 template <class Model, bool TREE, bool OBS>
 __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const int li, unsigned char* warp_base)
 {
@@ -2949,7 +2964,7 @@ int sm_count(const rewl_engine* e)
 // The serial chain reads the tables in global memory through L1, so its shared-memory carveout is
 // the smallest that still holds the blocks resident on an SM (the CUDA runtime's default split leaves
 // L1 far less); the tree keeps the walkers' surroundings in shared memory and takes all of it (with a
-// carveout just large enough, 512 walkers at L = 24 ran in two waves: 388 against 205 cycles per flip).
+// carveout just large enough, 512 walkers at L = 24 ran in two waves: 418 against 221 cycles per flip).
 int at_carveout(rewl_engine* e, Launch& l)
 {
     if (!l.tables) return REWL_OK;
@@ -3071,9 +3086,9 @@ int plan_launches(rewl_engine* e)
             int G = e->desc.persistent ? 1 : e->desc.walkers_per_warp;
             if (G == 0) {
                 // one walker per warp while the SM sub-partitions outnumber the walkers
-                // (the chain is latency-bound); two per warp beyond that (measured at L = 64: two
-                // per warp beat four from 2048 to 4096 walkers, 3.77e10 against 3.43e10 flips/s at
-                // 3072); four only for still larger batches
+                // (a block is latency-bound); two per warp beyond that (measured at L = 64, 3072 walkers,
+                // one / two / four per warp: 3.13 / 4.70 / 4.47e10 flips/s; 512 walkers 1.82 / 1.38e10);
+                // four only for still larger batches
                 G = n <= 4 * nsm ? 1 : (n <= 32 * nsm ? 2 : 4);
             }
             l.nbcap = (maxnb + 1) & ~1;
@@ -3113,8 +3128,8 @@ int plan_launches(rewl_engine* e)
                 const int fixed = (int)(sizeof(TableStage) + ((planes * maxN + 15) & ~15) + (corr ? (8 * planes * maxL + 15) & ~15 : 0));
                 // as much of every walker's table as the walkers sharing an SM leave room for, but no less than
                 // 2048 bins (the rest of the walkers then wait for a second wave): Ashkin-Teller L = 32 at bins
-                // of 0.05, 2048 walkers, 512 / 1024 / 2048 / 4096 bins 5.5 / 5.8 / 7.6 / 5.6e9 flips/s; 512
-                // walkers, 1024 / 2048 / 4096 / 8192 bins 3.0 / 4.1 / 5.1 / 3.1e9
+                // of 0.05, 2048 walkers, 512 / 1024 / 2048 bins 7.1 / 7.8 / 10.3e9 flips/s from flat tables and
+                // 7.1 / 7.6 / 9.6e9 in a longer run
                 const int per_sm = e->desc.persistent ? 8 : std::max(1, std::min(32, (e->nslots + nsm - 1) / nsm));
                 l.cache = l.tree ? 256 : 0;
                 while (l.cache && l.cache < maxnb && fixed + 24 * l.cache <= 200 * 1024 &&
