@@ -1384,6 +1384,7 @@ SweepKernel bins_kernel(int G, bool obs, bool cnt)
 // after each pass.  A window holds tens of thousands of bins, so its logDoS stays in global memory;
 // the part around the walker is held in shared memory (TableCache below).
 constexpr int kMinCache = 2048;
+constexpr int kTableReach = 512;           // serial chain: bins on either side prefetched per chunk
 
 // a Philox block gives four attempts' words, so that a warp draws 128 thresholds at a time (32 at a
 // time, one word a lane, was 700 cycles a chunk)
@@ -1391,13 +1392,14 @@ constexpr int kTableRing = 256;
 struct TableStage {
     longlong2 du[32 + 8];    // per site: {proposal, proposal after its left neighbour flipped in this chunk};
                              // tree: 32-bit, {proposal, change of it when the left neighbour flips}
-    long long T[kTableRing]; // acceptance thresholds, by attempt modulo kTableRing (serial chain: the chunk's)
     long long wcu;           // row-wrap correction of the last site when the chunk is a whole row
     int seq[32];             // bin after each step (observables)
     unsigned sink;           // counts the lanes off the path, read by nobody
-    unsigned pad[3];
+    unsigned pad[5];
+    long long T[kTableRing]; // acceptance thresholds, by attempt modulo kTableRing (serial chain: the chunk's 32)
 };
-static_assert(offsetof(TableStage, T) % 16 == 0 && sizeof(TableStage) % 16 == 0, "what follows is 16-byte aligned");
+constexpr int kSerialStage = offsetof(TableStage, T) + 32 * 8;         // what the serial chain has of it
+static_assert(kSerialStage % 16 == 0 && offsetof(TableStage, T) % 16 == 0 && sizeof(TableStage) % 16 == 0, "what follows is 16-byte aligned");
 
 // Chain state of one Ashkin-Teller walker (lane 0).  The energy is carried as its
 // position v = (E - E_lo) * bin_mul - gblo << bin_shift, in units of the bin
@@ -1648,7 +1650,7 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
     unsigned char* base = smem + (int)(warp_base - smem);
     const bool replay = !TREE && p.replay;
     TableStage* st = reinterpret_cast<TableStage*>(base);
-    int8_t* sp = reinterpret_cast<int8_t*>(st + 1);       // NP planes of N spins
+    int8_t* sp = reinterpret_cast<int8_t*>(base) + (TREE ? (int)sizeof(TableStage) : kSerialStage);     // NP planes of N spins
     const int64_t* hf = I.field_off >= 0 ? P.fields + I.field_off : nullptr;
 
     const int cfg = P.slot_cfg[s];
@@ -1769,7 +1771,17 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
             const int8_t* B = NP == 1 ? A : sp + (plane ^ 1) * N;
             for (int ch = 0, cc = 0, y = 0, c0 = 0, C = rc.len(0); ch < L * rc.n; ++ch) {
                 const int x0 = c0 - y * L;
-                if (TREE && !tab.within(b0, tab.size / 8)) tab.centre(b0, lane);
+                if (TREE) {
+                    if (!tab.within(b0, tab.size / 8)) tab.centre(b0, lane);
+                } else {
+                    // the lines of g within kTableReach bins of the walker's bin into L1 (the chunk's proposals
+                    // mostly fall there), one line per lane per 512 bins
+                    const int bcur = __shfl_sync(kFull, c.b, 0);
+                    for (int k = lane * 16 - kTableReach; k <= kTableReach; k += 32 * 16) {
+                        const int bb = bcur + k;
+                        if ((unsigned)bb < (unsigned)nb) asm volatile("prefetch.global.L1 [%0];" ::"l"(gg + bb));
+                    }
+                }
                 int ai = 0, sg[NM], far = 0;
                 for (int m = 0; m < NM; ++m) sg[m] = 0;
                 const Pos h = hnext;                   // (read while the chunk before it was decided)
@@ -3125,13 +3137,17 @@ int plan_launches(rewl_engine* e)
             } else {
                 const int planes = l.model == REWL_MODEL_ISING2D ? 1 : 2;
                 l.nbcap = 0;
-                const int fixed = (int)(sizeof(TableStage) + ((planes * maxN + 15) & ~15) + (corr ? (8 * planes * maxL + 15) & ~15 : 0));
+                // With observables and more walkers than one wave with that many bins holds, the serial chain:
+                // the moments' FP64 latency wants warps more than the tree (L = 32, moments, 1024 / 1536 / 2048
+                // walkers: tree 5.8 / 4.7 / 5.9, chain 4.5 / 5.9 / 6.6e9 flips/s)
+                const bool crowded = e->desc.observables && !e->desc.persistent && e->nslots > 7 * nsm;
+                l.cache = l.tree && !crowded ? 256 : 0;
+                const int fixed = (int)((l.cache ? sizeof(TableStage) : kSerialStage) + ((planes * maxN + 15) & ~15) + (corr ? (8 * planes * maxL + 15) & ~15 : 0));
                 // as much of every walker's table as the walkers sharing an SM leave room for, but no less than
                 // 2048 bins (the rest of the walkers then wait for a second wave): Ashkin-Teller L = 32 at bins
                 // of 0.05, 2048 walkers, 512 / 1024 / 2048 bins 7.1 / 7.8 / 10.3e9 flips/s from flat tables and
                 // 7.1 / 7.6 / 9.6e9 in a longer run
                 const int per_sm = e->desc.persistent ? 8 : std::max(1, std::min(32, (e->nslots + nsm - 1) / nsm));
-                l.cache = l.tree ? 256 : 0;
                 while (l.cache && l.cache < maxnb && fixed + 24 * l.cache <= 200 * 1024 &&
                        (l.cache < kMinCache || fixed + 24 * l.cache + 1040 <= 225 * 1024 / per_sm))
                     l.cache *= 2;
@@ -3141,7 +3157,7 @@ int plan_launches(rewl_engine* e)
         if (!l.bins) {
             l.smem_per_warp = (l.smem_per_warp + 15) & ~15;
             int wpb = e->desc.warps_per_block;
-            if (wpb == 0) wpb = l.tables || n <= nsm * 2 ? 1 : n <= nsm * 8 ? 2 : 4;
+            if (wpb == 0) wpb = (l.tables && l.cache) || n <= nsm * 2 ? 1 : n <= nsm * 8 ? 2 : 4;
             while (wpb > 1 && (size_t)wpb * l.smem_per_warp > 200 * 1024) wpb >>= 1;
             if ((size_t)l.smem_per_warp > 220 * 1024) return fail(REWL_EINVAL, "a walker needs %d bytes of shared memory (limit 220 KiB)", l.smem_per_warp);
             l.wpb = wpb;

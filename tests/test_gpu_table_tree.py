@@ -31,3 +31,29 @@ def test_positions_match_the_oracle(engine_lib, oracle_lib, case):
     finally:
         eng.close()
         orc.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("more", [0, 1])
+def test_crowded_launches_with_observables_run_the_same_trajectories(engine_lib, more):
+    """With observables, more than seven walkers per SM decide serially: an instance's tables and
+    averages are those of an engine of its own, on either side of the line."""
+    import torch
+    rg = engine_lib
+    n = 7 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    counts = [4] + [64] * ((n - 4) // 64) + ([(n - 4) % 64] if (n - 4) % 64 else [])
+    h = np.round(np.random.default_rng(3).normal(0, 0.5, 25) * 2**20) / 2**20
+
+    def engine(cs):
+        inss = [rg.Instance(model=rg.MODEL_ASHKIN_TELLER2D, L=5, K=0.5, fields=h, energy_min=-125.0, energy_max=0.0, bin_width=0.05,
+                            num_windows=1, replicas_per_window=r, seed=70 + i) for i, r in enumerate(cs)]
+        return rg.Engine(rg.Batch(instances=inss, sweeps_per_exchange=20, sweeps_per_check=40, mask_mode=rg.MASK_VISITED,
+                                  observables=2))
+    with engine(counts) as a, engine(counts[:1]) as b:
+        for e in (a, b):
+            e.run_cycles(2)
+        assert np.array_equal(a.window_logdos(0, 0), b.window_logdos(0, 0))
+        x, y = a.window_observables(0, 0), b.window_observables(0, 0)
+        assert np.array_equal(x[:, -1], y[:, -1])
+        # sums of at most 4000 terms in another order: 4000 x 2^-53 of the larger
+        np.testing.assert_allclose(x, y, rtol=1e-11, atol=1e-13)
