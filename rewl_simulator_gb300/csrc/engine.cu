@@ -1793,19 +1793,22 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
                     Model::flip_signs(ai, B[i], plane, sg);
                     const Pos d0 = Model::delta_at(A, B, i, nbr, cpl, TREE ? h : field(i));
                     const Pos dl = lane > 0 ? Model::flipped_at(A, B, i, nbr.left, cpl) : Pos(0);
+                    // where the chunk is a row: the change of its last site's once the first has flipped
+                    const Pos wrap = wraps && lane == C - 1 ? Model::flipped_at(A, B, i, nbr.right, cpl) >> even : Pos(0);
                     if constexpr (TREE) {
                         const int2 d = make_int2(d0 >> even, dl >> even);
+                        const int last = abs(wrap);
                         dx[lane] = d;
-                        far = (max(abs(d.x), abs(d.x + d.y)) >> shz) + 1;
+                        far = (max(abs(d.x), abs(d.x + d.y)) + last >> shz) + 1;
                     } else {
                         st->du[lane] = make_longlong2(d0, d0 + dl);
                     }
-                    if (wraps && lane == C - 1) st->wcu = Model::flipped_at(A, B, i, nbr.right, cpl) >> even;
+                    if (wraps && lane == C - 1) st->wcu = wrap;
                     if (!TREE && !replay) st->T[lane] = word_threshold(philox_word(seed, uid, attempt + (uint64_t)lane, kStreamWL));
                 }
-                // bins a block's nodes can lie away from its start: five steps (and a row's wrap term, part of
-                // an energy change as large)
-                const int reach = TREE ? (D + 1) * (int)__reduce_max_sync(kFull, (unsigned)far) : 0;
+                // bins a block's nodes can lie away from its start: five steps, the last site's with its wrap term
+                // (fields and the other bonds can cancel what it would be part of)
+                const int reach = TREE ? D * (int)__reduce_max_sync(kFull, (unsigned)far) : 0;
                 __syncwarp();
                 // the next chunk: position, first site, length
                 int cn = cc + 1, yn = y;
