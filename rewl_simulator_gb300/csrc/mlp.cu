@@ -19,7 +19,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -565,14 +567,17 @@ cudaError_t prepare_tc_kernels()
 }
 
 // a bounded wait in a tensor-core GEMM ran out since the last call: report it once
+int tc_timed_out()
+{
+    const int zero = 0;
+    cudaMemcpyToSymbol(g_tc_error, &zero, sizeof zero);
+    return mfail(REWL_EDEVICE, "a tensor-core GEMM timed out waiting for its MMAs (results discarded)");
+}
 int take_tc_error()
 {
     int v = 0;
     if (cudaMemcpyFromSymbol(&v, g_tc_error, sizeof v) != cudaSuccess) return mfail(REWL_EDEVICE, "reading the GEMM status failed");
-    if (!v) return REWL_OK;
-    const int zero = 0;
-    cudaMemcpyToSymbol(g_tc_error, &zero, sizeof zero);
-    return mfail(REWL_EDEVICE, "a tensor-core GEMM timed out waiting for its MMAs (results discarded)");
+    return v ? tc_timed_out() : REWL_OK;
 }
 
 constexpr int kColChunk = 256;                                 // rows per column-sum partial
@@ -952,13 +957,27 @@ __global__ void k_stage(const float* X, int n, int in_dim, int rows, bf16* H0)
     H0[i] = __float2bfloat16(r < n && c < in_dim ? X[(size_t)r * in_dim + c] : 0.f);
 }
 
-// the first column of the padded outputs; NaN while a GEMM's bounded wait has run out
-__global__ void k_take(const float* out, int n, float* y)
+// the first column of the padded outputs; NaN while a GEMM's bounded wait has run out.  Blocks read that
+// flag at different moments, and another network's product may raise it (or its call take it back) in
+// between, so each publishes the flag it acted on, behind the n results (acted not null).
+constexpr int kTakeRows = 256;
+int take_blocks(int n) { return (n + kTakeRows - 1) / kTakeRows; }
+__global__ void __launch_bounds__(kTakeRows) k_take(const float* out, int n, float* y, float* acted)
 {
+    __shared__ int flag;
     step_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool timed_out = *reinterpret_cast<const volatile int*>(&g_tc_error) != 0;
-    if (i < n) y[i] = timed_out ? __int_as_float(0x7FC00000) : out[(size_t)i * kOut];
+    if (threadIdx.x == 0) {
+        flag = *reinterpret_cast<const volatile int*>(&g_tc_error);
+        if (acted) acted[blockIdx.x] = flag ? 1.f : 0.f;
+    }
+    __syncthreads();
+    const int i = blockIdx.x * kTakeRows + threadIdx.x;
+    if (i < n) y[i] = flag ? __int_as_float(0x7FC00000) : out[(size_t)i * kOut];
+}
+// whether a block of k_take discarded its rows
+bool any_discarded(const float* acted, int n)
+{
+    return std::any_of(acted, acted + take_blocks(n), [](float f) { return f != 0.f; });
 }
 
 // the caller's n rows as they are to the device, and from there into rows x kIn bf16: the copy is
@@ -1099,13 +1118,18 @@ int rewl_mlp_predict(rewl_mlp* m, const float* X, int32_t n, int32_t in_dim, flo
     int rc = ensure_batch(m, Bp);
     if (rc) return rc;
     if ((rc = upload_features(m, X, n, in_dim, Bp, m->H[0].p)) || (rc = forward(m, Bp, false))) return rc;
-    // the last hidden layer's buffer is read by now: the first column goes there, n floats to the host
+    // the last hidden layer's buffer is read by now: the first column goes there and what k_take's blocks
+    // acted on behind it (the buffer has at least 128 bytes a row), in one copy to the host
     float* first = reinterpret_cast<float*>(m->H[m->layers].p);
-    MCUDA(launch_next(k_take, dim3((n + 255) / 256), 256, 0, m->stream, m->out.p, n, first));
+    const size_t words = (size_t)n + take_blocks(n);
+    const std::unique_ptr<float[]> h(new (std::nothrow) float[words]);
+    if (!h) return mfail(REWL_ENOMEM, "no host memory for %zu results", words);
+    MCUDA(launch_next(k_take, dim3(take_blocks(n)), kTakeRows, 0, m->stream, m->out.p, n, first, first + n));
     m->launches++;
-    MCUDA(cudaMemcpyAsync(y, first, (size_t)n * 4, cudaMemcpyDeviceToHost, m->stream));
+    MCUDA(cudaMemcpyAsync(h.get(), first, words * 4, cudaMemcpyDeviceToHost, m->stream));
     MCUDA(cudaStreamSynchronize(m->stream));
-    return y[0] == y[0] ? REWL_OK : take_tc_error();       // (NaN everywhere while the flag stands)
+    std::copy(h.get(), h.get() + n, y);
+    return any_discarded(h.get() + n, n) ? tc_timed_out() : REWL_OK;
 }
 
 // One forward + backward on the given rows (no update); gradients readable with
@@ -1336,7 +1360,7 @@ int predict_noalloc_on_device(rewl_mlp* m, const float* X, int32_t n, int32_t in
     const int L = m->layers;
     MCUDA(noalloc_layer<EPI_BIAS_F32>(st, cur, m->Pb.p + m->woff[L], rows, kOut, m->hidden, out, nullptr,
                                       m->P.p + m->boff[L]));
-    k_take<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(out, n, y);
+    k_take<<<take_blocks(n), kTakeRows, 0, st>>>(out, n, y, nullptr);
     MCUDA(cudaGetLastError());
     m->launches += L + 3;
     return REWL_OK;
