@@ -676,13 +676,18 @@ __global__ void k_adam(float* p, float* m, float* v, const float* grad, const fl
 {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int k = cur->k;
-    // the end of a training step, by the last block to have read the cursor: keep its loss, advance
+    // the end of a training step, by the last block to have read the cursor: keep its loss, advance (the
+    // fences order every block's read of the cursor before the write to it)
     __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(&cur->done, 1u) == gridDim.x - 1) {
-        losses[k] = *loss;
-        cur->step += 1;
-        cur->k = k + 1;
-        cur->done = 0;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&cur->done, 1u) == gridDim.x - 1) {
+            __threadfence();
+            losses[k] = *loss;
+            cur->step += 1;
+            cur->k = k + 1;
+            cur->done = 0;
+        }
     }
     if (i >= n) return;
     const float c1 = ctab[2 * k], c2 = ctab[2 * k + 1];
