@@ -274,8 +274,13 @@ int rewl_thermodynamics(const double* E, const double* lng, const double* obs, i
     std::vector<double> h(in);
     std::copy(E, E + nb, h.begin());
     std::copy(lng, lng + nb, h.begin() + nb);
+    bool finite = true;                                 // the averaged columns
     for (int k = 0; k < num_obs; ++k)
-        for (size_t b = 0; b < nb; ++b) h[nb * (2 + k) + b] = obs[b * num_obs + k];
+        for (size_t b = 0; b < nb; ++b) {
+            const double v = obs[b * num_obs + k];
+            h[nb * (2 + k) + b] = v;
+            finite = finite && (k == counts_col || std::isfinite(v));
+        }
     float2* x32 = reinterpret_cast<float2*>(h.data() + nb * (2 + num_obs));
     double e_max = 0, g_max = 0, counts = 0;
     for (size_t b = 0; b < nb; ++b) {
@@ -300,8 +305,9 @@ int rewl_thermodynamics(const double* E, const double* lng, const double* obs, i
     a.se = se; a.sg = sg;
     a.nb = nbins; a.K = num_obs; a.counts_col = counts_col; a.nT = num_T; a.trapezoid = trapezoid ? 1 : 0;
     a.N = system_size; a.Tmin = Tmin; a.dT = (Tmax - Tmin) / (double)num_T; a.counts_mean = counts / (double)nbins;
-    // single precision locates the levels that count while it can hold them
-    const bool filter = e_max < 1e18 && e_max < 1e30 * Tmin && g_max < 1e30 && Tmin > 1e-30;
+    // single precision locates the levels that count while it can hold them; a level of zero weight counts
+    // too where an average is not finite there (NaN or infinity times zero is NaN)
+    const bool filter = finite && e_max < 1e18 && e_max < 1e30 * Tmin && g_max < 1e30 && Tmin > 1e-30;
     a.e_max = filter ? std::nextafter((float)e_max, INFINITY) : -1.f;
     a.g_max = filter ? std::nextafter((float)g_max, INFINITY) : 0.f;
     cudaStream_t st;

@@ -1,0 +1,32 @@
+"""The temperature ladder (rewl_thermodynamics, csrc/thermo.cu) on inputs at the edge of what it takes."""
+import numpy as np
+import pytest
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("level", [0, 150, 299])
+@pytest.mark.parametrize("levels", [300, 5000])
+def test_averages_that_are_not_finite(engine_lib, value, level, levels):
+    """A column with a NaN or an infinity at one level averages to what its sum of products gives, whatever weight
+    the level has: NaN, or an infinity where the level's weight is not zero.  The other columns are as without it."""
+    from rewl_simulator_gb300.thermo import thermodynamics
+    E = np.linspace(-2048.0, 2048.0, levels)
+    lng = 700.0 * (1 - (E / 2048.0) ** 2)
+    obs = np.random.default_rng(1).uniform(0.1, 1.0, (levels, 3))
+    T, plain = thermodynamics(E, lng, 1024, obs=obs, counts_col=2, Tmin=0.05, Tmax=50.0, num_T=60)
+    obs[level, 1] = value
+    _, out = thermodynamics(E, lng, 1024, obs=obs, counts_col=2, Tmin=0.05, Tmax=50.0, num_T=60)
+    keep = [0, 1, 2, 3, 4, 5, 7]
+    np.testing.assert_allclose(out[:, keep], plain[:, keep], rtol=1e-9)
+    zero = 0
+    for i, t in enumerate(T):
+        x = lng - E / t
+        gap = x.max() - x[level]
+        if abs(gap - 745.2) < 1.0:                 # between zero and the smallest subnormal, as the rounding goes
+            continue
+        zero += gap > 745.2
+        with np.errstate(invalid="ignore"):
+            ref = value * (0.0 if gap > 745.2 else 1.0)
+        assert np.array_equal(out[i, 6], ref, equal_nan=True), (t, out[i, 6], ref)
+    assert (zero > 0) == (level > 0)               # the ground state always counts, the others not at every temperature
