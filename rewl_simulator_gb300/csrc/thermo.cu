@@ -293,7 +293,8 @@ int rewl_thermodynamics(const double* E, const double* lng, const double* obs, i
     int xe = 0, xg = 0;
     std::frexp(e_max, &xe);
     std::frexp(g_max * 1.45, &xg);
-    const int se = std::min(std::max(62 - xe, -900), 900), sg = std::min(std::max(60 - xg, -900), 900);
+    // (sg: a shift by sg - F >= sg - 52 bits has to stay below 64 where F is at least 24)
+    const int se = std::min(std::max(62 - xe, -900), 900), sg = std::min(std::max(60 - xg, -900), 86);
     long long* ints = reinterpret_cast<long long*>(h.data() + nb * (3 + num_obs));
     constexpr double kLog2e = 0x1.71547652b82fep+0, kLog2eLo = 0x1.777d0ffda0d24p-56;
     for (size_t b = 0; b < nb; ++b) {

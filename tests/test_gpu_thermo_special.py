@@ -30,3 +30,21 @@ def test_averages_that_are_not_finite(engine_lib, value, level, levels):
             ref = value * (0.0 if gap > 745.2 else 1.0)
         assert np.array_equal(out[i, 6], ref, equal_nan=True), (t, out[i, 6], ref)
     assert (zero > 0) == (level > 0)               # the ground state always counts, the others not at every temperature
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [0.0, 1e-300, 1e-30, 1e-18, 1e-15, 1e-12, 1e-9])
+def test_flat_density_of_states(engine_lib, scale):
+    """ln g of nearly nothing: the integer exponents keep every place that counts beside -E / T."""
+    from rewl_simulator_gb300.thermo import thermodynamics
+    r = np.random.default_rng(4)
+    E = np.sort(r.uniform(-64.0, 64.0, 400))
+    lng = scale * r.uniform(-1.0, 1.0, 400)
+    T, out = thermodynamics(E, lng, 64, Tmin=0.5, Tmax=40.0, num_T=50, trapezoid=False)
+    for i, t in enumerate(T):
+        x = lng - E / t
+        w = np.exp(x - x.max())
+        rel = 8 * 2.0**-52 * 64 / t + 1e-13
+        U = (w * E).sum() / w.sum() / 64
+        assert abs(out[i, 0] + t * (x.max() + np.log(w.sum())) / 64) <= rel * t / 64 + 1e-13 * abs(out[i, 0])
+        assert abs(out[i, 1] - U) <= rel * 64 / 64
