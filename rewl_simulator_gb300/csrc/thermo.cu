@@ -19,7 +19,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <string>
-#include <vector>
 
 #include "../../include/rewl.h"
 
@@ -49,6 +48,7 @@ struct ThermoArgs {
     const long long *Ei, *gi;          // E 2^se and ln g / ln 2 2^sg as integers (62 bits)
     int se, sg;
     const double* obs;                 // K columns of nb values
+    const int* not_finite;             // per block of k_levels: an averaged column holds a NaN or an infinity
     int nb, K, counts_col, nT, trapezoid;
     double N, Tmin, dT, counts_mean;
     float e_max, g_max;                // largest |E| and |ln g|; e_max < 0: no single-precision pass
@@ -99,6 +99,32 @@ __device__ __forceinline__ double pow2_fixed(long long d, int F, const unsigned 
     return __longlong_as_double(((long long)(k + 1022) << 52) + (long long)((w >> 11) + ((w >> 10) & 1ull)));
 }
 
+constexpr double kLog2e = 0x1.71547652b82fep+0, kLog2eLo = 0x1.777d0ffda0d24p-56;
+
+// The caller's levels as k_thermo reads them, a thread each: single precision, integers (ln g / ln 2 formed to
+// 106 bits), observables by column.  (On the host this was 90 us of a call with 4,095 levels.)
+constexpr int kLevelThreads = 128;
+__global__ void __launch_bounds__(kLevelThreads) k_levels(const ThermoArgs a, const double* rows, float2* x32, long long* Ei, long long* gi, double* cols,
+                         int* not_finite)
+{
+    const int b = blockIdx.x * kLevelThreads + threadIdx.x;
+    bool finite = true;
+    if (b < a.nb) {
+        const double e = a.E[b], l = a.lng[b];
+        x32[b] = make_float2((float)-e, (float)l);
+        const double g = __dmul_rn(l, kLog2e), rest = __dadd_rn(__fma_rn(l, kLog2e, -g), __dmul_rn(l, kLog2eLo));
+        Ei[b] = __double2ll_rn(ldexp(e, a.se));
+        gi[b] = __double2ll_rn(ldexp(g, a.sg)) + __double2ll_rn(ldexp(rest, a.sg));
+        for (int k = 0; k < a.K; ++k) {
+            const double v = rows[(size_t)b * a.K + k];
+            cols[(size_t)k * a.nb + b] = v;
+            finite = finite && (k == a.counts_col || isfinite(v));
+        }
+    }
+    const int any = __syncthreads_or(!finite);
+    if (threadIdx.x == 0) not_finite[blockIdx.x] = any;
+}
+
 // One warp per temperature.  Bound: the FP64 pipe -- an FP64 warp instruction occupies it for 32
 // cycles of the SM, as long as some sixty integer ones -- so what the sums do not need stays off it:
 //   * a level whose weight is zero in FP64 (more than 746 below the maximum) is found in single
@@ -131,13 +157,15 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
             sEi[b] = a.Ei[b];
             sgi[b] = a.gi[b];
         }
-    __syncthreads();
+    int special = 0;
+    for (int i = threadIdx.x; i < (a.nb + kLevelThreads - 1) / kLevelThreads; i += blockDim.x) special |= a.not_finite[i];
+    // (a level of zero weight counts too where an average is not finite there: NaN or infinity times zero is NaN)
+    const bool single = !__syncthreads_or(special) && a.e_max >= 0.f;
     const double* E = STAGED ? sE : a.E;
     const double* G = STAGED ? sG : a.lng;
     const float2* X = STAGED ? sX : a.x32;
     const long long* Ei = STAGED ? sEi : a.Ei;
     const long long* gi = STAGED ? sgi : a.gi;
-    constexpr double kLog2e = 0x1.71547652b82fep+0, kLog2eLo = 0x1.777d0ffda0d24p-56;
     const int lane = threadIdx.x & 31, nb = a.nb;
     for (int t = blockIdx.x * kWarps + (threadIdx.x >> 5); t < a.nT; t += gridDim.x * kWarps) {
         const double T = __dadd_rn(a.Tmin, __dmul_rn(a.dT, (double)t));    // rounded as the reference's Tmin + dT * i
@@ -148,7 +176,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
         // the largest one to the last bit
         const float r32 = (float)rT;
         const float err = 5e-7f * (a.e_max * r32 + a.g_max) + 1e-3f;
-        const bool filter = a.e_max >= 0.f && err < 50.f;
+        const bool filter = single && err < 50.f;
         double m;
         float floor32 = -INFINITY;
         int F = 0, top = 0;
@@ -268,59 +296,49 @@ int rewl_thermodynamics(const double* E, const double* lng, const double* obs, i
         if (!std::isfinite(E[b]) || !std::isfinite(lng[b])) return tfail(REWL_EINVAL, "non-finite energy or ln g at bin %d", b);
     if (cudaSetDevice(device) != cudaSuccess) return tfail(REWL_EDEVICE, "cannot use device %d", device);
     const size_t nrow = 5 + (size_t)num_obs, nb = (size_t)nbins;
-    // one buffer on the host and one on the device: E, ln g, observables by column, {-E, ln g} in
-    // single precision, E and ln g / ln 2 as integers; then (device) temperatures and rows
-    const size_t in = nb * (5 + num_obs), all = in + (size_t)num_T * (1 + nrow);
-    std::vector<double> h(in);
-    std::copy(E, E + nb, h.begin());
-    std::copy(lng, lng + nb, h.begin() + nb);
-    bool finite = true;                                 // the averaged columns
-    for (int k = 0; k < num_obs; ++k)
-        for (size_t b = 0; b < nb; ++b) {
-            const double v = obs[b * num_obs + k];
-            h[nb * (2 + k) + b] = v;
-            finite = finite && (k == counts_col || std::isfinite(v));
-        }
-    float2* x32 = reinterpret_cast<float2*>(h.data() + nb * (2 + num_obs));
     double e_max = 0, g_max = 0, counts = 0;
     for (size_t b = 0; b < nb; ++b) {
         e_max = std::max(e_max, std::fabs(E[b]));
         g_max = std::max(g_max, std::fabs(lng[b]));
         if (counts_col >= 0) counts += obs[b * num_obs + counts_col];
-        x32[b] = make_float2((float)-E[b], (float)lng[b]);
     }
-    // the integers: 2^62 above the largest energy, 2^60 above the largest ln g / ln 2 (formed to 106 bits)
+    // the integers: 2^62 above the largest energy, 2^60 above the largest ln g / ln 2
     int xe = 0, xg = 0;
     std::frexp(e_max, &xe);
     std::frexp(g_max * 1.45, &xg);
     // (sg: a shift by sg - F >= sg - 52 bits has to stay below 64 where F is at least 24)
     const int se = std::min(std::max(62 - xe, -900), 900), sg = std::min(std::max(60 - xg, -900), 86);
-    long long* ints = reinterpret_cast<long long*>(h.data() + nb * (3 + num_obs));
-    constexpr double kLog2e = 0x1.71547652b82fep+0, kLog2eLo = 0x1.777d0ffda0d24p-56;
-    for (size_t b = 0; b < nb; ++b) {
-        const double g = lng[b] * kLog2e, rest = std::fma(lng[b], kLog2e, -g) + lng[b] * kLog2eLo;
-        ints[b] = std::llrint(std::ldexp(E[b], se));
-        ints[nb + b] = std::llrint(std::ldexp(g, sg)) + std::llrint(std::ldexp(rest, sg));
-    }
     ThermoArgs a{};
     a.se = se; a.sg = sg;
     a.nb = nbins; a.K = num_obs; a.counts_col = counts_col; a.nT = num_T; a.trapezoid = trapezoid ? 1 : 0;
     a.N = system_size; a.Tmin = Tmin; a.dT = (Tmax - Tmin) / (double)num_T; a.counts_mean = counts / (double)nbins;
-    // single precision locates the levels that count while it can hold them; a level of zero weight counts
-    // too where an average is not finite there (NaN or infinity times zero is NaN)
-    const bool filter = finite && e_max < 1e18 && e_max < 1e30 * Tmin && g_max < 1e30 && Tmin > 1e-30;
+    // single precision locates the levels that count while it can hold them
+    const bool filter = e_max < 1e18 && e_max < 1e30 * Tmin && g_max < 1e30 && Tmin > 1e-30;
     a.e_max = filter ? std::nextafter((float)e_max, INFINITY) : -1.f;
     a.g_max = filter ? std::nextafter((float)g_max, INFINITY) : 0.f;
     cudaStream_t st;
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return tfail(REWL_EDEVICE, "stream creation failed");
+    // one buffer: E, ln g and the observables as the caller has them; what k_levels makes of them (columns, single
+    // precision, two integers a level); temperatures and rows;
+    // k_levels' flags
+    const size_t in = nb * (2 + num_obs), made = nb * (3 + num_obs);
+    const size_t blocks = (nb + kLevelThreads - 1) / kLevelThreads, all = in + made + (size_t)num_T * (1 + nrow) + (blocks + 1) / 2;
     double* d = nullptr;
     cudaError_t e = cudaMalloc(&d, all * sizeof(double));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d, h.data(), in * sizeof(double), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d, E, nb * 8, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d + nb, lng, nb * 8, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && num_obs) e = cudaMemcpyAsync(d + 2 * nb, obs, nb * num_obs * 8, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
-        a.E = d; a.lng = d + nb; a.obs = d + 2 * nb;
-        a.x32 = reinterpret_cast<const float2*>(d + nb * (2 + num_obs));
-        a.Ei = reinterpret_cast<const long long*>(d + nb * (3 + num_obs)); a.gi = a.Ei + nb;
-        a.temps = d + in; a.out = a.temps + num_T;
+        double* cols = d + in;
+        float2* x32 = reinterpret_cast<float2*>(cols + nb * num_obs);
+        long long* Ei = reinterpret_cast<long long*>(x32 + nb);
+        int* flags = reinterpret_cast<int*>(d + in + made + (size_t)num_T * (1 + nrow));
+        a.E = d; a.lng = d + nb; a.obs = cols; a.x32 = x32; a.Ei = Ei; a.gi = Ei + nb; a.not_finite = flags;
+        a.temps = d + in + made; a.out = a.temps + num_T;
+        k_levels<<<(unsigned)blocks, kLevelThreads, 0, st>>>(a, d + 2 * nb, x32, Ei, Ei + nb, cols, flags);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) {
         int nsm = 0;
         if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || nsm < 1) nsm = 152;
         const size_t table = kExpTable * sizeof(double), staged = table + nb * 48;
