@@ -9,7 +9,7 @@
 // F = -T (m + ln Z) / N, U = sum E w / (N Z), U2 = sum E^2 w / (N^2 Z), S = sum ln g w / (N Z),
 // C = N (U2 - U^2) / T^2, O_k = sum O_k w / Z, and the counts column averaged over the bins.
 // The reference loops over 50,000 temperatures serially (src/Simulation/main.cpp:13-15,
-// 339-351); here one warp reduces one temperature, all temperatures in one launch.
+// 339-351); here one warp (or a few) reduces one temperature, all temperatures in one launch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -49,7 +49,7 @@ struct ThermoArgs {
     int se, sg;
     const double* obs;                 // K columns of nb values
     const int* not_finite;             // per block of k_levels: an averaged column holds a NaN or an infinity
-    int nb, K, counts_col, nT, trapezoid;
+    int nb, K, counts_col, nT, trapezoid, team;
     double N, Tmin, dT, counts_mean;
     float e_max, g_max;                // largest |E| and |ln g|; e_max < 0: no single-precision pass
     double *temps, *out;
@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kLevelThreads) k_levels(const ThermoArgs a, co
     if (threadIdx.x == 0) not_finite[blockIdx.x] = any;
 }
 
-// One warp per temperature.  Bound: the FP64 pipe -- an FP64 warp instruction occupies it for 32
+// One warp per temperature; a team of warps where there are few (TEAM).  Bound: the FP64 pipe -- an FP64 warp instruction occupies it for 32
 // cycles of the SM, as long as some sixty integer ones -- so what the sums do not need stays off it:
 //   * a level whose weight is zero in FP64 (more than 746 below the maximum) is found in single
 //     precision, with its rounding error bounded and added to the margin, and skipped: half of the
@@ -137,11 +137,13 @@ __global__ void __launch_bounds__(kLevelThreads) k_levels(const ThermoArgs a, co
 // exponential for every level; the same sums with a table exponential in FP64 took 7.9 ms.
 // Where the integers could be coarser than FP64 -- energies whose largest values dwarf those that
 // count -- a temperature takes the FP64 form of the same sums.
-// STAGED: levels in shared memory.  KO: room for observable columns.
-template <bool STAGED, int KO>
+// STAGED: levels in shared memory.  KO: room for observable columns.  TEAM: a.team warps per temperature.
+template <bool STAGED, int KO, bool TEAM>
 __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
 {
     extern __shared__ __align__(16) double sm[];
+    __shared__ double part[TEAM ? kWarps : 1][4 + KO];
+    __shared__ int at[kWarps];
     unsigned long long* tab = reinterpret_cast<unsigned long long*>(sm);
     double *sE = sm + kExpTable, *sG = sE + a.nb, *sE2 = sG + a.nb;
     float2* sX = reinterpret_cast<float2*>(sE2 + a.nb);
@@ -166,8 +168,25 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
     const float2* X = STAGED ? sX : a.x32;
     const long long* Ei = STAGED ? sEi : a.Ei;
     const long long* gi = STAGED ? sgi : a.gi;
-    const int lane = threadIdx.x & 31, nb = a.nb;
-    for (int t = blockIdx.x * kWarps + (threadIdx.x >> 5); t < a.nT; t += gridDim.x * kWarps) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nb = a.nb;
+    // the warps of a temperature share its levels: this one's are first, first + stride ...
+    const int team = TEAM ? a.team : 1, teams = kWarps / team, lead = TEAM ? warp / team * team : warp;
+    const int first = TEAM ? 32 * (warp - lead) : 0, stride = 32 * team;
+    // a barrier of the team's own (teams at different temperatures take different branches)
+    auto team_sync = [&] { asm volatile("bar.sync %0, %1;" :: "r"(1 + warp / team), "r"(stride) : "memory"); };
+    // combine(v, w) of the values of a team's warps, w one of them, in every lane of all of them
+    auto team_all = [&](double v, auto combine) {
+        if (!TEAM) return v;
+        team_sync();
+        if (lane == 0) part[TEAM ? warp : 0][0] = v;
+        team_sync();
+        v = part[TEAM ? lead : 0][0];
+        for (int w = 1; w < team; ++w) v = combine(v, part[TEAM ? lead + w : 0][0]);
+        return v;
+    };
+    for (int t0 = blockIdx.x * teams + (TEAM ? 0 : warp); t0 < a.nT; t0 += gridDim.x * teams) {
+        const bool here = !TEAM || t0 + warp / team < a.nT;                // (all warps keep the barriers of a team)
+        const int t = !TEAM ? t0 : here ? t0 + warp / team : a.nT - 1;
         const double T = __dadd_rn(a.Tmin, __dmul_rn(a.dT, (double)t));    // rounded as the reference's Tmin + dT * i
         const double rT = 1.0 / T;
         auto exponent = [&](int b) { return G[b] - E[b] / T; };
@@ -183,7 +202,7 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
         long long c = 0;
         if (filter) {
             float best = -INFINITY;
-            for (int b = lane; b < nb; b += 32) {
+            for (int b = first + lane; b < nb; b += stride) {
                 const float2 v = X[b];
                 const float x = fmaf(v.x, r32, v.y);
                 if (x > best) { best = x; top = b; }
@@ -194,17 +213,28 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
                 const int i = __shfl_xor_sync(0xFFFFFFFFu, top, o);
                 if (x > best || (x == best && i < top)) { best = x; top = i; }
             }
+            if (TEAM) {
+                // the first of the team's largest
+                team_sync();
+                if (lane == 0) { part[TEAM ? warp : 0][0] = best; at[warp] = top; }
+                team_sync();
+                for (int w = lead; w < lead + team; ++w) {
+                    const float x = (float)part[TEAM ? w : 0][0];
+                    if (x > best || (x == best && at[w] < top)) { best = x; top = at[w]; }
+                }
+            }
             m = exponent(top);
             floor32 = best - 746.f - 2.f * err;
             // fixed point for the levels that count: their energies lie within `span` of the reference's
             float span = 0.f;
             const float2 ref = X[top];
-            for (int b = lane; b < nb; b += 32) {
+            for (int b = first + lane; b < nb; b += stride) {
                 const float2 v = X[b];
                 if (!(fmaf(v.x, r32, v.y) < floor32)) span = fmaxf(span, fabsf(v.x - ref.x));
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) span = fmaxf(span, __shfl_xor_sync(0xFFFFFFFFu, span, o));
+            span = (float)team_all(span, [](double x, double y) { return fmax(x, y); });
             span = 1.0001f * span + 2e-7f * a.e_max;
             const double ch = kLog2e * rT, cl = fma(kLog2e, rT, -ch) + (kLog2e * (fma(-rT, T, 1.0) * rT) + kLog2eLo * rT);
             const float bits = 1.45f * (2.f * span * r32 + 750.f + 2.f * err);     // bound of every exponent difference
@@ -219,16 +249,17 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
             }
         } else {
             m = -INFINITY;
-            for (int b = lane; b < nb; b += 32) m = fmax(m, exponent(b));
+            for (int b = first + lane; b < nb; b += stride) m = fmax(m, exponent(b));
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+            m = team_all(m, [](double x, double y) { return fmax(x, y); });
         }
 
         double z = 0.0, u = 0.0, u2 = 0.0, s = 0.0, o[KO + 1];
 #pragma unroll
         for (int k = 0; k < KO; ++k) o[k] = 0.0;
         const long long etop = Ei[top], gtop = gi[top];
-        for (int b0 = 0; b0 < nb; b0 += 32) {
+        for (int b0 = first; b0 < nb; b0 += stride) {
             const int b = b0 + lane;
             bool counts = b < nb;
             if (filter && counts) {
@@ -259,12 +290,32 @@ __global__ void __launch_bounds__(32 * kWarps, 1) k_thermo(const ThermoArgs a)
         u = warp_sum(u);
         u2 = warp_sum(u2);
         s = warp_sum(s);
+        if (TEAM) {
+#pragma unroll
+            for (int k = 0; k < KO; ++k)
+                if (k < a.K && k != a.counts_col) o[k] = warp_sum(o[k]);
+            double* p = part[TEAM ? warp : 0];
+            team_sync();
+            if (lane == 0) {
+                p[0] = z; p[1] = u; p[2] = u2; p[3] = s;
+#pragma unroll
+                for (int k = 0; k < KO; ++k) p[4 + k] = o[k];
+            }
+            team_sync();
+            if (warp != lead || !here) continue;
+            for (int w = 1; w < team; ++w) {
+                const double* v = part[TEAM ? lead + w : 0];
+                z += v[0]; u += v[1]; u2 += v[2]; s += v[3];
+#pragma unroll
+                for (int k = 0; k < KO; ++k) o[k] += v[4 + k];
+            }
+        }
         double* row = a.out + (size_t)t * (5 + a.K);
 #pragma unroll
         for (int k = 0; k < KO; ++k)
             if (k < a.K) {
                 if (k == a.counts_col) o[k] = a.counts_mean;
-                else o[k] = warp_sum(o[k]) / z;
+                else o[k] = (TEAM ? o[k] : warp_sum(o[k])) / z;
                 if (lane == 0) row[5 + k] = o[k];
             }
         if (lane == 0) {
@@ -325,9 +376,19 @@ int rewl_thermodynamics(const double* E, const double* lng, const double* obs, i
     const size_t blocks = (nb + kLevelThreads - 1) / kLevelThreads, all = in + made + (size_t)num_T * (1 + nrow) + (blocks + 1) / 2;
     double* d = nullptr;
     cudaError_t e = cudaMalloc(&d, all * sizeof(double));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d, E, nb * 8, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d + nb, lng, nb * 8, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && num_obs) e = cudaMemcpyAsync(d + 2 * nb, obs, nb * num_obs * 8, cudaMemcpyHostToDevice, st);
+    // (small inputs and results in one copy each: a copy is 5 to 10 us of a call of 200)
+    constexpr size_t kSmall = 4096;
+    double small[kSmall];
+    if (in <= kSmall) {
+        std::copy(E, E + nb, small);
+        std::copy(lng, lng + nb, small + nb);
+        std::copy(obs, obs + (num_obs ? nb * num_obs : 0), small + 2 * nb);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(d, small, in * 8, cudaMemcpyHostToDevice, st);
+    } else {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(d, E, nb * 8, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(d + nb, lng, nb * 8, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess && num_obs) e = cudaMemcpyAsync(d + 2 * nb, obs, nb * num_obs * 8, cudaMemcpyHostToDevice, st);
+    }
     if (e == cudaSuccess) {
         double* cols = d + in;
         float2* x32 = reinterpret_cast<float2*>(cols + nb * num_obs);
@@ -343,20 +404,37 @@ int rewl_thermodynamics(const double* E, const double* lng, const double* obs, i
         if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || nsm < 1) nsm = 152;
         const size_t table = kExpTable * sizeof(double), staged = table + nb * 48;
         const bool fits = staged <= 220 * 1024;        // levels up to 4,352 in shared memory
+        // Warps per temperature: one where the temperatures fill the device, else as many as keep all blocks
+        // in one wave (4,095 levels, 17 columns: 152 temperatures, teams of 1 / 4 / 8 / 16 warps 499 / 331 / 297 /
+        // 293 us; 500: 528 / 333 / 386 / 494; 1000, teams of 1 / 2 / 4: 527 / 397 / 421; 2432: 537 / 544 / 604)
+        a.team = 1;
+        while (a.team < kWarps && 32 * a.team < nbins && 2ll * a.team * num_T <= (long long)kWarps * nsm) a.team *= 2;
         using Kernel = void (*)(const ThermoArgs);
-        const Kernel kernels[2][3] = {{k_thermo<false, 0>, k_thermo<false, 6>, k_thermo<false, kMaxObs>},
-                                      {k_thermo<true, 0>, k_thermo<true, 6>, k_thermo<true, kMaxObs>}};
-        const Kernel fn = kernels[fits ? 1 : 0][num_obs == 0 ? 0 : num_obs <= 6 ? 1 : 2];
+        const Kernel kernels[2][2][3] = {{{k_thermo<false, 0, false>, k_thermo<false, 6, false>, k_thermo<false, kMaxObs, false>},
+                                          {k_thermo<true, 0, false>, k_thermo<true, 6, false>, k_thermo<true, kMaxObs, false>}},
+                                         {{k_thermo<false, 0, true>, k_thermo<false, 6, true>, k_thermo<false, kMaxObs, true>},
+                                          {k_thermo<true, 0, true>, k_thermo<true, 6, true>, k_thermo<true, kMaxObs, true>}}};
+        const Kernel fn = kernels[a.team > 1 ? 1 : 0][fits ? 1 : 0][num_obs == 0 ? 0 : num_obs <= 6 ? 1 : 2];
         e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
         if (e == cudaSuccess) {
-            const int grid = std::min((num_T + kWarps - 1) / kWarps, nsm);
+            const int teams = kWarps / a.team, grid = std::min((num_T + teams - 1) / teams, nsm);
             fn<<<grid, 32 * kWarps, fits ? staged : table, st>>>(a);
             e = cudaGetLastError();
         }
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, a.out, (size_t)num_T * nrow * 8, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(temperatures, a.temps, (size_t)num_T * 8, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    const size_t rows = (size_t)num_T * nrow, results = num_T + rows;
+    if (results <= kSmall) {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(small, a.temps, results * 8, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) {
+            std::copy(small, small + num_T, temperatures);
+            std::copy(small + num_T, small + results, out);
+        }
+    } else {
+        if (e == cudaSuccess) e = cudaMemcpyAsync(out, a.out, rows * 8, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(temperatures, a.temps, (size_t)num_T * 8, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    }
     cudaStreamDestroy(st);
     cudaFree(d);
     if (e != cudaSuccess) return tfail(REWL_EDEVICE, "thermodynamics: %s", cudaGetErrorString(e));

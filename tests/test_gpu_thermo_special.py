@@ -48,3 +48,30 @@ def test_flat_density_of_states(engine_lib, scale):
         U = (w * E).sum() / w.sum() / 64
         assert abs(out[i, 0] + t * (x.max() + np.log(w.sum())) / 64) <= rel * t / 64 + 1e-13 * abs(out[i, 0])
         assert abs(out[i, 1] - U) <= rel * 64 / 64
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("levels", [2, 33, 500, 4352, 4353])
+@pytest.mark.parametrize("columns", [0, 5, 17])
+def test_rows_do_not_depend_on_the_ladder(engine_lib, levels, columns):
+    """A temperature's row is the same in a ladder that fills the device (a warp a temperature) and in short ones
+    (teams of 2 to 16 warps a temperature), to the order of its sums: n terms, n x 2^-53 of the sum of magnitudes;
+    for the specific heat N (U2 - U^2) / T^2 those of its two terms."""
+    from rewl_simulator_gb300.thermo import thermodynamics
+    r = np.random.default_rng(levels)
+    E = np.linspace(-2.0, 2.0, levels) * 1024
+    lng = 710.0 * (1 - (E / 2048.0) ** 2)
+    obs = r.uniform(0.1, 1.0, (levels, columns)) if columns else None
+    step, low = 1.0 / 128, 0.5
+
+    def ladder(n):
+        return thermodynamics(E, lng, 1024, obs=obs, counts_col=columns - 1, Tmin=low, Tmax=low + step * n, num_T=n)
+    T, full = ladder(5000)
+    size = np.abs(full).max(axis=0)
+    for n in (1, 2, 151, 153, 305, 607, 609, 1217, 2433):
+        t, rows = ladder(n)
+        assert np.array_equal(t, T[:n])
+        off = np.abs(rows - full[:n])
+        heat = 1024 * (size[2] + 2 * size[1] ** 2) / t**2
+        assert np.all(np.delete(off, 4, axis=1) <= levels * 2.0**-50 * np.delete(size, 4))
+        assert np.all(off[:, 4] <= levels * 2.0**-50 * heat)
