@@ -792,7 +792,7 @@ struct MomentParts {
     __host__ __device__ explicit MomentParts(int N) : bits(N <= 8192 ? 18 : 16), visits(1u << (32 - bits)) {}
 };
 
-// shared memory of one walker: table with guards, lattice words, thresholds, two chunks' slots;
+// shared memory of one walker (of G a warp): table with guards, lattice words, thresholds, two chunks' slots;
 // with observables the bins of a chunk's steps and (acc) the
 // moments' integer sums, with correlators row and column sums and counts
 template <int G>
@@ -810,6 +810,13 @@ __host__ __device__ inline int bins_smem(int nbcap, int L, bool obs, bool corr, 
 // cycles per flip, 3072 walkers 4.62 -> 4.70e10 flips/s; L = 20, 32 walkers, whose rows had no chunk of
 // eight, 376 -> 71.
 //
+__host__ inline int bins_smem(int G, int nbcap, int L, bool obs, bool corr, bool cnt, bool acc)
+{
+    const int raw = G == 1 ? bins_smem<1>(nbcap, L, obs, corr, cnt, acc) : G == 2 ? bins_smem<2>(nbcap, L, obs, corr, cnt, acc)
+                                                                               : bins_smem<4>(nbcap, L, obs, corr, cnt, acc);
+    return ((raw + 127) & ~127) + 16;                          // + 16 skews the walkers' banks
+}
+
 // The sweeps of one warp's G walkers (launch position warp_index; its shared memory starts at
 // warp_base, one region of p.smem_per_warp bytes per walker).
 template <int G, bool OBS, bool CNT>
@@ -1364,20 +1371,28 @@ __device__ __forceinline__ void sweep_bins_warp(const SweepParams& p, const int 
     }
 }
 
-template <int G, bool OBS, bool CNT>
-__global__ void __launch_bounds__(128, 1) k_sweep_ising_bins(const SweepParams p)
+// BLOCKS: of 128 threads on an SM that the registers leave room for.  The observables take 190 to 212 registers,
+// which 8 to 10 warps of an SM have; with 168 it holds 12, the better form where there are as many (L = 64, moments,
+// 2944 walkers, two a warp: 26.2 -> 33.0e9 flips/s; 2048: 31.2 -> 30.6).
+template <int G, bool OBS, bool CNT, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) k_sweep_ising_bins(const SweepParams p)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int wib = threadIdx.x >> 5;
     sweep_bins_warp<G, OBS, CNT>(p, blockIdx.x * (blockDim.x >> 5) + wib, smem + (size_t)wib * G * p.smem_per_warp);
 }
 
-SweepKernel bins_kernel(int G, bool obs, bool cnt)
+template <int G>
+SweepKernel bins_kernel_t(bool obs, bool cnt, bool crowded)
 {
-    if (!cnt) return obs ? k_sweep_ising_bins<1, true, false> : k_sweep_ising_bins<1, false, false>;
-    if (G == 1) return obs ? k_sweep_ising_bins<1, true, true> : k_sweep_ising_bins<1, false, true>;
-    if (G == 2) return obs ? k_sweep_ising_bins<2, true, true> : k_sweep_ising_bins<2, false, true>;
-    return obs ? k_sweep_ising_bins<4, true, true> : k_sweep_ising_bins<4, false, true>;
+    if (!obs) return cnt ? k_sweep_ising_bins<G, false, true, 1> : k_sweep_ising_bins<G, false, false, 1>;
+    if (crowded) return cnt ? k_sweep_ising_bins<G, true, true, 3> : k_sweep_ising_bins<G, true, false, 3>;
+    return cnt ? k_sweep_ising_bins<G, true, true, 1> : k_sweep_ising_bins<G, true, false, 1>;
+}
+
+SweepKernel bins_kernel(int G, bool obs, bool cnt, bool crowded)
+{
+    return G == 1 ? bins_kernel_t<1>(obs, cnt, crowded) : G == 2 ? bins_kernel_t<2>(obs, cnt, crowded) : bins_kernel_t<4>(obs, cnt, crowded);
 }
 
 // Ashkin-Teller: sweep = sigma pass then tau pass (wang_landau.hpp:109-119); the flavour toggles
@@ -2501,6 +2516,8 @@ struct Launch {
     int walkers_per_warp = 1;
     int counts = 0;         // bin-tracking kernel: visit counts beside g in shared memory (16 bytes per bin)
     int moments = 0;        // bin-tracking kernel with observables: moment sums in shared memory
+    int crowded = 0;        // bin-tracking kernel with observables: the form of 168 registers
+    int maxL = 0;
     int tree = 0;           // the global-table kernel may decide on the tree of outcomes
     int tables = 0;         // the global-table kernel (k_sweep_tables)
     int cache = 0;          // its bins of each walker's table in shared memory (a power of two); 0: the serial chain
@@ -2998,6 +3015,56 @@ int at_carveout(rewl_engine* e, Launch& l)
     return REWL_OK;
 }
 
+// The time of a launch of n walkers of the bin-tracking kernel, G a warp, in cycles per flip of a walker: as many
+// warps as registers (12 warps) and shared memory hold on an SM run at once, in full waves and a last one, and take what
+// the busiest of its four schedulers does.  Measured at L = 48, windows of 114 bins, 1 to 3 warps a scheduler; equals
+// go to more walkers a warp, which shorter rows prefer (L = 16, 768 walkers, one a warp 2.67, two 2.58 ms).
+// What it decides (L = 64, e9 flips/s): visits beside g cost a bin 16 bytes instead of 8 and save the ordered stores of a
+// block's g (2048 walkers of 245 bins 39.5 against 32.3, of 865 bins 25.5 against 34.0, of 4097 bins 9.6 against 17.4);
+// moments in shared memory take 28 bytes a bin and save reductions to global memory (2048 walkers of 245 bins 31.2
+// against 29.0, 2944 walkers 26.2 against 33.0); two walkers a warp up to 24 walkers an SM, four beyond (4096 walkers of
+// 245 bins 41.1 against 55.2).
+double bins_cycles(int n, int nsm, int G, bool obs, bool cnt, bool mom, int smem)
+{
+    static const double kCycles[6][3][3] = {
+        {{72, 97, 132}, {98, 131, 177}, {120, 165, 219}},              // g alone
+        {{65, 88, 116}, {88, 114, 153}, {123, 159, 202}},              // visits beside g (one a warp: 84, 113 at L = 48)
+        {{108, 128, 161}, {153, 179, 221}, {226, 264, 320}},           // observables: g alone
+        {{95, 119, 159}, {128, 162, 216}, {196, 239, 285}},            //   moments in shared memory
+        {{101, 118, 147}, {142, 168, 208}, {230, 266, 303}},           //   visits beside g
+        {{88, 110, 145}, {119, 151, 200}, {199, 245, 290}}};           //   both
+    const auto& t = kCycles[obs ? 2 + 2 * cnt + mom : cnt][G == 1 ? 0 : G == 2 ? 1 : 2];
+    const int warps = ((n + G - 1) / G + nsm - 1) / nsm;
+    const int room = std::min(12, std::max(1, 228 * 1024 / (G * smem + 1024)));
+    const int waves = (warps - 1) / room, rest = warps - waves * room;
+    return waves * t[(room - 1) / 4] + t[(rest - 1) / 4];
+}
+
+// The shape of a launch group of the bin-tracking kernel: walkers per warp (G; 0: any), visits beside g and moments in
+// shared memory, the cheapest that fits; fewer walkers a warp where G's do not fit a block.
+void shape_bins(const rewl_engine* e, Launch& l, int nsm, int G)
+{
+    const bool obs = e->desc.observables != 0, corr = e->desc.observables == 2;
+    const int n = e->desc.persistent ? e->nslots : (int)l.slots.size();
+    double best = 0;
+    for (int g : {4, 2, 1}) {
+        if (G ? g > G : g > 1 && g > n) continue;
+        for (int c = 3; c >= 0; --c) {
+            const bool cnt = c & 1, mom = c & 2;
+            if (mom && !obs) continue;
+            const int smem = bins_smem(g, l.nbcap, l.maxL, obs, corr, cnt, mom);
+            if (g * smem > 200 * 1024 && (g > 1 || c > 0)) continue;
+            const double t = bins_cycles(n, nsm, g, obs, cnt, mom, smem);
+            if (best != 0 && t >= best) continue;
+            best = t;
+            l.walkers_per_warp = g; l.counts = cnt; l.moments = mom; l.smem_per_warp = smem;
+        }
+        if (G && best != 0) break;
+    }
+    l.crowded = obs && (n + l.walkers_per_warp - 1) / l.walkers_per_warp > 8 * nsm &&
+                228 * 1024 / (l.walkers_per_warp * l.smem_per_warp + 1024) > 8;
+}
+
 // A launch group's shape: walkers per warp (bin-tracking kernel) and warps per block, if the
 // block's shared memory fits.
 bool shape_fits(const Launch& l, int G, int wpb)
@@ -3098,35 +3165,17 @@ int plan_launches(rewl_engine* e)
         }
         const int n = (int)l.slots.size();
         if (l.bins) {
-            int G = e->desc.persistent ? 1 : e->desc.walkers_per_warp;
-            if (G == 0) {
-                // one walker per warp while the SM sub-partitions outnumber the walkers
-                // (a block is latency-bound); two per warp beyond that (measured at L = 64, 3072 walkers,
-                // one / two / four per warp: 3.13 / 4.70 / 4.47e10 flips/s; 512 walkers 1.82 / 1.38e10);
-                // four only for still larger batches
-                G = n <= 4 * nsm ? 1 : (n <= 32 * nsm ? 2 : 4);
-            }
+            const int G = e->desc.persistent ? 1 : e->desc.walkers_per_warp;
             l.nbcap = (maxnb + 1) & ~1;
-            const bool obs = e->desc.observables != 0;
-            // per walker, the largest of the shapes the autotuner may pick; +16 skews the walkers' banks
-            auto raw = [&](bool cnt, bool acc) {
-                return std::max({bins_smem<1>(l.nbcap, maxL, obs, corr, cnt, acc), bins_smem<2>(l.nbcap, maxL, obs, corr, cnt, acc),
-                                 bins_smem<4>(l.nbcap, maxL, obs, corr, cnt, acc)});
-            };
-            if ((size_t)raw(false, false) * G > 220 * 1024)
-                return fail(REWL_EINVAL, "a walker needs %d bytes of shared memory", raw(false, false));
-            l.counts = raw(true, false) + 144 <= 200 * 1024 / G;
-            if (!l.counts) G = 1;                                  // g alone: one walker per warp only
-            l.moments = obs && raw(l.counts, true) + 144 <= 200 * 1024 / G;
-            l.walkers_per_warp = G;
-            l.smem_per_warp = ((raw(l.counts, l.moments) + 127) & ~127) + 16;
-            int wpb = e->desc.warps_per_block;
-            if (wpb == 0) {
-                const int warps = (n + G - 1) / G;
-                wpb = warps <= nsm * 2 ? 1 : warps <= nsm * 8 ? 2 : 4;
-            }
+            l.maxL = maxL;
+            const int least = bins_smem(std::max(G, 1), l.nbcap, maxL, e->desc.observables != 0, corr, false, false);
+            if ((size_t)least * std::max(G, 1) > 220 * 1024) return fail(REWL_EINVAL, "a walker needs %d bytes of shared memory", least);
+            shape_bins(e, l, nsm, G);
+            // one warp a block: the schedulers fill evenly (L = 24, 5952 walkers, four a warp: blocks of four warps 44.5,
+            // of one 59.0e9 flips/s)
+            int wpb = e->desc.warps_per_block ? e->desc.warps_per_block : 1;
             wpb = std::min(wpb, 4);                                // the kernel's launch bounds: 128 threads
-            while (wpb > 1 && (size_t)wpb * G * l.smem_per_warp > 200 * 1024) wpb >>= 1;
+            while (wpb > 1 && (size_t)wpb * l.walkers_per_warp * l.smem_per_warp > 200 * 1024) wpb >>= 1;
             l.wpb = wpb;
         } else {
             const size_t ising_smem = (size_t)(((maxnb + 1) & ~1) * 8 + sizeof(Stage) + ((maxN + 15) & ~15) + (corr ? 8 * maxL : 0));
@@ -3183,8 +3232,8 @@ int plan_launches(rewl_engine* e)
             if (int rc = e->gsnap.alloc(e->table_total)) return rc;
     }
     for (int G : {1, 2, 4})
-        for (int o = 0; o < 4; ++o)
-            CUDA_TRY(cudaFuncSetAttribute(bins_kernel(G, o & 1, o & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        for (int o = 0; o < 8; ++o)
+            CUDA_TRY(cudaFuncSetAttribute(bins_kernel(G, o & 1, o & 2, o & 4), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     if (e->desc.persistent) return plan_fused(e, nsm);
     if (e->launches.size() > 1) {
         CUDA_TRY(cudaEventCreateWithFlags(&e->fork_ev, cudaEventDisableTiming));
@@ -3315,7 +3364,7 @@ int launch_group(rewl_engine* e, Launch& l, cudaStream_t stream, int nsweeps, co
         const int warps = (sp.nslots + G - 1) / G;
         const int blocks = (warps + l.wpb - 1) / l.wpb;
         const size_t smem = (size_t)l.wpb * G * l.smem_per_warp;
-        bins_kernel(G, P.obs != nullptr, l.counts)<<<blocks, 32 * l.wpb, smem, stream>>>(sp);
+        bins_kernel(G, P.obs != nullptr, l.counts, l.crowded)<<<blocks, 32 * l.wpb, smem, stream>>>(sp);
     } else {
         const int blocks = (sp.nslots + l.wpb - 1) / l.wpb;
         const size_t smem = (size_t)l.wpb * l.smem_per_warp;
@@ -4461,23 +4510,30 @@ int rewl_autotune(rewl_engine* e, int32_t sweeps)
                                            : (int)std::max<int64_t>(1, std::min<int64_t>(e->desc.sweeps_per_exchange,
                                                                                           20000000 / std::max<int64_t>(1, dof))));
         std::vector<std::pair<int, int>> cand;
+        const int planned = l.walkers_per_warp, nsm = sm_count(e);
+        auto shape = [&](int G, int W) {
+            if (l.bins) shape_bins(e, l, nsm, G);
+            l.wpb = W;
+            return !l.bins || l.walkers_per_warp == G;
+        };
+        std::pair<int, int> pick{planned, l.wpb};
         // the bin-tracking kernel takes at most 4 warps per block (its launch bounds); 4 walkers
         // per warp is left to the planner's rule for very large batches
-        for (int G : {1, 2}) {
-            if ((!l.counts && G > 1) || (l.bins && G > (int)l.slots.size())) continue;
+        for (int G : {1, 2, 4}) {
+            if (l.bins ? G > (int)l.slots.size() || (G == 4 && planned < 4) : G > 1) continue;
             if (e->desc.walkers_per_warp && l.bins && G != e->desc.walkers_per_warp) continue;
+            if (!shape(G, pick.second)) continue;
             for (int W : {1, 2, 4, 8}) {
                 if (l.bins && W > 4) continue;
                 if (e->desc.warps_per_block && W != std::min(e->desc.warps_per_block, l.bins ? 4 : 8)) continue;
                 if (shape_fits(l, G, W)) cand.push_back({G, W});
             }
         }
+        shape(pick.first, pick.second);
         if (cand.size() < 2) continue;
         float best = FLT_MAX;
-        std::pair<int, int> pick{l.walkers_per_warp, l.wpb};
         for (const auto& c : cand) {
-            l.walkers_per_warp = c.first;
-            l.wpb = c.second;
+            shape(c.first, c.second);
             if ((rc = at_carveout(e, l))) break;
             if ((rc = launch_group(e, l, e->stream, ts, P))) break;         // warm-up
             if (!ck(cudaEventRecord(a, e->stream))) break;
@@ -4487,8 +4543,7 @@ int rewl_autotune(rewl_engine* e, int32_t sweeps)
             if (!ck(cudaEventElapsedTime(&ms, a, b))) break;
             if (ms < best) { best = ms; pick = c; }
         }
-        l.walkers_per_warp = pick.first;
-        l.wpb = pick.second;
+        shape(pick.first, pick.second);
         if (int r2 = at_carveout(e, l)) if (rc == REWL_OK) rc = r2;
     }
     if (a) cudaEventDestroy(a);
