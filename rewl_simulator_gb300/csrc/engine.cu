@@ -19,6 +19,7 @@
 //   k_sweep_ising_bins  one, two or four walkers per warp; lattice, window table and
 //                   thresholds in shared memory; several sites decided at a time on
 //                   a binary tree of outcomes (the default Ising kernel)
+//   k_sweep_ising_rows  the same one decision after another: short rows in crowded launches
 //   k_sweep_ising   one warp per walker; lattice, g and H staged in shared
 //                   memory; lanes precompute a row-aligned chunk of <= 32 sites
 //                   (energy change with and without the left neighbour flipped,
@@ -1395,6 +1396,288 @@ SweepKernel bins_kernel(int G, bool obs, bool cnt, bool crowded)
     return G == 1 ? bins_kernel_t<1>(obs, cnt, crowded) : G == 2 ? bins_kernel_t<2>(obs, cnt, crowded) : bins_kernel_t<4>(obs, cnt, crowded);
 }
 
+// ---------------------------------------------------------------------------
+// The same sweeps one decision after another, for lattices whose rows are one chunk of C = 4, 8 or 16 sites, in crowded
+// launches.  A block of the tree costs the same however few sites the row leaves it, and the counts of a row are
+// formed anew for every few blocks; the chain's step is 16 instructions and a dependent shared load, which several
+// walkers a warp and several warps hide.  Per row the walker's lanes form each site's table offsets (without / with its left neighbour flipped; the last
+// site's wrap term) from the lattice before the row above is decided, and correct them for that row's flips; all lanes
+// then go through the row in lockstep, the two proposals a step may lead to formed while its predecessor is decided.
+// Measured against the tree, four walkers a warp, cycles per flip of a walker: 5952 walkers, L = 4 531 -> 266, L = 8
+// 315 -> 168 (with moments 500 -> 243), L = 16 249 -> 148 (364 -> 242); 1200 walkers 203 -> 157, 152 -> 96, 105 -> 79 (two
+// a warp); with correlators L = 16 202 -> 200 and 250 -> 313, which stays with the tree.
+// ---------------------------------------------------------------------------
+__host__ __device__ inline int rows_smem(int nbcap, int C, bool obs, bool corr)
+{
+    return (nbcap + 2 * kGuard) * 8 + C * C + 8 * C * 8 + 2 * C * 8 + (obs ? 4 * C : 0) + (corr ? 8 * C + 4 * nbcap : 0);
+}
+
+template <int G, int C, bool OBS>
+__global__ void __launch_bounds__(128, OBS ? 3 : 1) k_sweep_ising_rows(const SweepParams p)
+{
+    constexpr int P = 32 / G, N = C * C;
+    constexpr int SPL = (C + P - 1) / P;                       // sites per lane in a row
+    static_assert(C % 4 == 0 && C >= 4 && C <= 16 && G > 1, "rows");
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int grp = lane / P, q = lane - grp * P, gbase = grp * P;
+    const int li = (blockIdx.x * (blockDim.x >> 5) + wib) * G + grp;
+    const bool valid = li < p.nslots;
+    if (__ballot_sync(kFull, valid) == 0 || engine_failed_warp(p.P.counters)) return;   // no walkers, or stopped
+    const DevPtrs& P_ = p.P;
+    const int s = p.slots[valid ? li : 0];                     // idle groups shadow a walker, never write
+    const InstDev I = P_.inst[P_.slot_inst[s]];
+    const int w = P_.slot_win[s];
+    const WinDev W = P_.win[w];
+    const int nb = W.nb;
+    unsigned char* base = smem + (size_t)(wib * G + grp) * p.smem_per_warp;
+    long long* gs = reinterpret_cast<long long*>(base) + kGuard;                // gs[-kGuard .. nb + kGuard)
+    int8_t* lat = reinterpret_cast<int8_t*>(base + (p.nbcap + 2 * kGuard) * 8);
+    long long* Tb = reinterpret_cast<long long*>(lat + N);                      // 2 x 4C thresholds (+ ln f)
+    int2* Db = reinterpret_cast<int2*>(Tb + 8 * C);                             // 2 x C offset pairs
+    int* seqb = reinterpret_cast<int*>(Db + 2 * C);                             // a row's bins (observables)
+    int* rsum = seqb + C;                                                       // correlators: row sums,
+    int* csum = rsum + C;                                                       // column sums,
+    int* bcnt = csum + C;                                                       // bin counts modulo 1000
+    char* const sm = reinterpret_cast<char*>(smem);                             // table positions: bytes from here
+    const int gsoff = (int)(reinterpret_cast<char*>(gs) - sm);
+
+    const int cfg = P_.slot_cfg[s];
+    int8_t* gl = P_.spins + P_.cfg_off[cfg];
+    long long* gg = reinterpret_cast<long long*>(P_.g + P_.slot_tab[s]);
+    for (int i = q; i < N; i += P) lat[i] = gl[i];
+    for (int k = q - kGuard; k < nb + kGuard; k += P) gs[k] = k >= 0 && k < nb ? gg[k] : kGuardValue;
+    __syncwarp();
+    const bool corr = OBS && P_.corr;
+    if (corr) {
+        plane_sums(rsum, csum, C, q, [&](int i) { return (int)lat[i]; }, P);
+        const uint64_t* gv0 = P_.visits + P_.slot_tab[s];
+        for (int k = q; k < nb; k += P) bcnt[k] = mod_transform(gv0[k]);
+        __syncwarp();
+    }
+
+    const int J = (int)I.J_u, sh = I.bin_shift;
+    const int Ewlo = (int)W.elo_u;
+    const long long lnf = P_.win_lnf[w];
+    const uint64_t sweeps0 = P_.slot_sweeps[s];
+    const uint32_t uid = (uint32_t)(s - I.first_slot);
+    const uint32_t k0 = (uint32_t)I.seed ^ uid, k1 = (uint32_t)(I.seed >> 32);
+    const int E0 = (int)P_.cfg_E[cfg];
+    const int b0 = (E0 - Ewlo) >> sh;
+    const bool bad = ((E0 - Ewlo) & ((1 << sh) - 1)) != 0 || b0 < 0 || b0 >= nb;
+    if (__ballot_sync(kFull, valid && bad)) {
+        if (lane == 0) atomicOr(&P_.counters[0], ERR_BOUNDS);
+        return;
+    }
+    int M = P_.cfg_M[3 * cfg];
+    const double invN = 1.0 / (double)N;
+    double* ob = OBS ? P_.obs + (size_t)P_.slot_tab[s] * P_.obs_stride : nullptr;
+
+    // thresholds of the 4C attempts from `a0` on (a multiple of 4) into batch `buf`
+    auto draw = [&](uint64_t a0, int buf) {
+        longlong2* dst = reinterpret_cast<longlong2*>(Tb + buf * 4 * C);
+#pragma unroll
+        for (int k = 0; k < SPL; ++k) {
+            const int bi = q + k * P;
+            if (bi < C) {
+                const uint64_t blk = (a0 >> 2) + (uint64_t)bi;
+                const Philox4 r = philox4x32_10(Philox4{(uint32_t)blk, (uint32_t)(blk >> 32), kStreamWL, 0u}, k0, k1);
+                dst[2 * bi] = make_longlong2(word_threshold(r.x) + lnf, word_threshold(r.y) + lnf);
+                dst[2 * bi + 1] = make_longlong2(word_threshold(r.z) + lnf, word_threshold(r.w) + lnf);
+            }
+        }
+    };
+
+    // A row's sites as the lattice stands, before the flips of the row above: spin, energy change without / with the
+    // left neighbour flipped, the correction if the site above flips; the last site's if the first flips.
+    int ns[SPL], nd0[SPL], nd1[SPL], nup[SPL], nwrap = 0;
+    auto prepare = [&](int y) {
+        const int8_t *row = lat + y * C, *up = lat + (y == 0 ? C - 1 : y - 1) * C, *down = lat + (y == C - 1 ? 0 : y + 1) * C;
+#pragma unroll
+        for (int k = 0; k < SPL; ++k) {
+            const int x = q + k * P;
+            ns[k] = nd0[k] = nd1[k] = nup[k] = 0;
+            if (x < C) {
+                const int si = row[x], su = up[x], sl = row[x == 0 ? C - 1 : x - 1], sr = row[x == C - 1 ? 0 : x + 1];
+                ns[k] = si;
+                nd0[k] = 2 * J * si * (su + sl + sr + down[x]);
+                nd1[k] = x > 0 ? nd0[k] - 4 * J * si * sl : nd0[k];
+                nup[k] = 4 * J * si * su;
+                if (x == C - 1) nwrap = -4 * J * si * sr;
+            }
+        }
+    };
+    auto finish = [&](int k, unsigned flips) {                 // table offsets, the row above having flipped `flips`
+        const int c = (flips >> (q + k * P)) & 1u ? nup[k] : 0;
+        return make_int2(((nd0[k] - c) >> sh) * 8, ((nd1[k] - c) >> sh) * 8);
+    };
+    auto wrap_offset = [&] { return __shfl_sync(kFull, (nwrap >> sh) * 8, gbase + (C - 1) % P); };
+
+    const uint64_t A0 = sweeps0 * (uint64_t)N;
+    draw(A0, 0);
+    prepare(0);
+    int cs[SPL];                                               // spins of the current row
+#pragma unroll
+    for (int k = 0; k < SPL; ++k) {
+        cs[k] = ns[k];
+        if (q + k * P < C) Db[q + k * P] = finish(k, 0u);
+    }
+    int cwrap = wrap_offset();
+    __syncwarp();
+    int2 E4[4];                                                // offsets and thresholds of the row's first four sites
+    long long T4[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { E4[i] = Db[i]; T4[i] = Tb[i]; }
+
+    int bc = gsoff + b0 * 8;                                   // current bin, g there, proposal, g there
+    long long gcv = gs[b0];
+    int bp = bc + E4[0].x;
+    long long gp = lds64(sm, bp);
+    int q0 = bc + E4[1].x, q1 = bp + E4[1].y;                  // the next proposal: this one rejected / accepted
+    long long bound = gcv - lnf + T4[0];
+
+    const int64_t total = (int64_t)p.nsweeps * C;
+    int y = 0;
+    for (int64_t t = 0; t < total; ++t) {
+        const int64_t tn = t + 1;
+        const int yn = y + 1 == C ? 0 : y + 1;
+        const long long* Tc = Tb + ((t >> 2) & 1) * 4 * C + (t & 3) * C;
+        const long long* Tn = Tb + ((tn >> 2) & 1) * 4 * C + (tn & 3) * C;
+        const int2* Dc = Db + (t & 1) * C;
+        int2* Dn = Db + (tn & 1) * C;
+        if ((tn & 3) == 0 && tn < total) {                     // the next row opens a batch: its buffer is not in use
+            draw(A0 + (uint64_t)tn * C, (tn >> 2) & 1);
+            __syncwarp();
+        }
+        prepare(yn);
+        long long Tr[C + 1];
+        int2 Er[C];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { Tr[i] = T4[i]; Er[i] = E4[i]; }
+        Tr[C] = Tn[0];
+        unsigned acc = 0;
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+            if ((j & 1) == 0 && j + 6 <= C) {                  // inputs are read four sites ahead
+                const longlong2 tv = reinterpret_cast<const longlong2*>(Tc)[(j + 4) >> 1];
+                const int4 d = reinterpret_cast<const int4*>(Dc)[(j + 4) >> 1];
+                Tr[j + 4] = tv.x; Tr[j + 5] = tv.y;
+                Er[j + 4] = make_int2(d.x, d.y); Er[j + 5] = make_int2(d.z, d.w);
+            }
+            const bool a = gp < bound;
+            const long long sel = a ? gp : gcv;
+            const int bnew = a ? bp : bc;
+            gcv = sel + lnf;
+            sts64(sm, bnew, gcv);
+            if (OBS) seqb[j] = bnew;
+            if (a) acc |= 1u << j;
+            if (j == 1 || j == 3) {                            // the next row's first sites: those above them are decided
+#pragma unroll
+                for (int i = j - 1; i <= j; ++i) {
+                    const int2 v = finish(i / P, acc);
+                    E4[i] = make_int2(__shfl_sync(kFull, v.x, gbase + i % P), __shfl_sync(kFull, v.y, gbase + i % P));
+                }
+            }
+            bound = sel + Tr[j + 1];
+            bp = a ? q1 : q0;
+            gp = lds64(sm, bp);                                // after this step's store
+            const int2 ev = j + 2 < C ? Er[j + 2] : E4[j + 2 - C];
+            const int wv = j + 2 == C - 1 && (acc & 1u) ? cwrap : 0;           // a row's last site sees its first
+            q0 = bnew + ev.x + wv;
+            q1 = bp + ev.y + wv;
+            bc = bnew;
+        }
+        unsigned plus = 0;
+#pragma unroll
+        for (int k = 0; k < SPL; ++k) {
+            const int x = q + k * P;
+            const unsigned bal = __ballot_sync(kFull, x < C && cs[k] > 0);
+            plus |= ((bal >> gbase) & ((1u << P) - 1u)) << (k * P);
+            if (x < C && ((acc >> x) & 1u)) lat[y * C + x] = (int8_t)(-cs[k]);
+        }
+        if (OBS) {
+            __syncwarp();
+            int first[SPL], visits[SPL];                       // is the step its bin's first of the row; the row's visits to it
+#pragma unroll
+            for (int k = 0; k < SPL; ++k) {
+                const int x = q + k * P;
+                first[k] = visits[k] = 0;
+                if (!valid || x >= C) continue;
+                const int b = (seqb[x] - gsoff) >> 3;
+                const int32_t Mv[1] = {M + chunk_dm(acc, plus, x)};
+                Ising2dModel::add_observables(ob + (size_t)b * P_.obs_stride, Mv, invN, P_.corr);
+                if (corr) {
+                    // G(q_min) at the steps whose bin count before the visit is a multiple of 1000: bcnt before the row
+                    // and the row's earlier visits.  (The lattice already holds the row's flips.)
+                    int earlier = 0;
+#pragma unroll
+                    for (int j = 0; j < C; ++j) {
+                        const int eq = seqb[j] == seqb[x] ? 1 : 0;
+                        earlier += j < x ? eq : 0;
+                        visits[k] += eq;
+                    }
+                    first[k] = earlier == 0;
+                    if ((bcnt[b] + earlier) % (int)kCountsPerTransform == 0) {
+                        const double Gq = plane_corr(rsum, csum, P_.qtab + I.qtab_off, C, y, chunk_dm(acc, plus, x), 0, x, acc,
+                                                     [&](int i) { return -(int)lat[y * C + i]; });
+                        red_global_add(ob + (size_t)b * P_.obs_stride + 3, invN * invN * Gq);
+                    }
+                }
+            }
+            if (corr) {
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < SPL; ++k) {
+                    const int x = q + k * P;
+                    if (valid && x < C && ((acc >> x) & 1u)) csum[x] += 2 * (int)lat[y * C + x];
+                    if (first[k]) bcnt[(seqb[x] - gsoff) >> 3] += visits[k];
+                }
+                if (valid && q == 0) rsum[y] += chunk_dm(acc, plus, 31);
+            }
+        }
+        M += chunk_dm(acc, plus, 31);
+        // the next row
+#pragma unroll
+        for (int k = 0; k < SPL; ++k) {
+            cs[k] = ns[k];
+            if (q + k * P < C) Dn[q + k * P] = finish(k, acc);
+        }
+        cwrap = wrap_offset();
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) T4[i] = Tn[i];
+        y = yn;
+    }
+    __syncwarp();
+    if (valid) {
+        for (int i = q; i < N; i += P) gl[i] = lat[i];
+        uint32_t* gH = P_.H + P_.slot_tab[s];
+        uint64_t* gv = P_.visits + P_.slot_tab[s];
+        for (int k = q; k < nb; k += P) {
+            const long long gnew = gs[k];
+            const int e = commit_visits(gH, gv, k, (gnew - gg[k]) / lnf, gnew);
+            if (e) atomicOr(&P_.counters[0], e);
+            gg[k] = gnew;
+        }
+        if (q == 0) {
+            if ((unsigned)(bc - gsoff) >= (unsigned)(nb * 8)) atomicOr(&P_.counters[0], ERR_BOUNDS);
+            P_.cfg_E[cfg] = (long long)Ewlo + ((long long)((bc - gsoff) >> 3) << sh);
+            P_.cfg_M[3 * cfg] = M;
+            P_.slot_sweeps[s] = sweeps0 + (uint64_t)p.nsweeps;
+        }
+    }
+}
+
+template <int G>
+SweepKernel rows_kernel_t(int C, bool obs)
+{
+    if (C == 4) return obs ? k_sweep_ising_rows<G, 4, true> : k_sweep_ising_rows<G, 4, false>;
+    if (C == 8) return obs ? k_sweep_ising_rows<G, 8, true> : k_sweep_ising_rows<G, 8, false>;
+    return obs ? k_sweep_ising_rows<G, 16, true> : k_sweep_ising_rows<G, 16, false>;
+}
+
+SweepKernel rows_kernel(int G, int C, bool obs) { return G == 2 ? rows_kernel_t<2>(C, obs) : rows_kernel_t<4>(C, obs); }
+
 // Ashkin-Teller: sweep = sigma pass then tau pass (wang_landau.hpp:109-119); the flavour toggles
 // after each pass.  A window holds tens of thousands of bins, so its logDoS stays in global memory;
 // the part around the walker is held in shared memory (TableCache below).
@@ -2517,6 +2800,7 @@ struct Launch {
     int counts = 0;         // bin-tracking kernel: visit counts beside g in shared memory (16 bytes per bin)
     int moments = 0;        // bin-tracking kernel with observables: moment sums in shared memory
     int crowded = 0;        // bin-tracking kernel with observables: the form of 168 registers
+    int rows = 0;           // k_sweep_ising_rows in its place: sites of a row
     int maxL = 0;
     int tree = 0;           // the global-table kernel may decide on the tree of outcomes
     int tables = 0;         // the global-table kernel (k_sweep_tables)
@@ -3024,7 +3308,8 @@ int at_carveout(rewl_engine* e, Launch& l)
 // moments in shared memory take 28 bytes a bin and save reductions to global memory (2048 walkers of 245 bins 31.2
 // against 29.0, 2944 walkers 26.2 against 33.0); two walkers a warp up to 24 walkers an SM, four beyond (4096 walkers of
 // 245 bins 41.1 against 55.2).
-double bins_cycles(int n, int nsm, int G, bool obs, bool cnt, bool mom, int smem)
+// rows: k_sweep_ising_rows with rows of so many sites.
+double bins_cycles(int n, int nsm, int G, bool obs, bool cnt, bool mom, int rows, int smem)
 {
     static const double kCycles[6][3][3] = {
         {{72, 97, 132}, {98, 131, 177}, {120, 165, 219}},              // g alone
@@ -3033,7 +3318,9 @@ double bins_cycles(int n, int nsm, int G, bool obs, bool cnt, bool mom, int smem
         {{95, 119, 159}, {128, 162, 216}, {196, 239, 285}},            //   moments in shared memory
         {{101, 118, 147}, {142, 168, 208}, {230, 266, 303}},           //   visits beside g
         {{88, 110, 145}, {119, 151, 200}, {199, 245, 290}}};           //   both
-    const auto& t = kCycles[obs ? 2 + 2 * cnt + mom : cnt][G == 1 ? 0 : G == 2 ? 1 : 2];
+    static const double kRows[2][2][2][3] = {{{{117, 144, 185}, {97, 125, 168}}, {{200, 222, 258}, {178, 208, 245}}},      // 8
+                                             {{{79, 93, 120}, {88, 112, 149}}, {{124, 139, 170}, {179, 203, 245}}}};       // 16
+    const double* t = rows ? kRows[rows == 16][obs][G == 4] : kCycles[obs ? 2 + 2 * cnt + mom : cnt][G == 1 ? 0 : G == 2 ? 1 : 2];
     const int warps = ((n + G - 1) / G + nsm - 1) / nsm;
     const int room = std::min(12, std::max(1, 228 * 1024 / (G * smem + 1024)));
     const int waves = (warps - 1) / room, rest = warps - waves * room;
@@ -3041,12 +3328,26 @@ double bins_cycles(int n, int nsm, int G, bool obs, bool cnt, bool mom, int smem
 }
 
 // The shape of a launch group of the bin-tracking kernel: walkers per warp (G; 0: any), visits beside g and moments in
-// shared memory, the cheapest that fits; fewer walkers a warp where G's do not fit a block.
+// shared memory, the cheapest that fits; fewer walkers a warp where G's do not fit a block.  Rows of 4, 8 and 16 sites go
+// one decision after another (k_sweep_ising_rows) once there are more walkers than schedulers, but for L = 16 with
+// correlators.
 void shape_bins(const rewl_engine* e, Launch& l, int nsm, int G)
 {
     const bool obs = e->desc.observables != 0, corr = e->desc.observables == 2;
     const int n = e->desc.persistent ? e->nslots : (int)l.slots.size();
     double best = 0;
+    l.rows = 0;
+    if ((l.maxL == 4 || l.maxL == 8 || (l.maxL == 16 && !corr)) && !e->desc.persistent && n > 4 * nsm && G != 1) {
+        const int smem = ((rows_smem(l.nbcap, l.maxL, obs, corr) + 127) & ~127) + 16;
+        for (int g : {4, 2}) {
+            if ((G && g > G) || g * smem > 200 * 1024) continue;
+            const double t = bins_cycles(n, nsm, g, obs, false, false, l.maxL, smem);
+            if (best != 0 && (G || t >= best)) continue;
+            best = t;
+            l.walkers_per_warp = g; l.counts = l.moments = l.crowded = 0; l.smem_per_warp = smem; l.rows = l.maxL;
+        }
+        if (l.rows) return;
+    }
     for (int g : {4, 2, 1}) {
         if (G ? g > G : g > 1 && g > n) continue;
         for (int c = 3; c >= 0; --c) {
@@ -3054,7 +3355,7 @@ void shape_bins(const rewl_engine* e, Launch& l, int nsm, int G)
             if (mom && !obs) continue;
             const int smem = bins_smem(g, l.nbcap, l.maxL, obs, corr, cnt, mom);
             if (g * smem > 200 * 1024 && (g > 1 || c > 0)) continue;
-            const double t = bins_cycles(n, nsm, g, obs, cnt, mom, smem);
+            const double t = bins_cycles(n, nsm, g, obs, cnt, mom, 0, smem);
             if (best != 0 && t >= best) continue;
             best = t;
             l.walkers_per_warp = g; l.counts = cnt; l.moments = mom; l.smem_per_warp = smem;
@@ -3231,6 +3532,10 @@ int plan_launches(rewl_engine* e)
         if (l.tables && !l.cache && !e->gsnap.p && e->table_total > 0)
             if (int rc = e->gsnap.alloc(e->table_total)) return rc;
     }
+    for (int G : {2, 4})
+        for (int C : {4, 8, 16})
+            for (int o = 0; o < 2; ++o)
+                CUDA_TRY(cudaFuncSetAttribute(rows_kernel(G, C, o), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     for (int G : {1, 2, 4})
         for (int o = 0; o < 8; ++o)
             CUDA_TRY(cudaFuncSetAttribute(bins_kernel(G, o & 1, o & 2, o & 4), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
@@ -3364,7 +3669,8 @@ int launch_group(rewl_engine* e, Launch& l, cudaStream_t stream, int nsweeps, co
         const int warps = (sp.nslots + G - 1) / G;
         const int blocks = (warps + l.wpb - 1) / l.wpb;
         const size_t smem = (size_t)l.wpb * G * l.smem_per_warp;
-        bins_kernel(G, P.obs != nullptr, l.counts, l.crowded)<<<blocks, 32 * l.wpb, smem, stream>>>(sp);
+        const SweepKernel fn = l.rows ? rows_kernel(G, l.rows, P.obs != nullptr) : bins_kernel(G, P.obs != nullptr, l.counts, l.crowded);
+        fn<<<blocks, 32 * l.wpb, smem, stream>>>(sp);
     } else {
         const int blocks = (sp.nslots + l.wpb - 1) / l.wpb;
         const size_t smem = (size_t)l.wpb * l.smem_per_warp;

@@ -54,3 +54,36 @@ def test_walkers_per_warp_is_kept_where_it_fits(engine_lib, per_warp, obs):
             x, y = a.export_walker(w), b.export_walker(w)
             for k in x:
                 assert np.array_equal(x[k], y[k]), (w, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("obs", [0, 1, 2])
+@pytest.mark.parametrize("per_warp", [0, 2, 4])
+@pytest.mark.parametrize("L, windows, J", [(4, 1, 1.0), (8, 4, 1.0), (8, 3, -1.0), (16, 8, 1.0)])
+def test_short_rows_one_decision_after_another(engine_lib, L, windows, J, per_warp, obs):
+    """Rows of 4, 8 and 16 sites in launches of more walkers than schedulers (k_sweep_ising_rows): the first instance of
+    such a batch equals an engine of its own, whose walkers go through the tree.  (J = -1 turns the energies around;
+    enough visits for several transforms of the correlators.)"""
+    rg = engine_lib
+    N = L * L
+
+    def engine(instances, **kw):
+        inss = [rg.Instance(model=rg.MODEL_ISING2D, L=L, J=J, energy_min=-2.0 * N, energy_max=2.0 * N + 4, bin_width=4.0, num_windows=windows,
+                            replicas_per_window=8, init_mode=0, seed=40 + i) for i in range(instances)]
+        return rg.Engine(rg.Batch(instances=inss, sweeps_per_exchange=33, sweeps_per_check=99, observables=obs, **kw))
+    with engine(640 // (8 * windows) + 1, walkers_per_warp=per_warp) as a, engine(1, walkers_per_warp=1) as b:
+        # (L = 16 with correlators stays with the tree, whose choice is one walker a warp here)
+        assert a.launch_shapes()[0][2] in ((per_warp,) if per_warp else (1,) if L == 16 and obs == 2 else (2, 4))
+        for _ in range(3):
+            for e in (a, b):
+                e.run_cycles(1)
+            for w in range(b.num_walkers):
+                x, y = a.export_walker(w), b.export_walker(w)
+                for k in x:
+                    assert np.array_equal(x[k], y[k]), (w, k)
+        for w in range(windows if obs else 0):
+            x, y = a.window_observables(0, w), b.window_observables(0, w)
+            assert np.array_equal(x[:, -1], y[:, -1])
+            # sums of at most 8 x 297 N terms in another order, to 2^-53 of the sum each; the table of the
+            # correlators' transforms holds 60 places
+            np.testing.assert_allclose(x, y, rtol=8 * 297 * N * 2.0**-53, atol=1e-13)
