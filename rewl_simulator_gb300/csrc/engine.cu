@@ -426,7 +426,6 @@ struct SweepParams {
     int counts;              // bin-tracking kernel: visit counts beside g in shared memory
     int moments;             // bin-tracking kernel with observables: moment sums in shared memory
     int cache;               // global-table kernel: bins of each walker's table in shared memory
-    int replay;              // global-table kernel, serial chain: recorded uniforms
 };
 
 // Per-warp staging of one chunk for the lane-0 resolver: energy change without /
@@ -1706,31 +1705,35 @@ static_assert(kSerialStage % 16 == 0 && offsetof(TableStage, T) % 16 == 0 && siz
 struct TableChain {
     long long v, vn, gc, draws;
     long long G0, G1;        // logDoS loaded for step j's proposal if step j-1 was rejected / accepted
+    long long T;             // step j's threshold
     longlong2 q;             // step j+1's proposals
     int b, bn, err;
     bool inr, ap;            // step j's proposal in the window; step j-1 accepted
     unsigned acc;
 };
 
-// One step j of a chunk decided serially by lane 0, software-pipelined two deep: replayed runs,
-// whose recorded uniforms are consumed on demand, and windows whose bins the tree below cannot hold
-// in a register's high word.  On entry (vn, bn, inr) is step j's proposal, and its logDoS is G1 or G0
+// One step j of a chunk decided serially by lane 0, software-pipelined two deep: replayed runs
+// (REPLAY), whose recorded uniforms are consumed on demand, energy changes too large for the tree's
+// positions, and crowded launches with observables.  Unrolled by four, the next step's threshold read a
+// step ahead, the replayed form compiled apart: Ashkin-Teller L = 32, 2048 walkers 8.6 -> 9.2e9 flips/s, with moments
+// 6.6 -> 7.1e9.  On entry (vn, bn, inr) is step j's proposal, and its logDoS is G1 or G0
 // (as step j-1 was accepted or not), loaded during step j-1.  With PREFETCH the two proposals of step
 // j+1 (step j rejected: from v; accepted: from vn) are loaded first.  A value loaded before step j-1's
 // write to bin b is stale exactly when the proposal is b: gc replaces it.  LOADQ: step j+2 exists and
 // its proposals are read from shared memory now.  WRAPFIX: step j+1 is the last site of a whole-row
 // chunk, whose right neighbour is the row's first site, flipped in this chunk iff bit 0 of acc.
-template <bool OBS, bool PREFETCH, bool LOADQ, bool WRAPFIX>
+template <bool REPLAY, bool OBS, bool PREFETCH, bool LOADQ, bool WRAPFIX>
 __device__ __forceinline__ void serial_step(TableChain& c, const int j, TableStage* st, long long* gg, const int nb,
-                                        const int sh, const long long lnf, const DevPtrs& P, const bool replay,
+                                        const int sh, const long long lnf, const DevPtrs& P,
                                         const long long thr_off, const long long thr_n)
 {
-    long long t0 = 0, t1 = 0, G0 = 0, G1 = 0;
+    long long t0 = 0, t1 = 0, G0 = 0, G1 = 0, Tn = 0;
     longlong2 qn = make_longlong2(0, 0);
     int b0 = 0, b1 = 0;
     bool i0 = false, i1 = false;
     if (LOADQ) qn = st->du[j + 2];
     if (PREFETCH) {
+        if (!REPLAY) Tn = st->T[j + 1];
         t0 = c.v + c.q.x;
         t1 = c.vn + c.q.y;
         if (WRAPFIX) {
@@ -1748,8 +1751,8 @@ __device__ __forceinline__ void serial_step(TableChain& c, const int j, TableSta
     const long long gn = c.bn == c.b ? c.gc : (c.ap ? c.G1 : c.G0);
     const long long d = gn - c.gc;
     bool a;
-    if (!replay) {
-        a = c.inr && d < st->T[j];
+    if (!REPLAY) {
+        a = c.inr && (d < c.T);
     } else if (c.inr && d > 0) {
         if (c.draws >= thr_n) { c.err = ERR_REPLAY_EXHAUSTED; a = false; }
         else { a = d < P.thr[thr_off + c.draws]; ++c.draws; }
@@ -1765,6 +1768,7 @@ __device__ __forceinline__ void serial_step(TableChain& c, const int j, TableSta
         c.bn = a ? b1 : b0;
         c.inr = a ? i1 : i0;
         c.G0 = G0; c.G1 = G1; c.ap = a;
+        c.T = Tn;
         c.q = qn;
     }
 }
@@ -1930,7 +1934,9 @@ struct TableCache {
 // tree of 64-bit positions with 32 thresholds a draw, 122 now; 512 walkers 411, 210, 149; 2048 walkers 832,
 // 557, 411 (with the tables of a longer run 432, the chain 439: two waves of seven warps per SM, each with
 // its cached bins).
-template <class Model, bool TREE, bool OBS>
+enum TableMode : int { kTableSerial = 0, kTableTree = 1, kTableReplay = 2 };
+
+template <class Model, int MODE, bool OBS>
 __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const int li, unsigned char* warp_base)
 {
     constexpr int NP = Model::kPlanes, NM = Model::kMags, NC = Model::kCorrPlanes;
@@ -1946,7 +1952,7 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
     // from the start of shared memory, so that the accesses below are shared-memory accesses
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned char* base = smem + (int)(warp_base - smem);
-    const bool replay = !TREE && p.replay;
+    constexpr bool TREE = MODE == kTableTree, REPLAY = MODE == kTableReplay;
     TableStage* st = reinterpret_cast<TableStage*>(base);
     int8_t* sp = reinterpret_cast<int8_t*>(base) + (TREE ? (int)sizeof(TableStage) : kSerialStage);     // NP planes of N spins
     const int64_t* hf = I.field_off >= 0 ? P.fields + I.field_off : nullptr;
@@ -2013,7 +2019,7 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
         c.v = vr;
         c.b = (int)(vr >> sh);
         c.gc = gg[c.b];
-        if (replay) { c.draws = P.slot_draws[s]; thr_off = P.slot_thr_off[s]; thr_n = P.slot_thr_n[s]; }
+        if (REPLAY) { c.draws = P.slot_draws[s]; thr_off = P.slot_thr_off[s]; thr_n = P.slot_thr_n[s]; }
     }
     // the tree's position: bin, numerator within it in units of 2^zeros, and what is below them for good
     int b0 = (int)(vr >> sh), fr = (int)((vr >> zeros) & ((1ll << shz) - 1));
@@ -2102,7 +2108,7 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
                         st->du[lane] = make_longlong2(d0, d0 + dl);
                     }
                     if (wraps && lane == C - 1) st->wcu = wrap;
-                    if (!TREE && !replay) st->T[lane] = word_threshold(philox_word(seed, uid, attempt + (uint64_t)lane, kStreamWL));
+                    if (!TREE && !REPLAY) st->T[lane] = word_threshold(philox_word(seed, uid, attempt + (uint64_t)lane, kStreamWL));
                 }
                 // bins a block's nodes can lie away from its start: five steps, the last site's with its wrap term
                 // (fields and the other bonds can cancel what it would be part of)
@@ -2121,15 +2127,17 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
                         c.inr = (unsigned)c.bn < (unsigned)nb;
                         c.G0 = c.G1 = gg[min((unsigned)c.bn, (unsigned)(nb - 1))];
                         c.ap = false;
+                        if (!REPLAY) c.T = st->T[0];
                         if (C == 1) {
-                            serial_step<OBS, false, false, false>(c, 0, st, gg, nb, sh, lnf, P, replay, thr_off, thr_n);
+                            serial_step<REPLAY, OBS, false, false, false>(c, 0, st, gg, nb, sh, lnf, P, thr_off, thr_n);
                         } else {
                             c.q = st->du[1];
+#pragma unroll 4
                             for (int j = 0; j < C - 2; ++j)
-                                serial_step<OBS, true, true, false>(c, j, st, gg, nb, sh, lnf, P, replay, thr_off, thr_n);
-                            if (wraps) serial_step<OBS, true, false, true>(c, C - 2, st, gg, nb, sh, lnf, P, replay, thr_off, thr_n);
-                            else serial_step<OBS, true, false, false>(c, C - 2, st, gg, nb, sh, lnf, P, replay, thr_off, thr_n);
-                            serial_step<OBS, false, false, false>(c, C - 1, st, gg, nb, sh, lnf, P, replay, thr_off, thr_n);
+                                serial_step<REPLAY, OBS, true, true, false>(c, j, st, gg, nb, sh, lnf, P, thr_off, thr_n);
+                            if (wraps) serial_step<REPLAY, OBS, true, false, true>(c, C - 2, st, gg, nb, sh, lnf, P, thr_off, thr_n);
+                            else serial_step<REPLAY, OBS, true, false, false>(c, C - 2, st, gg, nb, sh, lnf, P, thr_off, thr_n);
+                            serial_step<REPLAY, OBS, false, false, false>(c, C - 1, st, gg, nb, sh, lnf, P, thr_off, thr_n);
                         }
                     }
                     acc = __shfl_sync(kFull, c.acc, 0);
@@ -2334,17 +2342,17 @@ __device__ __forceinline__ void sweep_tables_warp(const SweepParams& p, const in
         for (int m = 0; m < NM; ++m) P.cfg_M[3 * cfg + m] = M[m];
         P.slot_sweeps[s] = sweeps0 + (uint64_t)p.nsweeps;
         if (NP == 2) P.slot_flavour[s] = flavour;
-        if (replay) P.slot_draws[s] = c.draws;
+        if (REPLAY) P.slot_draws[s] = c.draws;
         if (c.err) atomicOr(&P.counters[0], c.err);
     }
 }
 
-template <class Model, bool TREE, bool OBS>
+template <class Model, int MODE, bool OBS>
 __global__ void __launch_bounds__(256, 2) k_sweep_tables(const SweepParams p)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int wib = threadIdx.x >> 5;
-    sweep_tables_warp<Model, TREE, OBS>(p, blockIdx.x * (blockDim.x >> 5) + wib, smem + (size_t)wib * p.smem_per_warp);
+    sweep_tables_warp<Model, MODE, OBS>(p, blockIdx.x * (blockDim.x >> 5) + wib, smem + (size_t)wib * p.smem_per_warp);
 }
 
 // --------------------------------------------------------------------------
@@ -2383,8 +2391,8 @@ __device__ __noinline__ void fused_bins(const SweepParams& p, int unit, unsigned
 template <class Model, bool OBS>
 __device__ __noinline__ void fused_tables(const SweepParams& p, int unit, unsigned char* base)
 {
-    if (p.cache) sweep_tables_warp<Model, true, OBS>(p, unit, base);
-    else sweep_tables_warp<Model, false, OBS>(p, unit, base);
+    if (p.cache) sweep_tables_warp<Model, kTableTree, OBS>(p, unit, base);
+    else sweep_tables_warp<Model, kTableSerial, OBS>(p, unit, base);
 }
 
 template <bool OBS>
@@ -2403,7 +2411,7 @@ __global__ void __launch_bounds__(128) k_sweep_fused(const FusedParams fp)
         const FusedGroup& G = fp.g[gi];
         SweepParams sp;
         sp.P = fp.P; sp.slots = G.slots; sp.nslots = G.nslots; sp.nsweeps = fp.nsweeps;
-        sp.smem_per_warp = G.smem_per_warp; sp.nbcap = G.nbcap; sp.counts = G.counts; sp.moments = G.moments; sp.cache = G.cache; sp.replay = 0;
+        sp.smem_per_warp = G.smem_per_warp; sp.nbcap = G.nbcap; sp.counts = G.counts; sp.moments = G.moments; sp.cache = G.cache;
         const int unit = t - G.first_task;
         switch (G.kind) {
         case kFusedBins: fused_bins<OBS>(sp, unit, base); break;
@@ -2810,16 +2818,17 @@ struct Launch {
 };
 
 template <class Model>
-SweepKernel table_kernel_t(bool tree, bool obs)
+SweepKernel table_kernel_t(int mode, bool obs)
 {
-    if (tree) return obs ? k_sweep_tables<Model, true, true> : k_sweep_tables<Model, true, false>;
-    return obs ? k_sweep_tables<Model, false, true> : k_sweep_tables<Model, false, false>;
+    if (mode == kTableTree) return obs ? k_sweep_tables<Model, kTableTree, true> : k_sweep_tables<Model, kTableTree, false>;
+    if (mode == kTableReplay) return obs ? k_sweep_tables<Model, kTableReplay, true> : k_sweep_tables<Model, kTableReplay, false>;
+    return obs ? k_sweep_tables<Model, kTableSerial, true> : k_sweep_tables<Model, kTableSerial, false>;
 }
 
-SweepKernel table_kernel(int model, bool tree, bool obs)
+SweepKernel table_kernel(int model, int mode, bool obs)
 {
-    return model == REWL_MODEL_ISING2D ? table_kernel_t<Ising2dModel>(tree, obs)
-                                       : table_kernel_t<AshkinTeller2dModel>(tree, obs);
+    return model == REWL_MODEL_ISING2D ? table_kernel_t<Ising2dModel>(mode, obs)
+                                       : table_kernel_t<AshkinTeller2dModel>(mode, obs);
 }
 
 } // namespace
@@ -3269,6 +3278,11 @@ int tree_eligible(const HostInst& H, const rewl_batch_desc& D)
     return 8.0 * std::ldexp(move, -even) * (double)(H.dev.bin_mul >> zeros) + std::ldexp(1.0, H.dev.bin_shift - zeros - even) < 2147483648.0 ? 1 : 0;
 }
 
+int table_mode(const rewl_engine* e, const Launch& l)
+{
+    return l.cache ? kTableTree : e->desc.rng_mode == REWL_RNG_REPLAY ? kTableReplay : kTableSerial;
+}
+
 // Streaming multiprocessors of the engine's device (152 on a GB300).
 int sm_count(const rewl_engine* e)
 {
@@ -3285,7 +3299,7 @@ int at_carveout(rewl_engine* e, Launch& l)
 {
     if (!l.tables) return REWL_OK;
     const int nsm = sm_count(e);
-    const SweepKernel fn = table_kernel(l.model, l.cache > 0, e->desc.observables != 0);
+    const SweepKernel fn = table_kernel(l.model, table_mode(e, l), e->desc.observables != 0);
     const int threads = 32 * l.wpb;
     const size_t smem = (size_t)l.wpb * l.smem_per_warp;
     int occ = 0;
@@ -3522,7 +3536,7 @@ int plan_launches(rewl_engine* e)
     CUDA_TRY(cudaFuncSetAttribute(k_sweep_ising<false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(k_sweep_ising<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     CUDA_TRY(cudaFuncSetAttribute(k_sweep_ising<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < 3; ++r)
         for (int o = 0; o < 2; ++o)
             for (int m : {REWL_MODEL_ISING2D, REWL_MODEL_ASHKIN_TELLER2D})
                 CUDA_TRY(cudaFuncSetAttribute(table_kernel(m, r, o), cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
@@ -3663,7 +3677,7 @@ int launch_group(rewl_engine* e, Launch& l, cudaStream_t stream, int nsweeps, co
     const bool replay = e->desc.rng_mode == REWL_RNG_REPLAY;
     SweepParams sp;
     sp.P = P; sp.slots = l.d_slots.p; sp.nslots = (int)l.slots.size(); sp.nsweeps = nsweeps;
-    sp.smem_per_warp = l.smem_per_warp; sp.nbcap = l.nbcap; sp.counts = l.counts; sp.moments = l.moments; sp.cache = l.cache; sp.replay = replay;
+    sp.smem_per_warp = l.smem_per_warp; sp.nbcap = l.nbcap; sp.counts = l.counts; sp.moments = l.moments; sp.cache = l.cache;
     if (l.bins) {
         const int G = l.walkers_per_warp;
         const int warps = (sp.nslots + G - 1) / G;
@@ -3675,7 +3689,7 @@ int launch_group(rewl_engine* e, Launch& l, cudaStream_t stream, int nsweeps, co
         const int blocks = (sp.nslots + l.wpb - 1) / l.wpb;
         const size_t smem = (size_t)l.wpb * l.smem_per_warp;
         if (l.tables) {
-            const SweepKernel fn = table_kernel(l.model, l.cache > 0, e->desc.observables != 0);
+            const SweepKernel fn = table_kernel(l.model, table_mode(e, l), e->desc.observables != 0);
             if (l.carveout >= 0) CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, l.carveout));
             fn<<<blocks, 32 * l.wpb, smem, stream>>>(sp);
         } else {
