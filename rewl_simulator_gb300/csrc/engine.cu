@@ -2395,8 +2395,9 @@ __device__ __noinline__ void fused_tables(const SweepParams& p, int unit, unsign
     else sweep_tables_warp<Model, kTableSerial, OBS>(p, unit, base);
 }
 
+// (three blocks an SM: without saying so the compiler settles at 128 registers and spills, 5 % slower on Ising L = 32)
 template <bool OBS>
-__global__ void __launch_bounds__(128) k_sweep_fused(const FusedParams fp)
+__global__ void __launch_bounds__(128, 3) k_sweep_fused(const FusedParams fp)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -3266,14 +3267,19 @@ bool bins_eligible(const InstDev& I, const rewl_batch_desc& D, int max_window_bi
 // in numerator units without the zeros that all changes end in (three changes more leave room for the
 // terms on the way): bins of 0.05 take single flips of up to 100 energy units, bins of 1 of up to 500.
 // Beyond that, the serial chain.
+double largest_move(const HostInst& H)                 // of a flip, in energy units
+{
+    double h = 0;
+    for (double f : H.fields) h = std::max(h, std::fabs(f));
+    return 2.0 * (4.0 * std::fabs((double)H.dev.J_u) + 4.0 * std::fabs((double)H.dev.K_u) + std::ldexp(h, H.dev.escale));
+}
+
 int tree_eligible(const HostInst& H, const rewl_batch_desc& D)
 {
     if (D.rng_mode != REWL_RNG_PHILOX) return 0;
     int zeros = 0;
     while (zeros < H.dev.bin_shift && (H.dev.bin_mul >> zeros & 1) == 0) ++zeros;
-    double h = 0;
-    for (double f : H.fields) h = std::max(h, std::fabs(f));
-    const double move = 2.0 * (4.0 * std::fabs((double)H.dev.J_u) + 4.0 * std::fabs((double)H.dev.K_u) + std::ldexp(h, H.dev.escale));
+    const double move = largest_move(H);
     const int even = zeros < H.dev.bin_shift ? 1 : 0;
     return 8.0 * std::ldexp(move, -even) * (double)(H.dev.bin_mul >> zeros) + std::ldexp(1.0, H.dev.bin_shift - zeros - even) < 2147483648.0 ? 1 : 0;
 }
@@ -3313,6 +3319,9 @@ int at_carveout(rewl_engine* e, Launch& l)
     return REWL_OK;
 }
 
+// Blocks of `smem` bytes that an SM's shared memory holds (228 KB, 1 KB of it per block reserved, in units of 128 bytes)
+int blocks_per_sm(int smem) { return std::max(1, 228 * 1024 / ((smem + 1024 + 127) & ~127)); }
+
 // The time of a launch of n walkers of the bin-tracking kernel, G a warp, in cycles per flip of a walker: as many
 // warps as registers (12 warps) and shared memory hold on an SM run at once, in full waves and a last one, and take what
 // the busiest of its four schedulers does.  Measured at L = 48, windows of 114 bins, 1 to 3 warps a scheduler; equals
@@ -3336,7 +3345,7 @@ double bins_cycles(int n, int nsm, int G, bool obs, bool cnt, bool mom, int rows
                                              {{{79, 93, 120}, {88, 112, 149}}, {{124, 139, 170}, {179, 203, 245}}}};       // 16
     const double* t = rows ? kRows[rows == 16][obs][G == 4] : kCycles[obs ? 2 + 2 * cnt + mom : cnt][G == 1 ? 0 : G == 2 ? 1 : 2];
     const int warps = ((n + G - 1) / G + nsm - 1) / nsm;
-    const int room = std::min(12, std::max(1, 228 * 1024 / (G * smem + 1024)));
+    const int room = std::min(12, blocks_per_sm(G * smem));
     const int waves = (warps - 1) / room, rest = warps - waves * room;
     return waves * t[(room - 1) / 4] + t[(rest - 1) / 4];
 }
@@ -3377,7 +3386,7 @@ void shape_bins(const rewl_engine* e, Launch& l, int nsm, int G)
         if (G && best != 0) break;
     }
     l.crowded = obs && (n + l.walkers_per_warp - 1) / l.walkers_per_warp > 8 * nsm &&
-                228 * 1024 / (l.walkers_per_warp * l.smem_per_warp + 1024) > 8;
+                blocks_per_sm(l.walkers_per_warp * l.smem_per_warp) > 8;
 }
 
 // A launch group's shape: walkers per warp (bin-tracking kernel) and warps per block, if the
@@ -3385,6 +3394,39 @@ void shape_bins(const rewl_engine* e, Launch& l, int nsm, int G)
 bool shape_fits(const Launch& l, int G, int wpb)
 {
     return (size_t)wpb * (l.bins ? G : 1) * l.smem_per_warp <= 200 * 1024;
+}
+
+// Bins of each walker's table that the global-table kernel's tree keeps in shared memory (a power of two; 0: the serial
+// chain is the better form, which only launches with observables take: the others are within 2 % in long launches, and
+// the chain's copy of the tables makes short ones 1.3 times as long), for n walkers of nb bins whose flips move them up to `move` bins; `fixed` bytes a walker beside
+// them, 12 a bin.  Time in cycles per flip of a walker: as many warps as registers (16) and shared memory hold run at
+// once, in full waves and a last one; the fewer moves the cached bins span, the more often the walker leaves them.
+// Measured on Ashkin-Teller L = 12 to 32, bins of 0.05, 0.25 and 1.0 (moves of 300, 60 and 15 bins), e9 flips/s:
+//   1024 walkers, 512 / 1024 / 2048 bins: bins of 0.05 4.0 / 6.3 / 8.9, of 0.25 11.6 / 12.9 / 13.4
+//   2048 walkers, 512 / 1024 / 2048 bins / chain: 0.05 7.0 / 7.5 / 9.5 / 9.2, 0.25 16.6 / 13.5 / 13.5 / 11.5; with moments
+//   5.2 / 4.9 / 5.8 / 7.1 and 9.6 / 7.1 / 7.3 / 8.4 (the moments' FP64 latency wants warps)
+// More than kMinCache bins only where all of the engine's walkers could have them (an uneven batch of 352 walkers, 256 of
+// them Ashkin-Teller: 4096 bins 10.4 ms, 8192 11.2).
+int table_cache(int n, int all, int nsm, int observables, int nb, double move, int fixed_tree, int fixed_chain)
+{
+    static const double kTree[4] = {150, 215, 265, 300}, kChain[4] = {310, 370, 440, 480};       // warps a scheduler
+    static const double kObs[2][3] = {{1.0, 1.7, 1.85}, {1.0, 1.3, 1.6}};
+    auto cycles = [&](const double* t, int smem) {
+        const int warps = (n + nsm - 1) / nsm, room = std::min(16, blocks_per_sm(smem));
+        const int waves = (warps - 1) / room, rest = warps - waves * room;
+        return waves * t[(room - 1) / 4] + t[(rest - 1) / 4];
+    };
+    int cache = 0;
+    double best = observables ? cycles(kChain, fixed_chain) * kObs[1][observables] : DBL_MAX;
+    for (int c = 256; fixed_tree + 12 * c <= 200 * 1024; c *= 2) {
+        if (c > kMinCache && blocks_per_sm(fixed_tree + 12 * c) < (all + nsm - 1) / nsm) break;
+        const double moves = c / move;
+        const double reach = c >= nb || moves >= 24 ? 1.0 : moves >= 12 ? 0.95 : moves >= 6 ? 0.9 : moves >= 3 ? 0.71 : moves >= 1.5 ? 0.5 : 0.35;
+        const double t = cycles(kTree, fixed_tree + 12 * c) * kObs[0][observables] / reach;
+        if (t <= best) { best = t; cache = c; }                // (equals go to more bins)
+        if (c >= nb) break;
+    }
+    return cache;
 }
 
 // The persistent launch: every group's walkers as tasks of one work-stealing kernel.  Groups are
@@ -3470,6 +3512,8 @@ int plan_launches(rewl_engine* e)
         }
         plans[idx].slots.push_back(s);
     }
+    int table_walkers = 0;                                     // of all groups that may have their tables in global memory
+    for (const auto& l : plans) table_walkers += l.bins ? 0 : (int)l.slots.size();
     for (auto& l : plans) {
         int maxN = 0, maxnb = 0, maxL = 0;
         const bool corr = e->desc.observables == 2;
@@ -3504,21 +3548,25 @@ int plan_launches(rewl_engine* e)
             } else {
                 const int planes = l.model == REWL_MODEL_ISING2D ? 1 : 2;
                 l.nbcap = 0;
-                // With observables and more walkers than one wave with that many bins holds, the serial chain:
-                // the moments' FP64 latency wants warps more than the tree (L = 32, moments, 1024 / 1536 / 2048
-                // walkers: tree 5.8 / 4.7 / 5.9, chain 4.5 / 5.9 / 6.6e9 flips/s)
-                const bool crowded = e->desc.observables && !e->desc.persistent && e->nslots > 7 * nsm;
-                l.cache = l.tree && !crowded ? 256 : 0;
-                const int fixed = (int)((l.cache ? sizeof(TableStage) : kSerialStage) + ((planes * maxN + 15) & ~15) + (corr ? (8 * planes * maxL + 15) & ~15 : 0));
-                // as much of every walker's table as the walkers sharing an SM leave room for, but no less than
-                // 2048 bins (the rest of the walkers then wait for a second wave): Ashkin-Teller L = 32 at bins
-                // of 0.05, 2048 walkers, 512 / 1024 / 2048 bins 7.1 / 7.8 / 10.3e9 flips/s from flat tables and
-                // 7.1 / 7.6 / 9.6e9 in a longer run
-                const int per_sm = e->desc.persistent ? 8 : std::max(1, std::min(32, (e->nslots + nsm - 1) / nsm));
-                while (l.cache && l.cache < maxnb && fixed + 24 * l.cache <= 200 * 1024 &&
-                       (l.cache < kMinCache || fixed + 24 * l.cache + 1040 <= 225 * 1024 / per_sm))
-                    l.cache *= 2;
-                l.smem_per_warp = fixed + 12 * l.cache;
+                auto fixed = [&](size_t stage) {
+                    return (int)(stage + ((planes * maxN + 15) & ~15) + (corr ? (8 * planes * maxL + 15) & ~15 : 0));
+                };
+                if (l.tree && e->desc.persistent) {
+                    // eight walkers an SM, but no less than 2048 bins
+                    l.cache = 256;
+                    const int f = fixed(sizeof(TableStage));
+                    while (l.cache < maxnb && f + 24 * l.cache <= 200 * 1024 &&
+                           (l.cache < kMinCache || f + 24 * l.cache + 1040 <= 225 * 1024 / 8))
+                        l.cache *= 2;
+                } else if (l.tree) {
+                    double move = 1.0;
+                    for (int s : l.slots) {
+                        const HostInst& H = e->inst[e->h_slot_inst[s]];
+                        move = std::max(move, std::ldexp(largest_move(H) * (double)H.dev.bin_mul, -H.dev.bin_shift));
+                    }
+                    l.cache = table_cache(table_walkers, e->nslots, nsm, e->desc.observables, maxnb, move, fixed(sizeof(TableStage)), fixed(kSerialStage));
+                }
+                l.smem_per_warp = fixed(l.cache ? sizeof(TableStage) : kSerialStage) + 12 * l.cache;
             }
         }
         if (!l.bins) {
