@@ -969,20 +969,23 @@ constexpr int kTakeRows = 256;
 int take_blocks(int n) { return (n + kTakeRows - 1) / kTakeRows; }
 __global__ void __launch_bounds__(kTakeRows) k_take(const float* out, int n, float* y, float* acted)
 {
-    __shared__ int flag;
     step_wait();
-    if (threadIdx.x == 0) {
-        flag = *reinterpret_cast<const volatile int*>(&g_tc_error);
-        if (acted) acted[blockIdx.x] = flag ? 1.f : 0.f;
-    }
-    __syncthreads();
     const int i = blockIdx.x * kTakeRows + threadIdx.x;
-    if (i < n) y[i] = flag ? __int_as_float(0x7FC00000) : out[(size_t)i * kOut];
+    const float v = i < n ? out[(size_t)i * kOut] : 0.f;
+    const int flag = __syncthreads_or(*reinterpret_cast<const volatile int*>(&g_tc_error));
+    if (i < n) y[i] = flag ? __int_as_float(0x7FC00000) : v;
+    if (acted && threadIdx.x == 0) acted[blockIdx.x] = flag ? 1.f : 0.f;
 }
-// whether a block of k_take discarded its rows
+// whether a block of k_take discarded its rows; whether one may have, by the first row of each
 bool any_discarded(const float* acted, int n)
 {
     return std::any_of(acted, acted + take_blocks(n), [](float f) { return f != 0.f; });
+}
+bool maybe_discarded(const float* y, int n)
+{
+    for (int i = 0; i < n; i += kTakeRows)
+        if (y[i] != y[i]) return true;
+    return false;
 }
 
 // the caller's n rows as they are to the device, and from there into rows x kIn bf16: the copy is
@@ -1123,18 +1126,19 @@ int rewl_mlp_predict(rewl_mlp* m, const float* X, int32_t n, int32_t in_dim, flo
     int rc = ensure_batch(m, Bp);
     if (rc) return rc;
     if ((rc = upload_features(m, X, n, in_dim, Bp, m->H[0].p)) || (rc = forward(m, Bp, false))) return rc;
-    // the last hidden layer's buffer is read by now: the first column goes there and what k_take's blocks
-    // acted on behind it (the buffer has at least 128 bytes a row), in one copy to the host
+    // the last hidden layer's buffer is read by now: the first column goes there, n floats to the host, and behind
+    // it what k_take's blocks acted on (the buffer has at least 128 bytes a row)
     float* first = reinterpret_cast<float*>(m->H[m->layers].p);
-    const size_t words = (size_t)n + take_blocks(n);
-    const std::unique_ptr<float[]> h(new (std::nothrow) float[words]);
-    if (!h) return mfail(REWL_ENOMEM, "no host memory for %zu results", words);
     MCUDA(launch_next(k_take, dim3(take_blocks(n)), kTakeRows, 0, m->stream, m->out.p, n, first, first + n));
     m->launches++;
-    MCUDA(cudaMemcpyAsync(h.get(), first, words * 4, cudaMemcpyDeviceToHost, m->stream));
+    MCUDA(cudaMemcpyAsync(y, first, (size_t)n * 4, cudaMemcpyDeviceToHost, m->stream));
     MCUDA(cudaStreamSynchronize(m->stream));
-    std::copy(h.get(), h.get() + n, y);
-    return any_discarded(h.get() + n, n) ? tc_timed_out() : REWL_OK;
+    if (!maybe_discarded(y, n)) return REWL_OK;
+    const std::unique_ptr<float[]> acted(new (std::nothrow) float[take_blocks(n)]);
+    if (!acted) return mfail(REWL_ENOMEM, "no host memory for the products' status");
+    MCUDA(cudaMemcpyAsync(acted.get(), first + n, (size_t)take_blocks(n) * 4, cudaMemcpyDeviceToHost, m->stream));
+    MCUDA(cudaStreamSynchronize(m->stream));
+    return any_discarded(acted.get(), n) ? tc_timed_out() : REWL_OK;
 }
 
 // One forward + backward on the given rows (no update); gradients readable with

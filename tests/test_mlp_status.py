@@ -16,6 +16,13 @@ int main(int argc, char**)
     float acted[5] = {};
     bool ok = blocks == 5 && !any_discarded(acted, n);
     for (float& a : acted) { a = 1.f; ok = ok && any_discarded(acted, n); a = 0.f; }
+    float rows[n] = {};
+    ok = ok && !maybe_discarded(rows, n);
+    for (int b = 0; b < blocks; ++b) {
+        for (int i = b * kTakeRows; i < n && i < (b + 1) * kTakeRows; ++i) rows[i] = NAN;
+        ok = ok && maybe_discarded(rows, n);
+        for (float& r : rows) r = 0.f;
+    }
     if (argc > 1) {
         // device: the kernel with the flag down and up
         float *out, *y, h[n + 5];
