@@ -3255,12 +3255,7 @@ bool bins_eligible(const InstDev& I, const rewl_batch_desc& D, int max_window_bi
     const long long maxbins = (8 * std::llabs(I.J_u)) >> I.bin_shift;
     if (5 * maxbins > kGuard) return false;
     // energies are -2 N J plus multiples of 4|J|: the bins' lower edges have to be energies
-    if (((-2 * (long long)I.N * I.J_u - I.eglo_u) & ((1LL << I.bin_shift) - 1)) != 0) {
-        // lattices cut into whole chunks of 4, 8, 16, 24 or 32 sites report this as an energy off its bin
-        const int C = I.chunk;
-        return (C == 32 || C == 24 || C == 16 || C == 8 || C == 4) && I.N % (4 * C) == 0;
-    }
-    return true;
+    return ((-2 * (long long)I.N * I.J_u - I.eglo_u) & ((1LL << I.bin_shift) - 1)) == 0;
 }
 
 // The global-table kernel's tree adds up to five energy changes to a position within a bin in 32 bits,
