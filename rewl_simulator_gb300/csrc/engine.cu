@@ -3426,8 +3426,8 @@ int table_cache(int n, int all, int nsm, int observables, int nb, double move, i
 
 // The persistent launch: every group's walkers as tasks of one work-stealing kernel.  Groups are
 // ordered by the expected cost of one walker's sweep (degrees of freedom x cycles per flip of
-// its kernel, measured: table kernel ~440, bin-tracking ~70), the dearest first, so that the
-// last tasks taken are short.  Every warp gets the largest shared-memory region any group needs.
+// its kernel, measured: table kernel ~130 on the tree and ~440 in the serial chain, bin-tracking
+// ~60), the dearest first, so that the last tasks taken are short.  Every warp gets the largest shared-memory region any group needs.
 int plan_fused(rewl_engine* e, int nsm)
 {
     if (e->launches.size() > (size_t)kMaxFusedGroups)
@@ -3438,7 +3438,7 @@ int plan_fused(rewl_engine* e, int nsm)
         const Launch& l = e->launches[gi];
         int ndof = 0;
         for (int s : l.slots) ndof = std::max(ndof, e->inst[e->h_slot_inst[s]].dev.ndof);
-        order.push_back({-(double)ndof * (l.bins ? 70.0 : 440.0), gi});
+        order.push_back({-(double)ndof * (l.bins ? 60.0 : l.cache ? 130.0 : 440.0), gi});
     }
     std::stable_sort(order.begin(), order.end());
     FusedParams& F = e->fused_p;
