@@ -992,17 +992,24 @@ bool maybe_discarded(const float* y, int n)
 // of in_dim floats a row, not of a row padded on the host (predicting 7900 rows, 7 features:
 // 224 us with padding on the host and all kOut columns back, 117 us with k_stage and k_take, 94 with
 // programmatic dependence and the status in k_take)
+// (at most kStageFloats of them at a time: the buffer stays, and a training set need not be held twice)
+constexpr size_t kStageFloats = 4u << 20;
 int upload_features(rewl_mlp* m, const float* X, int n, int in_dim, int rows, bf16* dst)
 {
-    const size_t need = (size_t)n * in_dim;
+    const int most = (int)(kStageFloats / in_dim);
+    const size_t need = (size_t)std::min(n, most) * in_dim;
     if (m->Xraw.n < need) {
         if (int rc = m->Xraw.alloc(need)) return rc;
         MCUDA(cudaStreamSynchronize(nullptr));         // zeroed before another stream writes
     }
-    MCUDA(cudaMemcpyAsync(m->Xraw.p, X, need * sizeof(float), cudaMemcpyHostToDevice, m->stream));
-    k_stage<<<(unsigned)(((size_t)rows * kIn + 255) / 256), 256, 0, m->stream>>>(m->Xraw.p, n, in_dim, rows, dst);
-    MCUDA(cudaGetLastError());
-    m->launches++;
+    for (int r = 0; r < n; r += most) {
+        const int part = std::min(most, n - r), out = r + part < n ? part : rows - r;
+        MCUDA(cudaMemcpyAsync(m->Xraw.p, X + (size_t)r * in_dim, (size_t)part * in_dim * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+        k_stage<<<(unsigned)(((size_t)out * kIn + 255) / 256), 256, 0, m->stream>>>(m->Xraw.p, part, in_dim, out, dst + (size_t)r * kIn);
+        MCUDA(cudaGetLastError());
+        m->launches++;
+        if (r + part >= n) break;                      // (r + most may pass the largest int)
+    }
     return REWL_OK;
 }
 
