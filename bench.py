@@ -56,11 +56,12 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 METRIC = "time to ln g within 1e-2 of exact, MLP warm-start vs plain WL, 1 GB300; flips/s"
-# Cycles per attempted flip of one walker at the speed of light of the sweep kernels' design, a
-# block of five decisions at a time, from probe kernels on a GB300: a dependent shared-memory load
-# of 16 bytes (33 cycles), a vote (12), a maximum over the warp (26) and fifteen dependent integer
-# instructions (4.5 each).
-CHAIN_FLOOR_CYCLES = 28.0
+# Cycles of a block of decisions of one walker at the speed of light of the sweep kernels' design, from
+# probe kernels on a GB300: a dependent shared-memory load of 16 bytes (33 cycles), a vote (12), a
+# maximum over the warp (26) and fifteen dependent integer instructions (4.5 each).  A block is five
+# decisions with one walker per warp, four with two, three with four.
+BLOCK_FLOOR_CYCLES = 139.0
+BLOCK_DECISIONS = {1: 5, 2: 4, 4: 3}
 
 
 def _ising_workload(name, L, nwin, R, se, sc, lnf_final, one_over_t, init_mode, profile):
@@ -909,11 +910,14 @@ def run_gpu(args):
         # one walker's blocks of decisions: cycles per attempted flip against the design's floor
         walker_flips = WORKLOAD["sweeps_per_exchange"] * ndof(WORKLOAD)
         cycles = avg_launch_ms * 1e-3 * sm_mhz * 1e6 / walker_flips
-        kind = "block floor: shared load (33) + vote (12) + warp maximum (26) + 15 dependent integer instructions (68) per five flips, measured on a GB300"
+        per_warp = int(shapes[0][2]) if shapes else 1
+        floor = BLOCK_FLOOR_CYCLES / BLOCK_DECISIONS[per_warp]
+        kind = ("block floor: shared load (33) + vote (12) + warp maximum (26) + 15 dependent integer instructions (68) per "
+                f"{BLOCK_DECISIONS[per_warp]} flips, measured on a GB300")
         if WORKLOAD["model"] != "ising2d":
             kind += "; this kernel holds only the bins around each walker in shared memory (tables of tens of thousands of bins)"
-        roofline.update({"unit": "cycles/flip", "achieved": cycles, "peak": CHAIN_FLOOR_CYCLES,
-                         "frac": CHAIN_FLOOR_CYCLES / cycles, "walkers_per_warp": int(shapes[0][2]) if shapes else 1,
+        roofline.update({"unit": "cycles/flip", "achieved": cycles, "peak": floor,
+                         "frac": floor / cycles, "walkers_per_warp": per_warp,
                          "peak_kind": kind,
                          "note": "per walker: launch time x median SM clock / flips of one walker; frac = floor / "
                                  "achieved"})

@@ -170,7 +170,7 @@ struct DevPtrs {
     int32_t* cfg_M;          // 3 per configuration
     int64_t* fields;         // Baxter field per site (units)
     int64_t* g;
-    int64_t* gsnap;          // logDoS at the start of an Ashkin-Teller sweep launch
+    int64_t* gsnap;          // global-table serial chain: logDoS at the start of a sweep launch
     uint32_t* H;
     uint64_t* visits;
     uint8_t* mask;
@@ -2887,7 +2887,7 @@ struct rewl_engine {
     DBuf<unsigned long long> stats;
     DBuf<int64_t> thr;
     DBuf<double> obs;           // per-bin observable sums (observables on)
-    DBuf<int64_t> gsnap;        // Ashkin-Teller engines: logDoS copy taken by each sweep launch
+    DBuf<int64_t> gsnap;        // global-table serial chain: logDoS copy taken by each sweep launch
     DBuf<double> qtab;          // correlator kernels (observables == 2)
     DBuf<int2> qfix;
     DBuf<unsigned long long> xround;   // exchange round and the exchange kernel's done-block count

@@ -7,7 +7,8 @@
 // Shapes: 7 inputs (padded to 64) -> 4 x 256 (GELU) -> 1 output (padded to 64).
 // A batch of 4096 is 4096 x 256 x 256 per hidden GEMM, i.e. latency-bound work.
 // The tiles are therefore small (128 x 64 on tcgen05, 64 x 64 on mma.sync) so
-// that a layer spans many blocks, and every GEMM of a step runs on one stream.
+// that a layer spans many blocks; the products that depend on one another run on one
+// stream, weight and bias gradients beside them.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -741,14 +742,14 @@ struct rewl_mlp {
     int hidden = 256, layers = 4;
     int batch_cap = 0;
     cudaStream_t stream = nullptr;
-    // layer l: weight [out_l x in_l] row-major, bias [out_l]; in_0 = 32, out_last = 64
+    // layer l: weight [out_l x in_l] row-major, bias [out_l]; in_0 = kIn, out_last = kOut
     std::vector<int> din, dout;
     std::vector<size_t> woff, boff;
     size_t nparams = 0;
     Buf<float> P, Mm, Vm, Gr, Mask;   // fp32 master params, Adam moments, grads, pad mask
     Buf<bf16> Pb;                     // bf16 params (weights used by the GEMMs)
     // activations for the current batch
-    std::vector<Buf<bf16>> H;         // H[0] = input (B x 32), H[l+1] = gelu(Z_l)
+    std::vector<Buf<bf16>> H;         // H[0] = input (B x kIn), H[l+1] = gelu(Z_l)
     std::vector<Buf<float>> Z;        // pre-activations (hidden layers)
     Buf<float> out, yb, loss, lossrow;
     Buf<bf16> dOut;
@@ -1210,7 +1211,7 @@ int rewl_mlp_train(rewl_mlp* m, int32_t steps, int32_t batch, float lr, float* l
     MCUDA(cudaStreamSynchronize(m->stream));       // the host copies above leave scope
 
     // one step: sample the batch, forward, backward, Adam, keep the loss and advance; captured as
-    // a CUDA graph and replayed `steps` times (about 30 launches a step, launch-bound otherwise)
+    // a CUDA graph and replayed `steps` times (33 launches a step, 12 of them in a row; launch-bound otherwise)
     const int64_t l0 = m->launches;
     auto enqueue_step = [&]() -> int {
         k_gather<<<(batch * kRowThreads + 127) / 128, 128, 0, m->stream>>>(m->Xall.p, m->yall.p, m->nall, m->H[0].p, m->yb.p, batch,
