@@ -645,8 +645,18 @@ __global__ void k_loss_grad(const float* out, const float* y, int B, bf16* dOut,
     *reinterpret_cast<uint4*>(dOut + (size_t)b * kOut + 8 * c) = v;
 }
 
-// loss = sum of rows[0..B): one block of 256 threads, strided partial sums, then a fixed tree
-__global__ void __launch_bounds__(256) k_loss_sum(const float* rows, int B, float* loss)
+// Device state of a training call: the network's step counter and the index of the step within
+// the call.  The kernels of a step read it, so that one captured step replays as the next.
+struct TrainCursor {
+    unsigned long long step;
+    int k;
+    int pad;
+};
+
+// loss = sum of rows[0..B): one block of 256 threads, strided partial sums, then a fixed tree.  In a training step
+// (cur not null) it also keeps the loss and moves the cursor on: k_gather, which reads the step, is done by then, and
+// k_adam, which reads the index, waits for this kernel.
+__global__ void __launch_bounds__(256) k_loss_sum(const float* rows, int B, float* loss, TrainCursor* cur, float* losses)
 {
     __shared__ float part[256];
     float s = 0.f;
@@ -657,39 +667,24 @@ __global__ void __launch_bounds__(256) k_loss_sum(const float* rows, int B, floa
         if ((int)threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *loss = part[0];
+    if (threadIdx.x == 0) {
+        *loss = part[0];
+        if (cur) {
+            losses[cur->k] = part[0];
+            cur->k += 1;
+            cur->step += 1;
+        }
+    }
 }
 
 // Adam on fp32 masters; refresh the bf16 copy.  mask zeroes the padded entries.
-// Device state of a training call: the network's step counter and the index of the step within
-// the call.  The kernels of a step read it, so that one captured step replays as the next.
-struct TrainCursor {
-    unsigned long long step;
-    int k;
-    unsigned done;                 // k_adam's blocks that are through with this step
-};
-
 // Adam with the bias corrections of the cursor's step (c1 = 1 - b1^t, c2 = 1 - b2^t, computed on
 // the host for every step of the call, two floats per step).
 __global__ void k_adam(float* p, float* m, float* v, const float* grad, const float* mask, bf16* pb, size_t n,
-                       float lr, float b1, float b2, float eps, const float* ctab, TrainCursor* cur, const float* loss,
-                       float* losses)
+                       float lr, float b1, float b2, float eps, const float* ctab, const TrainCursor* cur)
 {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = cur->k;
-    // the end of a training step, by the last block to have read the cursor: keep its loss, advance (the
-    // fences order every block's read of the cursor before the write to it)
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(&cur->done, 1u) == gridDim.x - 1) {
-            __threadfence();
-            losses[k] = *loss;
-            cur->step += 1;
-            cur->k = k + 1;
-            cur->done = 0;
-        }
-    }
+    const int k = cur->k - 1;                                  // (k_loss_sum has moved it on)
     if (i >= n) return;
     const float c1 = ctab[2 * k], c2 = ctab[2 * k + 1];
     const float gi = grad[i] * mask[i];
@@ -912,7 +907,7 @@ int bias_grad(rewl_mlp* m, cudaStream_t st, int l, const bf16* G, int B)
 // microseconds at most, so a step is bound by the number of launches that wait on one another:
 // 4096 rows, hidden 256 x 4: 30 launches in a row, 217 us a step; 14 in a row, 125 us; the chain with
 // programmatic dependence and shorter side work 103 us.
-int backward(rewl_mlp* m, int B)
+int backward(rewl_mlp* m, int B, TrainCursor* cur = nullptr, float* losses = nullptr)
 {
     const int L = m->layers;
     MCUDA(launch_next(k_loss_grad, dim3((B * kRowThreads + 127) / 128), 128, 0, m->stream, m->out.p, m->yb.p, B, m->dOut.p, m->lossrow.p));
@@ -924,7 +919,7 @@ int backward(rewl_mlp* m, int B)
         MCUDA(cudaStreamWaitEvent(sw, ev, 0));
         MCUDA(cudaStreamWaitEvent(sb, ev, 0));
         if (l == L) {
-            k_loss_sum<<<1, 256, 0, sb>>>(m->lossrow.p, B, m->loss.p);
+            k_loss_sum<<<1, 256, 0, sb>>>(m->lossrow.p, B, m->loss.p, cur, losses);
             m->launches++;
         }
         if (int rc = weight_grad(m, sw, l, A, m->H[l].p, B)) return rc;
@@ -1205,7 +1200,7 @@ int rewl_mlp_train(rewl_mlp* m, int32_t steps, int32_t batch, float lr, float* l
         ct[2 * s] = 1.f - std::pow(b1, t);
         ct[2 * s + 1] = 1.f - std::pow(b2, t);
     }
-    const TrainCursor c0{(unsigned long long)m->step, 0, 0u};
+    const TrainCursor c0{(unsigned long long)m->step, 0, 0};
     MCUDA(cudaMemcpyAsync(m->ctab.p, ct.data(), ct.size() * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     MCUDA(cudaMemcpyAsync(m->cursor.p, &c0, sizeof c0, cudaMemcpyHostToDevice, m->stream));
     MCUDA(cudaStreamSynchronize(m->stream));       // the host copies above leave scope
@@ -1218,10 +1213,10 @@ int rewl_mlp_train(rewl_mlp* m, int32_t steps, int32_t batch, float lr, float* l
                                                              m->seed, m->cursor.p);
         m->launches++;
         int r;
-        if ((r = forward(m, batch, true)) || (r = backward(m, batch))) return r;
+        if ((r = forward(m, batch, true)) || (r = backward(m, batch, m->cursor.p, m->lossv.p))) return r;
         k_adam<<<(unsigned)((m->nparams + 255) / 256), 256, 0, m->stream>>>(m->P.p, m->Mm.p, m->Vm.p, m->Gr.p, m->Mask.p,
                                                                             m->Pb.p, m->nparams, lr, b1, b2, eps,
-                                                                            m->ctab.p, m->cursor.p, m->loss.p, m->lossv.p);
+                                                                            m->ctab.p, m->cursor.p);
         m->launches++;
         MCUDA(cudaGetLastError());
         return REWL_OK;

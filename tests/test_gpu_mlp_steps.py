@@ -1,5 +1,5 @@
 """The training cursor on the device: steps of one call are those of as many calls of one step each, bit for bit
-(k_adam's blocks all read the step they belong to before its last block moves the cursor on, csrc/mlp.cu)."""
+(the kernel that sums a step's loss moves the cursor on, between the kernels that read it, csrc/mlp.cu)."""
 import numpy as np
 import pytest
 
