@@ -3393,8 +3393,8 @@ bool shape_fits(const Launch& l, int G, int wpb)
 
 // Bins of each walker's table that the global-table kernel's tree keeps in shared memory (a power of two; 0: the serial
 // chain is the better form, which only launches with observables take: the others are within 2 % in long launches, and
-// the chain's copy of the tables makes short ones 1.3 times as long), for n walkers of nb bins whose flips move them up to `move` bins; `fixed` bytes a walker beside
-// them, 12 a bin.  Time in cycles per flip of a walker: as many warps as registers (16) and shared memory hold run at
+// the chain's copy of the tables makes short ones 1.3 times as long), for n walkers of nb bins whose flips move them up
+// to `move` bins; `fixed` bytes a walker beside them, 12 a bin.  Time in cycles per flip of a walker: as many warps as registers (16) and shared memory hold run at
 // once, in full waves and a last one; the fewer moves the cached bins span, the more often the walker leaves them.
 // Measured on Ashkin-Teller L = 12 to 32, bins of 0.05, 0.25 and 1.0 (moves of 300, 60 and 15 bins), e9 flips/s:
 //   1024 walkers, 512 / 1024 / 2048 bins: bins of 0.05 4.0 / 6.3 / 8.9, of 0.25 11.6 / 12.9 / 13.4
@@ -3427,7 +3427,8 @@ int table_cache(int n, int all, int nsm, int observables, int nb, double move, i
 // The persistent launch: every group's walkers as tasks of one work-stealing kernel.  Groups are
 // ordered by the expected cost of one walker's sweep (degrees of freedom x cycles per flip of
 // its kernel, measured: table kernel ~130 on the tree and ~440 in the serial chain, bin-tracking
-// ~60), the dearest first, so that the last tasks taken are short.  Every warp gets the largest shared-memory region any group needs.
+// ~60), the dearest first, so that the last tasks taken are short.  Every warp gets the largest
+// shared-memory region any group needs.
 int plan_fused(rewl_engine* e, int nsm)
 {
     if (e->launches.size() > (size_t)kMaxFusedGroups)
@@ -3483,7 +3484,7 @@ int plan_fused(rewl_engine* e, int nsm)
 int plan_launches(rewl_engine* e)
 {
     const int nsm = sm_count(e);
-    // group walkers by (model, bin-tracking kernel, chunk, sites) so each launch has one
+    // group walkers by (model, bin-tracking kernel, sites, tree) so each launch has one
     // kernel shape and the walkers sharing a warp run the same number of chunks
     struct Key { int model, bins, sites, tree; };
     std::vector<Key> keys;
